@@ -233,6 +233,13 @@ typedef struct mxb_cds_desc {
     const int32_t *fpairx, *fpairy; int32_t fcount;
 } mxb_cds_desc;
 
+/* Test hook, no counterpart in the reference (host code only, no device needed): the task list of
+ * an FP64 evaluation (adjoint: of the transposed one) in claim order, as 64-byte task and 40-byte
+ * item records (csrc/f64_engine.h).  counts: tasks, items, counters per column tile, partial
+ * slots, column tiles, sub-block columns per stage, and the sub-blocks of the three pools. */
+MXB_API int32_t mxb_debug_f64_schedule(const mxb_cds_desc *desc, int32_t adjoint, int32_t nrhs, void *tasks,
+                                       int64_t task_cap, void *items, int64_t item_cap, int64_t *counts);
+
 /* Uploads and repacks the CDS for `precision`, builds the task lists; device = current.
  * desc->D, desc->B and desc->VT may be host arrays or device arrays of the current device
  * (e.g. blocks from mxb_kernel_blocks); the plan keeps its own copy either way. */
@@ -277,14 +284,15 @@ MXB_API int32_t mxb_plan_flops(const mxb_plan *plan, int32_t nrhs, uint64_t *flo
 MXB_API int32_t mxb_plan_info(const mxb_plan *plan, uint64_t *device_bytes, int32_t *launches,
                       int32_t *precision);
 /* Waits for the device and reports a kernel-side failure of earlier evaluations on the plan
- * (MXB_ERR_TIMEOUT when a bounded wait of a tensor-core kernel gave up); clears it. */
+ * (MXB_ERR_TIMEOUT when a bounded wait of an evaluation kernel gave up); clears it. */
 MXB_API int32_t mxb_plan_status(mxb_plan *plan);
 /* Test hook for failure detection, no counterpart in the reference.  With
  * MXB_DEBUG_STALL_ONE_WAIT, the first tensor-core launch of the next evaluations has one CTA
  * withhold a pipeline stage, so its bounded wait runs out: the CTA gives up, frees its TMEM
  * and mxb_plan_status() reports MXB_ERR_TIMEOUT, with the GPU context still usable.
  * wait_cycles > 0 shortens every kernel wait limit (default ~4e9 SM cycles).  flags = 0
- * restores normal operation.  Split-BF16 plans only. */
+ * restores normal operation.  The flags are for split-BF16 plans only; FP64 plans take
+ * wait_cycles (with flags = 0), the limit of every wait of their dataflow launch. */
 #define MXB_DEBUG_STALL_ONE_WAIT 1
 /* MXB_DEBUG_CHAIN_LEVELS: every run of consecutive up-sweep (or down-sweep) launches of one
  * product count runs as one launch whose levels wait for each other on the device (otherwise

@@ -10,6 +10,7 @@
 
 #include "matrox_b200.h"
 #include "mxb_internal.h"
+#include "f64_engine.h"
 #include "plan.h"
 
 using namespace mxb;
@@ -923,8 +924,7 @@ int32_t mxb_plan_info(const mxb_plan *plan, uint64_t *device_bytes, int32_t *lau
     const Plan *p = static_cast<const Plan *>(plan);
     if (device_bytes) *device_bytes = p->device_bytes;
     if (launches)
-        *launches = p->precision != MXB_PREC_FP64 ? (int32_t)split_bf16_launches(*p)
-                                                        : (int32_t)p->launches_fwd.size();
+        *launches = p->precision != MXB_PREC_FP64 ? (int32_t)split_bf16_launches(*p) : 1;
     if (precision) *precision = p->precision;
     return MXB_OK;
 }
@@ -1033,7 +1033,7 @@ int32_t mxb_plan_status(mxb_plan *plan)
     }
     Plan *p = static_cast<Plan *>(plan);
     API_CUDA(cudaDeviceSynchronize());
-    return split_bf16_status(*p);
+    return p->precision == MXB_PREC_FP64 ? f64_status(*p) : split_bf16_status(*p);
 }
 
 int32_t mxb_plan_read_workspaces(mxb_plan *plan, int32_t nrhs, const int32_t *wskeloffset, double *wskel,

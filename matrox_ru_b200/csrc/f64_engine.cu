@@ -1,0 +1,1168 @@
+// FP64 evaluation (Y = K~ W, and its adjoint) as ONE persistent launch on the FP64 tensor path.
+//
+// tcgen05.mma has no f64 kind, so FP64 products use the DMMA instruction mma.sync.m16n8k8.f64.
+//
+// Layout.  Every operand the products read is kept in DMMA fragment order, as 8 x 8 sub-blocks
+// of 64 doubles (512 bytes):
+//   A (the CDS, tiled once at plan creation): row-major sub-blocks, sub-block columns outermost,
+//     so a pipeline stage of a row tile is one run per sub-block column.  A lane takes the pair
+//     (k = 2a, 2a + 1) of its row as one 16-byte shared-memory read: the two DMMA steps of a
+//     sub-block use k = 2a and k = 2a + 1 (any order of k, the same for A and B, sums the same
+//     products).  A transposed product reads the same sub-blocks with k = a and k = a + 4,
+//     8-byte reads of 32 consecutive doubles: one copy of the CDS serves both directions.
+//   B (W, wskel, uskel): column-major sub-blocks, column sub-blocks of one row sub-block
+//     contiguous; element (k, n) at n * 8 + (k ^ 4 ((n >> 1) & 1)), which makes both read orders
+//     free of bank conflicts.  The skeleton vectors are written this way by the epilogue that
+//     computes them; W is rewritten by tasks of the same launch.
+// A stage is then filled by a few 1-D bulk copies on an mbarrier, issued by one warp, and the
+// product warps execute nothing but shared-memory reads and DMMAs.
+//
+// Schedule.  The tasks of all passes (rewriting W, up-sweep, far couplings, near field,
+// down-sweep, leaf down) form one list; a unit is a task and a column tile, claimed in list
+// order.  Units wait on per-node counters for the blocks they read, so no pass waits for the
+// last tile of the pass before.  The list comes from a list-scheduling simulation on the host
+// (longest remaining path first), every unit's inputs come earlier in it and a block runs its
+// units in claim order, so every wait ends; each is bounded all the same.  A long sum (a node
+// in many near or far lists) is cut along K into pieces whose partial tiles the last piece
+// adds up in piece order, so the result does not depend on timing.
+//
+// What bounds it: the DMMA pipe from about 32 right-hand sides on (89 % active in the middle of a
+// launch), HBM (the CDS, read once) below, and for small matrices the chain of node to node hops
+// (2 - 3 us each: publish, poll, load, multiply).  Measured on one B200, launch per pass with
+// cp.async tiles -> one dataflow launch: N = 65536 H2-b, 1024 right-hand sides 25.6 -> 23.3 ms
+// (33.7 TFLOP/s), 1 right-hand side 2563 -> 460 us (5.8 TB/s); N = 16384 HSS, 256 right-hand
+// sides 511 -> 351 us; N = 32768 adjoint, 64 right-hand sides (long near lists) 2946 -> 690 us;
+// N = 1024, 1 right-hand side 102 -> 30 us.
+#include <algorithm>
+#include <cstring>
+#include <functional>
+#include <queue>
+#include <string>
+
+#include "f64_engine.h"
+#include "plan.h"
+#include "tc_common.cuh"
+
+namespace mxb {
+namespace {
+
+enum : int16_t { F64_Y = 0, F64_WSKEL = 1, F64_USKEL = 2, F64_TILE_W = 3 };
+enum { BUF_W = 0, BUF_WSKEL = 1, BUF_USKEL = 2 };
+enum { CTL_CLAIM = 0, CTL_EXIT = 1, CTL_ERR = 2, CTL_FIRST = 16 };
+
+constexpr int WARPS = 4, THREADS = (WARPS + 1) * 32, RING = 4;
+constexpr int EAGER = 64;  // polls of a node counter before the first pause
+
+// BN: right-hand sides of a column tile.  BK8: sub-block columns of A per stage.  32 is the widest
+// tile: with 64 columns a unit takes twice as long on a shared SM, which the tree sweeps wait
+// for (N = 65536, 1024 right-hand sides: 24.2 ms against 23.3 ms; N = 16384 HSS, 256: 376 against
+// 354 us), and 16 re-reads A too often (418 us).  Stages of 4 sub-block columns beat 2 (24.8 ms)
+// because a warp pays ~100 cycles to move to the next stage; 3 blocks of 12 product warps per SM
+// beat 4 without fragment double-buffering (26.4 ms) and 2 (25 ms).
+template <int BN>
+struct Cfg {
+    static constexpr int N8 = BN / 8;
+    static constexpr int WN = N8 >= 4 ? 2 : 1, WM = WARPS / WN;   // product warps: rows x columns
+    static constexpr int MI = 8 / WM, NJ = N8 / WN;               // sub-blocks per warp
+    static constexpr int BK8 = 4;
+    static constexpr int A_BYTES = BK8 * 8 * 512, B_BYTES = BK8 * N8 * 512;
+    static constexpr int STAGE = A_BYTES + B_BYTES;
+    static constexpr int STAGES = 3;
+    static constexpr int CTAS = N8 >= 2 ? 3 : 4;                  // resident per SM
+    static constexpr int SMEM = STAGES * STAGE + 1024;            // + barriers and the unit ring
+};
+
+struct Args {
+    const double *pool[3];
+    double *buf[3];
+    const double *W;
+    double *Y;
+    const int32_t *wofs, *yofs;
+    const F64Task *tasks;
+    const F64Item *items;
+    double *partial;
+    int *ctl;
+    long long wait_cycles;
+    int units, ncol, nb, nrhs, beta, nctr;
+};
+
+struct Unit {  // ring slot: the claimed unit
+    F64Task task;
+    int32_t col, n8_0, n8, live;
+};
+
+// Two stacked 8 x 8 sub-blocks of A (rows g and g + 8 of a lane's fragment) times one of B.
+__device__ __forceinline__ void dmma(double (&c)[2], double (&d)[2], const double (&a0)[2], const double (&a1)[2],
+                                     const double (&b)[2])
+{
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(d[0]), "+d"(d[1])
+                 : "d"(a0[0]), "d"(a1[0]), "d"(a0[1]), "d"(a1[1]), "d"(b[0]), "d"(b[1]));
+}
+
+__device__ __forceinline__ int b_elem(int k, int n) { return n * 8 + (k ^ (((n >> 1) & 1) << 2)); }
+
+template <int BN>
+__global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(const Args g)
+{
+    using C = Cfg<BN>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
+    uint64_t *empty = full + C::STAGES;
+    uint64_t *ufull = empty + C::STAGES;
+    uint64_t *uempty = ufull + RING;
+    Unit *ring = reinterpret_cast<Unit *>(uempty + RING);
+    volatile int *meta = reinterpret_cast<volatile int *>(ring + RING);  // per stage: sub-block columns | trans << 8
+    volatile int *abort_word = meta + C::STAGES;
+    int *last_cta = const_cast<int *>(abort_word) + 1;
+    static_assert(sizeof(Unit) == 80 && (2 * C::STAGES + 2 * RING) * 8 + RING * 80 + C::STAGES * 4 + 8 <= 1024, "");
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int *counters = g.ctl + CTL_FIRST;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], WARPS);
+        }
+        for (int i = 0; i < RING; ++i) {
+            tc::mbar_init(&ufull[i], 1);
+            tc::mbar_init(&uempty[i], WARPS);
+        }
+        *abort_word = 0;
+        tc::fence_mbar_init();
+    }
+    __syncthreads();
+
+    if (warp == WARPS) {
+        // ---------------- producer: claims units, fills the stages ----------------
+        uint32_t st = 0;  // stages filled
+        int slot = 0;
+        bool ok = true;
+        while (ok) {
+            // claimed once the loads of the unit before are on their way, not earlier: a unit held
+            // back behind another would keep the units that read it waiting
+            int u = 0;
+            if (lane == 0) u = atomicAdd(g.ctl + CTL_CLAIM, 1);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            const int i = slot % RING;
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&uempty[i], ((slot / RING) & 1) ^ 1, abort_word, g.wait_cycles));
+            if (!ok) break;
+            ++slot;
+            Unit &un = ring[i];
+            if (u >= g.units) {
+                if (lane == 0) un.live = 0;
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&ufull[i])) : "memory");
+                break;
+            }
+            const int t = u / g.ncol, col = u - t * g.ncol;
+            // column tiles of nearly equal width: sub-blocks [n8_0, n8_0 + n8)
+            const int n8_0 = (int)((long long)g.nb * col / g.ncol);
+            const int n8 = (int)((long long)g.nb * (col + 1) / g.ncol) - n8_0;
+            if (lane < 16)
+                reinterpret_cast<int *>(&un.task)[lane] = __ldg(reinterpret_cast<const int *>(g.tasks + t) + lane);
+            if (lane == 16) un.col = col;
+            if (lane == 17) un.n8_0 = n8_0;
+            if (lane == 18) un.n8 = n8;
+            if (lane == 19) un.live = 1;
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&ufull[i])) : "memory");
+            const int item0 = un.task.item0, nitem = un.task.nitem, r8 = un.task.r8, m8 = un.task.m8;
+            for (int q = 0; q < nitem && ok; ++q) {
+                const F64Item it = g.items[item0 + q];
+                const double *a0 = it.a_pool == 0 ? g.pool[0] : (it.a_pool == 1 ? g.pool[1] : g.pool[2]);
+                const double *b0 = it.b_buf == 0 ? g.buf[0] : (it.b_buf == 1 ? g.buf[1] : g.buf[2]);
+                const uint8_t *A = reinterpret_cast<const uint8_t *>(a0 + it.a_off * 64);
+                const uint8_t *B = reinterpret_cast<const uint8_t *>(b0 + (it.b_base * g.nb + n8_0) * 64);
+                // stage f of the item: the CDS side (and the byte count of both), then B
+                auto load_a = [&](uint32_t f, int k0) {
+                    const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
+                    uint8_t *sa = smem + s * C::STAGE;
+                    if (lane == 0) {
+                        meta[s] = nk | (it.trans << 8);
+                        tc::mbar_expect_tx(&full[s], (uint32_t)(nk * (m8 + n8) * 512));
+                    }
+                    __syncwarp();
+                    if (it.trans) {  // one run per sub-block row of the tile
+                        if (lane < m8)
+                            tc::bulk_g2s(sa + lane * C::BK8 * 512, A + ((size_t)(r8 + lane) * it.lda + k0) * 512,
+                                         (uint32_t)nk * 512, &full[s]);
+                    } else if (lane < nk) {  // one run per sub-block column of the stage
+                        tc::bulk_g2s(sa + lane * 8 * 512, A + ((size_t)(k0 + lane) * it.lda + r8) * 512,
+                                     (uint32_t)m8 * 512, &full[s]);
+                    }
+                };
+                auto load_b = [&](uint32_t f, int k0) {
+                    const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
+                    if (lane < nk)
+                        tc::bulk_g2s(smem + s * C::STAGE + C::A_BYTES + lane * C::N8 * 512,
+                                     B + (size_t)(k0 + lane) * g.nb * 512, (uint32_t)n8 * 512, &full[s]);
+                };
+                int ahead = 0;  // sub-block columns whose A is on its way
+                if (it.dep >= 0) {
+                    const int *ctr = counters + it.dep * g.ncol + col;
+                    if (__any_sync(0xffffffffu, !tc::counter_reached(ctr, it.need))) {
+                        // B is not written yet: fill the free stages with A meanwhile
+                        for (uint32_t f = st; ahead < it.k8 && f < st + C::STAGES; ++f, ahead += C::BK8) {
+                            if (!__all_sync(0xffffffffu, tc::mbar_try_wait(&empty[f % C::STAGES], ((f / C::STAGES) & 1) ^ 1))) break;
+                            load_a(f, ahead);
+                        }
+                    }
+                    // every lane takes its own acquire: each issues copies of its own
+                    ok = __all_sync(0xffffffffu, tc::wait_counter(ctr, it.need, abort_word, g.wait_cycles, EAGER));
+                }
+                for (int k0 = 0; k0 < it.k8; k0 += C::BK8, ++st) {
+                    if (k0 >= ahead) {
+                        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st % C::STAGES], ((st / C::STAGES) & 1) ^ 1,
+                                                                        abort_word, g.wait_cycles));
+                        if (!ok) break;
+                        load_a(st, k0);
+                    }
+                    load_b(st, k0);  // also after a failed wait: a stage that was begun is filled
+                }
+            }
+        }
+        if (!ok && lane == 0) *abort_word = 1;
+        __syncwarp();
+        // every filled stage has landed before the block may exit
+        for (uint32_t f = st > C::STAGES ? st - C::STAGES : 0; f < st; ++f) {
+            volatile int never = 0;
+            tc::mbar_wait(&full[f % C::STAGES], (f / C::STAGES) & 1, &never, tc::WAIT_CYCLES);
+        }
+    } else {
+        // ---------------- product warps ----------------
+        const int wm = warp / C::WN, wn = warp % C::WN;
+        const int fr = lane >> 2, fa = lane & 3;  // fragment row (A) or column (B), and k
+        uint32_t st = 0;
+        for (int slot = 0;; ++slot) {
+            const int ri = slot % RING;
+            if (!tc::mbar_wait(&ufull[ri], (slot / RING) & 1, abort_word, g.wait_cycles)) {
+                *abort_word = 1;
+                break;
+            }
+            const Unit &un = ring[ri];
+            if (!un.live) break;
+            const int m8 = un.task.m8, n8 = un.n8, stages = un.task.stages;
+            // this warp's sub-blocks: rows [mb, mb + mi), columns [jb, jb + nj)
+            const int mb = m8 * wm / C::WM, mi = m8 * (wm + 1) / C::WM - mb;
+            const int jb = n8 * wn / C::WN, nj = n8 * (wn + 1) / C::WN - jb;
+            double acc[C::MI][C::NJ][2];
+#pragma unroll
+            for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+                for (int j = 0; j < C::NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+            // an accumulating unit starts from the old output, read while its first stages load
+            // (written by another unit of this launch where old_dep says so)
+            auto old_output = [&](const Unit &u) -> bool {
+                if (u.task.old_dep >= 0) {
+                    if (!__all_sync(0xffffffffu, tc::wait_counter(counters + u.task.old_dep * g.ncol + u.col, u.task.old_need,
+                                                                  abort_word, g.wait_cycles, EAGER)))
+                        return false;
+                }
+                if (u.task.kind == F64_Y) {
+                    const int rows = u.task.rows;
+                    const int r0 = (u.task.r8 + mb) * 8 + fr, c0 = (u.n8_0 + jb) * 8 + 2 * fa;
+                    const double *Y = g.Y + g.yofs[u.task.out] + r0 + (size_t)c0 * rows;
+#pragma unroll
+                    for (int j = 0; j < C::NJ; ++j, Y += (size_t)8 * rows)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (j >= nj || c0 + 8 * j + e >= g.nrhs) break;
+#pragma unroll
+                            for (int i = 0; i < C::MI; ++i)
+                                if (i < mi && r0 + 8 * i < rows) acc[i][j][e] = Y[(e ? rows : 0) + 8 * i];
+                        }
+                } else {
+                    const double *row = g.buf[BUF_USKEL] + ((u.task.out + u.task.r8 + mb) * (int64_t)g.nb + u.n8_0 + jb) * 64;
+                    const int e0 = b_elem(fr, 2 * fa), e1 = b_elem(fr, 2 * fa + 1);
+#pragma unroll
+                    for (int i = 0; i < C::MI; ++i, row += (size_t)g.nb * 64) {
+                        if (i >= mi) break;
+#pragma unroll
+                        for (int j = 0; j < C::NJ; ++j)
+                            if (j < nj) {
+                                acc[i][j][0] = row[j * 64 + e0];
+                                acc[i][j][1] = row[j * 64 + e1];
+                            }
+                    }
+                }
+                return true;
+            };
+            bool ok = true;
+            const int kind = un.task.kind, beta = un.task.beta == 2 ? g.beta : un.task.beta;
+            if (beta && kind != F64_TILE_W && un.task.npiece == 1) ok = old_output(un);
+            for (int q = 0; q < stages && ok; ++q, ++st) {
+                const int s = st % C::STAGES;
+                if (!tc::mbar_wait(&full[s], (st / C::STAGES) & 1, abort_word, g.wait_cycles)) {
+                    ok = false;
+                    break;
+                }
+                const int mt = meta[s], nk = mt & 0xFF;
+                const double *sa = reinterpret_cast<const double *>(smem + s * C::STAGE);
+                const double *sb = reinterpret_cast<const double *>(smem + s * C::STAGE + C::A_BYTES);
+                // ALL: every sub-block of the warp's tile and of the stage exists; the fragments of the
+                // next sub-block column are then read while this one's products run
+                auto products = [&](auto trans, auto whole) {
+                    constexpr bool T = decltype(trans)::value, ALL = decltype(whole)::value;
+                    const int sw = ((fr >> 1) & 1) << 2;
+                    const double *pb = sb + jb * 64 + fr * 8 + (T ? fa ^ sw : (2 * fa) ^ sw);
+                    const double *pa = T ? sa + mb * C::BK8 * 64 + fr + fa * 8 : sa + mb * 64 + fr * 8 + fa * 2;
+                    const int hop = T ? ((fa + 4) ^ sw) - (fa ^ sw) : 0;
+                    double a[2][C::MI][2], b[2][C::NJ][2];
+                    auto fetch = [&](int k, int h) {
+#pragma unroll
+                        for (int j = 0; j < C::NJ; ++j) {
+                            if (!ALL && j >= nj) break;
+                            const double *q = pb + (k * C::N8 + j) * 64;
+                            if constexpr (T) {
+                                b[h][j][0] = q[0];
+                                b[h][j][1] = q[hop];
+                            } else {
+                                const double2 v = *reinterpret_cast<const double2 *>(q);
+                                b[h][j][0] = v.x;
+                                b[h][j][1] = v.y;
+                            }
+                        }
+                        // rows come in pairs: past an odd count the stage holds older values, whose
+                        // products are never stored
+#pragma unroll
+                        for (int i = 0; i < C::MI; ++i) {
+                            if (!ALL && (i & ~1) >= mi) break;
+                            if constexpr (T) {
+                                a[h][i][0] = pa[(i * C::BK8 + k) * 64];
+                                a[h][i][1] = pa[(i * C::BK8 + k) * 64 + 32];
+                            } else {
+                                const double2 v = *reinterpret_cast<const double2 *>(pa + (k * 8 + i) * 64);
+                                a[h][i][0] = v.x;
+                                a[h][i][1] = v.y;
+                            }
+                        }
+                    };
+                    auto multiply = [&](int h) {
+#pragma unroll
+                        for (int i = 0; i < C::MI; i += 2) {
+                            if (!ALL && i >= mi) break;
+#pragma unroll
+                            for (int j = 0; j < C::NJ; ++j) {
+                                if (!ALL && j >= nj) break;
+                                dmma(acc[i][j], acc[i + 1][j], a[h][i], a[h][i + 1], b[h][j]);
+                            }
+                        }
+                    };
+                    if constexpr (ALL) {
+                        fetch(0, 0);
+#pragma unroll
+                        for (int k = 0; k < C::BK8; ++k) {
+                            if (k + 1 < C::BK8) fetch(k + 1, (k + 1) & 1);
+                            multiply(k & 1);
+                        }
+                    } else {
+                        for (int k = 0; k < nk; ++k) {
+                            fetch(k, 0);
+                            multiply(0);
+                        }
+                    }
+                };
+                const bool whole = mi == C::MI && nj == C::NJ && nk == C::BK8;
+                if (mt >> 8) {
+                    if (whole) products(std::true_type{}, std::true_type{});
+                    else products(std::true_type{}, std::false_type{});
+                } else {
+                    if (whole) products(std::false_type{}, std::true_type{});
+                    else products(std::false_type{}, std::false_type{});
+                }
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&empty[s])) : "memory");
+            }
+            if (!ok) {
+                *abort_word = 1;
+                break;
+            }
+            const int col = un.col, n8_0 = un.n8_0, sig = un.task.sig;
+            bool write = true;
+            if (un.task.npiece > 1) {
+                // K piece: leave the partial tile; the last piece of the tile to arrive adds all of
+                // them in piece order
+                constexpr int PER = C::MI * C::NJ * 2 * 32;  // partial values per warp
+                const size_t stride = (size_t)g.ncol * WARPS * PER;
+                double *base = g.partial + ((size_t)un.task.slot * g.ncol + col) * WARPS * PER + warp * PER + lane;
+                double *mine = base + un.task.piece * stride;
+#pragma unroll
+                for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < C::NJ; ++j) {
+                        __stcg(mine + ((i * C::NJ + j) * 2) * 32, acc[i][j][0]);
+                        __stcg(mine + ((i * C::NJ + j) * 2 + 1) * 32, acc[i][j][1]);
+                    }
+                __threadfence();
+                __syncwarp();
+                int seen = 0;
+                if (lane == 0) seen = atomicAdd(counters + un.task.piece_ctr * g.ncol + col * WARPS + warp, 1);
+                write = __shfl_sync(0xffffffffu, seen, 0) == un.task.npiece - 1;
+                if (write) {
+                    __threadfence();
+#pragma unroll
+                    for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+                        for (int j = 0; j < C::NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+                    if (beta && !old_output(un)) {
+                        *abort_word = 1;
+                        break;
+                    }
+                    for (int p = 0; p < un.task.npiece; ++p) {
+                        const double *src = base + p * stride;
+#pragma unroll
+                        for (int i = 0; i < C::MI; ++i)
+#pragma unroll
+                            for (int j = 0; j < C::NJ; ++j) {
+                                acc[i][j][0] += __ldcg(src + ((i * C::NJ + j) * 2) * 32);
+                                acc[i][j][1] += __ldcg(src + ((i * C::NJ + j) * 2 + 1) * 32);
+                            }
+                    }
+                }
+            }
+            if (write) {
+                if (kind == F64_Y) {
+                    const int rows = un.task.rows;
+                    const int r0 = (un.task.r8 + mb) * 8 + fr, c0 = (n8_0 + jb) * 8 + 2 * fa;
+                    double *Y = g.Y + g.yofs[un.task.out] + r0 + (size_t)c0 * rows;
+#pragma unroll
+                    for (int j = 0; j < C::NJ; ++j, Y += (size_t)8 * rows)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (j >= nj || c0 + 8 * j + e >= g.nrhs) break;
+                            double *y = Y + (e ? rows : 0);
+#pragma unroll
+                            for (int i = 0; i < C::MI; ++i)
+                                if (i < mi && r0 + 8 * i < rows) y[8 * i] = acc[i][j][e];
+                        }
+                } else if (kind == F64_TILE_W) {
+                    // W (column-major, leading dimension rows) -> sub-blocks of this column tile; a
+                    // warp takes 32 rows of 16 columns at a time, all its loads in flight (k past
+                    // the leaf and columns past nrhs are zero)
+                    const int rows = un.task.rows, r8 = un.task.r8;
+                    const double *W = g.W + g.wofs[un.task.out];
+                    double *dst = g.buf[BUF_W] + un.task.slot * (int64_t)g.nb * 64;
+                    const int nj2 = (n8 + 1) >> 1, steps = (m8 + 3) / 4 * nj2;
+                    for (int x = warp; x < steps; x += WARPS) {
+                        const int kq = x / nj2, j = 2 * (x - kq * nj2);
+                        const int k = r8 * 8 + kq * 32 + lane;
+                        double v[16];
+#pragma unroll
+                        for (int n = 0; n < 16; ++n) {
+                            const int c = (n8_0 + j) * 8 + n;
+                            v[n] = (k < rows && c < g.nrhs) ? W[(size_t)k + (size_t)c * rows] : 0.0;
+                        }
+                        if (k < (r8 + m8) * 8) {
+                            double *blk = dst + ((int64_t)(k >> 3) * g.nb + n8_0 + j) * 64;
+#pragma unroll
+                            for (int n = 0; n < 16; ++n)
+                                if (j + n / 8 < n8) blk[n / 8 * 64 + b_elem(k & 7, n & 7)] = v[n];
+                        }
+                    }
+                } else {
+                    double *buf = kind == F64_WSKEL ? g.buf[BUF_WSKEL] : g.buf[BUF_USKEL];
+                    double *row = buf + ((un.task.out + un.task.r8 + mb) * (int64_t)g.nb + n8_0 + jb) * 64;
+                    const int e0 = b_elem(fr, 2 * fa), e1 = b_elem(fr, 2 * fa + 1);
+#pragma unroll
+                    for (int i = 0; i < C::MI; ++i, row += (size_t)g.nb * 64) {
+                        if (i >= mi) break;
+#pragma unroll
+                        for (int j = 0; j < C::NJ; ++j)
+                            if (j < nj) {
+                                row[j * 64 + e0] = acc[i][j][0];
+                                row[j * 64 + e1] = acc[i][j][1];
+                            }
+                    }
+                }
+                if (sig >= 0) {
+                    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) atomicAdd(counters + sig * g.ncol + col, 1);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&uempty[ri])) : "memory");
+        }
+    }
+    __syncwarp();
+    __syncthreads();
+    // the last block out leaves the claim counter and every other counter at zero for the next launch
+    if (threadIdx.x == 0) {
+        if (*abort_word) atomicExch(g.ctl + CTL_ERR, MXB_ERR_TIMEOUT);
+        __threadfence();
+        *last_cta = atomicAdd(g.ctl + CTL_EXIT, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (*last_cta) {
+        __threadfence();
+        for (int i = threadIdx.x; i < g.nctr; i += THREADS) counters[i] = 0;
+        if (threadIdx.x == 0) g.ctl[CTL_CLAIM] = g.ctl[CTL_EXIT] = 0;
+    }
+}
+
+// CDS pool (column-major blocks) -> sub-blocks, one job per block.
+struct PoolJob {
+    uint64_t src;  // element offset
+    uint64_t dst;  // sub-block offset
+    int32_t ld, rows, cols, pad;
+};
+
+// A warp writes four sub-blocks (32 rows of 8 columns) at a time: reads of 32 consecutive rows.
+__global__ void __launch_bounds__(256) f64_tile_pool_kernel(const PoolJob *__restrict__ jobs, const double *__restrict__ src,
+                                                            double *__restrict__ dst)
+{
+    const PoolJob j = jobs[blockIdx.x];
+    const int m8 = (j.rows + 7) >> 3, k8 = (j.cols + 7) >> 3, mq = (m8 + 3) >> 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int x = blockIdx.y * 8 + warp; x < mq * k8; x += gridDim.y * 8) {
+        const int q = x % mq, k = x / mq;
+        const int r = q * 32 + lane;
+        double v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            v[e] = (r < j.rows && k * 8 + e < j.cols) ? src[j.src + (size_t)r + (size_t)(k * 8 + e) * j.ld] : 0.0;
+        if (r < m8 * 8) {
+            double *o = dst + (j.dst + (uint64_t)k * m8 + (r >> 3)) * 64 + (r & 7) * 8;
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) *reinterpret_cast<double2 *>(o + e) = make_double2(v[e], v[e + 1]);
+        }
+    }
+}
+
+int fail(const std::string &m, int code = MXB_ERR_CUDA)
+{
+    set_error(m);
+    return code;
+}
+
+#define F64_CUDA(call)                                                                    \
+    do {                                                                                  \
+        cudaError_t e_ = (call);                                                          \
+        if (e_ != cudaSuccess) return fail(std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    } while (0)
+
+int sm_count()
+{
+    static int n[128];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return 148;
+    if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return n[dev];
+}
+
+template <int BN>
+int launch(const Args &a, cudaStream_t stream)
+{
+    using C = Cfg<BN>;
+    static bool configured[128];
+    int dev = 0;
+    F64_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 128) return fail("device index out of range");
+    if (!configured[dev]) {
+        F64_CUDA(cudaFuncSetAttribute(f64_dataflow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        configured[dev] = true;
+    }
+    const int grid = std::min(a.units, sm_count() * C::CTAS);
+    f64_dataflow_kernel<BN><<<grid, THREADS, C::SMEM, stream>>>(a);
+    F64_CUDA(cudaGetLastError());
+    return MXB_OK;
+}
+
+struct Shape {  // of the kernel variant that runs `nb` column sub-blocks
+    int bn, bk8, ctas, ncol;
+};
+
+// The narrowest variant that holds all columns (8, 16), else tiles of at most 32: below 17 right-hand
+// sides the launch is bound by the CDS bytes, and a wider tile only adds padding products (16
+// right-hand sides, N = 32768: 237 us; 32: 382 us).
+Shape shape_for(int nb)
+{
+    if (nb <= 1) return {8, Cfg<8>::BK8, Cfg<8>::CTAS, 1};
+    if (nb <= 2) return {16, Cfg<16>::BK8, Cfg<16>::CTAS, 1};
+    return {32, Cfg<32>::BK8, Cfg<32>::CTAS, (nb + 3) / 4};
+}
+
+// A group of the schedule: the tasks of one output block in one pass.
+struct Group {
+    std::vector<F64Task> tasks;
+    std::vector<int> deps, cons;
+    double prio = -1, ready = 0, finish = 0;
+    int unplaced = 0, cost = 0;
+};
+
+}  // namespace
+
+// ---------------------------------------------------------------------------------------
+// creation: the CDS into sub-blocks
+// ---------------------------------------------------------------------------------------
+
+namespace {
+
+// Where every block of the CDS goes (host only), and the copies that put it there.
+void layout(Plan &p, std::vector<PoolJob> (&jobs)[3], uint64_t (&used)[3])
+{
+    F64Engine &E = *(p.f64 = new F64Engine());
+    auto ceil8 = [](int64_t v) { return (int32_t)((v + 7) / 8); };
+    auto add = [&](int pool, uint64_t src, int ld, int rows, int cols) {
+        F64Block b;
+        b.off = used[pool];
+        b.m8 = ceil8(rows);
+        b.k8 = ceil8(cols);
+        used[pool] += (uint64_t)b.m8 * b.k8;
+        if (rows > 0 && cols > 0) jobs[pool].push_back(PoolJob{src, b.off, ld, rows, cols, 0});
+        return b;
+    };
+    for (size_t k = 0; k < p.near_x.size(); ++k)
+        E.near.push_back(add(0, p.near_off[k], p.Ddim[p.near_x[k]], p.Ddim[p.near_x[k]], p.Ddim[p.near_y[k]]));
+    for (size_t k = 0; k < p.far_x.size(); ++k)
+        E.far.push_back(add(1, p.far_off[k], p.slen[p.far_x[k]], p.slen[p.far_x[k]], p.slen[p.far_y[k]]));
+    E.proj_l.resize(p.numnodes);
+    E.proj_r.resize(p.numnodes);
+    for (int v = 0; v < p.numnodes; ++v) {
+        if (v == p.root || p.slen[v] <= 0) continue;
+        const int s = p.slen[v];
+        if (p.lch[v] == -1) {
+            E.proj_l[v] = add(2, (uint64_t)p.VTptr[v], s, s, p.Ddim[p.lm[v]]);
+        } else {
+            const int l = p.slen[p.lch[v]], r = p.slen[p.rch[v]];
+            E.proj_l[v] = add(2, (uint64_t)p.VTptr[v], s, s, l);
+            E.proj_r[v] = add(2, (uint64_t)p.VTptr[v] + (uint64_t)s * l, s, s, r);
+        }
+    }
+    E.leaf8.resize(p.nleaf);
+    for (int i = 0; i < p.nleaf; ++i) {
+        E.leaf8[i] = E.leaf8_total;
+        E.leaf8_total += ceil8(p.Ddim[i]);
+    }
+    E.node8.assign(p.numnodes, 0);
+    for (int v : p.bfs) {
+        E.node8[v] = E.node8_total;
+        E.node8_total += ceil8(p.slen[v]);
+    }
+}
+
+}  // namespace
+
+int f64_create(Plan &p, const double *D, const double *B, const double *VT)
+{
+    std::vector<PoolJob> jobs[3];
+    uint64_t used[3] = {0, 0, 0};
+    layout(p, jobs, used);
+    F64Engine &E = *p.f64;
+    const double *src[3] = {D, B, VT};
+    const uint64_t len[3] = {p.D_len, p.B_len, p.VT_len};
+    // one allocation for the pools and one for the tiling jobs
+    int rc = p.alloc((void **)&E.pool[0], std::max<uint64_t>(used[0] + used[1] + used[2], 1) * 512);
+    if (rc) return rc;
+    E.pool[1] = E.pool[0] + used[0] * 64;
+    E.pool[2] = E.pool[1] + used[1] * 64;
+    std::vector<PoolJob> all;
+    for (const std::vector<PoolJob> &j : jobs) all.insert(all.end(), j.begin(), j.end());
+    if (all.empty()) return MXB_OK;
+    PoolJob *dj = nullptr;
+    double *copy[3] = {nullptr, nullptr, nullptr};
+    cudaError_t e = cudaMalloc(&dj, all.size() * sizeof(PoolJob));
+    if (e == cudaSuccess) e = cudaMemcpy(dj, all.data(), all.size() * sizeof(PoolJob), cudaMemcpyHostToDevice);
+    size_t first = 0;
+    for (int q = 0; q < 3 && e == cudaSuccess; first += jobs[q++].size()) {
+        if (jobs[q].empty()) continue;
+        // the caller's pool where this device holds it, else a copy for the time of the tiling
+        const double *dev = nullptr;
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, src[q]) != cudaSuccess) (void)cudaGetLastError();
+        else if (at.type == cudaMemoryTypeDevice && at.device == p.device) dev = src[q];
+        if (!dev) {
+            if (q > 0) {  // at most one copy at a time
+                e = cudaDeviceSynchronize();
+                if (copy[q - 1]) cudaFree(copy[q - 1]);
+                copy[q - 1] = nullptr;
+            }
+            if (e == cudaSuccess) e = cudaMalloc(&copy[q], len[q] * sizeof(double));
+            if (e == cudaSuccess) e = cudaMemcpy(copy[q], src[q], len[q] * sizeof(double), cudaMemcpyDefault);
+            if (e != cudaSuccess) break;
+            dev = copy[q];
+        }
+        f64_tile_pool_kernel<<<dim3((unsigned)jobs[q].size(), 4), 256>>>(dj + first, dev, E.pool[q]);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (dj) cudaFree(dj);
+    for (double *c : copy)
+        if (c) cudaFree(c);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        return fail("tiling the CDS: out of device memory", MXB_ERR_NOMEM);
+    }
+    if (e != cudaSuccess) return fail(std::string("tiling the CDS: ") + cudaGetErrorString(e));
+    return MXB_OK;
+}
+
+// ---------------------------------------------------------------------------------------
+// schedule
+// ---------------------------------------------------------------------------------------
+
+namespace {
+
+// Tasks in claim order for one direction and column count; see the file comment.
+int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> &out, std::vector<F64Item> &items,
+                   int &nctr, int64_t &slots)
+{
+    F64Engine &E = *p.f64;
+    auto projects = [&](int v) { return v != p.root && p.slen[v] > 0; };
+    auto has_down = [&](int v) { return p.parent[v] >= 0 && projects(p.parent[v]); };
+    auto ceil8 = [](int v) { return (v + 7) / 8; };
+    auto row_tiles = [&](int rows) { return std::max(1, (ceil8(rows) + 7) / 8); };
+    // counters (times the column count): per leaf W tiled and near field written; per node
+    // wskel, far part and uskel written
+    const int c_w = 0, c_near = p.nleaf, c_up = 2 * p.nleaf, c_far = c_up + p.numnodes, c_u = c_far + p.numnodes;
+    nctr = c_u + p.numnodes;
+    std::vector<Group> G;
+    std::vector<int> g_w(p.nleaf, -1), g_near(p.nleaf, -1), g_up(p.numnodes, -1), g_far(p.numnodes, -1), g_u(p.numnodes, -1);
+    struct Src {
+        F64Block a;
+        int pool, trans, buf, dep, need, group;
+        int64_t base;
+    };
+    auto block_item = [&](const Src &s) {
+        F64Item it{};
+        it.a_off = s.a.off;
+        it.lda = s.a.m8;
+        it.k8 = s.trans ? s.a.m8 : s.a.k8;
+        it.b_base = s.base;
+        it.dep = s.dep;
+        it.need = s.need;
+        it.a_pool = (int16_t)s.pool;
+        it.trans = (int16_t)s.trans;
+        it.b_buf = (int16_t)s.buf;
+        return it;
+    };
+    auto stages_of = [&](int k8) { return (k8 + sh.bk8 - 1) / sh.bk8; };
+    // one group: `rows` output rows, summing the sources
+    auto add_group = [&](int kind, int64_t o, int rows, const std::vector<Src> &srcs, int beta, int sig, int old_dep,
+                         int old_need, int old_group) {
+        Group g;
+        F64Task t{};
+        t.out = o;
+        t.item0 = (int)items.size();
+        t.rows = rows;
+        t.sig = sig;
+        t.old_dep = old_dep;
+        t.old_need = old_need;
+        t.piece_ctr = -1;
+        t.npiece = 1;
+        t.kind = (int16_t)kind;
+        t.beta = (int16_t)beta;
+        for (const Src &s : srcs) {
+            const F64Item it = block_item(s);
+            if (it.k8 <= 0) continue;
+            items.push_back(it);
+            t.stages += stages_of(it.k8);
+            if (s.group >= 0 && std::find(g.deps.begin(), g.deps.end(), s.group) == g.deps.end()) g.deps.push_back(s.group);
+        }
+        t.nitem = (int)items.size() - t.item0;
+        if (old_group >= 0) g.deps.push_back(old_group);
+        const int m8 = ceil8(rows), T = row_tiles(rows);
+        for (int i = 0; i < T; ++i) {  // row tiles of nearly equal height
+            t.r8 = (int)((int64_t)m8 * i / T);
+            t.m8 = (int)((int64_t)m8 * (i + 1) / T) - t.r8;
+            g.tasks.push_back(t);
+        }
+        G.push_back(std::move(g));
+        return (int)G.size() - 1;
+    };
+    const int WR = WARPS;  // every product warp of a tile counts itself
+    for (int i = 0; i < p.nleaf; ++i) {
+        Group g;
+        F64Task t{};
+        t.out = i;
+        t.rows = p.Ddim[i];
+        t.sig = c_w + i;
+        t.old_dep = t.piece_ctr = -1;
+        t.npiece = 1;
+        t.kind = F64_TILE_W;
+        t.slot = (int)E.leaf8[i];
+        const int m8 = ceil8(p.Ddim[i]), T = row_tiles(p.Ddim[i]);
+        for (int k = 0; k < T; ++k) {
+            t.r8 = (int)((int64_t)m8 * k / T);
+            t.m8 = (int)((int64_t)m8 * (k + 1) / T) - t.r8;
+            g.tasks.push_back(t);
+        }
+        G.push_back(std::move(g));
+        g_w[i] = (int)G.size() - 1;
+    }
+    auto w_src = [&](const F64Block &a, int pool, int trans, int leaf) {
+        return Src{a, pool, trans, BUF_W, c_w + leaf, WR * row_tiles(p.Ddim[leaf]), g_w[leaf], E.leaf8[leaf]};
+    };
+    auto up_src = [&](const F64Block &a, int pool, int trans, int v) {
+        return Src{a, pool, trans, BUF_WSKEL, c_up + v, WR * row_tiles(p.slen[v]), g_up[v], E.node8[v]};
+    };
+    auto u_src = [&](const F64Block &a, int pool, int trans, int v) {
+        return Src{a, pool, trans, BUF_USKEL, c_u + v, WR * row_tiles(p.slen[v]), g_u[v], E.node8[v]};
+    };
+    for (auto it = p.bfs.rbegin(); it != p.bfs.rend(); ++it) {  // children before parents
+        const int v = *it;
+        if (!projects(v)) continue;
+        std::vector<Src> s;
+        if (p.lch[v] == -1) {
+            s.push_back(w_src(E.proj_l[v], 2, 0, p.lm[v]));
+        } else {
+            if (p.slen[p.lch[v]] > 0) s.push_back(up_src(E.proj_l[v], 2, 0, p.lch[v]));
+            if (p.slen[p.rch[v]] > 0) s.push_back(up_src(E.proj_r[v], 2, 0, p.rch[v]));
+        }
+        g_up[v] = add_group(F64_WSKEL, E.node8[v], p.slen[v], s, 0, c_up + v, -1, 0, -1);
+    }
+    std::vector<std::vector<int>> far_of(p.numnodes), near_of(p.nleaf);
+    for (size_t k = 0; k < p.far_x.size(); ++k) far_of[adjoint ? p.far_y[k] : p.far_x[k]].push_back((int)k);
+    for (size_t k = 0; k < p.near_x.size(); ++k) near_of[adjoint ? p.near_y[k] : p.near_x[k]].push_back((int)k);
+    for (int v : p.bfs) {
+        if (!projects(v)) continue;
+        std::vector<Src> s;
+        for (int k : far_of[v]) {
+            const int o = adjoint ? p.far_x[k] : p.far_y[k];
+            if (p.slen[o] > 0) s.push_back(up_src(E.far[k], 1, adjoint ? 1 : 0, o));
+        }
+        if (s.empty() && has_down(v)) continue;
+        g_far[v] = add_group(F64_USKEL, E.node8[v], p.slen[v], s, 0, has_down(v) ? c_far + v : c_u + v, -1, 0, -1);
+        if (!has_down(v)) g_u[v] = g_far[v];
+    }
+    for (int v : p.bfs) {  // parents before children
+        if (!projects(v) || !has_down(v)) continue;
+        const int q = p.parent[v];
+        const bool far = g_far[v] >= 0;
+        g_u[v] = add_group(F64_USKEL, E.node8[v], p.slen[v],
+                           {u_src(v == p.rch[q] ? E.proj_r[q] : E.proj_l[q], 2, 1, q)}, far ? 1 : 0, c_u + v,
+                           far ? c_far + v : -1, WR * row_tiles(p.slen[v]), g_far[v]);
+    }
+    std::vector<int> leaf_node(p.nleaf, -1);
+    for (int v = 0; v < p.numnodes; ++v)
+        if (p.lch[v] == -1) leaf_node[p.lm[v]] = v;
+    for (int i = 0; i < p.nleaf; ++i) {
+        std::vector<Src> s;
+        for (int k : near_of[i]) s.push_back(w_src(E.near[k], 0, adjoint ? 1 : 0, adjoint ? p.near_x[k] : p.near_y[k]));
+        g_near[i] = add_group(F64_Y, i, p.Ddim[i], s, 2, c_near + i, -1, 0, -1);
+        const int v = leaf_node[i];
+        if (projects(v))
+            add_group(F64_Y, i, p.Ddim[i], {u_src(E.proj_l[v], 2, 1, v)}, 1, -1, c_near + i, WR * row_tiles(p.Ddim[i]), g_near[i]);
+    }
+
+    // Long sums are cut along K where one would keep a block busy for a large part of the
+    // launch: pieces of about an eighth of a block's share of all stages, at least 256 deep
+    // (N = 32768 adjoint, 64 right-hand sides: 707 us; a third of the share: 800 us; sixteenths
+    // only add partial tiles).
+    const int blocks = sm_count() * sh.ctas;
+    int64_t total = 0;
+    for (const Group &g : G)
+        for (const F64Task &t : g.tasks) total += (int64_t)t.stages * sh.ncol;
+    const int chunk = (int)std::max<int64_t>(32 / sh.bk8, total / (8 * (int64_t)blocks));
+    slots = 0;
+    for (Group &g : G) {
+        const F64Task t0 = g.tasks[0];
+        if (t0.stages <= chunk + chunk / 2) continue;
+        const int n = (t0.stages + chunk - 1) / chunk;
+        // item ranges of the pieces, cut at stage boundaries
+        std::vector<std::pair<int, int>> range;  // item0, nitem
+        std::vector<int> len;
+        int q = 0, off = 0;
+        const std::vector<F64Item> src(items.begin() + t0.item0, items.begin() + t0.item0 + t0.nitem);
+        for (int i = 0; i < n; ++i) {
+            int want = (int)((int64_t)t0.stages * (i + 1) / n) - (int)((int64_t)t0.stages * i / n);
+            range.push_back({(int)items.size(), 0});
+            len.push_back(want);
+            while (want > 0) {
+                F64Item it = src[q];
+                const int have = stages_of(it.k8 - off), take = std::min(want, have);
+                it.a_off += it.trans ? (uint64_t)off : (uint64_t)off * it.lda;
+                it.b_base += off;
+                it.k8 = std::min(take * sh.bk8, it.k8 - off);
+                items.push_back(it);
+                ++range.back().second;
+                want -= take;
+                off += take * sh.bk8;
+                if (take == have) {
+                    ++q;
+                    off = 0;
+                }
+            }
+        }
+        std::vector<F64Task> pieces;
+        for (const F64Task &base : g.tasks) {
+            for (int i = 0; i < n; ++i) {
+                F64Task t = base;
+                t.item0 = range[i].first;
+                t.nitem = range[i].second;
+                t.stages = len[i];
+                t.piece = i;
+                t.npiece = n;
+                t.piece_ctr = nctr;
+                t.slot = (int)slots;
+                pieces.push_back(t);
+            }
+            nctr += WARPS;  // one arrival counter per product warp
+            slots += n;
+        }
+        g.tasks = std::move(pieces);
+    }
+
+    // List scheduling, longest remaining path first among the groups whose inputs are written.  A
+    // worker stands for the blocks that run one task's column tiles side by side; it claims its
+    // next task once the loads of the current one are issued, STAGES before its products end.
+    // Times in stages of a busy SM (1.0 - 1.5 us): writing a tile out and publishing it takes
+    // about EPILOGUE, seeing it and loading from it about LATENCY.
+    const int EPILOGUE = sh.bn == 8 ? 4 : 2, LATENCY = 2, DEPTH = 3;
+    for (int i = 0; i < (int)G.size(); ++i) {
+        Group &g = G[i];
+        for (const F64Task &t : g.tasks) g.cost = std::max(g.cost, t.stages + EPILOGUE + LATENCY);
+        for (int d : g.deps) G[d].cons.push_back(i);
+        g.unplaced = (int)g.deps.size();
+    }
+    std::function<double(int)> prio = [&](int i) -> double {
+        Group &g = G[i];
+        if (g.prio >= 0) return g.prio;
+        double best = 0;
+        for (int c : g.cons) best = std::max(best, prio(c));
+        return g.prio = best + g.cost;
+    };
+    for (int i = 0; i < (int)G.size(); ++i) prio(i);
+    struct Worker {
+        double claim, free;
+        bool operator>(const Worker &o) const { return claim > o.claim; }
+    };
+    auto low = [&](int a, int b) { return G[a].prio != G[b].prio ? G[a].prio < G[b].prio : a > b; };
+    auto late = [&](int a, int b) { return G[a].ready != G[b].ready ? G[a].ready > G[b].ready : a > b; };
+    std::priority_queue<int, std::vector<int>, decltype(low)> ready(low);
+    std::priority_queue<int, std::vector<int>, decltype(late)> waiting(late);
+    std::priority_queue<Worker, std::vector<Worker>, std::greater<Worker>> workers;
+    for (int i = 0; i < std::max(1, blocks / sh.ncol); ++i) workers.push(Worker{0.0, 0.0});
+    for (int i = 0; i < (int)G.size(); ++i)
+        if (!G[i].unplaced) waiting.push(i);
+    out.clear();
+    for (size_t placed = 0; placed < G.size(); ++placed) {
+        const double now = workers.top().claim;
+        while (!waiting.empty() && G[waiting.top()].ready <= now) {
+            ready.push(waiting.top());
+            waiting.pop();
+        }
+        int i;
+        if (!ready.empty()) {
+            i = ready.top();
+            ready.pop();
+        } else if (!waiting.empty()) {
+            i = waiting.top();
+            waiting.pop();
+        } else {
+            return fail("FP64 schedule: a block's inputs are never written", MXB_ERR_STRUCTURE);
+        }
+        Group &g = G[i];
+        for (const F64Task &t : g.tasks) {
+            Worker w = workers.top();
+            workers.pop();
+            const double load = std::max(w.claim, g.ready), end = std::max(load + 1, w.free) + t.stages;
+            w.claim = std::max(load, end - DEPTH);
+            w.free = end + EPILOGUE;
+            workers.push(w);
+            g.finish = std::max(g.finish, w.free);
+            out.push_back(t);
+        }
+        for (int c : g.cons) {
+            G[c].ready = std::max(G[c].ready, g.finish + LATENCY);
+            if (--G[c].unplaced == 0) waiting.push(c);
+        }
+    }
+    return MXB_OK;
+}
+
+void free_buffer(Plan &p, void *q, size_t bytes)
+{
+    if (!q) return;
+    cudaFree(q);
+    p.allocations.erase(std::remove(p.allocations.begin(), p.allocations.end(), q), p.allocations.end());
+    p.device_bytes -= std::max<size_t>(bytes, 16);
+}
+
+int schedule_for(Plan &p, bool adjoint, const Shape &sh, F64Engine::Schedule **out)
+{
+    F64Engine &E = *p.f64;
+    for (F64Engine::Schedule &s : E.schedules)
+        if (s.adjoint == adjoint && s.ncol == sh.ncol && s.bn == sh.bn) {
+            *out = &s;
+            return MXB_OK;
+        }
+    std::vector<F64Task> tasks;
+    std::vector<F64Item> items;
+    F64Engine::Schedule s;
+    s.adjoint = adjoint;
+    s.ncol = sh.ncol;
+    s.bn = sh.bn;
+    int rc = build_schedule(p, adjoint, sh, tasks, items, s.nctr, s.slots);
+    if (rc) return rc;
+    s.ntasks = (int)tasks.size();
+    if ((int64_t)s.ntasks * sh.ncol > 0x3FFFFFFF) return fail("too many work units", MXB_ERR_UNSUPPORTED);
+    if (E.schedules.size() >= 8) {  // a bounded number of column counts is kept
+        cudaFree(E.schedules.front().tasks);
+        E.schedules.erase(E.schedules.begin());
+    }
+    const size_t tb = tasks.size() * sizeof(F64Task), ib = items.size() * sizeof(F64Item);
+    std::vector<uint8_t> both(tb + ib);
+    std::memcpy(both.data(), tasks.data(), tb);
+    if (ib) std::memcpy(both.data() + tb, items.data(), ib);
+    cudaError_t e = cudaMalloc(&s.tasks, std::max<size_t>(both.size(), 16));
+    if (e == cudaSuccess) e = cudaMemcpy(s.tasks, both.data(), both.size(), cudaMemcpyHostToDevice);
+    // the launch's stream does not wait for the legacy stream, and a copy from pageable memory
+    // may return before it has landed
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (e != cudaSuccess) {
+        if (s.tasks) cudaFree(s.tasks);
+        return fail(std::string("FP64 schedule: ") + cudaGetErrorString(e),
+                    e == cudaErrorMemoryAllocation ? MXB_ERR_NOMEM : MXB_ERR_CUDA);
+    }
+    s.items = reinterpret_cast<F64Item *>(s.tasks + tasks.size());
+    E.schedules.push_back(s);
+    *out = &E.schedules.back();
+    return MXB_OK;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------------------
+// evaluation
+// ---------------------------------------------------------------------------------------
+
+int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs,
+                 int nrhs, int accumulate, cudaStream_t stream)
+{
+    F64Engine &E = *p.f64;
+    const int nb = (nrhs + 7) / 8;
+    const Shape sh = shape_for(nb);
+    F64Engine::Schedule *s = nullptr;
+    int rc = schedule_for(p, adjoint, sh, &s);
+    if (rc) return rc;
+    if (nb > E.buf_nb) {
+        free_buffer(p, E.buf[0], (size_t)(E.leaf8_total + 2 * E.node8_total) * E.buf_nb * 512);
+        E.buf[0] = nullptr;
+        E.buf_nb = 0;
+        rc = p.alloc((void **)&E.buf[0], (size_t)(E.leaf8_total + 2 * E.node8_total) * nb * 512);
+        if (rc) return rc;
+        E.buf[1] = E.buf[0] + (size_t)E.leaf8_total * nb * 64;
+        E.buf[2] = E.buf[1] + (size_t)E.node8_total * nb * 64;
+        E.buf_nb = nb;
+    }
+    // counters (zero between launches: each launch's last block clears what it used), then the
+    // partial tiles
+    const size_t ctl = ((CTL_FIRST + (size_t)s->nctr * sh.ncol) * sizeof(int) + 511) / 512 * 512;
+    const size_t partial = (size_t)s->slots * sh.ncol * 64 * sh.bn * sizeof(double);
+    if (ctl > E.ctl_bytes || partial > E.partial_bytes) {
+        const size_t c = std::max(ctl, E.ctl_bytes), q = std::max(partial, E.partial_bytes);
+        free_buffer(p, E.ctl, E.ctl_bytes + E.partial_bytes);
+        E.ctl = nullptr;
+        E.ctl_bytes = E.partial_bytes = 0;
+        rc = p.alloc((void **)&E.ctl, c + q);
+        if (rc) return rc;
+        F64_CUDA(cudaMemset(E.ctl, 0, c));
+        F64_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        E.ctl_bytes = c;
+        E.partial_bytes = q;
+    }
+    Args a{};
+    for (int q = 0; q < 3; ++q) {
+        a.pool[q] = E.pool[q];
+        a.buf[q] = E.buf[q];
+    }
+    a.W = dW;
+    a.Y = dY;
+    a.wofs = wofs;
+    a.yofs = yofs;
+    a.tasks = s->tasks;
+    a.items = s->items;
+    a.partial = reinterpret_cast<double *>(E.ctl + E.ctl_bytes / sizeof(int));
+    a.ctl = E.ctl;
+    // ~2 s, and longer for evaluations that themselves take that long
+    a.wait_cycles = p.debug_wait_cycles > 0 ? p.debug_wait_cycles : tc::WAIT_CYCLES + (long long)(p.flops(nrhs) / 500);
+    a.units = s->ntasks * sh.ncol;
+    a.ncol = sh.ncol;
+    a.nb = nb;
+    a.nrhs = nrhs;
+    a.beta = accumulate ? 1 : 0;
+    a.nctr = s->nctr * sh.ncol;
+    switch (sh.bn) {
+    case 8: return launch<8>(a, stream);
+    case 16: return launch<16>(a, stream);
+    default: return launch<32>(a, stream);
+    }
+}
+
+int f64_status(Plan &p)
+{
+    if (!p.f64 || !p.f64->ctl) return MXB_OK;
+    int h = 0;
+    F64_CUDA(cudaMemcpy(&h, p.f64->ctl + CTL_ERR, sizeof(int), cudaMemcpyDeviceToHost));
+    if (!h) return MXB_OK;
+    F64_CUDA(cudaMemset(p.f64->ctl + CTL_ERR, 0, sizeof(int)));
+    F64_CUDA(cudaDeviceSynchronize());
+    return fail("an FP64 kernel wait timed out (MXB_ERR_TIMEOUT)", h);
+}
+
+// The last evaluation's skeleton vectors, node-blocked column-major (as skel_row * nrhs).
+int f64_read_skeletons(Plan &p, int nrhs, std::vector<double> &w, std::vector<double> &u)
+{
+    F64Engine &E = *p.f64;
+    const int64_t nb = (nrhs + 7) / 8;
+    if (nb > E.buf_nb) return fail("no evaluation with this nrhs has run on the plan", MXB_ERR_ARG);
+    F64_CUDA(cudaDeviceSynchronize());
+    std::vector<double> h((size_t)E.node8_total * nb * 64);
+    for (int which = 0; which < 2; ++which) {
+        std::vector<double> &o = which ? u : w;
+        o.assign((size_t)p.skel_total * nrhs, 0.0);
+        F64_CUDA(cudaMemcpy(h.data(), E.buf[which ? BUF_USKEL : BUF_WSKEL], h.size() * sizeof(double), cudaMemcpyDeviceToHost));
+        for (int v = 0; v < p.numnodes; ++v)
+            for (int c = 0; c < nrhs; ++c)
+                for (int r = 0; r < p.slen[v]; ++r)
+                    o[(size_t)p.skel_row[v] * nrhs + (size_t)c * p.slen[v] + r] =
+                        h[((size_t)(E.node8[v] + r / 8) * nb + c / 8) * 64 + (c % 8) * 8 + ((r % 8) ^ ((((c % 8) >> 1) & 1) << 2))];
+    }
+    return MXB_OK;
+}
+
+void f64_destroy(Plan &p)
+{
+    if (!p.f64) return;
+    for (F64Engine::Schedule &s : p.f64->schedules) cudaFree(s.tasks);
+    delete p.f64;
+    p.f64 = nullptr;
+}
+
+}  // namespace mxb
+
+// Test hook (no counterpart in the reference): the task list of the FP64 launch; host code only.
+extern "C" int32_t mxb_debug_f64_schedule(const mxb_cds_desc *desc, int32_t adjoint, int32_t nrhs, void *tasks,
+                                          int64_t task_cap, void *items, int64_t item_cap, int64_t *counts)
+{
+    if (!desc || nrhs < 1 || !tasks || !items || !counts) {
+        mxb::set_error("bad FP64 schedule arguments");
+        return MXB_ERR_ARG;
+    }
+    mxb::Plan p;
+    int rc = p.validate(*desc);
+    if (rc) return rc;
+    std::vector<mxb::PoolJob> jobs[3];
+    uint64_t used[3] = {0, 0, 0};
+    mxb::layout(p, jobs, used);
+    const mxb::Shape sh = mxb::shape_for((nrhs + 7) / 8);
+    std::vector<mxb::F64Task> t;
+    std::vector<mxb::F64Item> it;
+    int nctr = 0;
+    int64_t slots = 0;
+    rc = mxb::build_schedule(p, adjoint != 0, sh, t, it, nctr, slots);
+    if (rc) return rc;
+    const int64_t c[9] = {(int64_t)t.size(), (int64_t)it.size(), nctr, slots, sh.ncol, sh.bk8,
+                          (int64_t)used[0], (int64_t)used[1], (int64_t)used[2]};
+    std::memcpy(counts, c, sizeof(c));
+    if ((int64_t)t.size() > task_cap || (int64_t)it.size() > item_cap) {
+        mxb::set_error("output arrays too short");
+        return MXB_ERR_ARG;
+    }
+    std::memcpy(tasks, t.data(), t.size() * sizeof(mxb::F64Task));
+    std::memcpy(items, it.data(), it.size() * sizeof(mxb::F64Item));
+    return MXB_OK;
+}

@@ -1,4 +1,7 @@
-// FP64 grouped variable-size GEMM on the B200's FP64 tensor path.
+// FP64 grouped variable-size GEMM on the B200's FP64 tensor path, reading the caller's CDS pools in
+// place: the kernel of mxb_evaluate_noalloc, which may not hold a re-tiled copy of the CDS.  Plans
+// run the dataflow launch of f64_engine.cu instead (N = 65536, 1024 right-hand sides: 23.3 ms
+// against 25.6 ms here).
 //
 // tcgen05.mma has no f64 kind, so FP64 products use the DMMA instruction
 // mma.sync.m8n8k4.f64 (sm_80+).  One CTA computes a 64 x 64 tile of one task's output
@@ -276,15 +279,6 @@ cudaError_t launch_gemm_f64(const Task *tasks, const Item *items, int ntasks, co
     if (blocks > 0x7FFFFFFF) return cudaErrorInvalidConfiguration;
     gemm_f64_kernel<<<(unsigned)blocks, THREADS, SMEM_BYTES, stream>>>(tasks, items, ops);
     return cudaGetLastError();
-}
-
-int f64_row_tile() { return BM; }
-
-cudaError_t prepare_gemm_f64()
-{
-    Operands ops{};
-    ops.nrhs = 1;
-    return launch_gemm_f64(nullptr, nullptr, 0, ops, 0) == cudaSuccess ? cudaSuccess : cudaErrorUnknown;
 }
 
 }  // namespace mxb

@@ -71,8 +71,6 @@ struct Plan;
 cudaError_t launch_gemm_f64(const Task *tasks, const Item *items, int ntasks,
                             const Operands &ops, cudaStream_t stream);
 
-cudaError_t prepare_gemm_f64();  // sets the kernel's shared-memory limit (before any capture)
-
 // Row permutation between the caller's point order and the leaf-blocked tree order
 // (permute.cu): dir 0 gathers dst(leaf-blocked) = src[perm rows], dir 1 scatters
 // dst[perm rows] (+)= src(leaf-blocked).  The caller-order matrix has element (p, j) at

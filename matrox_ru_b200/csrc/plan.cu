@@ -1,6 +1,8 @@
 // Plan: validated structure, device copy of the CDS and the task lists of every pass.
 //
-// Schedule of one evaluation (the reference runs the same four phases,
+// FP64 plans evaluate in one dataflow launch (f64_engine.cu).  The launch-per-pass lists built
+// here are what mxb_evaluate_noalloc runs, and the pass-by-pass flop accounting of the profile.
+// Schedule of one such evaluation (the reference runs the same four phases,
 // symGen/HGEMM_gen.h:125-236, but as thousands of separate DGEMM calls):
 //   1. leaf up        wskel[v] = P_v W[leaf v]                          (one launch)
 //   2. transfer up    wskel[v] = P_v [wskel[l]; wskel[r]]    one launch per height, bottom-up
@@ -22,6 +24,7 @@
 
 #include "matrox_b200.h"
 #include "mxb_internal.h"
+#include "f64_engine.h"
 #include "plan.h"
 
 namespace mxb {
@@ -47,7 +50,7 @@ int row_tile_for(int precision);
 Plan::~Plan()
 {
     clear_graphs();
-    if (capture_stream) cudaStreamDestroy(capture_stream);
+    f64_destroy(*this);
     free_split_bf16();
     for (void *p : allocations) cudaFree(p);
 }
@@ -404,24 +407,21 @@ int Plan::create(const mxb_cds_desc &d, int prec, Plan **out)
     int rc = p->validate(d);
     if (rc) return rc;
     p->build_tasks(row_tile_for(prec));
-    // FP64 CDS (host or device arrays: cudaMemcpyDefault follows the pointers)
-    rc = p->alloc((void **)&p->dD, std::max<uint64_t>(d.D_len, 1) * sizeof(double));
-    if (rc) return rc;
-    MXB_CUDA(cudaMemcpy(p->dD, d.D, d.D_len * sizeof(double), cudaMemcpyDefault));
-    rc = p->alloc((void **)&p->dB, std::max<uint64_t>(d.B_len, 1) * sizeof(double));
-    if (rc) return rc;
-    if (d.B_len) MXB_CUDA(cudaMemcpy(p->dB, d.B, d.B_len * sizeof(double), cudaMemcpyDefault));
-    rc = p->alloc((void **)&p->dVT, std::max<uint64_t>(d.VT_len, 1) * sizeof(double));
-    if (rc) return rc;
-    if (d.VT_len) MXB_CUDA(cudaMemcpy(p->dVT, d.VT, d.VT_len * sizeof(double), cudaMemcpyDefault));
-    rc = p->alloc((void **)&p->dTasks, p->tasks.size() * sizeof(Task));
-    if (rc) return rc;
-    if (!p->tasks.empty())
-        MXB_CUDA(cudaMemcpy(p->dTasks, p->tasks.data(), p->tasks.size() * sizeof(Task), cudaMemcpyHostToDevice));
-    rc = p->alloc((void **)&p->dItems, p->items.size() * sizeof(Item));
-    if (rc) return rc;
-    if (!p->items.empty())
-        MXB_CUDA(cudaMemcpy(p->dItems, p->items.data(), p->items.size() * sizeof(Item), cudaMemcpyHostToDevice));
+    if (prec == MXB_PREC_FP64) {
+        rc = f64_create(*p, d.D, d.B, d.VT);
+        if (rc) return rc;
+    } else {
+        // FP64 CDS for the tiling (host or device arrays: cudaMemcpyDefault follows the pointers)
+        rc = p->alloc((void **)&p->dD, std::max<uint64_t>(d.D_len, 1) * sizeof(double));
+        if (rc) return rc;
+        MXB_CUDA(cudaMemcpy(p->dD, d.D, d.D_len * sizeof(double), cudaMemcpyDefault));
+        rc = p->alloc((void **)&p->dB, std::max<uint64_t>(d.B_len, 1) * sizeof(double));
+        if (rc) return rc;
+        if (d.B_len) MXB_CUDA(cudaMemcpy(p->dB, d.B, d.B_len * sizeof(double), cudaMemcpyDefault));
+        rc = p->alloc((void **)&p->dVT, std::max<uint64_t>(d.VT_len, 1) * sizeof(double));
+        if (rc) return rc;
+        if (d.VT_len) MXB_CUDA(cudaMemcpy(p->dVT, d.VT, d.VT_len * sizeof(double), cudaMemcpyDefault));
+    }
     rc = p->alloc((void **)&p->dOfs, 4 * (size_t)p->nleaf * sizeof(int32_t));
     if (rc) return rc;
     if (prec != MXB_PREC_FP64) {
@@ -436,34 +436,7 @@ int Plan::create(const mxb_cds_desc &d, int prec, Plan **out)
     return MXB_OK;
 }
 
-void Plan::clear_graphs()
-{
-    for (GraphEntry &g : graphs) cudaGraphExecDestroy(g.exec);
-    graphs.clear();
-    clear_split_graphs();
-}
-
-int Plan::ensure_scratch(int nrhs)
-{
-    const size_t need = (size_t)std::max<int64_t>(skel_total, 1) * nrhs;
-    if (need <= scratch_elems) return MXB_OK;
-    clear_graphs();
-    if (dWskel) {
-        cudaFree(dWskel);
-        cudaFree(dUskel);
-        allocations.erase(std::remove(allocations.begin(), allocations.end(), (void *)dWskel), allocations.end());
-        allocations.erase(std::remove(allocations.begin(), allocations.end(), (void *)dUskel), allocations.end());
-        device_bytes -= 2 * scratch_elems * sizeof(double);
-        dWskel = dUskel = nullptr;
-        scratch_elems = 0;
-    }
-    int rc = alloc((void **)&dWskel, need * sizeof(double));
-    if (rc) return rc;
-    rc = alloc((void **)&dUskel, need * sizeof(double));
-    if (rc) return rc;
-    scratch_elems = need;
-    return MXB_OK;
-}
+void Plan::clear_graphs() { clear_split_graphs(); }
 
 // Per-leaf offsets for one call; packed offsets when the caller passes none.
 int Plan::stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t stream)
@@ -507,53 +480,12 @@ int Plan::run(const std::vector<Launch> &L, const double *dW, double *dY, int nr
         set_error("plan used on a different device than it was created on");
         return MXB_ERR_ARG;
     }
-    int rc = precision == MXB_PREC_FP64 ? ensure_scratch(nrhs) : MXB_OK;  // FP64 skeleton scratch
-    if (rc) return rc;
-    rc = stage_offsets(0, wofs, nrhs, stream);
+    int rc = stage_offsets(0, wofs, nrhs, stream);
     if (rc) return rc;
     rc = stage_offsets(1, yofs, nrhs, stream);
     if (rc) return rc;
     if (precision != MXB_PREC_FP64) return run_split_bf16(L, dW, dY, nrhs, accumulate, stream);
-    MXB_CUDA(prepare_gemm_f64());
-    static const bool use_graphs = [] {
-        const char *e = getenv("MXB_NO_GRAPHS");
-        return !(e && *e && *e != '0');
-    }();
-    if (!use_graphs) return enqueue(L, dW, dY, nrhs, accumulate, stream);
-    // replay a captured graph of the whole evaluation: one launch instead of dozens
-    GraphEntry *hit = nullptr;
-    for (GraphEntry &g : graphs)
-        if (g.launches == &L && g.W == dW && g.Y == dY && g.nrhs == nrhs && g.accumulate == accumulate) hit = &g;
-    if (!hit) {
-        if (!capture_stream) MXB_CUDA(cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking));
-        MXB_CUDA(cudaStreamBeginCapture(capture_stream, cudaStreamCaptureModeThreadLocal));
-        rc = enqueue(L, dW, dY, nrhs, accumulate, capture_stream);
-        cudaGraph_t graph = nullptr;
-        cudaError_t e = cudaStreamEndCapture(capture_stream, &graph);
-        if (rc) {
-            if (graph) cudaGraphDestroy(graph);
-            return rc;
-        }
-        if (e != cudaSuccess) {
-            set_error(std::string("capturing the evaluation graph: ") + cudaGetErrorString(e));
-            return MXB_ERR_CUDA;
-        }
-        cudaGraphExec_t exec = nullptr;
-        e = cudaGraphInstantiate(&exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e != cudaSuccess) {
-            set_error(std::string("instantiating the evaluation graph: ") + cudaGetErrorString(e));
-            return MXB_ERR_CUDA;
-        }
-        if (graphs.size() >= 8) {
-            cudaGraphExecDestroy(graphs.front().exec);
-            graphs.erase(graphs.begin());
-        }
-        graphs.push_back(GraphEntry{&L, dW, dY, nrhs, accumulate, exec});
-        hit = &graphs.back();
-    }
-    MXB_CUDA(cudaGraphLaunch(hit->exec, stream));
-    return MXB_OK;
+    return f64_evaluate(*this, &L == &launches_adj, dW, dY, dOfs, dOfs + nleaf, nrhs, accumulate, stream);
 }
 
 // The caller's point order: perm[t] is the row of W / Y holding tree position t (the `lids`
@@ -631,32 +563,6 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
     return MXB_OK;
 }
 
-int Plan::enqueue(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, int accumulate,
-                  cudaStream_t stream)
-{
-    if (precision != MXB_PREC_FP64) return run_split_bf16(L, dW, dY, nrhs, accumulate, stream);
-    Operands ops{};
-    ops.pool[0] = dD;
-    ops.pool[1] = dB;
-    ops.pool[2] = dVT;
-    ops.W = dW;
-    ops.Y = dY;
-    ops.wskel = dWskel;
-    ops.uskel = dUskel;
-    ops.wofs = dOfs;
-    ops.yofs = dOfs + nleaf;
-    ops.nrhs = nrhs;
-    ops.beta_arg = accumulate ? 1 : 0;
-    for (const Launch &l : L) {
-        cudaError_t e = launch_gemm_f64(dTasks + l.task0, dItems, l.ntasks, ops, stream);
-        if (e != cudaSuccess) {
-            set_error(std::string("FP64 grouped GEMM launch: ") + cudaGetErrorString(e));
-            return MXB_ERR_CUDA;
-        }
-    }
-    return MXB_OK;
-}
-
 // Launch-by-launch timing of the forward evaluation (mxb_plan_profile).
 int Plan::profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, mxb_op_profile *out, int cap,
                   int *nops)
@@ -665,24 +571,25 @@ int Plan::profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, m
     if (rc) return rc;
     if (precision != MXB_PREC_FP64) return batch_profile(split_bf16_batch(*this), &dW, &dY, &nrhs, stream, out, cap, nops);
     const std::vector<Launch> &L = launches_fwd;
+    // one launch runs every pass: the first record carries its time, the others are chained to it
     const int tile = row_tile_for(precision), ncol = (int)((nrhs + tile - 1) / tile);
-    std::vector<cudaEvent_t> ev(L.size() + 1, nullptr);
+    cudaEvent_t ev[2] = {nullptr, nullptr};
     for (cudaEvent_t &e : ev)
         if (!rc && cudaEventCreate(&e) != cudaSuccess) {
             set_error("profile: creating CUDA events failed");
             rc = MXB_ERR_CUDA;
         }
+    float ms = 0.f;
     for (int rep = 0; rep < 2 && !rc; ++rep) {
         cudaEventRecord(ev[0], stream);
-        for (size_t i = 0; i < L.size() && !rc; ++i) {
-            rc = enqueue(std::vector<Launch>{L[i]}, dW, dY, nrhs, 0, stream);
-            cudaEventRecord(ev[i + 1], stream);
-        }
+        rc = run(L, dW, dY, nrhs, nullptr, nullptr, 0, stream);
+        cudaEventRecord(ev[1], stream);
         if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) {
             set_error("profile: stream synchronisation failed");
             rc = MXB_ERR_CUDA;
         }
     }
+    if (!rc) cudaEventElapsedTime(&ms, ev[0], ev[1]);
     if (nops) *nops = (int)L.size();
     for (size_t i = 0; i < L.size() && !rc && (int)i < cap && out; ++i) {
         const Launch &l = L[i];
@@ -700,7 +607,8 @@ int Plan::profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, m
                 o.issued_flops += 2.0 * tile * items[k].K * (double)ncol * tile;
             }
         }
-        cudaEventElapsedTime(&o.ms, ev[i], ev[i + 1]);
+        o.chained = i > 0;
+        o.ms = i ? 0.f : ms;
     }
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
@@ -713,14 +621,9 @@ int Plan::read_workspaces(int nrhs, const int32_t *wsko, double *wskel, const in
         set_error("skeleton workspaces are kept by FP64 plans only");
         return MXB_ERR_UNSUPPORTED;
     }
-    if (!dWskel || scratch_elems < (size_t)skel_total * nrhs) {
-        set_error("no evaluation with this nrhs has run on the plan");
-        return MXB_ERR_ARG;
-    }
-    MXB_CUDA(cudaDeviceSynchronize());
-    std::vector<double> w((size_t)skel_total * nrhs), u((size_t)skel_total * nrhs);
-    MXB_CUDA(cudaMemcpy(w.data(), dWskel, w.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    MXB_CUDA(cudaMemcpy(u.data(), dUskel, u.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    std::vector<double> w, u;
+    const int rc = f64_read_skeletons(*this, nrhs, w, u);
+    if (rc) return rc;
     for (int v = 0; v < numnodes; ++v) {
         const size_t n = (size_t)slen[v] * nrhs;
         if (!n) continue;

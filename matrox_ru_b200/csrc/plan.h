@@ -15,6 +15,7 @@ struct mxb_batch {
 
 namespace mxb {
 
+struct F64Engine;  // device state of the FP64 path (f64_engine.cu)
 struct SplitBF16;  // device state of the split-BF16 path (split_bf16.cu)
 struct Batch;     // merged launch sequence of several split-BF16 plans (split_bf16.cu)
 
@@ -40,18 +41,15 @@ struct Plan : public mxb_plan {
     std::vector<Launch> launches_fwd, launches_adj;
 
     // ---- device state ----
-    double *dD = nullptr, *dB = nullptr, *dVT = nullptr;
-    Task *dTasks = nullptr;
-    Item *dItems = nullptr;
+    double *dD = nullptr, *dB = nullptr, *dVT = nullptr;  // split-BF16: the FP64 CDS while it is being tiled
     int32_t *dOfs = nullptr;  // 4 x nleaf per-leaf offsets (slots: in, out, spare)
     std::vector<int32_t> ofs_host[4];
-    double *dWskel = nullptr, *dUskel = nullptr;
-    size_t scratch_elems = 0;
     // caller point order (mxb_plan_set_permutation): perm (rows_total entries) followed by
     // the first tree position of every leaf (nleaf + 1 entries)
     int32_t *dTree = nullptr;
     double *dTW = nullptr, *dTY = nullptr;  // leaf-blocked copies for the unfused caller-order path
     size_t order_elems = 0;
+    F64Engine *f64 = nullptr;
     SplitBF16 *bf16 = nullptr;
     int debug_flags = 0;              // test hooks (mxb_plan_set_test_hooks)
     long long debug_wait_cycles = 0;  // 0: default wait limit
@@ -64,7 +62,6 @@ struct Plan : public mxb_plan {
     void add_task(std::vector<Task> &tasks, int16_t c_kind, int64_t c_row, int ldc, int M, int item0,
                   int nitem, int16_t beta, int tile);
     int alloc(void **p, size_t bytes);
-    int ensure_scratch(int nrhs);
     int stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t stream);
     int run(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, const int32_t *wofs,
             const int32_t *yofs, int accumulate, cudaStream_t stream);
@@ -76,19 +73,7 @@ struct Plan : public mxb_plan {
     int read_workspaces(int nrhs, const int32_t *wsko, double *wskel, const int32_t *usko, double *uskel);
     uint64_t flops(int nrhs) const;
 
-    // evaluation replay: one CUDA graph per (operands, nrhs, accumulate, direction)
-    struct GraphEntry {
-        const void *launches;
-        const double *W;
-        double *Y;
-        int nrhs, accumulate;
-        cudaGraphExec_t exec;
-    };
-    std::vector<GraphEntry> graphs;
-    cudaStream_t capture_stream = nullptr;
     void clear_graphs();
-    int enqueue(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, int accumulate,
-                cudaStream_t stream);
 
     // split-BF16 path (split_bf16.cu)
     int setup_split_bf16(const mxb_cds_desc &d);

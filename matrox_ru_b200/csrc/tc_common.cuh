@@ -74,21 +74,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // Bounded wait until a global counter that other CTAs raise reaches `target` (acquire at GPU
 // scope), then a proxy fence so that the bulk copies this thread issues next (async proxy) see
 // the memory those CTAs wrote before raising it.  False when the wait gives up or an abort is
-// raised.
+// raised.  The first `eager` polls follow each other without a pause.
 __device__ __forceinline__ bool wait_counter(const int *ctr, int target, volatile int *abort_word,
-                                             long long limit = WAIT_CYCLES)
+                                             long long limit = WAIT_CYCLES, int eager = 0)
 {
     const long long t0 = clock64();
-    for (;;) {
+    for (int polls = 0;; ++polls) {
         int v;
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(ctr) : "memory");
         if (v >= target) break;
         if (*abort_word) return false;
         if (clock64() - t0 > limit) return false;
-        __nanosleep(32);
+        if (polls >= eager) __nanosleep(32);
     }
     asm volatile("fence.proxy.async.global;\n" ::: "memory");
     return true;
+}
+
+// Whether such a counter has reached `target` (no wait, nothing ordered after it).
+__device__ __forceinline__ bool counter_reached(const int *ctr, int target)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(ctr) : "memory");
+    return v >= target;
 }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns()

@@ -1,0 +1,75 @@
+"""GPU: the FP64 dataflow launch at the edges of its column tiles (8, 16 and 32 wide variants), with
+sums cut along K, odd ranks and leaves, operands that are only 8-byte aligned, and a wait that
+runs out."""
+import numpy as np
+import pytest
+
+import oracle as O
+from matrox_ru_b200 import _lib, hgemm as H, structure as S
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # the FP64 parity bar of the other GPU tests
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch as t
+    assert t.cuda.is_available(), "GPU tests need a CUDA device"
+    from matrox_ru_b200 import build
+    build.build()
+    return t
+
+
+@pytest.fixture(scope="module")
+def tall():
+    """Leaves of several row tiles and near lists long enough to be cut along K."""
+    X = S.gaussian_mixture(1501, 3, 3, 0.0, 2.0, 0.3, None, seed=5)
+    return S.build_cds(X, S.KernelSpec("gaussian", 0.4), leaf_size=200, budget=0.9, tol=1e-7, max_rank=149)
+
+
+@pytest.mark.parametrize("r", [1, 8, 9, 16, 17, 32, 33, 100])
+@pytest.mark.parametrize("name", ["tall", "ragged"])
+def test_column_tile_edges(torch, small_cases, tall, name, r):
+    cds = tall if name == "tall" else small_cases[name]
+    rng = np.random.default_rng(r)
+    TW, Y0 = rng.standard_normal((2, cds.n * r))
+    plan = H.Plan(cds, "fp64")
+    room = torch.zeros(2 * cds.n * r + 3, dtype=torch.float64, device="cuda")
+    w, y = room[1:1 + cds.n * r], room[2 + cds.n * r:2 + 2 * cds.n * r]  # 8-byte aligned
+    w.copy_(torch.as_tensor(TW))
+    for call, want in ((plan.evaluate, O.eval_h2b(cds, TW, r)), (plan.adjoint, O.adjoint(cds, TW, r))):
+        for accumulate in (False, True):
+            y.copy_(torch.as_tensor(Y0))
+            call(w, r, out=y, accumulate=accumulate)
+            ref = want + Y0 if accumulate else want
+            assert np.abs(y.cpu().numpy() - ref).max() <= TOL * np.abs(ref).max()
+            assert room[0] == 0 and room[1 + cds.n * r] == 0 and room[-1] == 0  # nothing else written
+    plan.status()
+
+
+def test_changing_column_counts_on_one_plan(torch, tall):
+    """Buffers and counters grow and are reused across right-hand-side counts and directions."""
+    plan = H.Plan(tall, "fp64")
+    for r in (3, 70, 16, 1, 70):
+        TW = np.random.default_rng(r).standard_normal(tall.n * r)
+        w = torch.as_tensor(TW, device="cuda")
+        got, adj = plan.evaluate(w, r).cpu().numpy(), plan.adjoint(w, r).cpu().numpy()
+        want, wadj = O.eval_h2b(tall, TW, r), O.adjoint(tall, TW, r)
+        assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+        assert np.abs(adj - wadj).max() <= TOL * np.abs(wadj).max()
+
+
+def test_wait_that_runs_out_reports_timeout(torch, tall):
+    r = 16
+    TW = np.random.default_rng(0).standard_normal(tall.n * r)
+    w = torch.as_tensor(TW, device="cuda")
+    plan = H.Plan(tall, "fp64")
+    plan.set_test_hooks(0, wait_cycles=1)  # the first wait that is not already over gives up
+    plan.evaluate(w, r)
+    with pytest.raises(_lib.MxbError) as e:
+        plan.status()
+    assert e.value.code == _lib.MXB_ERR_TIMEOUT
+    plan.set_test_hooks(0)
+    want = O.eval_h2b(tall, TW, r)
+    assert np.abs(plan.evaluate(w, r).cpu().numpy() - want).max() <= TOL * np.abs(want).max()
+    plan.status()
