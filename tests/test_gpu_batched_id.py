@@ -107,3 +107,31 @@ def test_build_cds_with_gpu_id(torch, name):
     want = O.eval_h2b(gpu, gpu.to_tree_order(W), r)
     got = H.Plan(gpu, "fp64").evaluate(torch.as_tensor(gpu.to_tree_order(W), device="cuda").reshape(-1), r)
     assert np.abs(got.cpu().numpy() - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("count,nr,nc,max_rank", [
+    (3, 301, 150, 256),    # clusters of 8, odd rows (8-byte columns)
+    (20, 128, 64, 64),     # clusters of 4
+    (40, 90, 45, 20),      # clusters of 2
+    (160, 64, 32, 32),     # one block per node
+    (2, 40, 100, 64),      # more columns than rows
+    (2, 700, 600, 300),    # ranks above 256
+    (1, 1100, 560, 540),   # ranks above 512: one block per node, in place
+    (1, 5800, 40, 40),     # too tall for four panel vectors in shared memory
+])
+def test_batched_id_shapes(torch, count, nr, nc, max_rank):
+    """The edges of the cluster kernel's range and of the kernel it leaves the rest to."""
+    rng = np.random.default_rng(nr + nc)
+    X = S.gaussian_mixture(nr + 2 * nc, 5, 5, -2.0, 2.0, 0.3, 1.0, seed=nc)
+    mats = []
+    for _ in range(count):
+        idx = rng.choice(X.shape[0], nr + nc - 1, replace=False)
+        c = nc - len(mats) % 2  # uneven nodes: later ones start at odd offsets
+        mats.append(S.kernel_matrix(X, idx[:nr], idx[nr - 1:nr - 1 + c], S.KernelSpec("imq", 0.3)))
+    pool = torch.as_tensor(np.concatenate([m.reshape(-1, order="F") for m in mats]), device="cuda")
+    got = H.batched_id(pool, [m.shape for m in mats], 1e-9, max_rank)
+    for b in range(0, count, max(1, count // 4)):
+        hpiv, hP = S.interpolative_decomposition(np.asfortranarray(mats[b]), 1e-9, max_rank)
+        piv, P = got[b]
+        assert np.array_equal(piv, hpiv), b
+        assert float(np.abs(P - hP).max()) <= 1e-8 * max(1.0, float(np.abs(hP).max())), b
