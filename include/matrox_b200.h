@@ -274,7 +274,7 @@ MXB_API int32_t mxb_plan_set_permutation(mxb_plan *plan, const int32_t *perm);
 MXB_API int32_t mxb_plan_evaluate_ordered(mxb_plan *plan, const double *dW, int64_t w_rs, int64_t w_cs,
                                           double *dY, int64_t y_rs, int64_t y_cs, int32_t nrhs,
                                           int32_t accumulate, void *stream);
-/* dGW (+)= K~^T dG in the caller's point order (permuted copies; the plans mxb_plan_adjoint takes). */
+/* dGW (+)= K~^T dG in the caller's point order, likewise (the plans mxb_plan_adjoint takes). */
 MXB_API int32_t mxb_plan_adjoint_ordered(mxb_plan *plan, const double *dG, int64_t g_rs, int64_t g_cs,
                                          double *dGW, int64_t gw_rs, int64_t gw_cs, int32_t nrhs,
                                          int32_t accumulate, void *stream);
@@ -302,7 +302,8 @@ MXB_API int32_t mxb_plan_status(mxb_plan *plan);
 #define MXB_DEBUG_CHAIN_LEVELS 2
 #define MXB_DEBUG_STALL_LEVEL 4
 /* MXB_DEBUG_ONE_LAUNCH: the plan's evaluation runs as one launch, as a batch in
- * MXB_BATCH_ONE_LAUNCH mode does (with MXB_DEBUG_STALL_LEVEL, its level barriers run out). */
+ * MXB_BATCH_ONE_LAUNCH mode does (with MXB_DEBUG_STALL_LEVEL, its first pass never reports its
+ * blocks written, so the waits of the units that read them run out). */
 #define MXB_DEBUG_ONE_LAUNCH 8
 MXB_API int32_t mxb_plan_set_test_hooks(mxb_plan *plan, int32_t flags, int64_t wait_cycles);
 /* Copies the last evaluation's skeleton workspaces (wskel, uskel) to host arrays laid out
@@ -315,11 +316,13 @@ MXB_API int32_t mxb_plan_read_workspaces(mxb_plan *plan, int32_t nrhs, const int
 /* No counterpart in the reference (which evaluates one matrix per HGEMM call).  A batch merges
  * the launch sequences of several split-BF16 plans (same device; uneven N, ranks and nrhs and
  * any mix of split modes allowed -- couplings of different product counts run in separate
- * launches): one tensor-core launch per level serves every plan, the whole evaluation is
- * captured as one CUDA graph, and the column-tile width of every launch is picked by timing
- * the candidates (64 / 128 / 256 right-hand sides) on the first evaluation of an nrhs
- * signature (MXB_AUTOTUNE=0 disables the measurement); runs of up-sweep or down-sweep levels
- * are chained into one launch with device-side level barriers where that measures faster.
+ * launches).  Up to 128 right-hand sides the passes of all plans run in one launch after the W
+ * split, each work unit waiting on the device for the blocks it reads.  Above, one tensor-core
+ * launch per level serves every plan, and the first evaluation of an nrhs signature picks by
+ * timing (MXB_AUTOTUNE=0 disables the measurement) the column-tile width of every launch (64 /
+ * 128 / 256 right-hand sides), which runs of up-sweep or down-sweep levels are chained into one
+ * launch, and up to 512 columns whether all passes run in one.  The whole evaluation is captured
+ * as one CUDA graph.
  * The plans must outlive the batch; dW[i] / dY[i] are packed leaf-blocked device arrays of
  * plan i with nrhs[i] columns. */
 typedef struct mxb_batch mxb_batch;
@@ -335,15 +338,14 @@ MXB_API int32_t mxb_batch_status(mxb_batch *batch);
 MXB_API int32_t mxb_batch_info(const mxb_batch *batch, int32_t *launches, int32_t *widths, int32_t cap,
                                int32_t *nwidths);
 /* How a batch evaluation is launched (no counterpart in the reference).
- * MXB_BATCH_LEVEL_LAUNCHES (default): a W-split launch, then one tensor-core launch per level of
- *   the merged sequence, runs of up-sweep or down-sweep levels chained into one launch where
- *   the autotuner measures that faster.
+ * MXB_BATCH_LEVEL_LAUNCHES (default): a W-split launch, then the tensor-core launches described
+ *   above.
  * MXB_BATCH_ONE_LAUNCH: the whole evaluation -- the W split, up-sweep, couplings, near field,
- *   down-sweep and leaf down of every plan -- is ONE launch of the persistent kernel: every
- *   level is a group of work units that waits on the device (bounded) until the level before
- *   it is written.  One column-tile width (64 or 128, timed on the first evaluation) and
- *   3-part stages serve every level; units of bf16x3 couplings load 2 parts and issue 3
- *   products.  W and Y leaf-blocked (MXB_ERR_UNSUPPORTED in the caller's point order).
+ *   down-sweep and leaf down of every plan -- is ONE launch of the persistent kernel at every
+ *   column count: each work unit waits on the device (bounded) until the blocks it reads are
+ *   written.  One column-tile width (64 up to 64 right-hand sides, else 128) and 3-part stages
+ *   serve every pass; units of bf16x3 couplings load 2 parts and issue 3 products.  W and Y
+ *   leaf-blocked (MXB_ERR_UNSUPPORTED in the caller's point order).
  * Changing the mode drops the batch's captured evaluations. */
 #define MXB_BATCH_LEVEL_LAUNCHES 0
 #define MXB_BATCH_ONE_LAUNCH 1
@@ -354,7 +356,7 @@ MXB_API int32_t mxb_batch_destroy(mxb_batch *batch);
  * call with omp_get_wtime in matroxTest-V1/main.cpp:94-108) ----
  * Evaluates Y = K~W (overwriting Y) once through the ordinary path, then twice launch by launch
  * outside any graph, bracketing every launch with CUDA events on `stream`, and reports the
- * second pass.  The launches are the ones the evaluation graph holds, in order, so Y on return
+ * second pass.  The launches are the ones an evaluation makes, in order, so Y on return
  * is the ordinary result.  The call synchronises `stream`. */
 #define MXB_PHASE_SPLIT_W 0        /* W -> bf16 operand tiles (split-BF16 plans) */
 #define MXB_PHASE_UP 1             /* leaf projection (level 0) or transfer at height `level` */

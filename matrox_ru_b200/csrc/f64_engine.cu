@@ -795,8 +795,8 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     auto w_src = [&](const F64Block &a, int pool, int trans, int leaf) {
         return Src{a, pool, trans, BUF_W, c_w + leaf, WR * row_tiles(p.Ddim[leaf]), g_w[leaf], E.leaf8[leaf]};
     };
-    auto up_src = [&](const F64Block &a, int pool, int trans, int v) {
-        return Src{a, pool, trans, BUF_WSKEL, c_up + v, WR * row_tiles(p.slen[v]), g_up[v], E.node8[v]};
+    auto up_src = [&](const F64Block &a, int pool, int trans, int v) {  // (nothing writes the root's block)
+        return Src{a, pool, trans, BUF_WSKEL, g_up[v] < 0 ? -1 : c_up + v, WR * row_tiles(p.slen[v]), g_up[v], E.node8[v]};
     };
     auto u_src = [&](const F64Block &a, int pool, int trans, int v) {
         return Src{a, pool, trans, BUF_USKEL, c_u + v, WR * row_tiles(p.slen[v]), g_u[v], E.node8[v]};

@@ -14,17 +14,29 @@
 // pipeline stage is filled by a few 1-D bulk copies (cp.async.bulk) on an mbarrier -- no
 // tensor maps, no per-element address math in the main loop.  The CDS operands (D, B, the
 // projections and their transposes) are tiled once when the plan is created; W is tiled per
-// evaluation by a split kernel, and the skeleton vectors are written as tiles directly by the
-// GEMM epilogue.
+// evaluation by a split kernel or by units of the GEMM kernel, and the skeleton vectors are
+// written as tiles directly by the GEMM epilogue.
 //
-// GEMM kernel (persistent, one CTA per SM, 10 warps), walking a list of work units
-// (task row tile x BN right-hand sides; BN = 64, 128 or 256, picked by the autotuner):
-//   warp 8 lane 0 : producer -- bulk copies of the A and B part tiles of each K step
-//   warp 9 lane 0 : MMA issuer -- tcgen05.mma M=128, N=BN, K=16, 3 or 6 per 16-K slice, one
-//                   fresh TMEM accumulator (of two) per 64-deep K tile
-//   warps 0-7     : drain every K tile's accumulator into round-to-nearest FP32 registers
-//                   (tcgen05.ld), then write Y (FP64), an FP32 block, or operand tiles
+// GEMM kernel (persistent, one CTA per SM), walking a list of work units (task row tile x BN
+// right-hand sides; BN = 64, 128 or 256).  E = 16 epilogue warps where BN <= 128 on single
+// CTAs, else 8:
+//   warps 0 - E-1  : drain every K tile's accumulator into round-to-nearest FP32 registers
+//                    (tcgen05.ld), then write Y (FP64), an FP32 block, or operand tiles
+//   warp E lane 0  : producer -- bulk copies of the A and B part tiles of each K step
+//   warp E+1 lane 0: MMA issuer -- tcgen05.mma M=128, N=BN, K=16, 3 or 6 per 16-K slice, one
+//                    fresh TMEM accumulator (of two or four) per 64-deep K tile
+//   warp E+2       : (single CTAs) publisher -- one device-scope fence and one counter
+//                    increment per unit once all its epilogue warps have written, so no
+//                    epilogue warp waits out a fence (about 1 us each in an up or down pass)
 // A task carries the index of its plan, so one launch can serve many H-matrices (batches).
+//
+// Launches: up to 128 columns, and where one SM's share of the products is not far above the
+// longest path through the tree (Batch::takes_flow), every pass of an evaluation runs in ONE
+// launch (the flow launch, Batch::flow_units), each unit waiting for the node blocks it reads.
+// Such evaluations were bound by the chain of launches, not by their products: with one launch
+// per pass or a barrier in between, N = 2048 x 32 took 104 us and N = 30011 x 130 645 us,
+// against 52 and 475 us.  Others time the launches per pass, chained passes and (near the line)
+// the flow launch against each other.
 // Every wait is bounded; a CTA that times out raises MXB_ERR_TIMEOUT in the error word,
 // drains its own copies and MMAs, frees its TMEM and exits.
 #include <algorithm>
@@ -67,11 +79,13 @@ enum BBuf { BUF_W, BUF_WSKEL, BUF_USKEL, NBUF };
 
 struct TcItem {
     uint64_t a_off;   // byte offset of A's tile (0, 0) in the plan's A pool `a_pool`
-    int64_t b_base;   // K-tile base of the B operand's node / leaf in the B buffer `b_buf`
+    int32_t b_base;   // K-tile base of the B operand's node / leaf in the B buffer `b_buf`
     int32_t KT;       // K tiles of this item
     int32_t K;        // K before padding to whole tiles (flop accounting)
-    int16_t a_pool;   // APool of A
-    int16_t b_buf;    // BBuf of B
+    int32_t dep;      // flow launches: the plan's counter of B's writer (FlowCounter; -1: none)
+    int16_t need;     // ... and its row tiles
+    int8_t a_pool;    // APool of A
+    int8_t b_buf;     // BBuf of B
     int32_t pad;
 };
 static_assert(sizeof(TcItem) == 32, "TcItem layout");
@@ -86,7 +100,7 @@ enum OutKind : int16_t {
 };
 
 struct TcTask {
-    int64_t c_row;   // leaf index (OUT_Y) or skeleton row offset (FP32 block)
+    int64_t c_row;   // leaf index (OUT_Y) or first 128-row tile of the node in the FP32 far results
     int64_t out_kt;  // K-tile base of the node in the tile buffer (OUT_TILES)
     int32_t ldc;
     int32_t M;       // rows of the whole output block
@@ -97,6 +111,22 @@ struct TcTask {
     int16_t out_kind;
     int16_t beta;    // 0 overwrite, 1 accumulate (OUT_TILES: add the FP32 block), 2 plan's arg
     int32_t t_buf;   // BBuf that OUT_TILES writes
+    // flow launches: the plan's counter raised once the tile is written, and the one to reach
+    // before the old output (Y, the far result) is read back (-1: none), with its row tiles
+    int32_t sig, old, old_need, pad;
+};
+static_assert(sizeof(TcTask) == 64, "TcTask layout");
+
+// Counters of one plan in a flow launch (times its column tiles, + column tile): per leaf W split
+// and near field written; per node wskel, far result and uskel written.
+struct FlowCounter {
+    int nleaf, numnodes;
+    int w(int leaf) const { return leaf; }
+    int near(int leaf) const { return nleaf + leaf; }
+    int up(int v) const { return 2 * nleaf + v; }
+    int far(int v) const { return 2 * nleaf + numnodes + v; }
+    int u(int v) const { return 2 * nleaf + 2 * numnodes + v; }
+    int count() const { return 2 * nleaf + 3 * numnodes; }
 };
 
 struct TcUnit {
@@ -134,7 +164,8 @@ struct PlanArgs {
     double *Y;
     const int32_t *wofs;
     const int32_t *yofs;
-    float *skel;         // FP32 far results awaiting the down launch
+    float *skel;         // FP32 far results awaiting the down launch: float4 of 4 columns at
+                         // (row tile * nq + column / 4) * 128 + row, so a warp moves 512 bytes at a time
     // caller point order (null: leaf-blocked W / Y at wofs / yofs): tree position t of leaf
     // i (t from tofs[i]) is row perm[t]; element (row, j) of W at row * w_rs + j * w_cs
     const int32_t *w_perm;
@@ -144,15 +175,20 @@ struct PlanArgs {
     int32_t NT;          // 128-column tiles per node in the B buffers (even)
     int32_t nrhs;
     int32_t beta_arg;
-    int32_t pad;
+    int32_t ctr0, ncol;  // flow launches: the plan's first counter, its column tiles
+    int32_t nq;          // column quads of a row tile of the FP32 far results
 };
+static_assert(sizeof(PlanArgs) % 8 == 0, "copied in 8-byte words");
 
 // Tree levels one tensor-core launch may chain (consecutive ops of one product count and tile,
 // e.g. the up-sweep heights): the units of level j wait on the device until every unit of
 // level j - 1 has been written.
 constexpr int MAX_CHAIN = 24;
-// Tile-code flag (above MXB_TILE_PAIR): the op runs in the launch of the op before it.
-constexpr int TILE_CHAIN = 1 << 13;
+// Tile-code flags (above MXB_TILE_PAIR): the op runs in the launch of the op before it; every op
+// runs in one flow launch.
+constexpr int TILE_CHAIN = 1 << 13, TILE_FLOW = 1 << 14;
+// Control words of a flow launch before its counters: claimed units, blocks that have left.
+constexpr int FLOW_CLAIM = 0, FLOW_EXIT = 1, FLOW_FIRST = 16;
 
 struct LaunchArgs {
     const PlanArgs *plans;
@@ -163,17 +199,24 @@ struct LaunchArgs {
     int *err;
     long long wait_cycles;  // limit of every wait in the kernel
     int nunits;
+    int nplans;
     int stall_test;         // test hook: CTA 0 withholds its first stage, so a wait runs out
     int kchain;             // K tiles accumulated per TMEM accumulator fill (1 or 2)
-    int nlevels;            // chained levels (1: none); a unit's level is in TcUnit::chain
+    int nlevels;            // levels chained by barriers (1: none); a unit's level is in TcUnit::chain
     int *level_done;        // per level: epilogue warps done with a unit of it (zero at launch)
     int stall_level;        // test hook: level 0 never reports done, so level 1's waits run out
-    // profiling of chained launches (null otherwise): [0] the earliest CTA start, [1 + j] the
-    // time the last unit of level j was written (%globaltimer, ns)
+    // profiling of a one-launch evaluation (null otherwise): [0] the earliest CTA start, [1 + j]
+    // the time the last unit of op j was written (%globaltimer, ns)
     unsigned long long *level_ns;
     // dataflow launches (null otherwise): per-node completion counters, zero at launch; units
     // wait for the nodes whose tiles they read instead of for whole levels (TcUnit::dep0/dep1)
     int *deps;
+    // flow launches (null otherwise): control words and counters, zero at launch and left zero by
+    // the last block; items and tasks name the counters they wait for and raise
+    int *flow;
+    int nflow;              // ints to clear
+    int skip_w;             // W was split by a launch before: nothing waits for it
+    PlanArgs plan0;         // the plan of a single-plan flow launch (plans is null then)
 };
 
 // ---------------------------------------------------------------------------------------
@@ -223,14 +266,17 @@ __global__ void __launch_bounds__(256) tile_pool_kernel(const PoolJob *__restric
 // B(n, k) = W[k + n ld]; rows n >= nrhs and k >= K are zero.  ORD: the evaluation reads W in
 // the caller's point order (PlanArgs::w_perm), a separate instantiation so the leaf-blocked
 // one keeps its small footprint.
+// Columns are filled up to whole groups of 16, which is all the launches read (splitting whole
+// 128-column tiles cost 11 us of the 104 at N = 2048 x 32).  plans null: the plan plan0.
 template <bool ORD>
-__global__ void __launch_bounds__(256) split_w_kernel(const SplitJob *__restrict__ jobs,
-                                                      const PlanArgs *__restrict__ plans)
+__global__ void __launch_bounds__(256) split_w_kernel(const SplitJob *__restrict__ jobs, const PlanArgs *__restrict__ plans,
+                                                      const __grid_constant__ PlanArgs plan0)
 {
     const SplitJob j = jobs[blockIdx.x];
-    const PlanArgs *pa = plans + j.plan;
+    const PlanArgs *pa = plans ? plans + j.plan : &plan0;
     const int kt = blockIdx.y, nt = blockIdx.z;
-    if (kt >= j.KT || nt >= pa->NT) return;
+    const int fill = ((pa->nrhs + 15) & ~15) - nt * 128;  // tile rows (columns of W) to fill
+    if (kt >= j.KT || fill <= 0) return;
     const int nrhs = pa->nrhs;
     uint8_t *tile0 = pa->buf[BUF_W] + ((size_t)j.dst_kt * pa->NT + (size_t)nt * j.KT + kt) * 3 * (size_t)TILE_BYTES;
     if (ORD && pa->w_perm) {
@@ -257,6 +303,7 @@ __global__ void __launch_bounds__(256) split_w_kernel(const SplitJob *__restrict
             __syncthreads();
             for (int q = threadIdx.x; q < 128 * 4; q += 256) {
                 const int c = q & 3, rr = q >> 2;
+                if (rr >= fill) break;
                 __nv_bfloat16 hi[8], mi[8], lo[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) tc::split3(stage[c * 8 + e][rr], hi[e], mi[e], lo[e]);
@@ -271,6 +318,7 @@ __global__ void __launch_bounds__(256) split_w_kernel(const SplitJob *__restrict
         const int idx = threadIdx.x + i * 256;
         const int c = idx % 8, r = idx / 8;
         const int n = nt * 128 + r;
+        if (r >= fill) break;
         __nv_bfloat16 h[8], m[8], l[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -306,6 +354,31 @@ __device__ __forceinline__ void transpose8(float (&x)[8], int lane)
     }
 }
 
+// Beside the stages: the unit and task records of the units in the ring (single CTAs; read from
+// there by the epilogue warps, whose global loads of them cost about 1 us per unit) and the first
+// plans' pointers.
+constexpr int RING_SLOTS = 16, SMEM_PLANS = 16;
+struct alignas(16) UnitRecord {
+    TcUnit unit;
+    TcTask task;
+};
+constexpr int RING_BYTES = RING_SLOTS * (int)sizeof(UnitRecord) + SMEM_PLANS * (int)sizeof(PlanArgs);
+
+// Columns of column tile `col` that hold right-hand sides, in whole 16-column groups (the smallest
+// MMA width): what lies past them is neither loaded, multiplied nor written.  A launch on CTA
+// pairs works on whole tiles.
+__host__ __device__ constexpr int tile_columns(int nrhs, int col, int bn)
+{
+    const int n = (nrhs - col * bn + 15) & ~15;
+    return n < bn ? n : bn;
+}
+
+__device__ __forceinline__ void add_or_store(double *y, double v, int beta)
+{
+    if (beta) asm volatile("red.global.add.f64 [%0], %1;\n" ::"l"(y), "d"(v) : "memory");
+    else *y = v;
+}
+
 // Launch shape.  PAIR: a cluster of two CTAs (one per SM) computes a 256-row x BN tile with
 // tcgen05.mma.cta_group::2; each CTA stages its own 128 rows of A and half of the BN rows of
 // B, so a pair moves a third less operand data per flop than two single CTAs and has room for
@@ -318,20 +391,17 @@ struct TcCfg {
     static constexpr int A_BYTES = P * TILE_BYTES;
     static constexpr int B_BYTES = P * B_ROWS_BYTES;
     static constexpr int STAGE = A_BYTES + B_BYTES;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 1024;  // + alignment, barriers, unit ring
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 1024 + RING_BYTES;  // + alignment, barriers, unit ring
     static constexpr int NPROD = P == 2 ? 3 : 6;
-    static constexpr int EPI_WARPS = 8;          // two per TMEM lane quarter, one per column half
-    static constexpr int RING = 16;              // work units published ahead of the readers
+    static constexpr int EPI_WARPS = (BN <= 128 && !PAIR) ? 16 : 8;  // 4 or 2 per TMEM lane quarter
+    static constexpr int RING = RING_SLOTS;      // work units published ahead of the readers
     // readers of a ring slot: MMA issuer and epilogue warps (+ the odd CTA's producer, relay
     // and epilogue warps in a pair)
-    static constexpr int RING_READERS = PAIR ? 2 * (1 + EPI_WARPS) + 1 : 1 + EPI_WARPS;
-    static constexpr int THREADS = (EPI_WARPS + 2) * 32;
+    static constexpr int RING_READERS = PAIR ? 2 * (1 + EPI_WARPS) + 1 : 2 + EPI_WARPS;
+    static constexpr int THREADS = (EPI_WARPS + (PAIR ? 2 : 3)) * 32;  // single CTAs: + the publishing warp
     // level-count increments per unit: one per epilogue warp (of both CTAs of a pair)
     static constexpr int UNIT_WRITERS = EPI_WARPS * (PAIR ? 2 : 1);
-    static constexpr int COLS = BN / 2;          // accumulator columns per epilogue thread
-    // old values loaded ahead of the stores in the epilogue's read-modify-writes (fewer where
-    // 128 accumulators already fill the registers)
-    static constexpr int RMW = COLS >= 128 ? 8 : 16;
+    static constexpr int COLS = BN * 4 / EPI_WARPS;  // accumulator columns per epilogue thread
     static constexpr int NACC = BN >= 256 ? 2 : 4;  // TMEM accumulator buffers (512 columns at most)
     static constexpr int TMEM_COLS = NACC * BN;
     static constexpr int M_MMA = PAIR ? 256 : 128;
@@ -358,9 +428,10 @@ struct TcCfg {
 // barrier, and the even CTA's commits arrive on both CTAs' barriers.  A failed wait in either
 // CTA sets both CTAs' abort words.
 template <int P, int BN, int STAGES_, bool PAIR, bool ORD>
-__global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_gemm_kernel(LaunchArgs la)
+__global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_gemm_kernel(const __grid_constant__ LaunchArgs la)
 {
     using C = TcCfg<P, BN, STAGES_, PAIR>;
+    constexpr bool FLOW = P == 3 && !PAIR && BN <= 128;  // flow and one-launch evaluations run on these
     constexpr int NB = C::STAGES;  // full / empty / pair barriers: one per stage
     constexpr int RING = C::RING;
     extern __shared__ uint8_t smem_raw[];
@@ -373,10 +444,14 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
     uint64_t *doneb = acce + C::NACC;     // every MMA of this CTA (pair) has completed
     uint64_t *ufull = doneb + 1;          // ring slot i holds a unit
     uint64_t *uempty = ufull + RING;      // every reader of ring slot i has taken its unit
-    volatile int *ring = reinterpret_cast<volatile int *>(uempty + RING);
+    uint64_t *written = uempty + RING;    // the epilogue warps have written the unit in ring slot i
+    volatile int *ring = reinterpret_cast<volatile int *>(written + RING);
     volatile int *ring_kt = ring + RING;  // K tiles of the unit in ring slot i
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(const_cast<int *>(ring_kt) + RING);
     volatile int *abort_word = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    UnitRecord *records = reinterpret_cast<UnitRecord *>(smem + C::STAGES * C::STAGE + 1024);
+    PlanArgs *splans = reinterpret_cast<PlanArgs *>(records + RING);
+    auto plan_args = [&](int p) -> const PlanArgs * { return p < SMEM_PLANS ? splans + p : la.plans + p; };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? tc::cluster_ctarank() : 0u;
@@ -394,10 +469,10 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(bar)) : "memory");
     };
     // Next unit of the ring for a reader (one thread): waits for slot `slot`, takes the unit,
-    // its K-tile count and its operand parts (published as ktiles | parts << 24, so the MMA
-    // issuer needs no global load per unit), and releases the slot to the producer (in the
+    // its K-tile count, operand parts and columns (published as ktiles | parts << 24 | columns / 16
+    // << 26, so the MMA issuer needs no global load per unit), and releases the slot to the producer (in the
     // even CTA of a pair).  -2: a wait gave up.
-    auto take_unit = [&](uint32_t &slot, int &ktiles, int *parts = nullptr) -> int {
+    auto take_unit = [&](uint32_t &slot, int &ktiles, int *parts = nullptr, int *columns = nullptr) -> int {
         const int i = (int)(slot % RING);
         const uint32_t parity = (slot / RING) & 1u;
         ++slot;
@@ -406,7 +481,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             u = ring[i];
             const int v = ring_kt[i];
             ktiles = v & 0xFFFFFF;
-            if (parts) *parts = v >> 24;
+            if (parts) *parts = (v >> 24) & 3;
+            if (columns) *columns = (v >> 26) * 16;
         }
         if constexpr (PAIR) {
             if (rank == 1) tc::mbar_arrive_remote(tc::peer_smem(&uempty[i], 0));
@@ -436,11 +512,14 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
         for (int i = 0; i < RING; ++i) {
             tc::mbar_init(&ufull[i], 1);
             tc::mbar_init(&uempty[i], C::RING_READERS);
+            tc::mbar_init(&written[i], C::EPI_WARPS);
         }
         *abort_word = 0;
 
         tc::fence_mbar_init();
     }
+    for (int i = threadIdx.x; i < min(la.nplans, SMEM_PLANS) * (int)(sizeof(PlanArgs) / 8); i += C::THREADS)
+        reinterpret_cast<uint64_t *>(splans)[i] = reinterpret_cast<const uint64_t *>(la.plans ? la.plans : &la.plan0)[i];
     if (warp == 0) {
         if constexpr (PAIR) tc::tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
         else tc::tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -470,7 +549,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             int nu = -1;
             TcUnit nun{};
             TcTask ntk{};
-            int nstate = 0;  // 0: nothing claimed, 1: claimed, 2: unit record loaded, 3: task loaded
+            TcItem nit{};
+            int nstate = 0;  // 0: nothing claimed, 1: claimed, 2: unit record loaded, 3: task, 4: first item
             auto advance = [&]() {
                 if (nstate == 0) {
                     nu = atomicAdd(la.next_unit, 1);
@@ -479,6 +559,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     if (nu >= 0) nun = la.units[nu];
                 } else if (nstate == 2) {
                     if (nu >= 0) ntk = la.tasks[nun.task];
+                } else if (nstate == 3) {
+                    if (nu >= 0 && ntk.nitem > 0) nit = la.items[ntk.item0];
                 }
                 ++nstate;
             };
@@ -486,17 +568,21 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 int u, kt_unit = 0;
                 TcUnit un{};
                 TcTask t{};
+                TcItem it_next{};
+                int left = 0;  // K tiles of the unit still to load
                 if (!PAIR || issuer) {
                     // take the claimed unit and publish it to every reader
-                    while (nstate < 3) advance();
+                    while (nstate < 4) advance();
                     u = nu;
                     un = nun;
                     t = ntk;
+                    it_next = nit;
                     nstate = 0;
                     int kt_pub = 0;
                     if (u >= 0) {
                         kt_unit = un.ktiles;
-                        kt_pub = un.ktiles | (unit_parts(un.chain) << 24);
+                        const int n = PAIR ? BN : tile_columns(plan_args(t.plan)->nrhs, un.col, BN);
+                        kt_pub = un.ktiles | (unit_parts(un.chain) << 24) | ((n / 16) << 26);
                     }
                     const int i = (int)(slot % RING);
                     const uint32_t round = slot / RING;
@@ -507,6 +593,12 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     }
                     ring[i] = u;
                     ring_kt[i] = kt_pub;
+                    if constexpr (!PAIR) {
+                        if (u >= 0) {
+                            records[i].unit = un;
+                            records[i].task = t;
+                        }
+                    }
                     if constexpr (PAIR) {
                         tc::st_remote_u32(tc::peer_smem((const void *)&ring[i], 1), (uint32_t)u);
                         tc::st_remote_u32(tc::peer_smem((const void *)&ring_kt[i], 1), (uint32_t)kt_pub);
@@ -522,6 +614,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     if (u >= 0) {
                         un = la.units[u];
                         t = la.tasks[un.task];
+                        if (t.nitem > 0) it_next = la.items[t.item0];
                     }
                 }
                 if (u < 0) break;
@@ -551,23 +644,32 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                         break;
                     }
                 }
-                const PlanArgs *pa = la.plans + t.plan;
+                const PlanArgs *pa = plan_args(t.plan);
                 const int NT = pa->NT;
                 const int cb = un.col * BN + (int)rank * C::B_ROWS;  // first B row staged here
                 const TcItem *ti = la.items + t.item0;
+                left = un.ktiles;
                 const int mt = t.m0 / 128 + (int)rank;
                 // the odd CTA's rows may lie past the block: its A tile does not exist, and the
                 // MMA rows it feeds are never stored
                 const bool a_ok = !PAIR || issuer || t.m0 + 128 < t.M;
                 const int up = unit_parts(un.chain);
-                const uint32_t tx = (a_ok ? (uint32_t)up * TILE_BYTES : 0u) + (uint32_t)up * C::B_ROWS_BYTES;
-                TcItem it_next{};
-                if (t.nitem > 0) it_next = ti[0];
+                const int b_rows = PAIR ? C::B_ROWS : tile_columns(pa->nrhs, un.col, BN);  // B rows to load
+                const uint32_t tx = (a_ok ? (uint32_t)up * TILE_BYTES : 0u) + (uint32_t)up * (uint32_t)b_rows * 128;
                 for (int q = 0; q < t.nitem && !stop; ++q) {
                     const TcItem it = it_next;
                     if (q + 1 < t.nitem) it_next = ti[q + 1];  // loaded while this item's copies go out
                     const uint8_t *a_pool = pa->pool[it.a_pool];
                     const uint8_t *b_pool = pa->buf[it.b_buf];
+                    if (FLOW && la.flow && it.dep >= 0 && !(la.skip_w && it.b_buf == BUF_W)) {
+                        // the writer of this item's B tiles has finished its row tiles of this column tile
+                        if (!tc::wait_counter(la.flow + FLOW_FIRST + pa->ctr0 + it.dep * pa->ncol + un.col,
+                                              it.need * C::UNIT_WRITERS, abort_word, la.wait_cycles, 64)) {
+                            raise_abort();
+                            stop = true;
+                            break;
+                        }
+                    }
                     for (int kt = 0; kt < it.KT; ++kt, ++g) {
                         const int s = g % C::STAGES;
                         const uint32_t round = g / C::STAGES;
@@ -587,6 +689,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                         if (C::B_ROWS >= 128) {
 #pragma unroll
                             for (int hh = 0; hh < C::B_ROWS / 128; ++hh) {
+                                const int rows = min(128, b_rows - hh * 128);
+                                if (rows <= 0) break;
                                 const size_t nt = (size_t)(cb >> 7) + hh;
                                 const uint8_t *gb =
                                     b_pool + ((size_t)it.b_base * NT + nt * it.KT + kt) * 3 * (size_t)TILE_BYTES;
@@ -594,7 +698,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                                 for (int p = 0; p < P; ++p)
                                     if (p < up)
                                         tc::bulk_g2s(sb + p * C::B_ROWS_BYTES + hh * TILE_BYTES,
-                                                     gb + (size_t)p * TILE_BYTES, TILE_BYTES, &full[s]);
+                                                     gb + (size_t)p * TILE_BYTES, (uint32_t)rows * 128, &full[s]);
                             }
                         } else {
                             // B_ROWS rows starting at row cb % 128 of a 128-row tile: contiguous, and
@@ -606,11 +710,13 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
 #pragma unroll
                             for (int p = 0; p < P; ++p)
                                 if (p < up)
-                                    tc::bulk_g2s(sb + p * C::B_ROWS_BYTES, gb + (size_t)p * TILE_BYTES, C::B_ROWS_BYTES,
-                                                 &full[s]);
+                                    tc::bulk_g2s(sb + p * C::B_ROWS_BYTES, gb + (size_t)p * TILE_BYTES,
+                                                 (uint32_t)b_rows * 128, &full[s]);
                         }
                         filled[s] = round + 1;
-                        if ((!PAIR || issuer) && nstate < 3) advance();
+                        // (flow launches claim late: a unit held behind another keeps its readers waiting)
+                        --left;
+                        if ((!PAIR || issuer) && nstate < 4 && (!FLOW || !la.flow || left < 4)) advance();
                     }
                 }
             }
@@ -633,8 +739,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             uint32_t slot = 0;  // ring counter
             bool any = false, stop = false;
             while (!stop) {
-                int ktiles = 0, up = P;
-                const int u = take_unit(slot, ktiles, &up);
+                int ktiles = 0, up = P, columns = BN;
+                const int u = take_unit(slot, ktiles, &up, &columns);
                 if (u < 0) {
                     if (u == -2) raise_abort();
                     break;
@@ -663,7 +769,8 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     const uint32_t dst = tmem + (uint32_t)(b * BN);
                     // the products of one K tile, fully unrolled for each product count (no
                     // run-time loop bound between the MMAs)
-                    auto issue = [&](auto np) {
+                    auto issue = [&](auto np, auto whole) {
+                        const uint32_t idesc = decltype(whole)::value ? IDESC : tc::idesc_bf16_f32(C::M_MMA, columns);
                         uint32_t accum = first ? 0u : 1u;
 #pragma unroll
                         for (int ks = 0; ks < 4; ++ks) {
@@ -671,14 +778,19 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                             for (int j = 0; j < decltype(np)::value; ++j) {
                                 const uint64_t ad = da + (uint64_t)((PA[j] * TILE_BYTES + ks * 32) >> 4);
                                 const uint64_t bd = db + (uint64_t)((PB[j] * C::B_ROWS_BYTES + ks * 32) >> 4);
-                                if constexpr (PAIR) tc::mma_bf16_pair(dst, ad, bd, IDESC, accum);
-                                else tc::mma_bf16(dst, ad, bd, IDESC, accum);
+                                if constexpr (PAIR) tc::mma_bf16_pair(dst, ad, bd, idesc, accum);
+                                else tc::mma_bf16(dst, ad, bd, idesc, accum);
                                 accum = 1;
                             }
                         }
                     };
-                    if (C::NPROD == 3 || nprod == 3) issue(std::integral_constant<int, 3>{});
-                    else issue(std::integral_constant<int, 6>{});
+                    if (columns == BN) {
+                        if (C::NPROD == 3 || nprod == 3) issue(std::integral_constant<int, 3>{}, std::true_type{});
+                        else issue(std::integral_constant<int, 6>{}, std::true_type{});
+                    } else {
+                        if (C::NPROD == 3 || nprod == 3) issue(std::integral_constant<int, 3>{}, std::false_type{});
+                        else issue(std::integral_constant<int, 6>{}, std::false_type{});
+                    }
                     if constexpr (PAIR) {
                         tc::mma_commit_pair(&empty[s]);
                         if (last) tc::mma_commit_pair(&accf[b]);
@@ -720,6 +832,40 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 }
             }
         }
+    } else if (!PAIR && warp == C::EPI_WARPS + 2) {
+        // ---------------- publisher (single CTAs) ----------------
+        // Counts written units for the units that read them.  The gpu-scope fence, which waits for
+        // the stores of a whole tile, is taken here instead of by the epilogue warps, which go on
+        // with the next unit (the stores reach this thread by the `written` barrier, and the fence
+        // covers what it has seen).
+        if (lane == 0) {
+            for (uint32_t slot = 0;; ++slot) {
+                const int i = (int)(slot % RING);
+                if (!tc::mbar_wait(&ufull[i], (slot / RING) & 1u, abort_word, la.wait_cycles)) {
+                    raise_abort();
+                    break;
+                }
+                if (ring[i] < 0) break;
+                const TcUnit &un = records[i].unit;
+                int *ctr = nullptr;
+                if (la.deps && un.sig >= 0 && !(la.stall_level && un.dep0 < 0)) ctr = la.deps + un.sig;  // (test hook: stall)
+                if (FLOW && la.flow && records[i].task.sig >= 0) {
+                    const PlanArgs *pa = plan_args(records[i].task.plan);
+                    ctr = la.flow + FLOW_FIRST + pa->ctr0 + records[i].task.sig * pa->ncol + un.col;
+                    if (la.stall_level && records[i].task.out_kind == OUT_SPLIT) ctr = nullptr;  // (test hook)
+                }
+                if (ctr || la.level_ns) {
+                    if (!tc::mbar_wait(&written[i], (slot / RING) & 1u, abort_word, la.wait_cycles)) {
+                        raise_abort();
+                        break;
+                    }
+                    asm volatile("fence.acq_rel.gpu;\n" ::: "memory");
+                    if (ctr) atomicAdd(ctr, C::UNIT_WRITERS);
+                    if (la.level_ns) atomicMax(la.level_ns + 1 + ((un.chain >> 20) & 0xFF), tc::globaltimer_ns());
+                }
+                arrive_local(&uempty[i]);
+            }
+        }
     } else {
         // ---------------- epilogue warps ----------------
         const int quarter = warp & 3, half = warp >> 2;
@@ -731,6 +877,10 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
         // are counted (after one fence for all their stores) when the warp takes its first unit
         // of a later level, or at the end: one fence and one atomic per level and warp.
         int pend_level = 0, pend = 0;
+        // the FP32 far result of row r (of a 4-column group starting at col)
+        auto skel_at = [&](const PlanArgs *pa, const TcTask &t, int r, int col) {
+            return pa->skel + (((size_t)t.c_row + (r >> 7)) * pa->nq + (col >> 2)) * 512 + (r & 127) * 4;
+        };
         auto flush = [&]() {
             if (!pend) return;
             asm volatile("fence.proxy.async.global;\n" ::: "memory");
@@ -743,21 +893,37 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             pend = 0;
         };
         for (;;) {
-            int u = 0, ktiles = 0;
-            if (lane == 0) u = take_unit(slot, ktiles);
-            u = __shfl_sync(0xffffffffu, u, 0);
-            ktiles = __shfl_sync(0xffffffffu, ktiles, 0);
+            int u = 0, ktiles = 0, columns = BN;
+            const int ri = (int)(slot % RING);
+            TcUnit unit_copy{};
+            TcTask task_copy{};
+            if constexpr (PAIR) {
+                if (lane == 0) u = take_unit(slot, ktiles);
+                u = __shfl_sync(0xffffffffu, u, 0);
+                ktiles = __shfl_sync(0xffffffffu, ktiles, 0);
+                if (u >= 0) {
+                    unit_copy = la.units[u];
+                    task_copy = la.tasks[unit_copy.task];
+                }
+            } else {  // the slot is released, with its records, at the end of the unit
+                const bool got = tc::mbar_wait(&ufull[ri], (slot / RING) & 1u, abort_word, la.wait_cycles);
+                ++slot;
+                u = __all_sync(0xffffffffu, got) ? ring[ri] : -2;
+                ktiles = ring_kt[ri] & 0xFFFFFF;
+                columns = (ring_kt[ri] >> 26) * 16;
+            }
+            columns -= half * C::COLS;  // of this warp's
+            const TcUnit &un = PAIR ? unit_copy : records[ri].unit;
+            const TcTask &t = PAIR ? task_copy : records[ri].task;
             if (u < 0) {
                 if (u == -2 && lane == 0) raise_abort();
                 if (u == -1) flush();
                 break;
             }
-            const TcUnit un = la.units[u];
             if (la.nlevels > 1 && ((un.chain >> 20) & 0xFF) != pend_level) {
                 flush();
                 pend_level = (un.chain >> 20) & 0xFF;
             }
-            const TcTask t = la.tasks[un.task];
             const int kc = unit_kchain(unit_parts(un.chain));
             const int fills = (ktiles + kc - 1) / kc;
             if (la.nlevels > 1 && ((un.chain >> 20) & 0xFF) > ewaited) {
@@ -783,12 +949,12 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 // flight per thread: ask L2 for them now, so the unit's MMAs cover the DRAM
                 // latency.  Lane j takes columns j, j + 32, ... of its warp's 32-row segment
                 // (128 bytes of FP32, 256 of FP64 per column).
-                const PlanArgs *pa = la.plans + t.plan;
+                const PlanArgs *pa = plan_args(t.plan);
                 const int r0 = t.m0 + (int)rank * 128 + quarter * 32;
                 const int c0 = un.col * BN + half * C::COLS;
                 const int beta = t.beta == 2 ? pa->beta_arg : t.beta;
                 const int nrhs = pa->nrhs;
-                const char *f32 = nullptr, *f64 = nullptr;
+                const char *f64 = nullptr;
                 if (ORD && t.out_kind == OUT_Y && beta && pa->y_perm) {
                     // caller point order: each lane asks for its own row's columns when they
                     // are contiguous (one 128-byte line per 16 columns)
@@ -801,19 +967,20 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     }
                 } else if (t.out_kind == OUT_Y && beta) {
                     f64 = reinterpret_cast<const char *>(pa->Y + pa->yofs[t.c_row] + r0);
-                } else if (t.out_kind == OUT_TILES && beta) {
-                    f32 = reinterpret_cast<const char *>(pa->skel + t.c_row * (int64_t)nrhs + r0);
+                } else if (t.out_kind == OUT_TILES && beta && r0 < t.M) {
+                    const char *q = reinterpret_cast<const char *>(skel_at(pa, t, r0, c0));
+                    for (int j = lane; j < C::COLS; j += 32)  // 4 lines per column quad
+                        if (c0 + (j & ~3) < pa->nq * 4)
+                            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + (size_t)(j >> 2) * 2048 + (j & 3) * 128));
                 }
-                if (r0 < t.M && (f32 || f64)) {
+                if (r0 < t.M && f64) {
                     for (int j = lane; j < C::COLS; j += 32) {
                         const int cc = c0 + j;
                         if (cc >= nrhs) break;
-                        if (f32) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(f32 + (size_t)cc * t.ldc * 4));
-                        if (f64) {  // rows r0 and r0 + 16 (only where they exist)
-                            const char *q = f64 + (size_t)cc * t.ldc * 8;
-                            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q));
-                            if (r0 + 16 < t.M) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + 128));
-                        }
+                        // rows r0 and r0 + 16 (only where they exist)
+                        const char *q = f64 + (size_t)cc * t.ldc * 8;
+                        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q));
+                        if (r0 + 16 < t.M) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + 128));
                     }
                 }
             }
@@ -832,7 +999,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 tc::fence_after_sync();
                 // 64 columns per load where the registers allow (one wait per 64 columns keeps
                 // the drain short); 128-column halves load 16 at a time to stay clear of spills
-                constexpr int LB = C::COLS == 64 ? 64 : (C::COLS >= 128 ? 16 : 32);
+                constexpr int LB = C::COLS == 64 ? 64 : (C::COLS == 32 ? 32 : 16);
 #pragma unroll
                 for (int c0 = 0; c0 < C::COLS; c0 += LB) {
                     float v[LB];
@@ -852,14 +1019,29 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 }
             }
             if (!ok || *abort_word) break;
-            const PlanArgs *pa = la.plans + t.plan;
+            const PlanArgs *pa = plan_args(t.plan);
             const int nrhs = pa->nrhs;
             const int r = t.m0 + (int)rank * 128 + quarter * 32 + lane;
             const int beta = t.beta == 2 ? pa->beta_arg : t.beta;
             const int col0 = un.col * BN + half * C::COLS;
-            // accumulating outputs: all old values of a 16-column chunk are loaded before any
-            // store, so the loads overlap instead of waiting on each other
-            if (ORD && t.out_kind == OUT_Y && pa->y_perm) {
+            if (FLOW && la.flow && t.old >= 0) {
+                // the old output comes from another unit of this launch: lane 0 waits, then every
+                // lane takes its own acquire of the completed count
+                const int *ctr = la.flow + FLOW_FIRST + pa->ctr0 + t.old * pa->ncol + un.col;
+                int done = 1;
+                if (lane == 0) done = tc::wait_counter(ctr, t.old_need * C::UNIT_WRITERS, abort_word, la.wait_cycles, 64);
+                done = __shfl_sync(0xffffffffu, done, 0);
+                if (!done) {
+                    if (lane == 0) raise_abort();
+                    break;
+                }
+                tc::acquire_counter(ctr);
+            }
+            // Y accumulates by reductions at L2 (each element has one writer, ordered after the old
+            // value's, so the sum is the same as load, add and store, without waiting for the load)
+            if (columns <= 0 && t.out_kind != OUT_SPLIT) {
+                // no right-hand sides in this warp's columns
+            } else if (ORD && t.out_kind == OUT_Y && pa->y_perm) {
                 // caller point order: row t of the leaf goes to row perm[t] of Y.  An 8 x 8
                 // transpose inside each group of 8 lanes gives every lane one column of 8
                 // consecutive tree rows, so each access covers 8 columns (64 bytes) of a row, 4
@@ -873,99 +1055,81 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     (lane & 7) < rows_ok ? (int64_t)pa->y_perm[pa->tofs[t.c_row] + rg + (lane & 7)] * pa->y_rs : 0;
                 const int64_t ycs = pa->y_cs;
                 double *ycol = pa->Y + (int64_t)(col0 + (lane & 7)) * ycs;  // advances 8 columns a group
-                // per batch: GB column groups x JB rows of old values in flight (fewer where 128
-                // accumulators already fill the registers)
-                constexpr int GB = C::COLS >= 128 ? 1 : 2;
-                constexpr int JB = C::COLS >= 128 ? 4 : 8;
 #pragma unroll
-                for (int g8 = 0; g8 < C::COLS / 8; g8 += GB) {
-                    float x[GB][8];
+                for (int g8 = 0; g8 < C::COLS / 8; ++g8) {
+                    float x[8];
 #pragma unroll
-                    for (int gb = 0; gb < GB; ++gb) {
+                    for (int j = 0; j < 8; ++j) x[j] = acc[8 * g8 + j];
+                    transpose8(x, lane);  // x[j]: row rg + j, column col0 + 8 g8 + (lane & 7)
+                    const bool col_ok = col0 + 8 * g8 + (lane & 7) < nrhs;
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) x[gb][j] = acc[8 * (g8 + gb) + j];
-                        transpose8(x[gb], lane);  // x[gb][j]: row rg + j, column col0 + 8 (g8 + gb) + (lane & 7)
+                    for (int j = 0; j < 8; ++j) {
+                        const int64_t ro = __shfl_sync(0xffffffffu, roff, (lane & ~7) | j);
+                        if (col_ok && j < rows_ok) add_or_store(ycol + ro, (double)x[j], beta);
                     }
-#pragma unroll
-                    for (int j0 = 0; j0 < 8; j0 += JB) {
-                        int64_t ro[JB];
-                        double old[GB][JB];
-#pragma unroll
-                        for (int j = 0; j < JB; ++j) ro[j] = __shfl_sync(0xffffffffu, roff, (lane & ~7) | (j0 + j));
-#pragma unroll
-                        for (int gb = 0; gb < GB; ++gb) {
-                            const bool col_ok = col0 + 8 * (g8 + gb) + (lane & 7) < nrhs;
-#pragma unroll
-                            for (int j = 0; j < JB; ++j)
-                                old[gb][j] = (beta && col_ok && j0 + j < rows_ok) ? ycol[ro[j] + 8 * gb * ycs] : 0.0;
-                        }
-#pragma unroll
-                        for (int gb = 0; gb < GB; ++gb) {
-                            const bool col_ok = col0 + 8 * (g8 + gb) + (lane & 7) < nrhs;
-#pragma unroll
-                            for (int j = 0; j < JB; ++j)
-                                if (col_ok && j0 + j < rows_ok) ycol[ro[j] + 8 * gb * ycs] = old[gb][j] + (double)x[gb][j0 + j];
-                        }
-                    }
-                    ycol += 8 * GB * ycs;
+                    ycol += 8 * ycs;
                 }
             } else if (t.out_kind == OUT_Y) {
                 if (r < t.M) {
-                    double *Yb = pa->Y + pa->yofs[t.c_row] + r;
+                    const int ldc = t.ldc, ncol = nrhs - col0;  // in registers: the stores below may alias the record
+                    double *Yb = pa->Y + pa->yofs[t.c_row] + r + (size_t)col0 * ldc;
+                    if (ncol >= C::COLS && beta) {
 #pragma unroll
-                    for (int c0 = 0; c0 < C::COLS; c0 += C::RMW) {
-                        double old[C::RMW];
+                        for (int e = 0; e < C::COLS; ++e, Yb += ldc) add_or_store(Yb, (double)acc[e], 1);
+                    } else {
 #pragma unroll
-                        for (int e = 0; e < C::RMW; ++e) {
-                            const int cc = col0 + c0 + e;
-                            old[e] = (beta && cc < nrhs) ? Yb[(size_t)cc * t.ldc] : 0.0;
-                        }
-#pragma unroll
-                        for (int e = 0; e < C::RMW; ++e) {
-                            const int cc = col0 + c0 + e;
-                            if (cc < nrhs) Yb[(size_t)cc * t.ldc] = old[e] + (double)acc[c0 + e];
-                        }
+                        for (int e = 0; e < C::COLS; ++e, Yb += ldc)
+                            if (e < ncol) add_or_store(Yb, (double)acc[e], beta);
                     }
                 }
             } else if (t.out_kind == OUT_F32) {
                 if (r < t.M) {
-                    float *Sb = pa->skel + t.c_row * (int64_t)nrhs + r;
+                    float4 *S = reinterpret_cast<float4 *>(skel_at(pa, t, r, col0));
+                    const int quads = min(pa->nq - (col0 >> 2), columns >> 2);
 #pragma unroll
-                    for (int e = 0; e < C::COLS; ++e) {
-                        const int cc = col0 + e;
-                        if (cc < nrhs) Sb[(size_t)cc * t.ldc] = acc[e];
-                    }
+                    for (int q = 0; q < C::COLS / 4; ++q)
+                        if (q < quads) S[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
                 }
-            } else if (t.out_kind == OUT_SPLIT) {
-                // no product: split one 128-column tile of a leaf's W block (FP64, leaf-blocked)
-                // into 3-part operand tiles, every K tile of the leaf, as split_w_kernel does.
-                // Columns past nrhs and points past M are zero.
-                const int nt = un.col;
+            } else if (FLOW && t.out_kind == OUT_SPLIT) {
+                // no product: split one column tile of a leaf's W block (FP64) into 3-part operand
+                // tiles, every K tile of the leaf, as split_w_kernel does.  Columns past nrhs and
+                // points past M are zero.  The tile is 128 columns wide, in flow launches BN (the
+                // columns that the unit's counter covers).
+                const int n0 = un.col * (la.flow ? BN : 128), nt = n0 >> 7;
+                const int rows = tile_columns(nrhs, un.col, la.flow ? BN : 128);  // tile rows: right-hand sides
                 const int KTv = (t.M + 63) / 64;
-                const double *src = pa->W + pa->wofs[t.c_row];
                 uint8_t *base = pa->buf[t.t_buf] + ((size_t)t.out_kt * pa->NT + (size_t)nt * KTv) * 3 * (size_t)TILE_BYTES;
                 const int tid = threadIdx.x;  // the epilogue warps are warps 0 .. EPI_WARPS - 1
                 constexpr int PER = 1024 / (C::EPI_WARPS * 32);  // 16-byte chunks per thread and K tile
+                const bool ordered = ORD && pa->w_perm;
+                const double *src = ordered ? pa->W : pa->W + pa->wofs[t.c_row];
+                const int32_t *perm = ordered ? pa->w_perm + pa->tofs[t.c_row] : nullptr;
                 for (int kt = 0; kt < KTv; ++kt) {
-                    // all of the thread's loads of the K tile in flight before any split
+                    // all of the thread's loads of the K tile in flight before any split.  Lanes run
+                    // along K in leaf-blocked W, along the right-hand sides in caller order.
                     double x[PER][8];
 #pragma unroll
                     for (int i = 0; i < PER; ++i) {
                         const int idx = tid + i * C::EPI_WARPS * 32;
-                        const int c = idx % 8, n = nt * 128 + idx / 8;
+                        if (idx >= rows * 8) break;
+                        const int c = ordered ? idx / rows : idx % 8, n = n0 + (ordered ? idx % rows : idx / 8);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             const int k = kt * 64 + c * 8 + e;
-                            x[i][e] = (n < nrhs && k < t.M) ? src[k + (size_t)n * t.ldc] : 0.0;
+                            const bool in = n < nrhs && k < t.M;
+                            if (ordered) x[i][e] = in ? src[(int64_t)perm[k] * pa->w_rs + (int64_t)n * pa->w_cs] : 0.0;
+                            else x[i][e] = in ? src[k + (size_t)n * t.ldc] : 0.0;
                         }
                     }
 #pragma unroll
                     for (int i = 0; i < PER; ++i) {
                         const int idx = tid + i * C::EPI_WARPS * 32;
+                        if (idx >= rows * 8) break;
+                        const int c = ordered ? idx / rows : idx % 8, r = (n0 & 127) + (ordered ? idx % rows : idx / 8);
                         __nv_bfloat16 h[8], m[8], l[8];
 #pragma unroll
                         for (int e = 0; e < 8; ++e) tc::split3(x[i][e], h[e], m[e], l[e]);
-                        store_parts(base + (size_t)kt * 3 * TILE_BYTES, 3, idx / 8, idx % 8, h, m, l);
+                        store_parts(base + (size_t)kt * 3 * TILE_BYTES, 3, r, c, h, m, l);
                     }
                 }
             } else {
@@ -975,53 +1139,66 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 // per part.  Rows past M carry zeros (A is zero-padded); rows past the node's
                 // K tiles are not written.
                 if (beta && r < t.M) {
-                    const float *Sb = pa->skel + t.c_row * (int64_t)nrhs + r;
+                    const float4 *S = reinterpret_cast<const float4 *>(skel_at(pa, t, r, col0));
+                    const int quads = min(pa->nq - (col0 >> 2), columns >> 2);
+                    constexpr int QB = C::COLS >= 128 ? 2 : (C::COLS < 32 ? C::COLS / 4 : 8);  // loads in flight
 #pragma unroll
-                    for (int c0 = 0; c0 < C::COLS; c0 += C::RMW) {
-                        float old[C::RMW];
+                    for (int q0 = 0; q0 < C::COLS / 4; q0 += QB) {
+                        float4 old[QB];
 #pragma unroll
-                        for (int e = 0; e < C::RMW; ++e) {
-                            const int cc = col0 + c0 + e;
-                            old[e] = cc < nrhs ? Sb[(size_t)cc * t.ldc] : 0.f;
+                        for (int q = 0; q < QB; ++q)
+                            old[q] = q0 + q < quads ? S[(q0 + q) * 128] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int q = 0; q < QB; ++q) {
+                            acc[4 * (q0 + q)] += old[q].x;
+                            acc[4 * (q0 + q) + 1] += old[q].y;
+                            acc[4 * (q0 + q) + 2] += old[q].z;
+                            acc[4 * (q0 + q) + 3] += old[q].w;
                         }
-#pragma unroll
-                        for (int e = 0; e < C::RMW; ++e) acc[c0 + e] += old[e];
                     }
                 }
                 const int KTv = (t.M + 63) / 64;
                 const int k0 = t.m0 + (int)rank * 128 + quarter * 32 + (lane & ~7);
                 const bool k_ok = k0 < KTv * 64;
-                const int kt = k0 >> 6;
-                const uint32_t kin = (uint32_t)(k0 & 63);
-                uint8_t *tbuf = pa->buf[t.t_buf];
-                const int NT = pa->NT;
+                // column col0 + 8 g8 + (lane & 7) of this thread's groups: one 128-column tile, and
+                // the same swizzle phase, so a group is 1024 bytes after the one before
+                uint8_t *out = pa->buf[t.t_buf] +
+                               ((size_t)t.out_kt * pa->NT + (size_t)(col0 >> 7) * KTv + (k0 >> 6)) * 3 * (size_t)TILE_BYTES +
+                               tc::swizzled_offset((col0 & 127) + (lane & 7), k0 & 63);
 #pragma unroll
                 for (int g8 = 0; g8 < C::COLS / 8; ++g8) {
                     float x[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) x[j] = acc[8 * g8 + j];
                     transpose8(x, lane);
-                    const int n = col0 + 8 * g8 + (lane & 7);
                     uint4 vh, vm, vl;
                     tc::split3x8(x, vh, vm, vl);
-                    if (k_ok) {
-                        uint8_t *tile0 = tbuf + ((size_t)t.out_kt * NT + (size_t)(n >> 7) * KTv + kt) * 3 *
-                                                    (size_t)TILE_BYTES;
-                        const uint32_t o = tc::swizzled_offset(n & 127, (int)kin);
-                        *reinterpret_cast<uint4 *>(tile0 + o) = vh;
-                        *reinterpret_cast<uint4 *>(tile0 + TILE_BYTES + o) = vm;
-                        *reinterpret_cast<uint4 *>(tile0 + 2 * TILE_BYTES + o) = vl;
+                    if (k_ok && g8 * 8 < columns) {
+                        *reinterpret_cast<uint4 *>(out + g8 * 1024) = vh;
+                        *reinterpret_cast<uint4 *>(out + g8 * 1024 + TILE_BYTES) = vm;
+                        *reinterpret_cast<uint4 *>(out + g8 * 1024 + 2 * TILE_BYTES) = vl;
                     }
                 }
             }
             if (la.nlevels > 1) ++pend;  // counted when the warp moves past this level
-            if (la.deps && un.sig >= 0) {
-                // dataflow: this warp's part of the unit is written; count it for the units
-                // that read it (the test hook keeps the units without inputs from counting)
-                asm volatile("fence.proxy.async.global;\n" ::: "memory");
-                __threadfence();
+            if constexpr (PAIR) {
+                if (la.deps && un.sig >= 0) {
+                    // dataflow: this warp's part of the unit is written; count it for the units
+                    // that read it (the test hook keeps the units without inputs from counting)
+                    asm volatile("fence.proxy.async.global;\n" ::: "memory");
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0 && !(la.stall_level && un.dep0 < 0)) atomicAdd(la.deps + un.sig, 1);
+                }
+            } else {
+                // written: the publishing warp counts the unit.  Operand tiles are read by bulk copies.
+                if (t.out_kind == OUT_TILES || t.out_kind == OUT_SPLIT) asm volatile("fence.proxy.async.global;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0 && !(la.stall_level && un.dep0 < 0)) atomicAdd(la.deps + un.sig, 1);
+                if (lane == 0) arrive_local(&written[ri]);
+            }
+            if constexpr (!PAIR) {
+                __syncwarp();
+                if (lane == 0) arrive_local(&uempty[ri]);
             }
         }
     }
@@ -1040,6 +1217,19 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
     if (warp == 0) {
         if constexpr (PAIR) tc::tmem_dealloc_pair(tmem, C::TMEM_COLS);
         else tc::tmem_dealloc(tmem, C::TMEM_COLS);
+    }
+    if (FLOW && la.flow) {
+        // the last block out leaves the control words and counters at zero for the next launch
+        volatile int *last = ring;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            *last = atomicAdd(la.flow + FLOW_EXIT, 1) == (int)gridDim.x - 1;
+        }
+        __syncthreads();
+        if (*last) {
+            __threadfence();
+            for (int i = threadIdx.x; i < la.nflow; i += C::THREADS) la.flow[i] = 0;
+        }
     }
 }
 
@@ -1197,9 +1387,10 @@ struct SplitBF16 {
     std::vector<TcItem> items;
     std::vector<SplitJob> jobs;
     std::vector<int64_t> leaf_kt, node_kt;  // K-tile bases
-    int64_t leaf_kt_total = 0, node_kt_total = 0;
+    std::vector<int64_t> node_rt;           // first 128-row tile of a node in the FP32 far results
+    int64_t leaf_kt_total = 0, node_kt_total = 0, node_rt_total = 0;
     int nt_cap = 0, nrhs_cap = 0;
-    int buf_gen = 0;  // counts reallocations of the buffers below (graphs hold their addresses)
+    int buf_gen = 0;  // counts reallocations of the buffers below (entries hold their addresses)
     uint8_t *Wt = nullptr, *wT = nullptr, *uT = nullptr;
     float *u32 = nullptr;  // FP32 far results awaiting the down launch
     int *dErr = nullptr;
@@ -1224,8 +1415,8 @@ struct Batch : public mxb_batch {
     std::vector<MOp> ops;
     std::vector<TcTask> tasks;
     std::vector<TcItem> items;
-    // One-launch mode: the W split and every tensor-core op run as the levels of a single
-    // launch of the kernel with 3-part stages (OUT_SPLIT tasks at [split_task0, + split_tasks)).
+    // One-launch mode: a flow launch whatever the column count, W split by units of the launch
+    // (OUT_SPLIT tasks at [split_task0, + split_tasks)).
     bool one_launch = false;
     int split_task0 = 0, split_tasks = 0;
     unsigned long long *level_ns = nullptr;  // while profiling a one-launch evaluation
@@ -1246,12 +1437,18 @@ struct Batch : public mxb_batch {
         std::vector<CallerOrder> order;  // per plan, when W / Y are in the caller's point order
         PlanArgs *dPlans = nullptr;
         TcUnit *dUnits = nullptr;
+        size_t units_cap = 0;
         std::vector<int> unit_first, unit_count;
         // dataflow launches: per op, whether its chained launch waits on node counters (the
         // counters of every such launch in one array, zeroed before each evaluation)
         std::vector<char> dataflow;
         int *dDeps = nullptr;
         int ndeps = 0;
+        // flow launch: control words and counters, and the host copy of the plan table
+        int *dFlow = nullptr;
+        int nflow = 0;
+        bool flow_w = false;           // the flow launch splits W too
+        std::vector<PlanArgs> pa;
         cudaGraphExec_t exec = nullptr;
     };
     std::vector<Entry> entries;
@@ -1274,6 +1471,9 @@ struct Batch : public mxb_batch {
         if (e.dPlans) cudaFree(e.dPlans);
         if (e.dUnits) cudaFree(e.dUnits);
         if (e.dDeps) cudaFree(e.dDeps);
+        if (e.dFlow) cudaFree(e.dFlow);
+        e.dFlow = nullptr;
+        e.nflow = 0;
         e.exec = nullptr;
         e.dPlans = nullptr;
         e.dUnits = nullptr;
@@ -1288,15 +1488,28 @@ struct Batch : public mxb_batch {
     int build(const std::vector<Plan *> &ps, bool adjoint = false);
     int evaluate(const double *const *W, double *const *Y, const int *nrhs, int accumulate, cudaStream_t stream,
                  int debug_flags, long long wait_cycles, const CallerOrder *order = nullptr);
+    cudaError_t split_w(const Entry &e, const MOp &m, cudaStream_t stream) const;
     int enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wait_cycles, const std::vector<int> &bn,
                 int only_op = -1);
-    int units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream);
+    int units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream, int only = -1);
     int dataflow_units(const Entry &e, size_t k, size_t end, const std::vector<int> &bn, std::vector<TcUnit> &units,
                        int &ndeps) const;
+    int flow_units(Entry &e, int w, std::vector<TcUnit> &units) const;
+    struct FlowGroup {
+        std::vector<int> tasks, deps, cons;
+        int ncol = 0, kt = 0, op = 0, cost = 0, unplaced = 0;
+        double prio = -1, ready = 0, finish = 0;
+    };
+    int flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const;
+    double flow_balance(Entry &e, int w) const;
+    bool takes_flow(Entry &e) const;
+    int flow_columns(Entry &e) const;
+    int task_parts(const TcTask &t) const;
+    int flow_width(const std::vector<int> &bn) const;  // column tile of a flow launch, 0: none
+    std::vector<int> flow_tiles(int w) const;
+    bool flow_splits_w(const Entry &e, int w) const;
     void chain_all(std::vector<int> &bn) const;
     int tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaStream_t stream, long long wait_cycles);
-    int tune_one_launch(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaStream_t stream,
-                        long long wait_cycles);
     Entry *find(const double *const *W, double *const *Y, const std::vector<int> &nr, int accumulate,
                 int debug_flags, const CallerOrder *order = nullptr);
     int profile(const double *const *W, double *const *Y, const int *nrhs, cudaStream_t stream, mxb_op_profile *out,
@@ -1368,7 +1581,7 @@ int Batch::build(const std::vector<Plan *> &ps, bool adjoint)
         }
         if (m.count > 0) ops.push_back(m);
     }
-    // the W split as tasks of the tensor-core kernel, for the one-launch mode
+    // the W split as tasks of the tensor-core kernel, for flow launches
     split_task0 = (int)tasks.size();
     for (const MOp &m : ops) {
         if (m.phase != PH_SPLITW) continue;
@@ -1382,6 +1595,8 @@ int Batch::build(const std::vector<Plan *> &ps, bool adjoint)
             t.plan = sj.plan;
             t.out_kind = OUT_SPLIT;
             t.t_buf = BUF_W;
+            t.sig = FlowCounter{ps[sj.plan]->nleaf, ps[sj.plan]->numnodes}.w((int)sj.src_row);
+            t.old = -1;
             tasks.push_back(t);
         }
     }
@@ -1437,8 +1652,8 @@ int64_t unit_group_bytes()
     return v;
 }
 
-// MXB_TC_DATAFLOW=0 keeps chained launches on level barriers (read when an evaluation graph is
-// built).
+// MXB_TC_DATAFLOW=0 keeps chained launches on level barriers (read when an evaluation is
+// prepared).
 bool dataflow_enabled()
 {
     const char *e = getenv("MXB_TC_DATAFLOW");
@@ -1642,7 +1857,7 @@ int Batch::dataflow_units(const Entry &e, size_t k, size_t end, const std::vecto
         for (int t : nd.tasks) {
             const TcTask &tk = tasks[t];
             for (int q = tk.item0; q < tk.item0 + tk.nitem; ++q) {
-                auto it = by_out.find(std::make_tuple(nd.plan, (int)items[q].b_buf, items[q].b_base));
+                auto it = by_out.find(std::make_tuple(nd.plan, (int)items[q].b_buf, (int64_t)items[q].b_base));
                 if (it == by_out.end()) continue;  // written before this launch
                 const int wn = it->second;
                 if (nodes[wn].level >= nd.level) return 0;
@@ -1653,47 +1868,257 @@ int Batch::dataflow_units(const Entry &e, size_t k, size_t end, const std::vecto
     return dataflow_schedule(nodes, pair ? sm_count() / 2 : sm_count(), units, ndeps);
 }
 
+int Batch::flow_width(const std::vector<int> &bn) const
+{
+    for (size_t k = 0; k < ops.size() && k < bn.size(); ++k)
+        if (ops[k].phase != PH_SPLITW) return (bn[k] & TILE_FLOW) ? tile_width(bn[k]) : 0;
+    return 0;
+}
+
+std::vector<int> Batch::flow_tiles(int w) const
+{
+    std::vector<int> bn(ops.size(), 0);
+    for (size_t k = 0; k < ops.size(); ++k)
+        if (ops[k].phase != PH_SPLITW) bn[k] = w | TILE_FLOW;
+    return bn;
+}
+
+// Whether a flow launch splits W itself: where each block gets at most one such unit (a column tile
+// of a leaf, 19 - 30 us for 256 points x 64 - 128 columns, which the unit's 8 warps cannot hide),
+// the launch saved is worth more.  N = 30011, 130 columns: 102 us of the launch against 22 us in
+// split_w_kernel; N = 2048, 32 columns: 4 us against 11 us.
+bool Batch::flow_splits_w(const Entry &e, int w) const
+{
+    int64_t n = 0;
+    for (size_t i = 0; i < plans.size(); ++i) n += (int64_t)plans[i]->nleaf * ceil_div(e.nrhs[i], w);
+    return one_launch || (plans.size() == 1 && n <= sm_count());
+}
+
+// The parts of a task's operands (2: bf16x3 products).
+int Batch::task_parts(const TcTask &t) const
+{
+    if (t.nitem == 0) return 3;
+    const int pool = items[t.item0].a_pool, prec = plans[t.plan]->precision;
+    if (pool == POOL_NEAR || pool == POOL_NEART) return prec == MXB_PREC_SPLIT_BF16_X6 ? 3 : 2;
+    if (pool == POOL_FAR || pool == POOL_FART) return prec == MXB_PREC_SPLIT_BF16 ? 2 : 3;
+    return 3;
+}
+
+// The groups of a flow launch (one output block: its row tiles times its column tiles) and what
+// each reads.  Returns 1, or 0 where the counters do not fit.
+int Batch::flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const
+{
+    std::map<std::pair<int, int>, int> writer;   // (plan, counter) -> group
+    std::map<std::pair<int, int64_t>, int> last;  // (plan, leaf) -> leaf-down group
+    int64_t nctr = 0;
+    for (size_t i = 0; i < plans.size(); ++i) {
+        e.pa[i].ctr0 = (int32_t)nctr;
+        e.pa[i].ncol = (int32_t)ceil_div(e.nrhs[i], w);
+        nctr += (int64_t)FlowCounter{plans[i]->nleaf, plans[i]->numnodes}.count() * e.pa[i].ncol;
+    }
+    if (nctr > 0x3FFFFFFF) return 0;
+    e.nflow = FLOW_FIRST + (int)nctr;
+    auto add = [&](int t, int kt, size_t op) {
+        const TcTask &tk = tasks[t];
+        int &g = tk.sig >= 0 ? writer.emplace(std::make_pair((int)tk.plan, (int)tk.sig), -1).first->second
+                             : last.emplace(std::make_pair((int)tk.plan, tk.c_row), -1).first->second;
+        if (g < 0) {
+            g = (int)G.size();
+            G.emplace_back();
+            G[g].ncol = e.pa[tk.plan].ncol;
+            G[g].kt = kt;
+            G[g].op = (int)std::min<size_t>(op, 255);
+        }
+        G[g].tasks.push_back(t);
+    };
+    e.flow_w = flow_splits_w(e, w);
+    if (e.flow_w)
+        for (int t = split_task0; t < split_task0 + split_tasks; ++t) add(t, (tasks[t].M + 63) / 64, 0);
+    for (size_t k = 0; k < ops.size(); ++k) {
+        const MOp &m = ops[k];
+        if (m.phase == PH_SPLITW) continue;
+        for (int t = m.first; t < m.first + m.count; ++t) {
+            int kt = 0;
+            for (int q = 0; q < tasks[t].nitem; ++q) kt += items[tasks[t].item0 + q].KT;
+            add(t, kt, k);
+        }
+    }
+    for (int i = 0; i < (int)G.size(); ++i) {
+        FlowGroup &g = G[i];
+        const TcTask &tk = tasks[g.tasks[0]];
+        auto depends = [&](int ctr, int need) {
+            auto it = writer.find(std::make_pair((int)tk.plan, ctr));
+            if (it == writer.end() || (int)G[it->second].tasks.size() != need) return false;
+            if (std::find(g.deps.begin(), g.deps.end(), it->second) == g.deps.end()) {
+                g.deps.push_back(it->second);
+                G[it->second].cons.push_back(i);
+            }
+            return true;
+        };
+        for (int q = 0; q < tk.nitem; ++q) {
+            const TcItem &it = items[tk.item0 + q];
+            if (it.dep < 0 || (it.b_buf == BUF_W && !e.flow_w)) continue;
+            if (!depends(it.dep, it.need)) return 0;
+        }
+        if (tk.old >= 0 && !depends(tk.old, tk.old_need)) return 0;
+    }
+    return 1;
+}
+
+// Work of one SM over the longest path of a flow launch with w-column tiles: what decides the
+// tiles of a flow launch and whether to take one.  In K tiles of 6 products (a K tile of 3
+// products takes about 0.4 of one); a unit costs 3 more, a step of the path 3.5.
+double Batch::flow_balance(Entry &e, int w) const
+{
+    std::vector<FlowGroup> G;
+    if (flow_groups(e, w, G) <= 0) return 1e30;
+    auto ktiles = [&](const FlowGroup &g) { return g.kt * (task_parts(tasks[g.tasks[0]]) == 3 ? 1.0 : 0.4); };
+    std::vector<double> path(G.size(), 0.0);  // up to the group's end
+    std::vector<int> open(G.size()), order;
+    for (size_t i = 0; i < G.size(); ++i)
+        if (!(open[i] = (int)G[i].deps.size())) order.push_back((int)i);
+    double work = 0, longest = 1;
+    for (size_t q = 0; q < order.size(); ++q) {
+        const FlowGroup &g = G[order[q]];
+        double &p = path[order[q]];
+        for (int d : g.deps) p = std::max(p, path[d]);
+        p += ktiles(g) + 3.5;
+        longest = std::max(longest, p);
+        work += (double)g.tasks.size() * g.ncol * (ktiles(g) + 3);
+        for (int c : g.cons)
+            if (--open[c] == 0) order.push_back(c);
+    }
+    return work / sm_count() / longest;
+}
+
+// Whether an evaluation takes the flow launch without timing the alternatives: up to FLOW_COLUMNS
+// right-hand sides, where no launch would use a wider tile, and where one SM's work is below FLOW_WORK
+// of the longest path.  It was the faster one by a tenth or more at every size tried (N = 1024 -
+// 131072, 1 - 512 columns: 56 against 72 us at N = 1024 x 128, 521 against 647 us at N = 65536 x 128,
+// 618 against 731 us at N = 30011 x 384, balance 2.9), and timing them all takes 4 - 44 ms of the
+// first evaluation.  Up to FLOW_TRIED it is one of the timed candidates: between them it is 1.18
+// times as fast (N = 65536 x 512 without a near field) to 0.9 times (N = 131072 x 256; 65536 x 512: 0.93).
+constexpr int FLOW_COLUMNS = 128;
+constexpr double FLOW_WORK = 3.5, FLOW_TRIED = 12;
+bool Batch::takes_flow(Entry &e) const
+{
+    return *std::max_element(e.nrhs.begin(), e.nrhs.end()) <= FLOW_COLUMNS || flow_balance(e, 128) < FLOW_WORK;
+}
+
+// Columns of a flow launch's tiles.  A step of the path is shorter on 64-column tiles and the
+// work smaller on 128-column ones (their A tiles are read for twice the columns): 64 columns
+// below FLOW_NARROW.  N = 4096, leaf 256, 128 columns (balance 0.3): 113 against 146 us; N = 16384,
+// 256 columns (1.6): 240 against 242 us; N = 65536, 128 columns (2.4): 427 against 406 us.
+int Batch::flow_columns(Entry &e) const
+{
+    constexpr double FLOW_NARROW = 1.3;
+    if (*std::max_element(e.nrhs.begin(), e.nrhs.end()) <= 64) return 64;
+    return flow_balance(e, 64) < FLOW_NARROW ? 64 : 128;
+}
+
+// Units of a flow launch: every op of the evaluation in one launch, each unit waiting for the
+// blocks it reads (per node and column tile) instead of for the passes before.  List scheduling,
+// longest remaining path first among the groups whose inputs are written; a worker is a block,
+// which claims its next unit about DEPTH K tiles before the products of the current one end.
+// Times in K tiles (about 0.7 us): an epilogue and its publication take about EPILOGUE, seeing it
+// and loading from it LATENCY.  A unit's inputs come earlier in the list, so every wait ends.
+// Returns 1, 0 where some input has no writer in the launch, or an error code.
+int Batch::flow_units(Entry &e, int w, std::vector<TcUnit> &units) const
+{
+    constexpr int EPILOGUE = 4, LATENCY = 2, DEPTH = 4;
+    std::vector<FlowGroup> G;
+    if (flow_groups(e, w, G) <= 0) return 0;
+    for (FlowGroup &g : G) {
+        g.cost = g.kt + EPILOGUE + LATENCY;
+        g.unplaced = (int)g.deps.size();
+    }
+    std::function<double(int)> prio = [&](int i) -> double {
+        if (G[i].prio >= 0) return G[i].prio;
+        double best = 0;
+        for (int c : G[i].cons) best = std::max(best, prio(c));
+        return G[i].prio = best + G[i].cost;
+    };
+    for (int i = 0; i < (int)G.size(); ++i) prio(i);
+    struct Worker {
+        double claim, mma, epi;
+        bool operator>(const Worker &o) const { return claim > o.claim; }
+    };
+    auto low = [&](int a, int b) { return G[a].prio != G[b].prio ? G[a].prio < G[b].prio : a > b; };
+    auto late = [&](int a, int b) { return G[a].ready != G[b].ready ? G[a].ready > G[b].ready : a > b; };
+    std::priority_queue<int, std::vector<int>, decltype(low)> ready(low);
+    std::priority_queue<int, std::vector<int>, decltype(late)> waiting(late);
+    std::priority_queue<Worker, std::vector<Worker>, std::greater<Worker>> workers;
+    for (int i = 0; i < sm_count(); ++i) workers.push(Worker{0.0, 0.0, 0.0});
+    for (int i = 0; i < (int)G.size(); ++i)
+        if (!G[i].unplaced) waiting.push(i);
+    for (size_t placed = 0; placed < G.size(); ++placed) {
+        const double now = workers.top().claim;
+        while (!waiting.empty() && G[waiting.top()].ready <= now) {
+            ready.push(waiting.top());
+            waiting.pop();
+        }
+        int i;
+        if (!ready.empty()) {
+            i = ready.top();
+            ready.pop();
+        } else if (!waiting.empty()) {
+            i = waiting.top();
+            waiting.pop();
+        } else {
+            return batch_fail("flow schedule: a block's inputs are never written");
+        }
+        FlowGroup &g = G[i];
+        for (int c = 0; c < g.ncol; ++c)
+            for (int t : g.tasks) {
+                Worker k = workers.top();
+                workers.pop();
+                const double load = std::max(k.claim, g.ready);
+                k.mma = std::max(load + 2, k.mma) + g.kt;
+                k.claim = std::max(load, k.mma - DEPTH);
+                k.epi = std::max(k.mma, k.epi) + EPILOGUE;
+                workers.push(k);
+                g.finish = std::max(g.finish, k.epi);
+                int kt = 0;
+                for (int q = 0; q < tasks[t].nitem; ++q) kt += items[tasks[t].item0 + q].KT;
+                units.push_back(TcUnit{t, c, kt, (task_parts(tasks[t]) << 28) | (g.op << 20), -1, -1, 0, -1});
+            }
+        for (int c : g.cons) {
+            G[c].ready = std::max(G[c].ready, g.finish + LATENCY);
+            if (--G[c].unplaced == 0) waiting.push(c);
+        }
+    }
+    return 1;
+}
+
 // Work units of every TC op for this entry's nrhs and column-tile choices.
-// The list is uploaded on `stream`, ahead of the launches that read it.
-int Batch::units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream)
+// The list is uploaded on `stream`, ahead of the launches that read it.  only >= 0: the launch of
+// that op alone (the autotuner's trials).
+int Batch::units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream, int only)
 {
     std::vector<TcUnit> units;
     e.unit_first.assign(ops.size(), 0);
     e.unit_count.assign(ops.size(), 0);
-    if (one_launch) {
-        // level k = op k: the W split (one unit per leaf and 128-column tile), then every
-        // tensor-core op in sequence, each unit tagged with its operand parts
-        if (ops.size() > (size_t)MAX_CHAIN) return batch_fail("too many levels for one launch");
-        for (size_t k = 0; k < ops.size(); ++k) {
-            const MOp &m = ops[k];
-            e.unit_first[k] = (int)units.size();
-            const int prev = k ? e.unit_count[k - 1] : 0;
-            if (prev > 0xFFFFF) return batch_fail("a level of the one-launch evaluation has too many units");
-            const int32_t chain = ((int32_t)k << 20) | prev;
-            if (m.phase == PH_SPLITW) {
-                // the 128-column tiles that the launch's units read (its tile is 64 or 128 wide)
-                for (int t = split_task0; t < split_task0 + split_tasks; ++t) {
-                    const int NT = (int)ceil_div(e.nrhs[tasks[t].plan], 128);
-                    for (int nt = 0; nt < NT; ++nt) units.push_back(TcUnit{t, nt, 0, chain | (3 << 28)});
-                }
-            } else {
-                const int w = tile_width(bn[k]);
-                for (int t = m.first; t < m.first + m.count; ++t) {
-                    int kt = 0;
-                    for (int q = tasks[t].item0; q < tasks[t].item0 + tasks[t].nitem; ++q) kt += items[q].KT;
-                    const int ncol = (int)ceil_div(e.nrhs[tasks[t].plan], w);
-                    for (int c = 0; c < ncol; ++c) units.push_back(TcUnit{t, c, kt, chain | (m.P << 28)});
-                }
-            }
-            e.unit_count[k] = (int)units.size() - e.unit_first[k];
-        }
-    }
     e.dataflow.assign(ops.size(), 0);
     int ndeps = 0;
-    for (size_t k = 0; k < ops.size() && !one_launch; ++k) {
+    const int flow = flow_width(bn);
+    if (e.dFlow) cudaFree(e.dFlow);
+    e.dFlow = nullptr;
+    e.nflow = 0;
+    if (flow) {
+        const int r = flow_units(e, flow, units);
+        if (r <= 0) return r < 0 ? r : batch_fail("no flow schedule for these plans");
+        e.unit_count[0] = (int)units.size();
+        cudaError_t ferr = cudaMalloc(&e.dFlow, (size_t)e.nflow * sizeof(int));
+        if (ferr == cudaSuccess) ferr = cudaMemsetAsync(e.dFlow, 0, (size_t)e.nflow * sizeof(int), stream);
+        // the plans' counters and column tiles
+        if (ferr == cudaSuccess && e.dPlans)
+            ferr = cudaMemcpyAsync(e.dPlans, e.pa.data(), e.pa.size() * sizeof(PlanArgs), cudaMemcpyHostToDevice, stream);
+        if (ferr != cudaSuccess) return batch_fail(std::string("flow counters: ") + cudaGetErrorString(ferr), MXB_ERR_CUDA);
+    }
+    for (size_t k = 0; k < ops.size() && !flow; ++k) {
         const MOp &m = ops[k];
         e.unit_first[k] = (int)units.size();
-        if (m.phase == PH_SPLITW) continue;
+        if (m.phase == PH_SPLITW || (only >= 0 && (int)k != only)) continue;
         if (!(bn[k] & TILE_CHAIN) && dataflow_enabled()) {
             // a chain head: its run waits on node counters where the sweep's dependencies allow
             size_t end = k + 1;
@@ -1773,8 +2198,6 @@ int Batch::units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream)
         }
         e.unit_count[k] = (int)units.size() - e.unit_first[k];
     }
-    if (e.dUnits) cudaFree(e.dUnits);
-    e.dUnits = nullptr;
     if (e.dDeps) cudaFree(e.dDeps);
     e.dDeps = nullptr;
     e.ndeps = ndeps;
@@ -1782,7 +2205,13 @@ int Batch::units_for(Entry &e, const std::vector<int> &bn, cudaStream_t stream)
         const cudaError_t derr = cudaMalloc(&e.dDeps, (size_t)ndeps * sizeof(int));
         if (derr != cudaSuccess) return batch_fail(std::string("node counters: ") + cudaGetErrorString(derr), MXB_ERR_NOMEM);
     }
-    cudaError_t err = cudaMalloc(&e.dUnits, std::max<size_t>(units.size(), 1) * sizeof(TcUnit));
+    cudaError_t err = cudaSuccess;
+    if (!e.dUnits || units.size() > e.units_cap) {
+        if (e.dUnits) cudaFree(e.dUnits);
+        e.dUnits = nullptr;
+        e.units_cap = std::max<size_t>(units.size(), 1);
+        err = cudaMalloc(&e.dUnits, e.units_cap * sizeof(TcUnit));
+    }
     if (err == cudaSuccess && !units.empty())
         err = cudaMemcpyAsync(e.dUnits, units.data(), units.size() * sizeof(TcUnit), cudaMemcpyHostToDevice, stream);
     if (err != cudaSuccess) return batch_fail(std::string("work units: ") + cudaGetErrorString(err), MXB_ERR_CUDA);
@@ -1793,13 +2222,61 @@ namespace {
 int kchain_for(int P);
 }
 
+// W -> operand tiles.
+cudaError_t Batch::split_w(const Entry &e, const MOp &m, cudaStream_t stream) const
+{
+    int tiles = 1;
+    for (int r : e.nrhs) tiles = std::max<int>(tiles, (int)ceil_div(r, 128));
+    const dim3 grid(m.count, m.max_kt, tiles);
+    const PlanArgs *table = plans.size() == 1 ? nullptr : e.dPlans;
+    if (e.order.empty()) split_w_kernel<false><<<grid, 256, 0, stream>>>(dJobs + m.first, table, e.pa[0]);
+    else split_w_kernel<true><<<grid, 256, 0, stream>>>(dJobs + m.first, table, e.pa[0]);
+    return cudaGetLastError();
+}
 
 int Batch::enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wait_cycles, const std::vector<int> &bn,
                    int only_op)
 {
     bool first_tc = true;
-    int maxnt = 0;
-    for (Plan *p : plans) maxnt = std::max(maxnt, p->bf16->nt_cap);
+    if (const int flow = flow_width(bn)) {
+        if (one_launch && only_op > 0) return MXB_OK;  // (profiling asks for op 0 to time the launch)
+        if (one_launch) only_op = -1;
+        for (size_t k = 0; k < ops.size(); ++k) {
+            if (only_op >= 0 && (int)k != only_op) {
+                if (ops[k].phase != PH_SPLITW) break;
+                continue;
+            }
+            cudaError_t err = cudaSuccess;
+            if (ops[k].phase == PH_SPLITW) {
+                if (e.flow_w) continue;
+                err = split_w(e, ops[k], stream);
+            } else {
+                LaunchArgs a{};
+                a.plans = plans.size() == 1 ? nullptr : e.dPlans;
+                a.plan0 = e.pa[0];
+                a.nplans = (int)plans.size();
+                a.tasks = dTasks;
+                a.items = dItems;
+                a.units = e.dUnits;
+                a.nunits = e.unit_count[0];
+                a.next_unit = e.dFlow + FLOW_CLAIM;
+                a.err = plans[0]->bf16->dErr;
+                a.wait_cycles = wait_cycles > 0 ? wait_cycles : tc::WAIT_CYCLES;
+                a.stall_test = (debug_flags & MXB_DEBUG_STALL_ONE_WAIT) != 0;
+                a.kchain = kchain_for(3);
+                a.nlevels = 1;
+                a.level_ns = level_ns;
+                a.stall_level = (debug_flags & MXB_DEBUG_STALL_LEVEL) != 0;
+                a.flow = e.dFlow;
+                a.nflow = e.nflow;
+                a.skip_w = e.flow_w ? 0 : 1;
+                err = launch_tc(3, flow, false, !e.order.empty(), a, stream);
+            }
+            if (err != cudaSuccess) return batch_fail(std::string("flow launch: ") + cudaGetErrorString(err), MXB_ERR_CUDA);
+            if (ops[k].phase != PH_SPLITW) break;
+        }
+        return MXB_OK;
+    }
     // work-unit and level counters of the tensor-core launches start at zero (both arrays in
     // one allocation: dLevel follows dNext)
     const size_t nops = std::max<size_t>(ops.size(), 1);
@@ -1807,35 +2284,6 @@ int Batch::enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wai
     if (zerr == cudaSuccess && e.ndeps && (only_op < 0 || (only_op < (int)e.dataflow.size() && e.dataflow[only_op])))
         zerr = cudaMemsetAsync(e.dDeps, 0, (size_t)e.ndeps * sizeof(int), stream);
     if (zerr != cudaSuccess) return batch_fail(std::string("work-unit counters: ") + cudaGetErrorString(zerr), MXB_ERR_CUDA);
-    if (one_launch) {
-        // every op is a level of the launch of op 0 (profiling asks for op 0 to time it)
-        if (only_op > 0) return MXB_OK;
-        int w = 128;
-        for (size_t k = 0; k < ops.size(); ++k)
-            if (ops[k].phase != PH_SPLITW) {
-                w = tile_width(bn[k]) >= 128 ? 128 : 64;
-                break;
-            }
-        LaunchArgs a{};
-        a.plans = e.dPlans;
-        a.tasks = dTasks;
-        a.items = dItems;
-        a.units = e.dUnits;
-        a.nunits = 0;
-        for (int c : e.unit_count) a.nunits += c;
-        a.next_unit = dNext;
-        a.err = plans[0]->bf16->dErr;
-        a.wait_cycles = wait_cycles > 0 ? wait_cycles : tc::WAIT_CYCLES;
-        a.stall_test = (debug_flags & MXB_DEBUG_STALL_ONE_WAIT) != 0;
-        a.kchain = kchain_for(3);
-        a.nlevels = (int)ops.size();
-        a.level_done = dLevel;
-        a.stall_level = (debug_flags & MXB_DEBUG_STALL_LEVEL) != 0;
-        a.level_ns = level_ns;
-        const cudaError_t err = launch_tc(3, w, false, false, a, stream);
-        if (err != cudaSuccess) return batch_fail(std::string("one-launch evaluation: ") + cudaGetErrorString(err), MXB_ERR_CUDA);
-        return MXB_OK;
-    }
     for (size_t k = 0; k < ops.size(); ++k) {
         const MOp &m = ops[k];
         const bool run = only_op < 0 || (int)k == only_op;
@@ -1843,16 +2291,14 @@ int Batch::enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wai
         if (m.phase != PH_SPLITW && (bn[k] & TILE_CHAIN)) continue;  // runs in its chain head's launch
         if (m.phase == PH_SPLITW) {
             if (run) {
-                if (e.order.empty())
-                    split_w_kernel<false><<<dim3(m.count, m.max_kt, maxnt), 256, 0, stream>>>(dJobs + m.first, e.dPlans);
-                else
-                    split_w_kernel<true><<<dim3(m.count, m.max_kt, maxnt), 256, 0, stream>>>(dJobs + m.first, e.dPlans);
-                err = cudaGetLastError();
+                err = split_w(e, m, stream);
             }
         } else {
             if (run) {
                 LaunchArgs a{};
-                a.plans = e.dPlans;
+                a.plans = plans.size() == 1 ? nullptr : e.dPlans;
+                a.plan0 = e.pa[0];
+                a.nplans = (int)plans.size();
                 a.tasks = dTasks;
                 a.items = dItems;
                 a.units = e.dUnits + e.unit_first[k];
@@ -1875,7 +2321,7 @@ int Batch::enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wai
                     a.deps = e.dDeps;
                 }
                 a.stall_level = (debug_flags & MXB_DEBUG_STALL_LEVEL) != 0;
-                        int total = 0;
+                int total = 0;
                 for (size_t j = k; j < end; ++j) total += e.unit_count[j];
                 a.nunits = total;
                 err = launch_tc(m.P, tile_width(bn[k]), tile_pair(bn[k]), writes_y && !e.order.empty(), a, stream);
@@ -1888,6 +2334,9 @@ int Batch::enqueue(Entry &e, cudaStream_t stream, int debug_flags, long long wai
 }
 
 namespace {
+
+// Column quads of a row tile of the FP32 far results (64-column tiles write whole quads).
+int far_quads(int nrhs) { return 16 * (int)ceil_div(nrhs, 64); }
 
 int split_buffers(Plan &p, SplitBF16 &S, int nrhs)
 {
@@ -1908,7 +2357,7 @@ int split_buffers(Plan &p, SplitBF16 &S, int nrhs)
     int rc = p.alloc((void **)&S.Wt, std::max<int64_t>(S.leaf_kt_total, 1) * NT * tile3);
     if (!rc) rc = p.alloc((void **)&S.wT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
     if (!rc) rc = p.alloc((void **)&S.uT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
-    if (!rc) rc = p.alloc((void **)&S.u32, std::max<int64_t>(p.skel_total, 1) * (size_t)nrhs * sizeof(float));
+    if (!rc) rc = p.alloc((void **)&S.u32, std::max<int64_t>(S.node_rt_total, 1) * (size_t)far_quads(nrhs) * 512 * sizeof(float));
     if (rc) return rc;
     S.nt_cap = NT;
     S.nrhs_cap = nrhs;
@@ -1925,7 +2374,7 @@ int default_bn(int P, int nrhs_max)
 
 // MXB_TC_TILE=<code> runs every tensor-core launch with that tile (width, + MXB_TILE_PAIR for
 // pairs), mapped to the nearest variant the launch's product count has; read when an
-// evaluation graph is built.  For tests that must reach one kernel variant.
+// evaluation is prepared.  For tests that must reach one kernel variant.
 int forced_tile(int P)
 {
     const char *e = getenv("MXB_TC_TILE");
@@ -1960,7 +2409,7 @@ bool pairs_enabled()
 
 // MXB_TC_CHAIN=0 keeps every tree level in a launch of its own; MXB_TC_CHAIN=2 chains every run
 // of sweep levels that share a product count and a tile, without timing the alternatives (read
-// when an evaluation graph is built).
+// when an evaluation is prepared).
 bool chains_enabled()
 {
     const char *e = getenv("MXB_TC_CHAIN");
@@ -1972,7 +2421,14 @@ bool chains_forced()
     return e && *e == '2';
 }
 
-// MXB_AUTOTUNE=0 keeps the default tiles (read when an evaluation graph is built).
+// MXB_TC_FLOW=0 keeps the passes in launches of their own (read when an evaluation is prepared).
+bool flow_enabled()
+{
+    const char *e = getenv("MXB_TC_FLOW");
+    return !(e && *e == '0') && chains_enabled() && !chains_forced();
+}
+
+// MXB_AUTOTUNE=0 keeps the default tiles (read when an evaluation is prepared).
 bool autotune_enabled()
 {
     const char *e = getenv("MXB_AUTOTUNE");
@@ -1984,72 +2440,8 @@ bool autotune_enabled()
 // Autotuner: runs the op sequence once; every tensor-core op is timed with each candidate
 // column-tile width (second of two runs, CUDA events) with the Y outputs redirected to
 // scratch, and the fastest width is kept.  Each op's outputs are left in place for the next.
-// One-launch mode: the whole evaluation is one launch, so its one column-tile width (64 or 128)
-// is picked by timing the launch with each (Y redirected to scratch).
-int Batch::tune_one_launch(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaStream_t stream,
-                           long long wait_cycles)
-{
-    const int np = (int)plans.size();
-    std::vector<double *> scratch(np, nullptr);
-    PlanArgs *dTune = nullptr;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    Entry te;
-    te.nrhs = e.nrhs;
-    int rc = MXB_OK;
-    for (int i = 0; i < np && !rc; ++i) {
-        Plan &p = *plans[i];
-        size_t ext = 0;
-        for (int l = 0; l < p.nleaf; ++l)
-            ext = std::max<size_t>(ext, (size_t)p.ofs_host[1][l] + (size_t)p.Ddim[l] * e.nrhs[i]);
-        if (cudaMalloc(&scratch[i], std::max<size_t>(ext, 1) * sizeof(double)) != cudaSuccess)
-            rc = batch_fail("autotune scratch allocation failed", MXB_ERR_NOMEM);
-        else
-            pa[i].Y = scratch[i];
-        pa[i].y_perm = nullptr;
-    }
-    if (!rc && cudaMalloc(&dTune, np * sizeof(PlanArgs)) != cudaSuccess)
-        rc = batch_fail("autotune table allocation failed", MXB_ERR_NOMEM);
-    if (!rc && cudaMemcpyAsync(dTune, pa.data(), np * sizeof(PlanArgs), cudaMemcpyHostToDevice, stream) != cudaSuccess)
-        rc = batch_fail("autotune table upload failed", MXB_ERR_CUDA);
-    te.dPlans = dTune;
-    if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
-        rc = batch_fail("autotune events", MXB_ERR_CUDA);
-    float best = 1e30f;
-    int best_w = 128;
-    for (int w : {128, 64}) {
-        if (rc) break;
-        std::vector<int> trial = bn;
-        for (size_t k = 0; k < ops.size(); ++k)
-            if (ops[k].phase != PH_SPLITW) trial[k] = w;
-        rc = units_for(te, trial, stream);
-        float ms = 0.f;
-        for (int rep = 0; rep < 2 && !rc; ++rep) {
-            cudaEventRecord(e0, stream);
-            rc = enqueue(te, stream, 0, wait_cycles, trial, -1);
-            cudaEventRecord(e1, stream);
-            if (!rc && cudaEventSynchronize(e1) != cudaSuccess) rc = batch_fail("autotune sync", MXB_ERR_CUDA);
-            if (!rc) cudaEventElapsedTime(&ms, e0, e1);
-        }
-        if (!rc && ms < best) {
-            best = ms;
-            best_w = w;
-        }
-    }
-    for (size_t k = 0; k < ops.size(); ++k)
-        if (ops[k].phase != PH_SPLITW) bn[k] = best_w;
-    if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) rc = batch_fail("autotune sync", MXB_ERR_CUDA);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
-    if (te.dUnits) cudaFree(te.dUnits);
-    if (dTune) cudaFree(dTune);
-    for (double *x : scratch)
-        if (x) cudaFree(x);
-    return rc;
-}
-
 int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaStream_t stream, long long wait_cycles)
 {
-    if (one_launch) return tune_one_launch(e, pa, bn, stream, wait_cycles);
     const int np = (int)plans.size();
     const int maxn = *std::max_element(e.nrhs.begin(), e.nrhs.end());
     std::vector<double *> scratch(np, nullptr);
@@ -2058,6 +2450,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
     Entry te;
     te.nrhs = e.nrhs;
     te.order = e.order;  // the same kernel instantiations as the evaluation (Y goes to scratch)
+    te.pa.resize(np);
     int rc = MXB_OK;
     for (int i = 0; i < np && !rc; ++i) {
         Plan &p = *plans[i];
@@ -2069,6 +2462,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
         else
             pa[i].Y = scratch[i];
         pa[i].y_perm = nullptr;  // the scratch is leaf-blocked (packed offsets)
+        te.pa[i] = pa[i];
     }
     if (!rc && cudaMalloc(&dTune, np * sizeof(PlanArgs)) != cudaSuccess)
         rc = batch_fail("autotune table allocation failed", MXB_ERR_NOMEM);
@@ -2080,7 +2474,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
     std::vector<float> op_ms(ops.size(), 0.f);
     for (size_t k = 0; k < ops.size() && !rc; ++k) {
         if (ops[k].phase == PH_SPLITW) {
-            rc = units_for(te, bn, stream);
+            rc = units_for(te, bn, stream, (int)k);
             if (!rc) rc = enqueue(te, stream, 0, wait_cycles, bn, (int)k);
             continue;
         }
@@ -2095,7 +2489,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
             if (tile_width(c) > 2 * std::max(64, maxn)) continue;
             std::vector<int> trial = bn;
             trial[k] = c;
-            rc = units_for(te, trial, stream);
+            rc = units_for(te, trial, stream, (int)k);
             float ms = 0.f;
             bool refused = false;
             for (int rep = 0; rep < 2 && !rc && !refused; ++rep) {
@@ -2121,7 +2515,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
         }
         bn[k] = best_bn;
         op_ms[k] = best;
-        if (!rc) rc = units_for(te, bn, stream);
+        if (!rc) rc = units_for(te, bn, stream, (int)k);
         if (!rc) rc = enqueue(te, stream, 0, wait_cycles, bn, (int)k);
     }
     // Chains: a run of consecutive up-sweep launches (or down-sweep launches, leaf down
@@ -2180,10 +2574,36 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
         k = j;
     }
     if (!rc) rc = units_for(te, bn, stream);
+    // The whole evaluation in one flow launch, against the launches chosen above.  Its tiles are
+    // at most 128 columns of single CTAs with 3-part stages, which wide coupling launches outrun.
+    if (!rc && flow_enabled() && flow_balance(te, 128) < FLOW_TRIED) {
+        auto time_all = [&](const std::vector<int> &tiles, float &best) {
+            best = 1e30f;
+            for (int rep = 0; rep < 4 && !rc; ++rep) {
+                float ms = 0.f;
+                cudaEventRecord(e0, stream);
+                rc = enqueue(te, stream, 0, wait_cycles, tiles, -1);
+                cudaEventRecord(e1, stream);
+                if (!rc && cudaEventSynchronize(e1) != cudaSuccess) rc = batch_fail("autotune sync", MXB_ERR_CUDA);
+                if (!rc) cudaEventElapsedTime(&ms, e0, e1);
+                if (rep) best = std::min(best, ms);
+            }
+        };
+        float best = 0.f;
+        time_all(bn, best);
+        const std::vector<int> trial = flow_tiles(flow_columns(te));
+        if (!rc && units_for(te, trial, stream) == MXB_OK) {  // (no schedule: not a candidate)
+            float ms = 0.f;
+            time_all(trial, ms);
+            if (!rc && ms < best) bn = trial;
+        }
+    }
     if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) rc = batch_fail("autotune sync", MXB_ERR_CUDA);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (te.dUnits) cudaFree(te.dUnits);
+    if (te.dDeps) cudaFree(te.dDeps);
+    if (te.dFlow) cudaFree(te.dFlow);
     if (dTune) cudaFree(dTune);
     for (double *s : scratch)
         if (s) cudaFree(s);
@@ -2238,6 +2658,7 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
             pa[i].skel = S.u32;
             pa[i].NT = S.nt_cap;
             pa[i].nrhs = nr[i];
+            pa[i].nq = far_quads(nr[i]);
             pa[i].beta_arg = accumulate ? 1 : 0;
             if (order) {
                 pa[i].w_perm = pa[i].y_perm = order[i].perm;
@@ -2248,9 +2669,16 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
                 pa[i].y_cs = order[i].y_cs;
             }
         }
-        cudaError_t err = cudaMalloc(&e.dPlans, np * sizeof(PlanArgs));
-        // on the evaluation stream, ahead of the graph launch that reads it
-        if (err == cudaSuccess)
+        // preparing allocates, and uploads from temporary host memory: not while the stream captures
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        MXB_CUDA_OR(cudaStreamIsCapturing(stream, &cap));
+        if (cap != cudaStreamCaptureStatusNone) {
+            return batch_fail("the first evaluation of these operands cannot be captured: evaluate them once before",
+                              MXB_ERR_UNSUPPORTED);
+        }
+        // several plans: their table, on the evaluation stream ahead of the graph launch that reads it
+        cudaError_t err = np > 1 ? cudaMalloc(&e.dPlans, np * sizeof(PlanArgs)) : cudaSuccess;
+        if (err == cudaSuccess && np > 1)
             err = cudaMemcpyAsync(e.dPlans, pa.data(), np * sizeof(PlanArgs), cudaMemcpyHostToDevice, stream);
         if (err != cudaSuccess) {
             release(e);
@@ -2261,12 +2689,21 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
         std::vector<int> bn(ops.size(), 0);
         for (size_t k = 0; k < ops.size(); ++k)
             if (ops[k].phase != PH_SPLITW) bn[k] = default_bn(ops[k].P, maxn);
+        e.pa = pa;
         auto t = tuned.find(nr);
-        if (forced_tile(2)) {
+        if (t != tuned.end() && flow_width(t->second) && (debug_flags & (MXB_DEBUG_CHAIN_LEVELS | MXB_DEBUG_STALL_LEVEL)))
+            t = tuned.end();  // the hooks of chained levels: default tiles, chained below
+        if (one_launch) {
+            // the whole evaluation in one flow launch, W split included
+            bn = flow_tiles(flow_columns(e));
+        } else if (forced_tile(2)) {
             for (size_t k = 0; k < ops.size(); ++k)
                 if (ops[k].phase != PH_SPLITW) bn[k] = forced_tile(ops[k].P);
         } else if (t != tuned.end()) {
             bn = t->second;
+        } else if (autotune_enabled() && !debug_flags && flow_enabled() && takes_flow(e)) {
+            bn = flow_tiles(flow_columns(e));
+            tuned[nr] = bn;
         } else if (autotune_enabled() && !debug_flags) {
             int rc = tune(e, pa, bn, stream, wait_cycles);
             if (rc) {
@@ -2275,20 +2712,16 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
             }
             tuned[nr] = bn;
         }
-        if ((debug_flags & (MXB_DEBUG_CHAIN_LEVELS | MXB_DEBUG_STALL_LEVEL)) || chains_forced()) chain_all(bn);
-        if (one_launch) {
-            // one tile for the whole launch: the first tensor-core op's width, 64 or 128
-            int w = 0;
-            for (size_t k = 0; k < ops.size() && !w; ++k)
-                if (ops[k].phase != PH_SPLITW) w = tile_width(bn[k]) >= 128 ? 128 : 64;
-            for (size_t k = 0; k < ops.size(); ++k)
-                if (ops[k].phase != PH_SPLITW) bn[k] = w;
-        }
+        if (!one_launch && ((debug_flags & (MXB_DEBUG_CHAIN_LEVELS | MXB_DEBUG_STALL_LEVEL)) || chains_forced())) chain_all(bn);
         e.bn = bn;
         int rc = units_for(e, bn, stream);
         if (rc) {
             release(e);
             return rc;
+        }
+        if (np == 1) {  // a handful of launches that take the operands as arguments: no graph
+            entries.push_back(std::move(e));
+            return enqueue(entries.back(), stream, debug_flags, wait_cycles, bn);
         }
         if (!capture_stream && cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking) != cudaSuccess) {
             release(e);
@@ -2314,6 +2747,21 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
         }
         entries.push_back(std::move(e));
         hit = &entries.back();
+    } else if (!hit->exec) {
+        // a single plan's launches take the operands as arguments: nothing is kept by their address
+        PlanArgs &pa = hit->pa[0];
+        pa.W = W[0];
+        pa.Y = Y[0];
+        pa.beta_arg = accumulate ? 1 : 0;
+        if (order) {
+            pa.w_perm = pa.y_perm = order[0].perm;
+            pa.tofs = order[0].tofs;
+            pa.w_rs = order[0].w_rs;
+            pa.w_cs = order[0].w_cs;
+            pa.y_rs = order[0].y_rs;
+            pa.y_cs = order[0].y_cs;
+        }
+        return enqueue(*hit, stream, debug_flags, wait_cycles, hit->bn);
     }
     MXB_CUDA_OR(cudaGraphLaunch(hit->exec, stream));
     return MXB_OK;
@@ -2324,7 +2772,8 @@ Batch::Entry *Batch::find(const double *const *W, double *const *Y, const std::v
 {
     Entry *hit = nullptr;
     for (Entry &e : entries) {
-        bool same = e.accumulate == accumulate && e.nrhs == nr && e.debug_flags == debug_flags &&
+        if (!e.exec && e.nrhs == nr && e.debug_flags == debug_flags && e.order.empty() == !order) return &e;  // one plan
+        bool same = e.exec && e.accumulate == accumulate && e.nrhs == nr && e.debug_flags == debug_flags &&
                     e.order.empty() == !order;
         for (size_t i = 0; same && order && i < plans.size(); ++i) {
             const CallerOrder &a = e.order[i], &b = order[i];
@@ -2338,18 +2787,18 @@ Batch::Entry *Batch::find(const double *const *W, double *const *Y, const std::v
 }
 
 // Launch-by-launch timing of one evaluation (mxb_batch_profile / mxb_plan_profile); the
-// evaluation graph of these operands has been built (and run) by the caller.
+// evaluation of these operands has been prepared (and run) by the caller.
 int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cudaStream_t stream, mxb_op_profile *out,
                    int cap, int *nops)
 {
     const std::vector<int> nr(nrhs, nrhs + plans.size());
     Entry *e = find(W, Y, nr, 0, 0);
-    if (!e) return batch_fail("profile: no evaluation graph for these operands");
+    if (!e) return batch_fail("profile: these operands have not been evaluated");
     std::vector<cudaEvent_t> ev(ops.size() + 1, nullptr);
     int rc = MXB_OK;
     for (cudaEvent_t &x : ev)
         if (!rc && cudaEventCreate(&x) != cudaSuccess) rc = batch_fail("profile: creating CUDA events failed", MXB_ERR_CUDA);
-    // one launch: each level's span on the device, from the kernel's own timestamps
+    // one launch: each op's span on the device, from the kernel's own timestamps
     std::vector<unsigned long long> lns(ops.size() + 1, 0);
     if (!rc && one_launch) {
         if (cudaMalloc(&level_ns, lns.size() * sizeof(unsigned long long)) != cudaSuccess) {
@@ -2395,6 +2844,8 @@ int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cu
         }
         for (int t = ops[k].first; t < ops[k].first + ops[k].count; ++t) task_op[t] = (int)k;
     }
+    int first_tc = 0;
+    while (first_tc < (int)ops.size() && ops[first_tc].phase == PH_SPLITW) ++first_tc;
     for (size_t k = 0; k < ops.size() && !rc && (int)k < cap && out; ++k) {
         const MOp &m = ops[k];
         mxb_op_profile &o = out[k];
@@ -2403,11 +2854,21 @@ int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cu
         o.level = m.level;
         o.width = tile_width(e->bn[k]);
         o.pair = tile_pair(e->bn[k]) ? 1 : 0;
-        o.chained = one_launch ? (k > 0) : ((m.phase != PH_SPLITW && (e->bn[k] & TILE_CHAIN)) ? 1 : 0);
+        o.chained = one_launch ? (k > 0) : flow_width(e->bn) ? (m.phase == PH_SPLITW ? e->flow_w : (int)k != first_tc) : ((m.phase != PH_SPLITW && (e->bn[k] & TILE_CHAIN)) ? 1 : 0);
         cudaEventElapsedTime(&o.ms, ev[k], ev[k + 1]);
         if (o.chained) o.ms = 0.f;
-        if (one_launch && lns[k + 1] >= lns[k] && lns[0] != ~0ull)
-            o.level_ms = (float)((double)(lns[k + 1] - (k ? lns[k] : lns[0])) * 1e-6);
+    }
+    if (!rc && one_launch && out && lns[0] != ~0ull) {
+        // the passes overlap: each gets the time from the end of the one that ended before it
+        std::vector<int> by(ops.size());
+        for (size_t k = 0; k < by.size(); ++k) by[k] = (int)k;
+        std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return lns[a + 1] < lns[b + 1]; });
+        unsigned long long last = lns[0];
+        for (int k : by) {
+            const unsigned long long end = std::max(lns[k + 1], last + 1);
+            if (k < cap) out[k].level_ms = (float)((double)(end - last) * 1e-6);
+            last = end;
+        }
     }
     for (size_t u = 0; u < units.size() && !rc && out; ++u) {
         const TcTask &t = tasks[units[u].task];
@@ -2451,9 +2912,12 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
         S->leaf_kt_total += KT(Ddim[i]);
     }
     S->node_kt.assign(numnodes, 0);
+    S->node_rt.assign(numnodes, 0);
     for (int v : bfs) {
         S->node_kt[v] = S->node_kt_total;
         S->node_kt_total += KT(slen[v]);
+        S->node_rt[v] = S->node_rt_total;
+        S->node_rt_total += RT(slen[v]);
     }
 
     // ---- CDS pools: tiling jobs ----
@@ -2556,8 +3020,10 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
         o.count = (o.phase == PH_SPLITW ? (int)S->jobs.size() : (int)S->tasks.size()) - o.first;
         if (o.count == 0) op_list->pop_back();
     };
+    const FlowCounter fc{nleaf, numnodes};
+    auto row_tiles = [](int rows) { return (rows + 127) / 128; };
     auto add_tasks = [&](int16_t out_kind, int64_t c_row, int64_t out_kt, int ldc, int M, int item0,
-                         int16_t beta, int t_buf) {
+                         int16_t beta, int t_buf, int sig, int old = -1) {
         for (int m0 = 0; m0 < M; m0 += 128) {
             TcTask t{};
             t.c_row = c_row;
@@ -2571,15 +3037,22 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             t.out_kind = out_kind;
             t.beta = beta;
             t.t_buf = t_buf;
+            t.sig = sig;
+            t.old = old;
+            t.old_need = row_tiles(M);  // of the same block
             S->tasks.push_back(t);
         }
     };
-    auto item = [&](int a_pool, uint64_t a_off, int b_buf, int64_t b_base, int K) {
+    // B from buffer b_buf of leaf (W) or node `from`, whose K is K
+    auto item = [&](int a_pool, uint64_t a_off, int b_buf, int from, int K) {
         TcItem it{};
-        it.a_pool = (int16_t)a_pool;
+        it.a_pool = (int8_t)a_pool;
         it.a_off = a_off;
-        it.b_buf = (int16_t)b_buf;
-        it.b_base = b_base;
+        it.b_buf = (int8_t)b_buf;
+        it.b_base = (int32_t)(b_buf == BUF_W ? S->leaf_kt[from] : S->node_kt[from]);
+        it.dep = b_buf == BUF_W ? fc.w(from) : (b_buf == BUF_WSKEL ? fc.up(from) : fc.u(from));
+        if (b_buf != BUF_W && !projects(from)) it.dep = -1;  // (the root's block) nothing writes it
+        it.need = (int16_t)(b_buf == BUF_W ? 1 : row_tiles(K));
         it.KT = KT(K);
         it.K = K;
         if (it.KT > 0) S->items.push_back(it);
@@ -2605,12 +3078,12 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             if (height[v] != h || !projects(v)) continue;
             const int item0 = (int)S->items.size();
             if (lch[v] == -1) {
-                item(POOL_VU3, up_a[v], BUF_W, S->leaf_kt[lm[v]], Ddim[lm[v]]);
+                item(POOL_VU3, up_a[v], BUF_W, lm[v], Ddim[lm[v]]);
             } else {
-                if (slen[lch[v]] > 0) item(POOL_VU3, up_a[v], BUF_WSKEL, S->node_kt[lch[v]], slen[lch[v]]);
-                if (slen[rch[v]] > 0) item(POOL_VU3, up_b[v], BUF_WSKEL, S->node_kt[rch[v]], slen[rch[v]]);
+                if (slen[lch[v]] > 0) item(POOL_VU3, up_a[v], BUF_WSKEL, lch[v], slen[lch[v]]);
+                if (slen[rch[v]] > 0) item(POOL_VU3, up_b[v], BUF_WSKEL, rch[v], slen[rch[v]]);
             }
-            add_tasks(OUT_TILES, skel_row[v], S->node_kt[v], slen[v], slen[v], item0, 0, BUF_WSKEL);
+            add_tasks(OUT_TILES, S->node_rt[v], S->node_kt[v], slen[v], slen[v], item0, 0, BUF_WSKEL, fc.up(v));
         }
         end_op();
     }
@@ -2628,8 +3101,8 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             if (lch[v] != -1) continue;
             const int x = lm[v];
             const int item0 = (int)S->items.size();
-            for (int k : near_out[x]) item(POOL_NEAR, near_a[k], BUF_W, S->leaf_kt[near_y[k]], Ddim[near_y[k]]);
-            add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W);
+            for (int k : near_out[x]) item(POOL_NEAR, near_a[k], BUF_W, near_y[k], Ddim[near_y[k]]);
+            add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W, fc.near(x));
         }
     };
     const bool near_with_far = near_parts == far_parts;
@@ -2638,9 +3111,9 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
         if (!projects(c)) continue;
         const int item0 = (int)S->items.size();
         for (int k : far_out[c])
-            if (slen[far_y[k]] > 0) item(POOL_FAR, far_a[k], BUF_WSKEL, S->node_kt[far_y[k]], slen[far_y[k]]);
-        add_tasks(has_down(c) ? OUT_F32 : OUT_TILES, skel_row[c], S->node_kt[c], slen[c], slen[c], item0, 0,
-                  BUF_USKEL);
+            if (slen[far_y[k]] > 0) item(POOL_FAR, far_a[k], BUF_WSKEL, far_y[k], slen[far_y[k]]);
+        add_tasks(has_down(c) ? OUT_F32 : OUT_TILES, S->node_rt[c], S->node_kt[c], slen[c], slen[c], item0, 0,
+                  BUF_USKEL, has_down(c) ? fc.far(c) : fc.u(c));
     }
     if (near_with_far) near_tasks();
     end_op();
@@ -2649,8 +3122,8 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
         for (int c : bfs) {
             if (depth[c] != dd || !projects(c) || !has_down(c)) continue;
             const int item0 = (int)S->items.size();
-            item(POOL_VD3, down_child[c], BUF_USKEL, S->node_kt[parent[c]], slen[parent[c]]);
-            add_tasks(OUT_TILES, skel_row[c], S->node_kt[c], slen[c], slen[c], item0, 1, BUF_USKEL);
+            item(POOL_VD3, down_child[c], BUF_USKEL, parent[c], slen[parent[c]]);
+            add_tasks(OUT_TILES, S->node_rt[c], S->node_kt[c], slen[c], slen[c], item0, 1, BUF_USKEL, fc.u(c), fc.far(c));
         }
         end_op();
     }
@@ -2664,8 +3137,8 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
     for (int v : bfs) {
         if (lch[v] != -1 || !projects(v)) continue;
         const int item0 = (int)S->items.size();
-        item(POOL_VD3, down_a[v], BUF_USKEL, S->node_kt[v], slen[v]);
-        add_tasks(OUT_Y, lm[v], 0, Ddim[lm[v]], Ddim[lm[v]], item0, 1, BUF_W);
+        item(POOL_VD3, down_a[v], BUF_USKEL, v, slen[v]);
+        add_tasks(OUT_Y, lm[v], 0, Ddim[lm[v]], Ddim[lm[v]], item0, 1, BUF_W, -1, fc.near(lm[v]));
     }
     end_op();
 
@@ -2686,8 +3159,8 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
                 if (lch[v] != -1) continue;
                 const int x = lm[v];
                 const int item0 = (int)S->items.size();
-                for (int k : near_in[x]) item(POOL_NEART, neart_a[k], BUF_W, S->leaf_kt[near_x[k]], Ddim[near_x[k]]);
-                add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W);
+                for (int k : near_in[x]) item(POOL_NEART, neart_a[k], BUF_W, near_x[k], Ddim[near_x[k]]);
+                add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W, fc.near(x));
             }
         };
         begin_op(near_with_far ? PH_FARNEAR : PH_FAR, 0, far_parts);
@@ -2695,9 +3168,9 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             if (!projects(c)) continue;
             const int item0 = (int)S->items.size();
             for (int k : far_in[c])
-                if (slen[far_x[k]] > 0) item(POOL_FART, fart_a[k], BUF_WSKEL, S->node_kt[far_x[k]], slen[far_x[k]]);
-            add_tasks(has_down(c) ? OUT_F32 : OUT_TILES, skel_row[c], S->node_kt[c], slen[c], slen[c], item0, 0,
-                      BUF_USKEL);
+                if (slen[far_x[k]] > 0) item(POOL_FART, fart_a[k], BUF_WSKEL, far_x[k], slen[far_x[k]]);
+            add_tasks(has_down(c) ? OUT_F32 : OUT_TILES, S->node_rt[c], S->node_kt[c], slen[c], slen[c], item0, 0,
+                      BUF_USKEL, has_down(c) ? fc.far(c) : fc.u(c));
         }
         if (near_with_far) near_tasks_t();
         end_op();
@@ -2770,6 +3243,7 @@ int launch_count(const Batch *b)
     int n = (int)b->ops.size();
     if (!b->entries.empty()) {
         const std::vector<int> &bn = b->entries.back().bn;
+        if (b->flow_width(bn)) return b->entries.back().flow_w ? 1 : 2;
         for (size_t k = 0; k < bn.size() && k < b->ops.size(); ++k)
             if (b->ops[k].phase != PH_SPLITW && (bn[k] & TILE_CHAIN)) --n;
     }

@@ -453,7 +453,7 @@ class Plan:
 
 class Batch:
     """Several split-BF16 plans evaluated by one merged, graph-captured launch sequence
-    (``mxb_batch_*``); the column-tile widths are tuned by measurement on first use."""
+    (``mxb_batch_*``); beyond 128 columns the launches are tuned by measurement on first use."""
 
     def __init__(self, plans):
         if not plans:
@@ -465,8 +465,8 @@ class Batch:
         self._h = h
 
     def set_one_launch(self, on: bool = True) -> None:
-        """Evaluate the whole batch as one launch with device-side level barriers
-        (MXB_BATCH_ONE_LAUNCH), or as a sequence of level launches (the default)."""
+        """Evaluate the whole batch as one launch whose work units wait on the device for the
+        blocks they read (MXB_BATCH_ONE_LAUNCH), or as a launch sequence (the default)."""
         mode = _lib.BATCH_ONE_LAUNCH if on else _lib.BATCH_LEVEL_LAUNCHES
         check(_lib.load().mxb_batch_set_launch_mode(self._h, mode), "mxb_batch_set_launch_mode")
 
