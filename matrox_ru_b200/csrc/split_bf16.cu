@@ -23,7 +23,7 @@
 //   warps 0 - E-1  : drain every K tile's accumulator into round-to-nearest FP32 registers
 //                    (tcgen05.ld), then write Y (FP64), an FP32 block, or operand tiles
 //   warp E lane 0  : producer -- bulk copies of the A and B part tiles of each K step
-//   warp E+1 lane 0: MMA issuer -- tcgen05.mma M=128, N=BN, K=16, 3 or 6 per 16-K slice, one
+//   warp E+1       : MMA issuer (one elected lane) -- tcgen05.mma M=128, N=BN, K=16, 3 or 6 per 16-K slice, one
 //                    fresh TMEM accumulator (of two or four) per 64-deep K tile
 //   warp E+2       : (single CTAs) publisher -- one device-scope fence and one counter
 //                    increment per unit once all its epilogue warps have written, so no
@@ -357,6 +357,9 @@ __device__ __forceinline__ void transpose8(float (&x)[8], int lane)
 // Beside the stages: the unit and task records of the units in the ring (single CTAs; read from
 // there by the epilogue warps, whose global loads of them cost about 1 us per unit) and the first
 // plans' pointers.
+// Epilogue state of a unit: its OutKind, whether the old output is added, whether the thread's row and
+// its operand chunks exist, whether Y is in the caller's point order.
+constexpr uint32_t MODE_KIND = 3, MODE_ADD = 4, MODE_ROW = 8, MODE_K = 16, MODE_ORDERED = 32;
 constexpr int RING_SLOTS = 16, SMEM_PLANS = 16;
 struct alignas(16) UnitRecord {
     TcUnit unit;
@@ -729,22 +732,32 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             }
         }
     } else if (warp == C::EPI_WARPS + 1) {
-        if (lane == 0 && issuer) {
+        if (issuer) {
             // ---------------- MMA issuer ----------------
+            // The whole warp walks the units, so that addresses and descriptors are warp-uniform, and
+            // one elected lane issues.  With one lane walking alone a 128 x 128 x 16 MMA took 94 - 114
+            // cycles to issue (64 at the tensor core's rate): the couplings of N = 65536 x 1024 on
+            // 128-column tiles went from 1849 to 1772 us, the leaf projections from 231 to 214 us.
             constexpr uint32_t IDESC = tc::idesc_bf16_f32(C::M_MMA, BN);
             constexpr int PA[6] = {0, 0, 1, 0, 1, 2};
             constexpr int PB[6] = {0, 1, 0, 2, 1, 0};
+            const bool leader = tc::elect_one();
             uint32_t g = 0;     // K-tile (stage) counter
             uint32_t ga = 0;    // accumulator-fill counter
-            uint32_t slot = 0;  // ring counter
             bool any = false, stop = false;
-            while (!stop) {
-                int ktiles = 0, up = P, columns = BN;
-                const int u = take_unit(slot, ktiles, &up, &columns);
+            for (uint32_t slot = 0; !stop; ++slot) {
+                const int ri = (int)(slot % RING);
+                const bool got = wait_x(&ufull[ri], (slot / RING) & 1u, abort_word);
+                int u = got ? ring[ri] : -2, v = ring_kt[ri];
+                u = __shfl_sync(0xffffffffu, __all_sync(0xffffffffu, got) ? u : -2, 0);
+                v = __shfl_sync(0xffffffffu, v, 0);
+                __syncwarp();
+                if (leader) arrive_local(&uempty[ri]);
                 if (u < 0) {
                     if (u == -2) raise_abort();
                     break;
                 }
+                const int ktiles = v & 0xFFFFFF, up = (v >> 24) & 3, columns = (v >> 26) * 16;
                 const int nprod = up == 2 ? 3 : 6;
                 const int kc = unit_kchain(up);
                 for (int i = 0; i < ktiles; ++i, ++g) {
@@ -754,9 +767,10 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     const uint32_t use = ga / C::NACC;
                     const bool first = i % kc == 0;
                     const bool last = i % kc == kc - 1 || i == ktiles - 1;
-                    if ((first && !wait_x(&acce[b], (use & 1) ^ 1, abort_word)) ||
-                        !tc::mbar_wait(&full[s], round & 1, abort_word, la.wait_cycles) ||
-                        (PAIR && !wait_x(&pfull[s], round & 1, abort_word))) {
+                    const bool ready = (!first || wait_x(&acce[b], (use & 1) ^ 1, abort_word)) &&
+                                       tc::mbar_wait(&full[s], round & 1, abort_word, la.wait_cycles) &&
+                                       (!PAIR || wait_x(&pfull[s], round & 1, abort_word));
+                    if (!__all_sync(0xffffffffu, ready)) {
                         raise_abort();
                         stop = true;
                         break;
@@ -784,6 +798,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                             }
                         }
                     };
+                    if (leader) {
                     if (columns == BN) {
                         if (C::NPROD == 3 || nprod == 3) issue(std::integral_constant<int, 3>{}, std::true_type{});
                         else issue(std::integral_constant<int, 6>{}, std::true_type{});
@@ -791,23 +806,28 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                         if (C::NPROD == 3 || nprod == 3) issue(std::integral_constant<int, 3>{}, std::false_type{});
                         else issue(std::integral_constant<int, 6>{}, std::false_type{});
                     }
-                    if constexpr (PAIR) {
-                        tc::mma_commit_pair(&empty[s]);
-                        if (last) tc::mma_commit_pair(&accf[b]);
-                    } else {
-                        tc::mma_commit(&empty[s]);
-                        if (last) tc::mma_commit(&accf[b]);
+                    }
+                    if (leader) {
+                        if constexpr (PAIR) {
+                            tc::mma_commit_pair(&empty[s]);
+                            if (last) tc::mma_commit_pair(&accf[b]);
+                        } else {
+                            tc::mma_commit(&empty[s]);
+                            if (last) tc::mma_commit(&accf[b]);
+                        }
                     }
                     if (last) ++ga;
                     any = true;
                 }
             }
-            if (any) {
-                if constexpr (PAIR) tc::mma_commit_pair(doneb);
-                else tc::mma_commit(doneb);
-            } else {
-                tc::mbar_expect_tx(doneb, 0);  // nothing issued: complete the barrier's phase now
-                if constexpr (PAIR) tc::mbar_arrive_remote(tc::peer_smem(doneb, 1));
+            if (leader) {
+                if (any) {
+                    if constexpr (PAIR) tc::mma_commit_pair(doneb);
+                    else tc::mma_commit(doneb);
+                } else {
+                    tc::mbar_expect_tx(doneb, 0);  // nothing issued: complete the barrier's phase now
+                    if constexpr (PAIR) tc::mbar_arrive_remote(tc::peer_smem(doneb, 1));
+                }
             }
         } else if (lane == 0 && PAIR) {
             // ---------------- relay (odd CTA of a pair) ----------------
@@ -944,43 +964,69 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 }
                 tc::acquire_counter(ctr);
             }
+            // What the output needs, in registers before the products are waited for: shared memory
+            // answers late while MMAs read their operands from it (reading the records where they
+            // are used took 600 - 1600 cycles of each unit).  Few registers: the drain needs the rest.
+            uint32_t mode = 0;       // OutKind | MODE_* bits
+            int n1 = 0, n2 = 0;      // Y: leading dimension, columns; else column quads of S, columns
+            float4 *S = nullptr;     // the FP32 far result at (row, col0)
+            uint8_t *out = nullptr;  // Y at (row, col0), or the tile chunk at (k0, col0 + lane % 8)
+            int old_ctr = -1, old_target = 0;  // of the old output, where another unit of this launch writes it
             {
+                const PlanArgs *pa = plan_args(t.plan);
+                const int kind = t.out_kind, M = t.M, nrhs = pa->nrhs;
+                const int r0 = t.m0 + (int)rank * 128 + quarter * 32, r = r0 + lane;
+                const int col0 = un.col * BN + half * C::COLS;
+                const int beta = t.beta == 2 ? pa->beta_arg : t.beta;
+                const bool ordered = ORD && kind == OUT_Y && pa->y_perm;
+                // OUT_TILES: column col0 + 8 g8 + (lane & 7) of this thread's groups: one 128-column tile,
+                // and the same swizzle phase, so a group is 1024 bytes after the one before.  Rows past
+                // the node's K tiles are not written.
+                const int k0 = r0 + (lane & ~7), KTv = (M + 63) / 64;
+                mode = (uint32_t)kind | (beta ? MODE_ADD : 0u) | (r < M ? MODE_ROW : 0u) |
+                       (k0 < KTv * 64 ? MODE_K : 0u) | (ordered ? MODE_ORDERED : 0u);
+                n1 = min(pa->nq - (col0 >> 2), columns >> 2);
+                n2 = columns;
+                if (kind == OUT_F32 || (kind == OUT_TILES && beta)) S = reinterpret_cast<float4 *>(skel_at(pa, t, r, col0));
+                if (kind == OUT_TILES) {
+                    out = pa->buf[t.t_buf] +
+                          ((size_t)t.out_kt * pa->NT + (size_t)(col0 >> 7) * KTv + (k0 >> 6)) * 3 * (size_t)TILE_BYTES +
+                          tc::swizzled_offset((col0 & 127) + (lane & 7), k0 & 63);
+                } else if (kind == OUT_Y && !ordered) {
+                    n1 = t.ldc;
+                    n2 = nrhs - col0;
+                    out = reinterpret_cast<uint8_t *>(pa->Y + pa->yofs[t.c_row] + r + (size_t)col0 * n1);
+                }
+                if (FLOW && la.flow && t.old >= 0) {
+                    old_ctr = FLOW_FIRST + pa->ctr0 + t.old * pa->ncol + un.col;
+                    old_target = t.old_need * C::UNIT_WRITERS;
+                }
                 // The output phase reads old values (Y, the far result) with a few loads in
                 // flight per thread: ask L2 for them now, so the unit's MMAs cover the DRAM
                 // latency.  Lane j takes columns j, j + 32, ... of its warp's 32-row segment
                 // (128 bytes of FP32, 256 of FP64 per column).
-                const PlanArgs *pa = plan_args(t.plan);
-                const int r0 = t.m0 + (int)rank * 128 + quarter * 32;
-                const int c0 = un.col * BN + half * C::COLS;
-                const int beta = t.beta == 2 ? pa->beta_arg : t.beta;
-                const int nrhs = pa->nrhs;
-                const char *f64 = nullptr;
-                if (ORD && t.out_kind == OUT_Y && beta && pa->y_perm) {
+                if (ordered && beta) {
                     // caller point order: each lane asks for its own row's columns when they
                     // are contiguous (one 128-byte line per 16 columns)
-                    const int rl = r0 + lane;
-                    if (rl < t.M && pa->y_cs == 1) {
+                    if (r < M && pa->y_cs == 1) {
                         const char *q = reinterpret_cast<const char *>(
-                            pa->Y + (int64_t)pa->y_perm[pa->tofs[t.c_row] + rl] * pa->y_rs + c0);
-                        const int ncol = min(C::COLS, nrhs - c0);
+                            pa->Y + (int64_t)pa->y_perm[pa->tofs[t.c_row] + r] * pa->y_rs + col0);
+                        const int ncol = min(C::COLS, nrhs - col0);
                         for (int j = 0; j < ncol; j += 16) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + j * 8));
                     }
-                } else if (t.out_kind == OUT_Y && beta) {
-                    f64 = reinterpret_cast<const char *>(pa->Y + pa->yofs[t.c_row] + r0);
-                } else if (t.out_kind == OUT_TILES && beta && r0 < t.M) {
-                    const char *q = reinterpret_cast<const char *>(skel_at(pa, t, r0, c0));
+                } else if (kind == OUT_TILES && beta && r0 < M) {
+                    const char *q = reinterpret_cast<const char *>(S) - lane * 16;
                     for (int j = lane; j < C::COLS; j += 32)  // 4 lines per column quad
-                        if (c0 + (j & ~3) < pa->nq * 4)
+                        if (col0 + (j & ~3) < pa->nq * 4)
                             asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + (size_t)(j >> 2) * 2048 + (j & 3) * 128));
-                }
-                if (r0 < t.M && f64) {
+                } else if (kind == OUT_Y && beta && r0 < M) {
+                    const uint8_t *f64 = out - lane * 8;
                     for (int j = lane; j < C::COLS; j += 32) {
-                        const int cc = c0 + j;
-                        if (cc >= nrhs) break;
+                        if (j >= n2) break;
                         // rows r0 and r0 + 16 (only where they exist)
-                        const char *q = f64 + (size_t)cc * t.ldc * 8;
+                        const uint8_t *q = f64 + (size_t)j * n1 * 8;
                         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q));
-                        if (r0 + 16 < t.M) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + 128));
+                        if (r0 + 16 < M) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + 128));
                     }
                 }
             }
@@ -998,8 +1044,10 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 }
                 tc::fence_after_sync();
                 // 64 columns per load where the registers allow (one wait per 64 columns keeps
-                // the drain short); 128-column halves load 16 at a time to stay clear of spills
-                constexpr int LB = C::COLS == 64 ? 64 : (C::COLS == 32 ? 32 : 16);
+                // the drain short), else 16 at a time to stay clear of spills (32 at a time of
+                // 32 columns spilled 36 - 160 bytes, and N = 65536 x 1024's last down pass took
+                // 258 us against 213)
+                constexpr int LB = C::COLS == 64 ? 64 : 16;
 #pragma unroll
                 for (int c0 = 0; c0 < C::COLS; c0 += LB) {
                     float v[LB];
@@ -1019,34 +1067,32 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                 }
             }
             if (!ok || *abort_word) break;
-            const PlanArgs *pa = plan_args(t.plan);
-            const int nrhs = pa->nrhs;
-            const int r = t.m0 + (int)rank * 128 + quarter * 32 + lane;
-            const int beta = t.beta == 2 ? pa->beta_arg : t.beta;
-            const int col0 = un.col * BN + half * C::COLS;
-            if (FLOW && la.flow && t.old >= 0) {
+            if (FLOW && old_ctr >= 0) {
                 // the old output comes from another unit of this launch: lane 0 waits, then every
                 // lane takes its own acquire of the completed count
-                const int *ctr = la.flow + FLOW_FIRST + pa->ctr0 + t.old * pa->ncol + un.col;
                 int done = 1;
-                if (lane == 0) done = tc::wait_counter(ctr, t.old_need * C::UNIT_WRITERS, abort_word, la.wait_cycles, 64);
+                if (lane == 0) done = tc::wait_counter(la.flow + old_ctr, old_target, abort_word, la.wait_cycles, 64);
                 done = __shfl_sync(0xffffffffu, done, 0);
                 if (!done) {
                     if (lane == 0) raise_abort();
                     break;
                 }
-                tc::acquire_counter(ctr);
+                tc::acquire_counter(la.flow + old_ctr);
             }
             // Y accumulates by reductions at L2 (each element has one writer, ordered after the old
             // value's, so the sum is the same as load, add and store, without waiting for the load)
-            if (columns <= 0 && t.out_kind != OUT_SPLIT) {
+            const int kind = (int)(mode & MODE_KIND);
+            const bool beta = mode & MODE_ADD;
+            if (columns <= 0 && kind != OUT_SPLIT) {
                 // no right-hand sides in this warp's columns
-            } else if (ORD && t.out_kind == OUT_Y && pa->y_perm) {
+            } else if (ORD && (mode & MODE_ORDERED)) {
                 // caller point order: row t of the leaf goes to row perm[t] of Y.  An 8 x 8
                 // transpose inside each group of 8 lanes gives every lane one column of 8
                 // consecutive tree rows, so each access covers 8 columns (64 bytes) of a row, 4
                 // rows per warp instruction, instead of 32 rows.  All lanes take part in the
                 // shuffles; rows past M are masked at the accesses.
+                const PlanArgs *pa = plan_args(t.plan);
+                const int nrhs = pa->nrhs, col0 = un.col * BN + half * C::COLS;
                 const int rg = t.m0 + (int)rank * 128 + quarter * 32 + (lane & ~7);  // group's first row
                 const int rows_ok = t.M - rg;  // rows rg + j with j < rows_ok exist
                 // lane 8g + i holds the element offset of caller row perm[rg + i]; the others
@@ -1069,10 +1115,10 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     }
                     ycol += 8 * ycs;
                 }
-            } else if (t.out_kind == OUT_Y) {
-                if (r < t.M) {
-                    const int ldc = t.ldc, ncol = nrhs - col0;  // in registers: the stores below may alias the record
-                    double *Yb = pa->Y + pa->yofs[t.c_row] + r + (size_t)col0 * ldc;
+            } else if (kind == OUT_Y) {
+                if (mode & MODE_ROW) {
+                    const int ldc = n1, ncol = n2;
+                    double *Yb = reinterpret_cast<double *>(out);
                     if (ncol >= C::COLS && beta) {
 #pragma unroll
                         for (int e = 0; e < C::COLS; ++e, Yb += ldc) add_or_store(Yb, (double)acc[e], 1);
@@ -1082,65 +1128,53 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                             if (e < ncol) add_or_store(Yb, (double)acc[e], beta);
                     }
                 }
-            } else if (t.out_kind == OUT_F32) {
-                if (r < t.M) {
-                    float4 *S = reinterpret_cast<float4 *>(skel_at(pa, t, r, col0));
-                    const int quads = min(pa->nq - (col0 >> 2), columns >> 2);
+            } else if (kind == OUT_F32) {
+                if (mode & MODE_ROW) {
+                    const int quads = n1;
 #pragma unroll
                     for (int q = 0; q < C::COLS / 4; ++q)
                         if (q < quads) S[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
                 }
-            } else if (FLOW && t.out_kind == OUT_SPLIT) {
+            } else if (FLOW && kind == OUT_SPLIT) {
                 // no product: split one column tile of a leaf's W block (FP64) into 3-part operand
                 // tiles, every K tile of the leaf, as split_w_kernel does.  Columns past nrhs and
-                // points past M are zero.  The tile is 128 columns wide, in flow launches BN (the
-                // columns that the unit's counter covers).
-                const int n0 = un.col * (la.flow ? BN : 128), nt = n0 >> 7;
-                const int rows = tile_columns(nrhs, un.col, la.flow ? BN : 128);  // tile rows: right-hand sides
-                const int KTv = (t.M + 63) / 64;
+                // points past M are zero.
+                const PlanArgs *pa = plan_args(t.plan);
+                const int nrhs = pa->nrhs, M = t.M, KTv = (M + 63) / 64;
+                const int n0 = un.col * BN, nt = n0 >> 7;
+                const int rows = tile_columns(nrhs, un.col, BN);  // tile rows: right-hand sides
                 uint8_t *base = pa->buf[t.t_buf] + ((size_t)t.out_kt * pa->NT + (size_t)nt * KTv) * 3 * (size_t)TILE_BYTES;
-                const int tid = threadIdx.x;  // the epilogue warps are warps 0 .. EPI_WARPS - 1
-                constexpr int PER = 1024 / (C::EPI_WARPS * 32);  // 16-byte chunks per thread and K tile
-                const bool ordered = ORD && pa->w_perm;
-                const double *src = ordered ? pa->W : pa->W + pa->wofs[t.c_row];
-                const int32_t *perm = ordered ? pa->w_perm + pa->tofs[t.c_row] : nullptr;
-                for (int kt = 0; kt < KTv; ++kt) {
-                    // all of the thread's loads of the K tile in flight before any split.  Lanes run
-                    // along K in leaf-blocked W, along the right-hand sides in caller order.
-                    double x[PER][8];
+                const bool gather = ORD && pa->w_perm;
+                const double *src = gather ? pa->W : pa->W + pa->wofs[t.c_row];
+                const int32_t *perm = gather ? pa->w_perm + pa->tofs[t.c_row] : nullptr;
+                // 16-byte chunks of a K tile, one at a time per thread (two at 128 columns in flight spilled
+                // the registers of the loops above).  Lanes run along K in leaf-blocked W, along the
+                // right-hand sides in caller order.
+#pragma unroll 1
+                for (int q = threadIdx.x; q < KTv * BN * 8; q += C::EPI_WARPS * 32) {  // (warps 0 .. EPI_WARPS - 1)
+                    const int kt = q / (BN * 8), idx = q % (BN * 8);
+                    if (idx >= rows * 8) continue;
+                    const int c = gather ? idx / rows : idx % 8, n = gather ? idx % rows : idx / 8;
+                    const int k0 = kt * 64 + c * 8;
+                    double x[8];
 #pragma unroll
-                    for (int i = 0; i < PER; ++i) {
-                        const int idx = tid + i * C::EPI_WARPS * 32;
-                        if (idx >= rows * 8) break;
-                        const int c = ordered ? idx / rows : idx % 8, n = n0 + (ordered ? idx % rows : idx / 8);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const int k = kt * 64 + c * 8 + e;
-                            const bool in = n < nrhs && k < t.M;
-                            if (ordered) x[i][e] = in ? src[(int64_t)perm[k] * pa->w_rs + (int64_t)n * pa->w_cs] : 0.0;
-                            else x[i][e] = in ? src[k + (size_t)n * t.ldc] : 0.0;
-                        }
+                    for (int e = 0; e < 8; ++e) {
+                        const bool in = n0 + n < nrhs && k0 + e < M;
+                        if (gather) x[e] = in ? src[(int64_t)perm[k0 + e] * pa->w_rs + (int64_t)(n0 + n) * pa->w_cs] : 0.0;
+                        else x[e] = in ? src[k0 + e + (size_t)(n0 + n) * t.ldc] : 0.0;
                     }
+                    __nv_bfloat16 h[8], m[8], l[8];
 #pragma unroll
-                    for (int i = 0; i < PER; ++i) {
-                        const int idx = tid + i * C::EPI_WARPS * 32;
-                        if (idx >= rows * 8) break;
-                        const int c = ordered ? idx / rows : idx % 8, r = (n0 & 127) + (ordered ? idx % rows : idx / 8);
-                        __nv_bfloat16 h[8], m[8], l[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) tc::split3(x[i][e], h[e], m[e], l[e]);
-                        store_parts(base + (size_t)kt * 3 * TILE_BYTES, 3, r, c, h, m, l);
-                    }
+                    for (int e = 0; e < 8; ++e) tc::split3(x[e], h[e], m[e], l[e]);
+                    store_parts(base + (size_t)kt * 3 * TILE_BYTES, 3, (n0 & 127) + n, c, h, m, l);
                 }
             } else {
                 // OUT_TILES: (optionally) add the FP32 far result, then write this row's values
                 // as 3-part bf16 operand tiles.  The lane holds one K index; a transpose in
                 // groups of 8 lanes gives it 8 consecutive K of one column: one 16-byte chunk
-                // per part.  Rows past M carry zeros (A is zero-padded); rows past the node's
-                // K tiles are not written.
-                if (beta && r < t.M) {
-                    const float4 *S = reinterpret_cast<const float4 *>(skel_at(pa, t, r, col0));
-                    const int quads = min(pa->nq - (col0 >> 2), columns >> 2);
+                // per part.  Rows past M carry zeros (A is zero-padded).
+                if (beta && (mode & MODE_ROW)) {
+                    const int quads = n1;
                     constexpr int QB = C::COLS >= 128 ? 2 : (C::COLS < 32 ? C::COLS / 4 : 8);  // loads in flight
 #pragma unroll
                     for (int q0 = 0; q0 < C::COLS / 4; q0 += QB) {
@@ -1157,14 +1191,6 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                         }
                     }
                 }
-                const int KTv = (t.M + 63) / 64;
-                const int k0 = t.m0 + (int)rank * 128 + quarter * 32 + (lane & ~7);
-                const bool k_ok = k0 < KTv * 64;
-                // column col0 + 8 g8 + (lane & 7) of this thread's groups: one 128-column tile, and
-                // the same swizzle phase, so a group is 1024 bytes after the one before
-                uint8_t *out = pa->buf[t.t_buf] +
-                               ((size_t)t.out_kt * pa->NT + (size_t)(col0 >> 7) * KTv + (k0 >> 6)) * 3 * (size_t)TILE_BYTES +
-                               tc::swizzled_offset((col0 & 127) + (lane & 7), k0 & 63);
 #pragma unroll
                 for (int g8 = 0; g8 < C::COLS / 8; ++g8) {
                     float x[8];
@@ -1173,7 +1199,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     transpose8(x, lane);
                     uint4 vh, vm, vl;
                     tc::split3x8(x, vh, vm, vl);
-                    if (k_ok && g8 * 8 < columns) {
+                    if ((mode & MODE_K) && g8 * 8 < n2) {
                         *reinterpret_cast<uint4 *>(out + g8 * 1024) = vh;
                         *reinterpret_cast<uint4 *>(out + g8 * 1024 + TILE_BYTES) = vm;
                         *reinterpret_cast<uint4 *>(out + g8 * 1024 + 2 * TILE_BYTES) = vl;
@@ -1191,14 +1217,12 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     if (lane == 0 && !(la.stall_level && un.dep0 < 0)) atomicAdd(la.deps + un.sig, 1);
                 }
             } else {
-                // written: the publishing warp counts the unit.  Operand tiles are read by bulk copies.
-                if (t.out_kind == OUT_TILES || t.out_kind == OUT_SPLIT) asm volatile("fence.proxy.async.global;\n" ::: "memory");
+                // written: the publishing warp counts the unit
                 __syncwarp();
-                if (lane == 0) arrive_local(&written[ri]);
-            }
-            if constexpr (!PAIR) {
-                __syncwarp();
-                if (lane == 0) arrive_local(&uempty[ri]);
+                if (lane == 0) {
+                    arrive_local(&written[ri]);
+                    arrive_local(&uempty[ri]);
+                }
             }
         }
     }

@@ -139,6 +139,14 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P1;\n\telect.sync _|P1, 0xffffffff;\n\tselp.b32 %0, 1, 0, P1;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
 // Shared-memory matrix descriptor of a K-major, 128-byte-swizzled tile (8-row groups 1024
 // bytes apart).  Bits: start address >> 4 [0,14), leading byte offset >> 4 [16,30) (unused
 // with this swizzle, 1 by convention), stride byte offset >> 4 [32,46), fixed version 1 at
