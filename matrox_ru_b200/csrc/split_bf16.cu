@@ -2017,11 +2017,12 @@ double Batch::flow_balance(Entry &e, int w) const
 
 // Whether an evaluation takes the flow launch without timing the alternatives: up to FLOW_COLUMNS
 // right-hand sides, where no launch would use a wider tile, and where one SM's work is below FLOW_WORK
-// of the longest path.  It was the faster one by a tenth or more at every size tried (N = 1024 -
-// 131072, 1 - 512 columns: 56 against 72 us at N = 1024 x 128, 521 against 647 us at N = 65536 x 128,
-// 618 against 731 us at N = 30011 x 384, balance 2.9), and timing them all takes 4 - 44 ms of the
-// first evaluation.  Up to FLOW_TRIED it is one of the timed candidates: between them it is 1.18
-// times as fast (N = 65536 x 512 without a near field) to 0.9 times (N = 131072 x 256; 65536 x 512: 0.93).
+// of the longest path.  There it was the faster one at every size tried (N = 1024 - 131072, 1 - 768
+// columns: 69 against 103 us at N = 4096 x 128, 500 against 607 us at N = 65536 x 128, 577 against
+// 671 us at N = 30011 x 384, balance 2.9, 447 against 468 us at N = 16384 x 768, balance 3.2), and
+// timing them all takes 4 - 44 ms of the first evaluation.  Up to FLOW_TRIED it is one of the timed
+// candidates: it takes 0.83 (N = 65536 x 384 without a near field, six products) to 1.08 (N = 16384
+// x 1536) of the separate launches' time.
 constexpr int FLOW_COLUMNS = 128;
 constexpr double FLOW_WORK = 3.5, FLOW_TRIED = 12;
 bool Batch::takes_flow(Entry &e) const
@@ -2031,11 +2032,12 @@ bool Batch::takes_flow(Entry &e) const
 
 // Columns of a flow launch's tiles.  A step of the path is shorter on 64-column tiles and the
 // work smaller on 128-column ones (their A tiles are read for twice the columns): 64 columns
-// below FLOW_NARROW.  N = 4096, leaf 256, 128 columns (balance 0.3): 113 against 146 us; N = 16384,
-// 256 columns (1.6): 240 against 242 us; N = 65536, 128 columns (2.4): 427 against 406 us.
+// below FLOW_NARROW.  N = 16384, 128 columns (balance 0.8): 165 against 188 us; N = 4096 with
+// leaves of 64 points, 256 columns (1.04): 106 against 87 us; N = 65536, 128 columns (2.4): 404 against
+// 379 us.
 int Batch::flow_columns(Entry &e) const
 {
-    constexpr double FLOW_NARROW = 1.3;
+    constexpr double FLOW_NARROW = 1.0;
     if (*std::max_element(e.nrhs.begin(), e.nrhs.end()) <= 64) return 64;
     return flow_balance(e, 64) < FLOW_NARROW ? 64 : 128;
 }
@@ -2603,7 +2605,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
     if (!rc && flow_enabled() && flow_balance(te, 128) < FLOW_TRIED) {
         auto time_all = [&](const std::vector<int> &tiles, float &best) {
             best = 1e30f;
-            for (int rep = 0; rep < 4 && !rc; ++rep) {
+            for (int rep = 0; rep < 2 && !rc; ++rep) {
                 float ms = 0.f;
                 cudaEventRecord(e0, stream);
                 rc = enqueue(te, stream, 0, wait_cycles, tiles, -1);
