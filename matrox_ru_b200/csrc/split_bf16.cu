@@ -1932,20 +1932,24 @@ int Batch::task_parts(const TcTask &t) const
 // each reads.  Returns 1, or 0 where the counters do not fit.
 int Batch::flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const
 {
-    std::map<std::pair<int, int>, int> writer;   // (plan, counter) -> group
-    std::map<std::pair<int, int64_t>, int> last;  // (plan, leaf) -> leaf-down group
+    // the group that raises each counter of a plan (its leaf-down groups, which raise none, after them)
+    std::vector<size_t> first(plans.size() + 1, 0);
     int64_t nctr = 0;
     for (size_t i = 0; i < plans.size(); ++i) {
+        const int n = FlowCounter{plans[i]->nleaf, plans[i]->numnodes}.count();
         e.pa[i].ctr0 = (int32_t)nctr;
         e.pa[i].ncol = (int32_t)ceil_div(e.nrhs[i], w);
-        nctr += (int64_t)FlowCounter{plans[i]->nleaf, plans[i]->numnodes}.count() * e.pa[i].ncol;
+        nctr += (int64_t)n * e.pa[i].ncol;
+        first[i + 1] = first[i] + (size_t)n + (size_t)plans[i]->nleaf;
     }
     if (nctr > 0x3FFFFFFF) return 0;
+    std::vector<int> writer(first.back(), -1);
+    G.reserve(first.back());
     e.nflow = FLOW_FIRST + (int)nctr;
     auto add = [&](int t, int kt, size_t op) {
         const TcTask &tk = tasks[t];
-        int &g = tk.sig >= 0 ? writer.emplace(std::make_pair((int)tk.plan, (int)tk.sig), -1).first->second
-                             : last.emplace(std::make_pair((int)tk.plan, tk.c_row), -1).first->second;
+        const FlowCounter fc{plans[tk.plan]->nleaf, plans[tk.plan]->numnodes};
+        int &g = writer[first[tk.plan] + (tk.sig >= 0 ? tk.sig : fc.count() + (int)tk.c_row)];
         if (g < 0) {
             g = (int)G.size();
             G.emplace_back();
@@ -1971,11 +1975,11 @@ int Batch::flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const
         FlowGroup &g = G[i];
         const TcTask &tk = tasks[g.tasks[0]];
         auto depends = [&](int ctr, int need) {
-            auto it = writer.find(std::make_pair((int)tk.plan, ctr));
-            if (it == writer.end() || (int)G[it->second].tasks.size() != need) return false;
-            if (std::find(g.deps.begin(), g.deps.end(), it->second) == g.deps.end()) {
-                g.deps.push_back(it->second);
-                G[it->second].cons.push_back(i);
+            const int d = writer[first[tk.plan] + ctr];
+            if (d < 0 || (int)G[d].tasks.size() != need) return false;
+            if (std::find(g.deps.begin(), g.deps.end(), d) == g.deps.end()) {
+                g.deps.push_back(d);
+                G[d].cons.push_back(i);
             }
             return true;
         };
