@@ -710,7 +710,7 @@ def main():
     if best == "fp64":
         roof = {"bound": "tensor", "achieved": round(flops / (gms * 1e-3) / 1e12, 3), "peak": round(fp64_peak, 2),
                 "unit": "TFLOP/s", "peak_source": "measured in this run: cuBLAS DGEMM 8192^3 (torch.matmul f64)",
-                "kernel": "gemm_f64_kernel", "flops_counted": "algorithmic FP64 flops (computeFlops)",
+                "kernel": "f64_dataflow_kernel", "flops_counted": "algorithmic FP64 flops (computeFlops)",
                 "per_launch_flops": flops // nl}
     else:
         roof = {"bound": "tensor", "achieved": round(exec_flops[best] / (gms * 1e-3) / 1e12, 3),
