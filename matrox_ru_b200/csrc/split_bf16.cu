@@ -1053,7 +1053,6 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     float v[LB];
                     const uint32_t ta = tmem + lane_base + (uint32_t)(b * BN + half * C::COLS + c0);
                     if constexpr (LB == 64) tc::tmem_ld64(ta, v);
-                    else if constexpr (LB == 32) tc::tmem_ld32(ta, v);
                     else tc::tmem_ld16(ta, v);
 #pragma unroll
                     for (int e = 0; e < LB; ++e) acc[c0 + e] += v[e];
