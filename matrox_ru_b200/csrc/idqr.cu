@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(CL_THREADS, 1) id_cluster_kernel(const IdJob *
         if (lane == 0) vn1[l] = vn2[l] = sqrt(t);
     }
     __syncthreads();
+    if (C > 1) cluster_barrier();  // every block runs before another writes to its shared memory
 
     const int kmax = min(ns, nc);
     int s = min(kmax, max_rank), i0 = 0, slot = 0;

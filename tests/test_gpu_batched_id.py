@@ -135,3 +135,25 @@ def test_batched_id_shapes(torch, count, nr, nc, max_rank):
         piv, P = got[b]
         assert np.array_equal(piv, hpiv), b
         assert float(np.abs(P - hP).max()) <= 1e-8 * max(1.0, float(np.abs(hP).max())), b
+
+
+def test_batched_id_beside_other_work(torch):
+    """Clusters whose blocks start at different times (another stream holds SMs) give what they
+    give on an idle GPU, bit for bit: no block writes to a peer that has not started."""
+    shapes = [(301 + 8 * b, 150 - b) for b in range(12)]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    pool = torch.randn(sum(r * c for r, c in shapes), dtype=torch.float64, device="cuda", generator=g)
+    want = H.batched_id(pool.clone(), shapes, 1e-9, 128)
+    side = torch.cuda.Stream()
+    x = torch.randn(2048, 2048, device="cuda")
+    for _ in range(4):
+        p = pool.clone()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for _ in range(20):
+                y = x @ x
+        got = H.batched_id(p, shapes, 1e-9, 128)
+        for (a, P), (b, Q) in zip(want, got):
+            assert np.array_equal(a, b) and np.array_equal(P, Q)
+    side.synchronize()
