@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
         uint32_t st = 0;
         for (int slot = 0;; ++slot) {
             const int ri = slot % RING;
-            if (!tc::mbar_wait(&ufull[ri], (slot / RING) & 1, abort_word, g.wait_cycles)) {
+            if (!tc::mbar_wait_warp(&ufull[ri], (slot / RING) & 1, abort_word, g.wait_cycles)) {
                 *abort_word = 1;
                 break;
             }
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
             if (beta && kind != F64_TILE_W && un.task.npiece == 1) ok = old_output(un);
             for (int q = 0; q < stages && ok; ++q, ++st) {
                 const int s = st % C::STAGES;
-                if (!tc::mbar_wait(&full[s], (st / C::STAGES) & 1, abort_word, g.wait_cycles)) {
+                if (!tc::mbar_wait_warp(&full[s], (st / C::STAGES) & 1, abort_word, g.wait_cycles)) {
                     ok = false;
                     break;
                 }

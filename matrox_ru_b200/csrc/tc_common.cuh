@@ -71,6 +71,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     return true;
 }
 
+// The same for a whole converged warp, which gets one answer: some lane can see the barrier complete
+// where another's limit runs out, and a lane that left alone would be missed by the warp's next vote
+// or shuffle.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_word,
+                                               long long limit = WAIT_CYCLES)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)))
+        if (__any_sync(0xffffffffu, *abort_word || clock64() - t0 > limit)) return false;
+    return true;
+}
+
 // Bounded wait until a global counter that other CTAs raise reaches `target` (acquire at GPU
 // scope), then a proxy fence so that the bulk copies this thread issues next (async proxy) see
 // the memory those CTAs wrote before raising it.  False when the wait gives up or an abort is

@@ -73,3 +73,26 @@ def test_wait_that_runs_out_reports_timeout(torch, tall):
     want = O.eval_h2b(tall, TW, r)
     assert np.abs(plan.evaluate(w, r).cpu().numpy() - want).max() <= TOL * np.abs(want).max()
     plan.status()
+
+
+@pytest.mark.parametrize("r", [5, 16, 70])
+def test_waits_of_any_limit_end_with_a_status(torch, tall, r):
+    """Limits from nothing to a few polls: some lanes of a warp find a barrier complete where others
+    give up.  Every such evaluation returns, with a timeout or with the product, and the plan
+    computes correctly after it."""
+    TW = np.random.default_rng(r).standard_normal(tall.n * r)
+    w = torch.as_tensor(TW, device="cuda")
+    plan = H.Plan(tall, "fp64")
+    want = O.eval_h2b(tall, TW, r)
+    for limit in (1, 30, 100, 300, 1000, 3000, 10000, 30000):
+        plan.set_test_hooks(0, wait_cycles=limit)
+        got = plan.evaluate(w, r).cpu().numpy()
+        try:
+            plan.status()
+        except _lib.MxbError as e:
+            assert e.code == _lib.MXB_ERR_TIMEOUT
+        else:
+            assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+    plan.set_test_hooks(0)
+    assert np.abs(plan.evaluate(w, r).cpu().numpy() - want).max() <= TOL * np.abs(want).max()
+    plan.status()
