@@ -1033,11 +1033,11 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
             float acc[C::COLS];
 #pragma unroll
             for (int e = 0; e < C::COLS; ++e) acc[e] = 0.f;
-            bool ok = !*abort_word;
+            bool ok = __all_sync(0xffffffffu, !*abort_word);  // (a warp leaves as a whole)
             for (int i = 0; i < fills && ok; ++i, ++g) {
                 const int b = g % C::NACC;
                 const uint32_t use = g / C::NACC;
-                if (!wait_x(&accf[b], use & 1, abort_word)) {
+                if (!__all_sync(0xffffffffu, wait_x(&accf[b], use & 1, abort_word))) {
                     raise_abort();
                     ok = false;
                     break;
@@ -1065,7 +1065,7 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                                       : "memory");
                 }
             }
-            if (!ok || *abort_word) break;
+            if (!ok) break;
             if (FLOW && old_ctr >= 0) {
                 // the old output comes from another unit of this launch: lane 0 waits, then every
                 // lane takes its own acquire of the completed count

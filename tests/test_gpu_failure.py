@@ -129,3 +129,26 @@ def test_one_launch_plan_and_its_level_barrier(torch, small_cases):
     again = plan.evaluate(tw, r).cpu().numpy()
     plan.status()
     assert np.linalg.norm(again - want) / np.linalg.norm(want) <= 1e-5
+
+
+@pytest.mark.parametrize("tile", [64, 128, 256])
+def test_timeout_on_each_column_tile(torch, small_cases, monkeypatch, tile):
+    """A stalled stage in the kernels of every column tile (16 and 8 epilogue warps): all warps of
+    the block leave, the plan reports MXB_ERR_TIMEOUT and then computes correctly."""
+    monkeypatch.setenv("MXB_TC_TILE", str(tile))
+    cds = small_cases["h2b"]
+    r = 200
+    TW = np.random.default_rng(tile).standard_normal(cds.n * r)
+    want = O.eval_h2b(cds, TW, r)
+    plan = H.Plan(cds, "split_bf16")
+    tw = torch.as_tensor(TW, device="cuda")
+    for _ in range(3):
+        plan.set_test_hooks(_lib.DEBUG_STALL_ONE_WAIT, wait_cycles=20_000_000)  # ~10 ms limit
+        plan.evaluate(tw, r)
+        with pytest.raises(_lib.MxbError) as e:
+            plan.status()
+        assert e.value.code == _lib.MXB_ERR_TIMEOUT
+        plan.set_test_hooks(0)
+        got = plan.evaluate(tw, r).cpu().numpy()
+        plan.status()
+        assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-5
