@@ -723,12 +723,13 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     }
                 }
             }
-            // every stage this thread filled must have landed before the CTA may exit
+            // every stage this thread filled must have landed before the CTA may exit, whatever the
+            // limit of the waits above
 #pragma unroll
             for (int s = 0; s < C::STAGES; ++s) {
                 if (!filled[s]) continue;
                 volatile int never = 0;
-                tc::mbar_wait(&full[s], (filled[s] - 1) & 1, &never, la.wait_cycles);
+                tc::mbar_wait(&full[s], (filled[s] - 1) & 1, &never, tc::WAIT_CYCLES);
             }
         }
     } else if (warp == C::EPI_WARPS + 1) {
@@ -1227,10 +1228,14 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
     }
     __syncwarp();
     __syncthreads();
-    // all MMAs must be complete before TMEM is released (bounded, also after an abort)
+    // all MMAs must be complete before TMEM is released (bounded, also after an abort, and by the
+    // full limit where a shorter one was asked for)
     if (threadIdx.x == 0) {
         volatile int never = 0;
-        if (!wait_x(doneb, 0, &never)) *abort_word = 1;
+        bool done;
+        if constexpr (PAIR) done = tc::mbar_wait_cluster(doneb, 0, &never, tc::WAIT_CYCLES);
+        else done = tc::mbar_wait(doneb, 0, &never, tc::WAIT_CYCLES);
+        if (!done) *abort_word = 1;
     }
     __syncthreads();
     if constexpr (PAIR) tc::cluster_sync();  // no traffic between the two CTAs after this point

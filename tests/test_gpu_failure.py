@@ -152,3 +152,31 @@ def test_timeout_on_each_column_tile(torch, small_cases, monkeypatch, tile):
         got = plan.evaluate(tw, r).cpu().numpy()
         plan.status()
         assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-5
+
+
+@pytest.mark.parametrize("flow", ["1", "0"])
+@pytest.mark.parametrize("r", [5, 130])
+def test_waits_of_any_limit_end_with_a_status(torch, small_cases, monkeypatch, flow, r):
+    """Limits from nothing to a few polls, in the flow launch and in separate launches: every
+    evaluation returns (its copies landed, its products done) with a timeout or with the product,
+    and the plan computes correctly after it."""
+    monkeypatch.setenv("MXB_TC_FLOW", flow)
+    cds = small_cases["h2b"]
+    TW = np.random.default_rng(r).standard_normal(cds.n * r)
+    want = O.eval_h2b(cds, TW, r)
+    tw = torch.as_tensor(TW, device="cuda")
+    plan = H.Plan(cds, "split_bf16")
+    plan.evaluate(tw, r)  # tuned without a short limit
+    for limit in (1, 100, 1000, 3000, 10000, 30000):
+        plan.set_test_hooks(0, wait_cycles=limit)
+        got = plan.evaluate(tw, r).cpu().numpy()
+        try:
+            plan.status()
+        except _lib.MxbError as e:
+            assert e.code == _lib.MXB_ERR_TIMEOUT
+        else:
+            assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-5
+    plan.set_test_hooks(0)
+    got = plan.evaluate(tw, r).cpu().numpy()
+    plan.status()
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-5
