@@ -48,7 +48,7 @@ namespace {
 
 enum : int16_t { F64_Y = 0, F64_WSKEL = 1, F64_USKEL = 2, F64_TILE_W = 3 };
 enum { BUF_W = 0, BUF_WSKEL = 1, BUF_USKEL = 2 };
-enum { CTL_CLAIM = 0, CTL_EXIT = 1, CTL_ERR = 2, CTL_FIRST = 16 };
+enum { CTL_CLAIM = 0, CTL_EXIT = 1, CTL_FIRST = 16 };
 
 constexpr int WARPS = 4, THREADS = (WARPS + 1) * 32, RING = 4;
 constexpr int EAGER = 64;  // polls of a node counter before the first pause
@@ -81,7 +81,7 @@ struct Args {
     const F64Task *tasks;
     const F64Item *items;
     double *partial;
-    int *ctl;
+    int *ctl, *err;
     long long wait_cycles;
     int units, ncol, nb, nrhs, beta, nctr;
 };
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
     __syncthreads();
     // the last block out leaves the claim counter and every other counter at zero for the next launch
     if (threadIdx.x == 0) {
-        if (*abort_word) atomicExch(g.ctl + CTL_ERR, MXB_ERR_TIMEOUT);
+        if (*abort_word) atomicExch(g.err, MXB_ERR_TIMEOUT);
         __threadfence();
         *last_cta = atomicAdd(g.ctl + CTL_EXIT, 1) == (int)gridDim.x - 1;
     }
@@ -653,11 +653,16 @@ int f64_create(Plan &p, const double *D, const double *B, const double *VT)
     F64Engine &E = *p.f64;
     const double *src[3] = {D, B, VT};
     const uint64_t len[3] = {p.D_len, p.B_len, p.VT_len};
-    // one allocation for the pools and one for the tiling jobs
-    int rc = p.alloc((void **)&E.pool[0], std::max<uint64_t>(used[0] + used[1] + used[2], 1) * 512);
+    // one allocation for the pools and the error word, and one for the tiling jobs.  The error word
+    // stays where it is until the plan is destroyed: it holds a failure until it is asked for, also
+    // where the workspaces of the failed evaluation have been replaced since.
+    const uint64_t total = used[0] + used[1] + used[2];
+    int rc = p.alloc((void **)&E.pool[0], total * 512 + 512);
     if (rc) return rc;
     E.pool[1] = E.pool[0] + used[0] * 64;
     E.pool[2] = E.pool[1] + used[1] * 64;
+    E.err = reinterpret_cast<int *>(E.pool[0] + total * 64);
+    F64_CUDA(cudaMemset(E.err, 0, sizeof(int)));
     std::vector<PoolJob> all;
     for (const std::vector<PoolJob> &j : jobs) all.insert(all.end(), j.begin(), j.end());
     if (all.empty()) return MXB_OK;
@@ -1077,6 +1082,7 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
     a.items = s->items;
     a.partial = reinterpret_cast<double *>(E.ctl + E.ctl_bytes / sizeof(int));
     a.ctl = E.ctl;
+    a.err = E.err;
     // ~2 s, and longer for evaluations that themselves take that long
     a.wait_cycles = p.debug_wait_cycles > 0 ? p.debug_wait_cycles : tc::WAIT_CYCLES + (long long)(p.flops(nrhs) / 500);
     a.units = s->ntasks * sh.ncol;
@@ -1094,11 +1100,11 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
 
 int f64_status(Plan &p)
 {
-    if (!p.f64 || !p.f64->ctl) return MXB_OK;
+    if (!p.f64 || !p.f64->err) return MXB_OK;
     int h = 0;
-    F64_CUDA(cudaMemcpy(&h, p.f64->ctl + CTL_ERR, sizeof(int), cudaMemcpyDeviceToHost));
+    F64_CUDA(cudaMemcpy(&h, p.f64->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!h) return MXB_OK;
-    F64_CUDA(cudaMemset(p.f64->ctl + CTL_ERR, 0, sizeof(int)));
+    F64_CUDA(cudaMemset(p.f64->err, 0, sizeof(int)));
     F64_CUDA(cudaDeviceSynchronize());
     return fail("an FP64 kernel wait timed out (MXB_ERR_TIMEOUT)", h);
 }

@@ -57,7 +57,8 @@ struct F64Engine {
     double *pool[3] = {nullptr, nullptr, nullptr};  // near, far, projections
     double *buf[3] = {nullptr, nullptr, nullptr};   // W, wskel, uskel sub-blocks
     int64_t buf_nb = 0;                             // column sub-blocks the buffers hold
-    int *ctl = nullptr;                             // claim, exits, error, counters; then partial tiles
+    int *ctl = nullptr;                             // claim, exits, counters; then partial tiles
+    int *err = nullptr;                             // sticky error word, behind the pools
     size_t ctl_bytes = 0, partial_bytes = 0;
     struct Schedule {                               // tasks in claim order for one column count
         bool adjoint = false;

@@ -96,3 +96,24 @@ def test_waits_of_any_limit_end_with_a_status(torch, tall, r):
     plan.set_test_hooks(0)
     assert np.abs(plan.evaluate(w, r).cpu().numpy() - want).max() <= TOL * np.abs(want).max()
     plan.status()
+
+
+def test_timeout_outlives_the_workspaces_it_happened_in(torch, tall):
+    """A timed-out evaluation, then one that needs more counters and partial tiles (the workspaces
+    are replaced) and one in the other direction: status() still reports the first."""
+    rng = np.random.default_rng(2)
+    plan = H.Plan(tall, "fp64")
+    w = torch.as_tensor(rng.standard_normal(tall.n * 8), device="cuda")
+    plan.set_test_hooks(0, wait_cycles=1)
+    plan.evaluate(w, 8)
+    plan.set_test_hooks(0)
+    TW = rng.standard_normal(tall.n * 200)
+    wide = torch.as_tensor(TW, device="cuda")
+    got = plan.evaluate(wide, 200).cpu().numpy()
+    plan.adjoint(wide, 200)
+    want = O.eval_h2b(tall, TW, 200)
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+    with pytest.raises(_lib.MxbError) as e:
+        plan.status()
+    assert e.value.code == _lib.MXB_ERR_TIMEOUT
+    plan.status()
