@@ -248,7 +248,12 @@ MXB_API int32_t mxb_plan_destroy(mxb_plan *plan);
 /* dY (+)= K~ dW on `stream` (a cudaStream_t, 0 = legacy default).  dW / dY are device
  * arrays in the leaf-blocked layout with per-leaf offsets wptr / uptr (host arrays, nleaf
  * entries; NULL = packed: offset of leaf i = (sum of Ddim[<i]) * nrhs).  accumulate = 1
- * adds to dY (H2-b reference semantics), 0 overwrites it.  Asynchronous. */
+ * adds to dY (H2-b reference semantics), 0 overwrites it.  Asynchronous.
+ * An evaluation that has run once (same column count, direction, layout and offsets) can be
+ * captured in the caller's graph, with any operands; others return MXB_ERR_UNSUPPORTED on a
+ * capturing stream.  From then on the plan keeps the workspaces, offsets and task lists that the
+ * graph points to, also those it replaces, until it is destroyed: the graph may be replayed
+ * between any other calls on the plan, not after mxb_plan_destroy. */
 MXB_API int32_t mxb_plan_evaluate(mxb_plan *plan, const double *dW, double *dY, int32_t nrhs,
                           const int32_t *wptr, const int32_t *uptr, int32_t accumulate,
                           void *stream);

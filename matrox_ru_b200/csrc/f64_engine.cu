@@ -978,15 +978,11 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     return MXB_OK;
 }
 
-void free_buffer(Plan &p, void *q, size_t bytes)
-{
-    if (!q) return;
-    cudaFree(q);
-    p.allocations.erase(std::remove(p.allocations.begin(), p.allocations.end(), q), p.allocations.end());
-    p.device_bytes -= std::max<size_t>(bytes, 16);
-}
+// Task lists of a plan, in bytes, above which the oldest go (N = 65536 with leaves of 256 points: 1.4
+// MB each).  Those a caller's graph may replay stay.
+constexpr size_t SCHEDULE_BYTES = 64 << 20;
 
-int schedule_for(Plan &p, bool adjoint, const Shape &sh, F64Engine::Schedule **out)
+int schedule_for(Plan &p, bool adjoint, const Shape &sh, bool capturing, F64Engine::Schedule **out)
 {
     F64Engine &E = *p.f64;
     for (F64Engine::Schedule &s : E.schedules)
@@ -994,6 +990,7 @@ int schedule_for(Plan &p, bool adjoint, const Shape &sh, F64Engine::Schedule **o
             *out = &s;
             return MXB_OK;
         }
+    if (capturing) return refuse_unprepared();
     std::vector<F64Task> tasks;
     std::vector<F64Item> items;
     F64Engine::Schedule s;
@@ -1004,11 +1001,15 @@ int schedule_for(Plan &p, bool adjoint, const Shape &sh, F64Engine::Schedule **o
     if (rc) return rc;
     s.ntasks = (int)tasks.size();
     if ((int64_t)s.ntasks * sh.ncol > 0x3FFFFFFF) return fail("too many work units", MXB_ERR_UNSUPPORTED);
-    if (E.schedules.size() >= 8) {  // a bounded number of column counts is kept
+    const size_t tb = tasks.size() * sizeof(F64Task), ib = items.size() * sizeof(F64Item);
+    s.bytes = tb + ib;
+    size_t held = s.bytes;
+    for (const F64Engine::Schedule &o : E.schedules) held += o.bytes;
+    while (!p.recorded && !E.schedules.empty() && held > SCHEDULE_BYTES) {
+        held -= E.schedules.front().bytes;
         cudaFree(E.schedules.front().tasks);
         E.schedules.erase(E.schedules.begin());
     }
-    const size_t tb = tasks.size() * sizeof(F64Task), ib = items.size() * sizeof(F64Item);
     std::vector<uint8_t> both(tb + ib);
     std::memcpy(both.data(), tasks.data(), tb);
     if (ib) std::memcpy(both.data() + tb, items.data(), ib);
@@ -1040,11 +1041,15 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
     F64Engine &E = *p.f64;
     const int nb = (nrhs + 7) / 8;
     const Shape sh = shape_for(nb);
+    bool capturing = false;
+    int rc = is_capturing(stream, &capturing);
+    if (rc) return rc;
     F64Engine::Schedule *s = nullptr;
-    int rc = schedule_for(p, adjoint, sh, &s);
+    rc = schedule_for(p, adjoint, sh, capturing, &s);
     if (rc) return rc;
     if (nb > E.buf_nb) {
-        free_buffer(p, E.buf[0], (size_t)(E.leaf8_total + 2 * E.node8_total) * E.buf_nb * 512);
+        if (capturing) return refuse_unprepared();
+        p.release(E.buf[0], (size_t)(E.leaf8_total + 2 * E.node8_total) * E.buf_nb * 512);
         E.buf[0] = nullptr;
         E.buf_nb = 0;
         rc = p.alloc((void **)&E.buf[0], (size_t)(E.leaf8_total + 2 * E.node8_total) * nb * 512);
@@ -1059,7 +1064,8 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
     const size_t partial = (size_t)s->slots * sh.ncol * 64 * sh.bn * sizeof(double);
     if (ctl > E.ctl_bytes || partial > E.partial_bytes) {
         const size_t c = std::max(ctl, E.ctl_bytes), q = std::max(partial, E.partial_bytes);
-        free_buffer(p, E.ctl, E.ctl_bytes + E.partial_bytes);
+        if (capturing) return refuse_unprepared();
+        p.release(E.ctl, E.ctl_bytes + E.partial_bytes);
         E.ctl = nullptr;
         E.ctl_bytes = E.partial_bytes = 0;
         rc = p.alloc((void **)&E.ctl, c + q);
@@ -1069,6 +1075,7 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
         E.ctl_bytes = c;
         E.partial_bytes = q;
     }
+    if (capturing) p.record();
     Args a{};
     for (int q = 0; q < 3; ++q) {
         a.pool[q] = E.pool[q];

@@ -65,6 +65,7 @@ struct F64Engine {
         int ncol = 0, bn = 0;
         int ntasks = 0, nctr = 0;
         int64_t slots = 0;                          // partial slots (times ncol)
+        size_t bytes = 0;                           // of tasks and items
         F64Task *tasks = nullptr;                   // followed by the items
         F64Item *items = nullptr;
     };

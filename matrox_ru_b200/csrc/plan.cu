@@ -68,6 +68,39 @@ int Plan::alloc(void **p, size_t bytes)
     return MXB_OK;
 }
 
+void Plan::release(void *q, size_t bytes)
+{
+    if (!q || recorded) return;
+    cudaFree(q);
+    allocations.erase(std::remove(allocations.begin(), allocations.end(), q), allocations.end());
+    device_bytes -= std::max<size_t>(bytes, 16);
+}
+
+void Plan::record()
+{
+    recorded = true;
+    for (int slot = 0; slot < 2; ++slot) {
+        if (ofs[slot] != &ofs_own[slot]) continue;
+        ofs_kept.push_back(std::move(ofs_own[slot]));
+        ofs_own[slot] = Offsets{};
+        ofs[slot] = &ofs_kept.back();
+    }
+}
+
+int is_capturing(cudaStream_t stream, bool *yes)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    MXB_CUDA(cudaStreamIsCapturing(stream, &st));
+    *yes = st != cudaStreamCaptureStatusNone;
+    return MXB_OK;
+}
+
+int refuse_unprepared()
+{
+    set_error("the first evaluation of a column count, direction or layout cannot be captured: evaluate it once before");
+    return MXB_ERR_UNSUPPORTED;
+}
+
 // ---------------------------------------------------------------------------------------
 // validation of the host structure
 // ---------------------------------------------------------------------------------------
@@ -422,8 +455,9 @@ int Plan::create(const mxb_cds_desc &d, int prec, Plan **out)
         if (rc) return rc;
         if (d.VT_len) MXB_CUDA(cudaMemcpy(p->dVT, d.VT, d.VT_len * sizeof(double), cudaMemcpyDefault));
     }
-    rc = p->alloc((void **)&p->dOfs, 4 * (size_t)p->nleaf * sizeof(int32_t));
+    rc = p->alloc((void **)&p->ofs_own[0].dev, 2 * (size_t)p->nleaf * sizeof(int32_t));
     if (rc) return rc;
+    p->ofs_own[1].dev = p->ofs_own[0].dev + p->nleaf;
     if (prec != MXB_PREC_FP64) {
         rc = p->setup_split_bf16(d);
         if (rc) return rc;
@@ -439,12 +473,11 @@ int Plan::create(const mxb_cds_desc &d, int prec, Plan **out)
 void Plan::clear_graphs() { clear_split_graphs(); }
 
 // Per-leaf offsets for one call; packed offsets when the caller passes none.
-int Plan::stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t stream)
+int Plan::stage_offsets(int slot, const int32_t *given, int nrhs, cudaStream_t stream)
 {
-    std::vector<int32_t> &host = ofs_host[slot];
     std::vector<int32_t> want(nleaf);
-    if (ofs) {
-        std::memcpy(want.data(), ofs, sizeof(int32_t) * nleaf);
+    if (given) {
+        std::memcpy(want.data(), given, sizeof(int32_t) * nleaf);
         for (int i = 0; i < nleaf; ++i)
             if (want[i] < 0) return fail("negative leaf offset");
     } else {
@@ -454,12 +487,27 @@ int Plan::stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t str
             want[i] = (int32_t)o;
         }
     }
-    if (want != host) {
-        host = want;
-        MXB_CUDA(cudaMemcpyAsync(dOfs + (size_t)slot * nleaf, host.data(), sizeof(int32_t) * nleaf,
-                                 cudaMemcpyHostToDevice, stream));
+    if (ofs[slot] && ofs[slot]->host == want) return MXB_OK;
+    for (const Offsets &k : ofs_kept)
+        if (k.host == want) {
+            ofs[slot] = &k;
+            return MXB_OK;
+        }
+    Offsets &own = ofs_own[slot];
+    if (own.host != want) {
+        bool capturing = false;
+        int rc = is_capturing(stream, &capturing);
+        if (rc) return rc;
+        if (capturing) return refuse_unprepared();
+        if (!own.dev) {
+            rc = alloc((void **)&own.dev, sizeof(int32_t) * nleaf);
+            if (rc) return rc;
+        }
+        own.host = std::move(want);
+        MXB_CUDA(cudaMemcpyAsync(own.dev, own.host.data(), sizeof(int32_t) * nleaf, cudaMemcpyHostToDevice, stream));
         MXB_CUDA(cudaStreamSynchronize(stream));
     }
+    ofs[slot] = &own;
     return MXB_OK;
 }
 
@@ -485,7 +533,7 @@ int Plan::run(const std::vector<Launch> &L, const double *dW, double *dY, int nr
     rc = stage_offsets(1, yofs, nrhs, stream);
     if (rc) return rc;
     if (precision != MXB_PREC_FP64) return run_split_bf16(L, dW, dY, nrhs, accumulate, stream);
-    return f64_evaluate(*this, &L == &launches_adj, dW, dY, dOfs, dOfs + nleaf, nrhs, accumulate, stream);
+    return f64_evaluate(*this, &L == &launches_adj, dW, dY, ofs[0]->dev, ofs[1]->dev, nrhs, accumulate, stream);
 }
 
 // The caller's point order: perm[t] is the row of W / Y holding tree position t (the `lids`
@@ -541,25 +589,26 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
     }
     const size_t need = (size_t)std::max<int64_t>(n, 1) * nrhs;
     if (need > order_elems) {
+        bool capturing = false;
+        int rc = is_capturing(stream, &capturing);
+        if (rc) return rc;
+        if (capturing) return refuse_unprepared();
         for (double **q : {&dTW, &dTY}) {
-            if (!*q) continue;
-            cudaFree(*q);
-            allocations.erase(std::remove(allocations.begin(), allocations.end(), (void *)*q), allocations.end());
+            release(*q, order_elems * sizeof(double));
             *q = nullptr;
         }
-        device_bytes -= 2 * order_elems * sizeof(double);
         order_elems = 0;
-        int rc = alloc((void **)&dTW, need * sizeof(double));
+        rc = alloc((void **)&dTW, need * sizeof(double));
         if (!rc) rc = alloc((void **)&dTY, need * sizeof(double));
         if (rc) return rc;
         order_elems = need;
     }
     int rc = stage_offsets(0, nullptr, nrhs, stream);  // packed blocks of the leaf-blocked copies
     if (rc) return rc;
-    MXB_CUDA(launch_permute(dTree, dTree + n, dOfs, nleaf, n, dW, dTW, w_rs, w_cs, nrhs, 0, 0, stream));
+    MXB_CUDA(launch_permute(dTree, dTree + n, ofs[0]->dev, nleaf, n, dW, dTW, w_rs, w_cs, nrhs, 0, 0, stream));
     rc = run(L, dTW, dTY, nrhs, nullptr, nullptr, 0, stream);
     if (rc) return rc;
-    MXB_CUDA(launch_permute(dTree, dTree + n, dOfs + nleaf, nleaf, n, dTY, dY, y_rs, y_cs, nrhs, 1, accumulate,
+    MXB_CUDA(launch_permute(dTree, dTree + n, ofs[1]->dev, nleaf, n, dTY, dY, y_rs, y_cs, nrhs, 1, accumulate,
                             stream));
     return MXB_OK;
 }

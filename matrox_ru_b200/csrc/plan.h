@@ -1,6 +1,7 @@
 // Plan object behind the mxb_plan_* C-ABI.
 #pragma once
 #include <cstdint>
+#include <list>
 #include <vector>
 
 #include "matrox_b200.h"
@@ -42,8 +43,19 @@ struct Plan : public mxb_plan {
 
     // ---- device state ----
     double *dD = nullptr, *dB = nullptr, *dVT = nullptr;  // split-BF16: the FP64 CDS while it is being tiled
-    int32_t *dOfs = nullptr;  // 4 x nleaf per-leaf offsets (slots: in, out, spare)
-    std::vector<int32_t> ofs_host[4];
+    // per-leaf offsets of W (slot 0) and Y (slot 1): the set the evaluation uses, and the slot's own
+    // set, which is overwritten by the next offsets
+    struct Offsets {
+        std::vector<int32_t> host;
+        int32_t *dev = nullptr;
+    };
+    Offsets ofs_own[2];
+    std::list<Offsets> ofs_kept;  // of recorded evaluations: never overwritten
+    const Offsets *ofs[2] = {nullptr, nullptr};
+    // An evaluation was recorded in a caller's stream capture.  What its launches point to (offsets,
+    // workspaces, task lists) then stays as it is until the plan is destroyed, so the caller's graph
+    // can be replayed whatever the plan evaluates in between.
+    bool recorded = false;
     // caller point order (mxb_plan_set_permutation): perm (rows_total entries) followed by
     // the first tree position of every leaf (nleaf + 1 entries)
     int32_t *dTree = nullptr;
@@ -62,6 +74,8 @@ struct Plan : public mxb_plan {
     void add_task(std::vector<Task> &tasks, int16_t c_kind, int64_t c_row, int ldc, int M, int item0,
                   int nitem, int16_t beta, int tile);
     int alloc(void **p, size_t bytes);
+    void release(void *q, size_t bytes);  // of alloc; kept until destruction once recorded
+    void record();                        // the evaluation now enqueued is being captured
     int stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t stream);
     int run(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, const int32_t *wofs,
             const int32_t *yofs, int accumulate, cudaStream_t stream);
@@ -84,6 +98,9 @@ struct Plan : public mxb_plan {
 };
 
 const char *last_error();
+// Whether `stream` is being captured; MXB_ERR_CUDA where it cannot be asked.
+int is_capturing(cudaStream_t stream, bool *yes);
+int refuse_unprepared();  // MXB_ERR_UNSUPPORTED: preparing allocates and copies, which a capture cannot hold
 int row_tile_for(int precision);
 int split_bf16_launches(const Plan &p);
 int split_bf16_prepare();

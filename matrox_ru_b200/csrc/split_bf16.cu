@@ -1455,7 +1455,8 @@ struct Batch : public mxb_batch {
     int *dNext = nullptr;  // work-unit counter per op
     int *dLevel = nullptr; // per op: epilogue warps done with its units (chained launches)
     std::vector<void *> allocations;
-    struct Entry {                     // one captured evaluation
+    bool recorded = false;             // see Plan::recorded: what entries hold is then kept
+    struct Entry {                     // one prepared evaluation
         std::vector<const double *> W;
         std::vector<double *> Y;
         std::vector<int> nrhs;
@@ -1493,13 +1494,13 @@ struct Batch : public mxb_batch {
         if (capture_stream) cudaStreamDestroy(capture_stream);
         for (void *p : allocations) cudaFree(p);
     }
-    static void release(Entry &e)
+    void release(Entry &e)
     {
         if (e.exec) cudaGraphExecDestroy(e.exec);
-        if (e.dPlans) cudaFree(e.dPlans);
-        if (e.dUnits) cudaFree(e.dUnits);
-        if (e.dDeps) cudaFree(e.dDeps);
-        if (e.dFlow) cudaFree(e.dFlow);
+        for (void *q : {(void *)e.dPlans, (void *)e.dUnits, (void *)e.dDeps, (void *)e.dFlow}) {
+            if (q && recorded) allocations.push_back(q);
+            else if (q) cudaFree(q);
+        }
         e.dFlow = nullptr;
         e.nflow = 0;
         e.exec = nullptr;
@@ -2372,22 +2373,18 @@ namespace {
 // Column quads of a row tile of the FP32 far results (64-column tiles write whole quads).
 int far_quads(int nrhs) { return 16 * (int)ceil_div(nrhs, 64); }
 
-int split_buffers(Plan &p, SplitBF16 &S, int nrhs)
+int split_buffers(Plan &p, SplitBF16 &S, int nrhs, bool capturing)
 {
     const int NT = 2 * (int)ceil_div(nrhs, 256);  // even: BN = 256 launches read tile pairs
     if (NT <= S.nt_cap && nrhs <= S.nrhs_cap) return MXB_OK;
-    auto release = [&](void *q) {
-        if (!q) return;
-        cudaFree(q);
-        p.allocations.erase(std::remove(p.allocations.begin(), p.allocations.end(), q), p.allocations.end());
-    };
-    release(S.Wt);
-    release(S.wT);
-    release(S.uT);
-    release(S.u32);
+    if (capturing) return refuse_unprepared();
+    const size_t tile3 = 3 * (size_t)TILE_BYTES;
+    p.release(S.Wt, std::max<int64_t>(S.leaf_kt_total, 1) * S.nt_cap * tile3);
+    p.release(S.wT, std::max<int64_t>(S.node_kt_total, 1) * S.nt_cap * tile3);
+    p.release(S.uT, std::max<int64_t>(S.node_kt_total, 1) * S.nt_cap * tile3);
+    p.release(S.u32, std::max<int64_t>(S.node_rt_total, 1) * (size_t)far_quads(S.nrhs_cap) * 512 * sizeof(float));
     S.Wt = S.wT = S.uT = nullptr;
     S.u32 = nullptr;
-    const size_t tile3 = 3 * (size_t)TILE_BYTES;
     int rc = p.alloc((void **)&S.Wt, std::max<int64_t>(S.leaf_kt_total, 1) * NT * tile3);
     if (!rc) rc = p.alloc((void **)&S.wT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
     if (!rc) rc = p.alloc((void **)&S.uT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
@@ -2490,7 +2487,7 @@ int Batch::tune(Entry &e, std::vector<PlanArgs> pa, std::vector<int> &bn, cudaSt
         Plan &p = *plans[i];
         size_t ext = 0;
         for (int l = 0; l < p.nleaf; ++l)
-            ext = std::max<size_t>(ext, (size_t)p.ofs_host[1][l] + (size_t)p.Ddim[l] * e.nrhs[i]);
+            ext = std::max<size_t>(ext, (size_t)p.ofs[1]->host[l] + (size_t)p.Ddim[l] * e.nrhs[i]);
         if (cudaMalloc(&scratch[i], std::max<size_t>(ext, 1) * sizeof(double)) != cudaSuccess)
             rc = batch_fail("autotune scratch allocation failed", MXB_ERR_NOMEM);
         else
@@ -2653,18 +2650,28 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
     if (cur != device) return batch_fail("batch used on a different device than it was created on");
     std::vector<int> nr(nrhs, nrhs + np);
     if (one_launch && order) return batch_fail("the one-launch mode takes leaf-blocked W and Y", MXB_ERR_UNSUPPORTED);
-    bool realloc = false;
+    bool capturing = false, realloc = false;
+    if (int rc = is_capturing(stream, &capturing)) return rc;
     if (buf_gens.size() != (size_t)np) buf_gens.assign(np, -1);
     for (int i = 0; i < np; ++i) {
         if (nr[i] < 1 || !W[i] || !Y[i]) return batch_fail("bad operand or nrhs in batch");
-        int rc = split_buffers(*plans[i], *plans[i]->bf16, nr[i]);
+        int rc = split_buffers(*plans[i], *plans[i]->bf16, nr[i], capturing);
         if (rc) return rc;
         realloc |= plans[i]->bf16->buf_gen != buf_gens[i];
-        buf_gens[i] = plans[i]->bf16->buf_gen;
     }
-    if (realloc) clear();
+    if (realloc) {
+        if (capturing) return refuse_unprepared();
+        for (int i = 0; i < np; ++i) buf_gens[i] = plans[i]->bf16->buf_gen;
+        clear();
+    }
     MXB_CUDA_OR(configure_all_tc());
     Entry *hit = find(W, Y, nr, accumulate, debug_flags, order);
+    // preparing allocates, and uploads from temporary host memory: not while the stream captures
+    if (capturing && !hit) return refuse_unprepared();
+    if (capturing) {
+        recorded = true;
+        for (Plan *p : plans) p->record();
+    }
     if (!hit) {
         if (entries.size() >= 8) {
             release(entries.front());
@@ -2687,8 +2694,8 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
             pa[i].buf[BUF_USKEL] = S.uT;
             pa[i].W = W[i];
             pa[i].Y = Y[i];
-            pa[i].wofs = p.dOfs;
-            pa[i].yofs = p.dOfs + p.nleaf;
+            pa[i].wofs = p.ofs[0]->dev;
+            pa[i].yofs = p.ofs[1]->dev;
             pa[i].skel = S.u32;
             pa[i].NT = S.nt_cap;
             pa[i].nrhs = nr[i];
@@ -2702,13 +2709,6 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
                 pa[i].y_rs = order[i].y_rs;
                 pa[i].y_cs = order[i].y_cs;
             }
-        }
-        // preparing allocates, and uploads from temporary host memory: not while the stream captures
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        MXB_CUDA_OR(cudaStreamIsCapturing(stream, &cap));
-        if (cap != cudaStreamCaptureStatusNone) {
-            return batch_fail("the first evaluation of these operands cannot be captured: evaluate them once before",
-                              MXB_ERR_UNSUPPORTED);
         }
         // several plans: their table, on the evaluation stream ahead of the graph launch that reads it
         cudaError_t err = np > 1 ? cudaMalloc(&e.dPlans, np * sizeof(PlanArgs)) : cudaSuccess;
@@ -2786,6 +2786,8 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
         PlanArgs &pa = hit->pa[0];
         pa.W = W[0];
         pa.Y = Y[0];
+        pa.wofs = plans[0]->ofs[0]->dev;
+        pa.yofs = plans[0]->ofs[1]->dev;
         pa.beta_arg = accumulate ? 1 : 0;
         if (order) {
             pa.w_perm = pa.y_perm = order[0].perm;
@@ -2814,7 +2816,9 @@ Batch::Entry *Batch::find(const double *const *W, double *const *Y, const std::v
             same = a.perm == b.perm && a.tofs == b.tofs && a.w_rs == b.w_rs && a.w_cs == b.w_cs && a.y_rs == b.y_rs &&
                    a.y_cs == b.y_cs;
         }
-        for (size_t i = 0; same && i < plans.size(); ++i) same = e.W[i] == W[i] && e.Y[i] == Y[i];
+        for (size_t i = 0; same && i < plans.size(); ++i)
+            same = e.W[i] == W[i] && e.Y[i] == Y[i] && e.pa[i].wofs == plans[i]->ofs[0]->dev &&
+                   e.pa[i].yofs == plans[i]->ofs[1]->dev;
         if (same) hit = &e;
     }
     return hit;
