@@ -533,6 +533,7 @@ __global__ void __launch_bounds__(256) f64_tile_pool_kernel(const PoolJob *__res
 
 int fail(const std::string &m, int code = MXB_ERR_CUDA)
 {
+    (void)cudaGetLastError();  // reported here, not by the next launch
     set_error(m);
     return code;
 }

@@ -60,6 +60,8 @@ int Plan::alloc(void **p, size_t bytes)
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
+        *p = nullptr;
+        (void)cudaGetLastError();  // not for the check behind the next launch
         set_error(std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
         return e == cudaErrorMemoryAllocation ? MXB_ERR_NOMEM : MXB_ERR_CUDA;
     }

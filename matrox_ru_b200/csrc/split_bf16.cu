@@ -1400,6 +1400,7 @@ struct Op {             // one op of one plan
 
 int batch_fail(const std::string &m, int code = MXB_ERR_ARG)
 {
+    if (code != MXB_ERR_ARG) (void)cudaGetLastError();  // reported here, not by the next launch
     set_error(m);
     return code;
 }
@@ -2379,17 +2380,27 @@ int split_buffers(Plan &p, SplitBF16 &S, int nrhs, bool capturing)
     if (NT <= S.nt_cap && nrhs <= S.nrhs_cap) return MXB_OK;
     if (capturing) return refuse_unprepared();
     const size_t tile3 = 3 * (size_t)TILE_BYTES;
-    p.release(S.Wt, std::max<int64_t>(S.leaf_kt_total, 1) * S.nt_cap * tile3);
-    p.release(S.wT, std::max<int64_t>(S.node_kt_total, 1) * S.nt_cap * tile3);
-    p.release(S.uT, std::max<int64_t>(S.node_kt_total, 1) * S.nt_cap * tile3);
-    p.release(S.u32, std::max<int64_t>(S.node_rt_total, 1) * (size_t)far_quads(S.nrhs_cap) * 512 * sizeof(float));
-    S.Wt = S.wT = S.uT = nullptr;
-    S.u32 = nullptr;
-    int rc = p.alloc((void **)&S.Wt, std::max<int64_t>(S.leaf_kt_total, 1) * NT * tile3);
-    if (!rc) rc = p.alloc((void **)&S.wT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
-    if (!rc) rc = p.alloc((void **)&S.uT, std::max<int64_t>(S.node_kt_total, 1) * NT * tile3);
-    if (!rc) rc = p.alloc((void **)&S.u32, std::max<int64_t>(S.node_rt_total, 1) * (size_t)far_quads(nrhs) * 512 * sizeof(float));
-    if (rc) return rc;
+    auto leaf_tiles = [&](int nt) { return std::max<int64_t>(S.leaf_kt_total, 1) * nt * tile3; };
+    auto node_tiles = [&](int nt) { return std::max<int64_t>(S.node_kt_total, 1) * nt * tile3; };
+    auto far_results = [&](int r) { return std::max<int64_t>(S.node_rt_total, 1) * (size_t)far_quads(r) * 512 * sizeof(float); };
+    auto release = [&](int nt, int r) {
+        p.release(S.Wt, leaf_tiles(nt));
+        p.release(S.wT, node_tiles(nt));
+        p.release(S.uT, node_tiles(nt));
+        p.release(S.u32, far_results(r));
+        S.Wt = S.wT = S.uT = nullptr;
+        S.u32 = nullptr;
+        S.nt_cap = S.nrhs_cap = 0;
+    };
+    release(S.nt_cap, S.nrhs_cap);
+    int rc = p.alloc((void **)&S.Wt, leaf_tiles(NT));
+    if (!rc) rc = p.alloc((void **)&S.wT, node_tiles(NT));
+    if (!rc) rc = p.alloc((void **)&S.uT, node_tiles(NT));
+    if (!rc) rc = p.alloc((void **)&S.u32, far_results(nrhs));
+    if (rc) {
+        release(NT, nrhs);
+        return rc;
+    }
     S.nt_cap = NT;
     S.nrhs_cap = nrhs;
     ++S.buf_gen;
