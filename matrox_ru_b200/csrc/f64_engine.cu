@@ -464,14 +464,18 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
                     double *buf = kind == F64_WSKEL ? g.buf[BUF_WSKEL] : g.buf[BUF_USKEL];
                     double *row = buf + ((un.task.out + un.task.r8 + mb) * (int64_t)g.nb + n8_0 + jb) * 64;
                     const int e0 = b_elem(fr, 2 * fa), e1 = b_elem(fr, 2 * fa + 1);
+                    // rows past the block are K padding of the units that read it: zero, not the sum
+                    // of zeros times what may be infinite
+                    const int left = un.task.rows - (un.task.r8 + mb) * 8 - fr;
 #pragma unroll
                     for (int i = 0; i < C::MI; ++i, row += (size_t)g.nb * 64) {
                         if (i >= mi) break;
+                        const bool in = 8 * i < left;
 #pragma unroll
                         for (int j = 0; j < C::NJ; ++j)
                             if (j < nj) {
-                                row[j * 64 + e0] = acc[i][j][0];
-                                row[j * 64 + e1] = acc[i][j][1];
+                                row[j * 64 + e0] = in ? acc[i][j][0] : 0.0;
+                                row[j * 64 + e1] = in ? acc[i][j][1] : 0.0;
                             }
                     }
                 }

@@ -1,6 +1,8 @@
 """GPU: the FP64 dataflow launch at the edges of its column tiles (8, 16 and 32 wide variants), with
 sums cut along K, odd ranks and leaves, operands that are only 8-byte aligned, and a wait that
 runs out."""
+import copy
+
 import numpy as np
 import pytest
 
@@ -116,4 +118,31 @@ def test_timeout_outlives_the_workspaces_it_happened_in(torch, tall):
     with pytest.raises(_lib.MxbError) as e:
         plan.status()
     assert e.value.code == _lib.MXB_ERR_TIMEOUT
+    plan.status()
+
+
+@pytest.mark.parametrize("r", [5, 16, 40])
+@pytest.mark.parametrize("name", ["hss", "h2b", "ragged"])
+def test_infinities_stay_infinities(torch, small_cases, name, r):
+    """Ranks and leaves off the multiples of 8 on positive blocks: an infinite right-hand side gives
+    infinities, as the oracle's loops do, and NaN only where it gives NaN (the padding of the 8 x 8
+    sub-blocks multiplies nothing that is not finite)."""
+    cds = copy.copy(small_cases[name])
+    for pool in ("D", "B", "VT"):
+        setattr(cds, pool, np.abs(getattr(cds, pool)) + 0.125)
+    TW = np.random.default_rng(r).standard_normal((cds.n, r))
+    TW[3, 0], TW[-2, 1], TW[5, 2], TW[5, 3] = np.inf, -np.inf, np.nan, 1e307
+    lo = cds.leaf_lids_offset
+    TW = np.concatenate([TW[lo[i]:lo[i + 1]].reshape(-1, order="F") for i in range(cds.nleaf)])
+    plan = H.Plan(cds, "fp64")
+    w = torch.as_tensor(TW, device="cuda")
+    with np.errstate(all="ignore"):
+        for call, want in ((plan.evaluate, O.eval_h2b(cds, TW, r)), (plan.adjoint, O.adjoint(cds, TW, r))):
+            got = call(w, r).cpu().numpy()
+            assert np.isinf(want).any() and np.isnan(want).any()
+            assert np.array_equal(np.isnan(got), np.isnan(want))
+            assert np.array_equal(np.isposinf(got), np.isposinf(want))
+            assert np.array_equal(np.isneginf(got), np.isneginf(want))
+            ok = np.isfinite(want)
+            assert np.abs(got[ok] - want[ok]).max() <= TOL * np.abs(want[ok]).max()
     plan.status()
