@@ -112,10 +112,14 @@ struct TcTask {
     int16_t beta;    // 0 overwrite, 1 accumulate (OUT_TILES: add the FP32 block), 2 plan's arg
     int32_t t_buf;   // BBuf that OUT_TILES writes
     // flow launches: the plan's counter raised once the tile is written, and the one to reach
-    // before the old output (Y, the far result) is read back (-1: none), with its row tiles
+    // before the old output (Y, the far result) is read back (-1: none), with its row tiles.  A Y
+    // block that is no product of its own leaf's W waits for the split of that W (old_need
+    // NEED_OWN_W): Y may be W.
     int32_t sig, old, old_need, pad;
 };
 static_assert(sizeof(TcTask) == 64, "TcTask layout");
+
+constexpr int NEED_OWN_W = -1;
 
 // Counters of one plan in a flow launch (times its column tiles, + column tile): per leaf W split
 // and near field written; per node wskel, far result and uskel written.
@@ -998,9 +1002,9 @@ __global__ void __launch_bounds__(TcCfg<P, BN, STAGES_, PAIR>::THREADS, 1) tc_ge
                     n2 = nrhs - col0;
                     out = reinterpret_cast<uint8_t *>(pa->Y + pa->yofs[t.c_row] + r + (size_t)col0 * n1);
                 }
-                if (FLOW && la.flow && t.old >= 0) {
+                if (FLOW && la.flow && t.old >= 0 && !(t.old_need == NEED_OWN_W && la.skip_w)) {
                     old_ctr = FLOW_FIRST + pa->ctr0 + t.old * pa->ncol + un.col;
-                    old_target = t.old_need * C::UNIT_WRITERS;
+                    old_target = (t.old_need == NEED_OWN_W ? 1 : t.old_need) * C::UNIT_WRITERS;
                 }
                 // The output phase reads old values (Y, the far result) with a few loads in
                 // flight per thread: ask L2 for them now, so the unit's MMAs cover the DRAM
@@ -1994,7 +1998,8 @@ int Batch::flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const
             if (it.dep < 0 || (it.b_buf == BUF_W && !e.flow_w)) continue;
             if (!depends(it.dep, it.need)) return 0;
         }
-        if (tk.old >= 0 && !depends(tk.old, tk.old_need)) return 0;
+        if (tk.old >= 0 && tk.old_need != NEED_OWN_W && !depends(tk.old, tk.old_need)) return 0;
+        if (tk.old >= 0 && tk.old_need == NEED_OWN_W && e.flow_w && !depends(tk.old, 1)) return 0;
     }
     return 1;
 }
@@ -3092,6 +3097,11 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             S->tasks.push_back(t);
         }
     };
+    auto add_near = [&](int leaf, int item0, bool own) {  // own: W of the leaf itself is an input
+        const size_t first = S->tasks.size();
+        add_tasks(OUT_Y, leaf, 0, Ddim[leaf], Ddim[leaf], item0, 2, BUF_W, fc.near(leaf), own ? -1 : fc.w(leaf));
+        for (size_t t = first; t < S->tasks.size() && !own; ++t) S->tasks[t].old_need = NEED_OWN_W;
+    };
     // B from buffer b_buf of leaf (W) or node `from`, whose K is K
     auto item = [&](int a_pool, uint64_t a_off, int b_buf, int from, int K) {
         TcItem it{};
@@ -3150,8 +3160,12 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
             if (lch[v] != -1) continue;
             const int x = lm[v];
             const int item0 = (int)S->items.size();
-            for (int k : near_out[x]) item(POOL_NEAR, near_a[k], BUF_W, near_y[k], Ddim[near_y[k]]);
-            add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W, fc.near(x));
+            bool own = false;
+            for (int k : near_out[x]) {
+                item(POOL_NEAR, near_a[k], BUF_W, near_y[k], Ddim[near_y[k]]);
+                own |= near_y[k] == x;
+            }
+            add_near(x, item0, own);
         }
     };
     const bool near_with_far = near_parts == far_parts;
@@ -3208,8 +3222,12 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
                 if (lch[v] != -1) continue;
                 const int x = lm[v];
                 const int item0 = (int)S->items.size();
-                for (int k : near_in[x]) item(POOL_NEART, neart_a[k], BUF_W, near_x[k], Ddim[near_x[k]]);
-                add_tasks(OUT_Y, x, 0, Ddim[x], Ddim[x], item0, 2, BUF_W, fc.near(x));
+                bool own = false;
+                for (int k : near_in[x]) {
+                    item(POOL_NEART, neart_a[k], BUF_W, near_x[k], Ddim[near_x[k]]);
+                    own |= near_x[k] == x;
+                }
+                add_near(x, item0, own);
             }
         };
         begin_op(near_with_far ? PH_FARNEAR : PH_FAR, 0, far_parts);

@@ -1,6 +1,8 @@
 """GPU: split-BF16 evaluations in one flow launch (every pass in one launch, units waiting on
 per-node counters) against the same plans with a launch per pass.  The products, their order and
 the splits are the same, so results are bit-identical at every column count and layout."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -111,4 +113,24 @@ def test_replay_of_a_captured_evaluation(torch, small_cases, precision):
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(Ys, plan.evaluate(Ws, r))
+    plan.status()
+
+
+@pytest.mark.parametrize("hooks", [0, _lib.DEBUG_ONE_LAUNCH])
+def test_in_place_without_diagonal_blocks(torch, small_cases, hooks):
+    """Y = W on near lists without a leaf's own block: a Y block is written once the W it replaces
+    has been split, as with a launch per pass."""
+    full, r = small_cases["h2b"], 100
+    keep = np.flatnonzero((full.npairx != full.npairy) & (full.npairx % 2 == 0))
+    cds = dataclasses.replace(full, npairx=full.npairx[keep], npairy=full.npairy[keep], Dptr=full.Dptr[keep])
+    plan = H.Plan(cds, "split_bf16", adjoint=True)
+    plan.set_test_hooks(hooks)
+    W = torch.randn(cds.n * r, dtype=torch.float64, device="cuda")
+    for call in (plan.evaluate, plan.adjoint):
+        want = call(W, r).clone()
+        assert plan.info()["launches"] == 1
+        for _ in range(20):
+            x = W.clone()
+            call(x, r, out=x)
+            assert torch.equal(x, want)
     plan.status()
