@@ -506,16 +506,15 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
     }
 }
 
-// CDS pool (column-major blocks) -> sub-blocks, one job per block.
+// CDS blocks (column-major) -> sub-blocks, one job per block.
 struct PoolJob {
-    uint64_t src;  // element offset
-    uint64_t dst;  // sub-block offset
+    const double *src;  // device address
+    uint64_t dst;       // sub-block offset from the first pool
     int32_t ld, rows, cols, pad;
 };
 
 // A warp writes four sub-blocks (32 rows of 8 columns) at a time: reads of 32 consecutive rows.
-__global__ void __launch_bounds__(256) f64_tile_pool_kernel(const PoolJob *__restrict__ jobs, const double *__restrict__ src,
-                                                            double *__restrict__ dst)
+__global__ void __launch_bounds__(256) f64_tile_pool_kernel(const PoolJob *__restrict__ jobs, double *__restrict__ dst)
 {
     const PoolJob j = jobs[blockIdx.x];
     const int m8 = (j.rows + 7) >> 3, k8 = (j.cols + 7) >> 3, mq = (m8 + 3) >> 2;
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(256) f64_tile_pool_kernel(const PoolJob *__res
         double v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            v[e] = (r < j.rows && k * 8 + e < j.cols) ? src[j.src + (size_t)r + (size_t)(k * 8 + e) * j.ld] : 0.0;
+            v[e] = (r < j.rows && k * 8 + e < j.cols) ? j.src[(size_t)r + (size_t)(k * 8 + e) * j.ld] : 0.0;
         if (r < m8 * 8) {
             double *o = dst + (j.dst + (uint64_t)k * m8 + (r >> 3)) * 64 + (r & 7) * 8;
 #pragma unroll
@@ -605,8 +604,15 @@ struct Group {
 
 namespace {
 
-// Where every block of the CDS goes (host only), and the copies that put it there.
-void layout(Plan &p, std::vector<PoolJob> (&jobs)[3], uint64_t (&used)[3])
+// Where every block of the CDS goes (host only), and where it comes from.
+struct BlockSource {
+    uint64_t src;  // element offset in the caller's pool
+    uint64_t dst;  // sub-block offset in the pool
+    int32_t ld, rows, cols;
+    uint64_t end() const { return src + (uint64_t)(cols - 1) * ld + rows; }
+};
+
+void layout(Plan &p, std::vector<BlockSource> (&blocks)[3], uint64_t (&used)[3])
 {
     F64Engine &E = *(p.f64 = new F64Engine());
     auto ceil8 = [](int64_t v) { return (int32_t)((v + 7) / 8); };
@@ -616,7 +622,7 @@ void layout(Plan &p, std::vector<PoolJob> (&jobs)[3], uint64_t (&used)[3])
         b.m8 = ceil8(rows);
         b.k8 = ceil8(cols);
         used[pool] += (uint64_t)b.m8 * b.k8;
-        if (rows > 0 && cols > 0) jobs[pool].push_back(PoolJob{src, b.off, ld, rows, cols, 0});
+        if (rows > 0 && cols > 0) blocks[pool].push_back(BlockSource{src, b.off, ld, rows, cols});
         return b;
     };
     for (size_t k = 0; k < p.near_x.size(); ++k)
@@ -650,15 +656,18 @@ void layout(Plan &p, std::vector<PoolJob> (&jobs)[3], uint64_t (&used)[3])
 
 }  // namespace
 
+// Device memory for the tiling besides the pools, at most: pools on the host go through it piece by
+// piece (a block larger than it alone), so a plan needs little more than its own size.
+constexpr size_t STAGING_BYTES = 64 << 20;
+
 int f64_create(Plan &p, const double *D, const double *B, const double *VT)
 {
-    std::vector<PoolJob> jobs[3];
+    std::vector<BlockSource> blocks[3];
     uint64_t used[3] = {0, 0, 0};
-    layout(p, jobs, used);
+    layout(p, blocks, used);
     F64Engine &E = *p.f64;
     const double *src[3] = {D, B, VT};
-    const uint64_t len[3] = {p.D_len, p.B_len, p.VT_len};
-    // one allocation for the pools and the error word, and one for the tiling jobs.  The error word
+    // one allocation for the pools and the error word, and one for the tiling.  The error word
     // stays where it is until the plan is destroyed: it holds a failure until it is asked for, also
     // where the workspaces of the failed evaluation have been replaced since.
     const uint64_t total = used[0] + used[1] + used[2];
@@ -668,43 +677,72 @@ int f64_create(Plan &p, const double *D, const double *B, const double *VT)
     E.pool[2] = E.pool[1] + used[1] * 64;
     E.err = reinterpret_cast<int *>(E.pool[0] + total * 64);
     F64_CUDA(cudaMemset(E.err, 0, sizeof(int)));
-    std::vector<PoolJob> all;
-    for (const std::vector<PoolJob> &j : jobs) all.insert(all.end(), j.begin(), j.end());
-    if (all.empty()) return MXB_OK;
-    PoolJob *dj = nullptr;
-    double *copy[3] = {nullptr, nullptr, nullptr};
-    cudaError_t e = cudaMalloc(&dj, all.size() * sizeof(PoolJob));
-    if (e == cudaSuccess) e = cudaMemcpy(dj, all.data(), all.size() * sizeof(PoolJob), cudaMemcpyHostToDevice);
-    size_t first = 0;
-    for (int q = 0; q < 3 && e == cudaSuccess; first += jobs[q++].size()) {
-        if (jobs[q].empty()) continue;
-        // the caller's pool where this device holds it, else a copy for the time of the tiling
-        const double *dev = nullptr;
+    // pieces: runs of blocks whose part of the caller's pool fits the staging, several pools together
+    // where they do.  The caller's pool is read in place where this device holds it.
+    struct Copy {
+        const double *from;
+        size_t to, len;  // elements
+    };
+    struct Piece {
+        std::vector<Copy> copies;
+        size_t job0, jobs;
+    };
+    std::vector<PoolJob> jobs;
+    std::vector<Piece> pieces(1, Piece{{}, 0, 0});
+    std::vector<std::pair<const double *, uint64_t>> from;  // per job: the pool (null: the staging), and where in it
+    size_t fill = 0, staging = 0;
+    uint64_t first = 0;        // of the pool's sub-blocks
+    for (int q = 0; q < 3; first += used[q++]) {
+        std::vector<BlockSource> &bl = blocks[q];
         cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, src[q]) != cudaSuccess) (void)cudaGetLastError();
-        else if (at.type == cudaMemoryTypeDevice && at.device == p.device) dev = src[q];
-        if (!dev) {
-            if (q > 0) {  // at most one copy at a time
-                e = cudaDeviceSynchronize();
-                if (copy[q - 1]) cudaFree(copy[q - 1]);
-                copy[q - 1] = nullptr;
+        bool here = false;
+        if (!bl.empty() && cudaPointerGetAttributes(&at, src[q]) != cudaSuccess) (void)cudaGetLastError();
+        else here = at.type == cudaMemoryTypeDevice && at.device == p.device;
+        if (!here)
+            std::sort(bl.begin(), bl.end(), [](const BlockSource &a, const BlockSource &b) { return a.src < b.src; });
+        for (size_t i = 0; i < bl.size();) {
+            size_t n = 1;
+            uint64_t end = bl[i].end();
+            const size_t room = STAGING_BYTES / sizeof(double);
+            auto joins = [&](uint64_t e) { return here || std::max(end, e) - bl[i].src <= room; };
+            while (i + n < bl.size() && joins(bl[i + n].end())) end = std::max(end, bl[i + n++].end());
+            if (!here) {
+                const size_t len = (size_t)(end - bl[i].src);
+                if (fill && fill + len > room) {
+                    pieces.push_back(Piece{{}, jobs.size(), 0});
+                    fill = 0;
+                }
+                pieces.back().copies.push_back(Copy{src[q] + bl[i].src, fill, len});
             }
-            if (e == cudaSuccess) e = cudaMalloc(&copy[q], len[q] * sizeof(double));
-            if (e == cudaSuccess) e = cudaMemcpy(copy[q], src[q], len[q] * sizeof(double), cudaMemcpyDefault);
-            if (e != cudaSuccess) break;
-            dev = copy[q];
+            for (size_t k = i; k < i + n; ++k) {
+                jobs.push_back(PoolJob{nullptr, first + bl[k].dst, bl[k].ld, bl[k].rows, bl[k].cols, 0});
+                from.push_back({here ? src[q] : nullptr, here ? bl[k].src : fill + (bl[k].src - bl[i].src)});
+            }
+            pieces.back().jobs += n;
+            if (!here) {
+                fill += (size_t)(end - bl[i].src);
+                staging = std::max(staging, fill);
+            }
+            i += n;
         }
-        f64_tile_pool_kernel<<<dim3((unsigned)jobs[q].size(), 4), 256>>>(dj + first, dev, E.pool[q]);
+    }
+    if (jobs.empty()) return MXB_OK;
+    const size_t job_bytes = (jobs.size() * sizeof(PoolJob) + 255) / 256 * 256;
+    uint8_t *work = nullptr;
+    cudaError_t e = cudaMalloc(&work, job_bytes + staging * sizeof(double));
+    double *stage = reinterpret_cast<double *>(work + job_bytes);
+    for (size_t k = 0; k < jobs.size(); ++k) jobs[k].src = (from[k].first ? from[k].first : stage) + from[k].second;
+    if (e == cudaSuccess) e = cudaMemcpy(work, jobs.data(), jobs.size() * sizeof(PoolJob), cudaMemcpyHostToDevice);
+    for (const Piece &pc : pieces) {  // (on the legacy stream: a piece's copies wait for the kernel before)
+        for (const Copy &c : pc.copies)
+            if (e == cudaSuccess) e = cudaMemcpy(stage + c.to, c.from, c.len * sizeof(double), cudaMemcpyDefault);
+        if (e != cudaSuccess || !pc.jobs) continue;
+        f64_tile_pool_kernel<<<dim3((unsigned)pc.jobs, 4), 256>>>(reinterpret_cast<PoolJob *>(work) + pc.job0, E.pool[0]);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (dj) cudaFree(dj);
-    for (double *c : copy)
-        if (c) cudaFree(c);
-    if (e == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();
-        return fail("tiling the CDS: out of device memory", MXB_ERR_NOMEM);
-    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+    if (work) cudaFree(work);
+    if (e == cudaErrorMemoryAllocation) return fail("tiling the CDS: out of device memory", MXB_ERR_NOMEM);
     if (e != cudaSuccess) return fail(std::string("tiling the CDS: ") + cudaGetErrorString(e));
     return MXB_OK;
 }
@@ -1163,9 +1201,9 @@ extern "C" int32_t mxb_debug_f64_schedule(const mxb_cds_desc *desc, int32_t adjo
     mxb::Plan p;
     int rc = p.validate(*desc);
     if (rc) return rc;
-    std::vector<mxb::PoolJob> jobs[3];
+    std::vector<mxb::BlockSource> blocks[3];
     uint64_t used[3] = {0, 0, 0};
-    mxb::layout(p, jobs, used);
+    mxb::layout(p, blocks, used);
     const mxb::Shape sh = mxb::shape_for((nrhs + 7) / 8);
     std::vector<mxb::F64Task> t;
     std::vector<mxb::F64Item> it;

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from matrox_ru_b200 import _lib, hgemm as H
+from matrox_ru_b200 import _lib, hgemm as H, structure as S
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +42,22 @@ def test_workspaces_that_do_not_fit(torch, small_cases, precision):
     del hog, W, Y
     torch.cuda.empty_cache()
     assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+def test_plan_creation_needs_little_more_than_the_plan(torch):
+    """FP64 plans copy a host CDS through a bounded staging buffer, in several pieces, not beside a
+    second copy of it.  170 MB of near blocks, 110 MB to spare."""
+    X = S.gaussian_mixture(16384, 3, 3, 0.0, 2.0, 0.3, None, seed=5)
+    cds = S.build_cds(X, S.KernelSpec("gaussian", 0.4), leaf_size=256, budget=0.1, tol=1e-3, max_rank=9)
+    size = 8 * (cds.D.size + cds.B.size + cds.VT.size)
+    assert size > 160e6
+    H.Plan(cds, "fp64").close()  # loads the kernels
+    torch.zeros(1, device="cuda")
+    hog = fill(torch, size + (110 << 20))
+    plan = H.Plan(cds, "fp64")
+    del hog
+    torch.cuda.empty_cache()
+    TW = np.random.default_rng(1).standard_normal(cds.n * 3)
+    got = plan.evaluate(torch.as_tensor(TW, device="cuda"), 3).cpu().numpy()
+    want = O.eval_h2b(cds, TW, 3)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
