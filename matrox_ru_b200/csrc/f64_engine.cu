@@ -657,8 +657,10 @@ void layout(Plan &p, std::vector<BlockSource> (&blocks)[3], uint64_t (&used)[3])
 }  // namespace
 
 // Device memory for the tiling besides the pools, at most: pools on the host go through it piece by
-// piece (a block larger than it alone), so a plan needs little more than its own size.
-constexpr size_t STAGING_BYTES = 64 << 20;
+// piece (a block larger than it alone), so a plan needs little more than its own size.  Mapping and
+// unmapping it costs more than the copies it saves: 72 MB of CDS take 6.8 - 7.5 ms in pieces of 8
+// MB, 7.1 - 7.4 in 64, 8.1 in 1; 2.8 MB take 0.7 ms in pieces of 1 MB and 1.3 ms in one.
+constexpr size_t STAGING_BYTES = 8 << 20, SMALL_STAGING_BYTES = 1 << 20;
 
 int f64_create(Plan &p, const double *D, const double *B, const double *VT)
 {
@@ -691,6 +693,7 @@ int f64_create(Plan &p, const double *D, const double *B, const double *VT)
     std::vector<Piece> pieces(1, Piece{{}, 0, 0});
     std::vector<std::pair<const double *, uint64_t>> from;  // per job: the pool (null: the staging), and where in it
     size_t fill = 0, staging = 0;
+    const size_t room = (total * 512 <= STAGING_BYTES ? SMALL_STAGING_BYTES : STAGING_BYTES) / sizeof(double);
     uint64_t first = 0;        // of the pool's sub-blocks
     for (int q = 0; q < 3; first += used[q++]) {
         std::vector<BlockSource> &bl = blocks[q];
@@ -703,7 +706,6 @@ int f64_create(Plan &p, const double *D, const double *B, const double *VT)
         for (size_t i = 0; i < bl.size();) {
             size_t n = 1;
             uint64_t end = bl[i].end();
-            const size_t room = STAGING_BYTES / sizeof(double);
             auto joins = [&](uint64_t e) { return here || std::max(end, e) - bl[i].src <= room; };
             while (i + n < bl.size() && joins(bl[i + n].end())) end = std::max(end, bl[i + n++].end());
             if (!here) {
