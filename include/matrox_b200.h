@@ -362,7 +362,8 @@ MXB_API int32_t mxb_batch_destroy(mxb_batch *batch);
  * Evaluates Y = K~W (overwriting Y) once through the ordinary path, then twice launch by launch
  * outside any graph, bracketing every launch with CUDA events on `stream`, and reports the
  * second pass.  The launches are the ones an evaluation makes, in order, so Y on return
- * is the ordinary result.  The call synchronises `stream`. */
+ * is the ordinary result.  The call synchronises `stream`.  A launch that runs several passes has
+ * one record per pass (FP64 plans: the rewriting of W counts with the first). */
 #define MXB_PHASE_SPLIT_W 0        /* W -> bf16 operand tiles (split-BF16 plans) */
 #define MXB_PHASE_UP 1             /* leaf projection (level 0) or transfer at height `level` */
 #define MXB_PHASE_FAR 2            /* far couplings of every depth (one launch) */
@@ -385,9 +386,10 @@ typedef struct mxb_op_profile {
     int32_t chained;      /* 1: ran inside the launch of the record before it, as a later tree
                              level that waits on the device for the level before; ms is 0 and
                              that launch's ms covers both */
-    float level_ms;       /* one-launch batches: this level's span inside the launch, from the
-                             kernel's own timer (last unit of the level before to its own last
-                             unit written); 0 elsewhere */
+    float level_ms;       /* launches that run several passes at once (FP64 plans, one-launch
+                             batches): this pass's span inside the launch, from the kernel's own
+                             timer (last unit of the pass that ended before it to its own last unit
+                             written); 0 elsewhere */
 } mxb_op_profile;
 /* `*nops` receives the number of launches; at most `cap` records are written. */
 MXB_API int32_t mxb_plan_profile(mxb_plan *plan, const double *dW, double *dY, int32_t nrhs, void *stream,

@@ -84,11 +84,15 @@ struct Args {
     int *ctl, *err;
     long long wait_cycles;
     int units, ncol, nb, nrhs, beta, nctr;
+    // profiling (null otherwise): [0] the earliest block's start, [1 + p] the time the last tile of
+    // pass p was written (%globaltimer, ns); the pass of each task
+    unsigned long long *pass_ns;
+    const uint8_t *pass_of;
 };
 
 struct Unit {  // ring slot: the claimed unit
     F64Task task;
-    int32_t col, n8_0, n8, live;
+    int32_t col, n8_0, n8, live, index, pad;
 };
 
 // Two stacked 8 x 8 sub-blocks of A (rows g and g + 8 of a lane's fragment) times one of B.
@@ -115,7 +119,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
     volatile int *meta = reinterpret_cast<volatile int *>(ring + RING);  // per stage: sub-block columns | trans << 8
     volatile int *abort_word = meta + C::STAGES;
     int *last_cta = const_cast<int *>(abort_word) + 1;
-    static_assert(sizeof(Unit) == 80 && (2 * C::STAGES + 2 * RING) * 8 + RING * 80 + C::STAGES * 4 + 8 <= 1024, "");
+    static_assert(sizeof(Unit) == 88 && (2 * C::STAGES + 2 * RING) * 8 + RING * 88 + C::STAGES * 4 + 8 <= 1024, "");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *counters = g.ctl + CTL_FIRST;
@@ -132,6 +136,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
         tc::fence_mbar_init();
     }
     __syncthreads();
+    if (g.pass_ns && threadIdx.x == 0) atomicMin(g.pass_ns, tc::globaltimer_ns());
 
     if (warp == WARPS) {
         // ---------------- producer: claims units, fills the stages ----------------
@@ -165,6 +170,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
             if (lane == 17) un.n8_0 = n8_0;
             if (lane == 18) un.n8 = n8;
             if (lane == 19) un.live = 1;
+            if (lane == 20) un.index = t;
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&ufull[i])) : "memory");
             const int item0 = un.task.item0, nitem = un.task.nitem, r8 = un.task.r8, m8 = un.task.m8;
@@ -485,6 +491,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
                     __syncwarp();
                     if (lane == 0) atomicAdd(counters + sig * g.ncol + col, 1);
                 }
+                if (g.pass_ns && lane == 0) atomicMax(g.pass_ns + 1 + g.pass_of[un.index], tc::globaltimer_ns());
             }
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&uempty[ri])) : "memory");
@@ -1080,8 +1087,10 @@ int schedule_for(Plan &p, bool adjoint, const Shape &sh, bool capturing, F64Engi
 // evaluation
 // ---------------------------------------------------------------------------------------
 
-int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs,
-                 int nrhs, int accumulate, cudaStream_t stream)
+namespace {
+
+int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs, int nrhs,
+             int accumulate, cudaStream_t stream, unsigned long long *pass_ns, const uint8_t *pass_of)
 {
     F64Engine &E = *p.f64;
     const int nb = (nrhs + 7) / 8;
@@ -1143,11 +1152,136 @@ int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int3
     a.nrhs = nrhs;
     a.beta = accumulate ? 1 : 0;
     a.nctr = s->nctr * sh.ncol;
+    a.pass_ns = pass_ns;
+    a.pass_of = pass_of;
     switch (sh.bn) {
     case 8: return launch<8>(a, stream);
     case 16: return launch<16>(a, stream);
     default: return launch<32>(a, stream);
     }
+}
+
+// Rows of the products that a variant's warps issue for a tile of m8 sub-block rows: its share of
+// them in pairs, per warp.
+int issued_rows(int bn, int m8)
+{
+    const int wm = bn >= 32 ? Cfg<32>::WM : Cfg<8>::WM;
+    int rows = 0;
+    for (int w = 0; w < wm; ++w) rows += (m8 * (w + 1) / wm - m8 * w / wm + 1) / 2 * 16;
+    return rows;
+}
+
+}  // namespace
+
+int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs,
+                 int nrhs, int accumulate, cudaStream_t stream)
+{
+    return evaluate(p, adjoint, dW, dY, wofs, yofs, nrhs, accumulate, stream, nullptr, nullptr);
+}
+
+// The one launch of a forward evaluation by passes: a record per up-sweep height (the rewriting of W
+// with the first), far + down depth, and the near field with leaf down.  Flops come from the
+// structure, units and issued flops from the task list that ran, spans from the kernel's own timer.
+int f64_profile(Plan &p, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs, int nrhs,
+                cudaStream_t stream, mxb_op_profile *out, int cap, int *nops)
+{
+    F64Engine &E = *p.f64;
+    const int nb = (nrhs + 7) / 8;
+    const Shape sh = shape_for(nb);
+    F64Engine::Schedule *s = nullptr;
+    int rc = schedule_for(p, false, sh, false, &s);
+    if (rc) return rc;
+    std::vector<F64Task> tasks(s->ntasks);
+    std::vector<F64Item> items((s->bytes - tasks.size() * sizeof(F64Task)) / sizeof(F64Item));
+    F64_CUDA(cudaMemcpy(tasks.data(), s->tasks, tasks.size() * sizeof(F64Task), cudaMemcpyDeviceToHost));
+    if (!items.empty())
+        F64_CUDA(cudaMemcpy(items.data(), s->items, items.size() * sizeof(F64Item), cudaMemcpyDeviceToHost));
+
+    std::vector<mxb_op_profile> rec;
+    auto record = [&](int phase, int level) {
+        mxb_op_profile o{};
+        o.phase = phase;
+        o.level = level;
+        o.width = sh.bn;
+        o.chained = rec.empty() ? 0 : 1;
+        rec.push_back(o);
+        return (int)rec.size() - 1;
+    };
+    auto projects = [&](int v) { return v != p.root && p.slen[v] > 0; };
+    int top = 0, deep = 0;
+    for (int v = 0; v < p.numnodes; ++v)
+        if (projects(v)) {
+            top = std::max(top, p.height[v]);
+            deep = std::max(deep, p.depth[v]);
+        }
+    std::vector<int> up(top + 1, -1), down(deep + 1, -1);
+    for (int h = 0; h <= top; ++h)
+        for (int v = 0; v < p.numnodes && up[h] < 0; ++v)
+            if (projects(v) && p.height[v] == h) up[h] = record(MXB_PHASE_UP, h);
+    for (int d = 1; d <= deep; ++d)
+        for (int v = 0; v < p.numnodes && down[d] < 0; ++v)
+            if (projects(v) && p.depth[v] == d) down[d] = record(MXB_PHASE_FAR_DOWN, d);
+    const int near = record(MXB_PHASE_NEAR_LEAF_DOWN, 0);
+    for (int v = 0; v < p.numnodes; ++v) {
+        if (!projects(v)) continue;
+        const bool leaf = p.lch[v] == -1;
+        const double cols = leaf ? p.Ddim[p.lm[v]] : p.slen[p.lch[v]] + p.slen[p.rch[v]];
+        rec[up[p.height[v]]].flops += 2.0 * p.slen[v] * cols * nrhs;
+        if (leaf) rec[near].flops += 2.0 * p.slen[v] * cols * nrhs;
+        if (p.parent[v] >= 0 && projects(p.parent[v]))
+            rec[down[p.depth[v]]].flops += 2.0 * p.slen[v] * p.slen[p.parent[v]] * nrhs;
+    }
+    for (size_t k = 0; k < p.far_x.size(); ++k)
+        if (projects(p.far_x[k])) rec[down[p.depth[p.far_x[k]]]].flops += 2.0 * p.slen[p.far_x[k]] * p.slen[p.far_y[k]] * nrhs;
+    for (size_t k = 0; k < p.near_x.size(); ++k) rec[near].flops += 2.0 * p.Ddim[p.near_x[k]] * p.Ddim[p.near_y[k]] * nrhs;
+
+    std::vector<int> node_at(E.node8_total + 1, -1);  // by sub-block row
+    for (int v = 0; v < p.numnodes; ++v)
+        if (projects(v)) node_at[E.node8[v]] = v;
+    std::vector<uint8_t> pass(tasks.size());
+    for (size_t t = 0; t < tasks.size(); ++t) {
+        const F64Task &tk = tasks[t];
+        const int k = tk.kind == F64_TILE_W ? 0 : tk.kind == F64_Y ? near
+                      : tk.kind == F64_WSKEL ? up[p.height[node_at[tk.out]]] : down[p.depth[node_at[tk.out]]];
+        pass[t] = (uint8_t)std::min(k, 255);
+        rec[k].units += sh.ncol;
+        for (int q = tk.item0; q < tk.item0 + tk.nitem; ++q)
+            rec[k].issued_flops += 2.0 * issued_rows(sh.bn, tk.m8) * (8.0 * items[q].k8) * (8.0 * nb);
+    }
+
+    // [start, passes], then the pass of each task
+    std::vector<unsigned long long> ends(rec.size() + 1, 0);
+    const size_t times = ends.size() * sizeof(unsigned long long);
+    uint8_t *work = nullptr;
+    F64_CUDA(cudaMalloc(&work, times + pass.size()));
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    cudaError_t e = cudaMemcpy(work + times, pass.data(), pass.size(), cudaMemcpyHostToDevice);
+    for (cudaEvent_t &x : ev)
+        if (e == cudaSuccess) e = cudaEventCreate(&x);
+    for (int rep = 0; rep < 2 && !rc && e == cudaSuccess; ++rep) {
+        cudaMemsetAsync(work, 0, times, stream);
+        cudaMemsetAsync(work, 0xff, sizeof(unsigned long long), stream);  // start: minimum of
+        cudaEventRecord(ev[0], stream);
+        rc = evaluate(p, false, dW, dY, wofs, yofs, nrhs, 0, stream, reinterpret_cast<unsigned long long *>(work), work + times);
+        cudaEventRecord(ev[1], stream);
+        e = cudaStreamSynchronize(stream);
+    }
+    float ms = 0.f;
+    if (!rc && e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev[0], ev[1]);
+    if (!rc && e == cudaSuccess) e = cudaMemcpy(ends.data(), work, times, cudaMemcpyDeviceToHost);
+    for (cudaEvent_t x : ev)
+        if (x) cudaEventDestroy(x);
+    cudaFree(work);
+    if (rc) return rc;
+    if (e != cudaSuccess) return fail(std::string("profile: ") + cudaGetErrorString(e));
+    const std::vector<float> spans = pass_spans(ends);
+    for (size_t k = 0; k < rec.size(); ++k) {
+        rec[k].ms = k ? 0.f : ms;
+        rec[k].level_ms = spans[k];
+        if (out && (int)k < cap) out[k] = rec[k];
+    }
+    if (nops) *nops = (int)rec.size();
+    return MXB_OK;
 }
 
 int f64_status(Plan &p)

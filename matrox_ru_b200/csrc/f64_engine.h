@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "matrox_b200.h"
 #include "mxb_internal.h"
 
 namespace mxb {
@@ -75,6 +76,8 @@ struct F64Engine {
 int f64_create(Plan &p, const double *D, const double *B, const double *VT);
 int f64_evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs,
                  int nrhs, int accumulate, cudaStream_t stream);
+int f64_profile(Plan &p, const double *dW, double *dY, const int32_t *wofs, const int32_t *yofs, int nrhs,
+                cudaStream_t stream, mxb_op_profile *out, int cap, int *nops);
 int f64_status(Plan &p);
 int f64_read_skeletons(Plan &p, int nrhs, std::vector<double> &w, std::vector<double> &u);
 void f64_destroy(Plan &p);

@@ -615,56 +615,32 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
     return MXB_OK;
 }
 
-// Launch-by-launch timing of the forward evaluation (mxb_plan_profile).
+// Timing of the forward evaluation by launches and passes (mxb_plan_profile).
 int Plan::profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, mxb_op_profile *out, int cap,
                   int *nops)
 {
     int rc = run(launches_fwd, dW, dY, nrhs, nullptr, nullptr, 0, stream);  // checks, offsets, graphs, tuning
     if (rc) return rc;
     if (precision != MXB_PREC_FP64) return batch_profile(split_bf16_batch(*this), &dW, &dY, &nrhs, stream, out, cap, nops);
-    const std::vector<Launch> &L = launches_fwd;
-    // one launch runs every pass: the first record carries its time, the others are chained to it
-    const int tile = row_tile_for(precision), ncol = (int)((nrhs + tile - 1) / tile);
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    for (cudaEvent_t &e : ev)
-        if (!rc && cudaEventCreate(&e) != cudaSuccess) {
-            set_error("profile: creating CUDA events failed");
-            rc = MXB_ERR_CUDA;
-        }
-    float ms = 0.f;
-    for (int rep = 0; rep < 2 && !rc; ++rep) {
-        cudaEventRecord(ev[0], stream);
-        rc = run(L, dW, dY, nrhs, nullptr, nullptr, 0, stream);
-        cudaEventRecord(ev[1], stream);
-        if (!rc && cudaStreamSynchronize(stream) != cudaSuccess) {
-            set_error("profile: stream synchronisation failed");
-            rc = MXB_ERR_CUDA;
-        }
+    return f64_profile(*this, dW, dY, ofs[0]->dev, ofs[1]->dev, nrhs, stream, out, cap, nops);
+}
+
+std::vector<float> pass_spans(const std::vector<unsigned long long> &ends)
+{
+    const int n = (int)ends.size() - 1;
+    std::vector<float> ms(n, 0.f);
+    if (ends[0] == ~0ull) return ms;
+    std::vector<int> by(n);
+    for (int k = 0; k < n; ++k) by[k] = k;
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return ends[a + 1] < ends[b + 1]; });
+    unsigned long long last = ends[0];
+    for (int k : by) {
+        if (!ends[k + 1]) continue;
+        const unsigned long long end = std::max(ends[k + 1], last + 1);
+        ms[k] = (float)((double)(end - last) * 1e-6);
+        last = end;
     }
-    if (!rc) cudaEventElapsedTime(&ms, ev[0], ev[1]);
-    if (nops) *nops = (int)L.size();
-    for (size_t i = 0; i < L.size() && !rc && (int)i < cap && out; ++i) {
-        const Launch &l = L[i];
-        mxb_op_profile &o = out[i];
-        o = mxb_op_profile{};
-        o.phase = l.kind;
-        o.level = l.level;
-        o.width = tile;
-        o.units = l.ntasks * ncol;
-        for (int t = l.task0; t < l.task0 + l.ntasks; ++t) {
-            const Task &T = tasks[t];
-            const double rows = std::min(tile, T.M - T.m0);
-            for (int k = T.item0; k < T.item0 + T.nitem; ++k) {
-                o.flops += 2.0 * rows * items[k].K * nrhs;
-                o.issued_flops += 2.0 * tile * items[k].K * (double)ncol * tile;
-            }
-        }
-        o.chained = i > 0;
-        o.ms = i ? 0.f : ms;
-    }
-    for (cudaEvent_t e : ev)
-        if (e) cudaEventDestroy(e);
-    return rc;
+    return ms;
 }
 
 int Plan::read_workspaces(int nrhs, const int32_t *wsko, double *wskel, const int32_t *usko, double *uskel)

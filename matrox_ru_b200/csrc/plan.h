@@ -100,6 +100,9 @@ struct Plan : public mxb_plan {
 const char *last_error();
 // Whether `stream` is being captured; MXB_ERR_CUDA where it cannot be asked.
 int is_capturing(cudaStream_t stream, bool *yes);
+// Time of each pass inside a launch that overlaps them, in ms: from the end of the pass that ended
+// before it to its own end.  ends[0]: the launch's start, ends[1 + k]: pass k (0: not in the launch), ns.
+std::vector<float> pass_spans(const std::vector<unsigned long long> &ends);
 int refuse_unprepared();  // MXB_ERR_UNSUPPORTED: preparing allocates and copies, which a capture cannot hold
 int row_tile_for(int precision);
 int split_bf16_launches(const Plan &p);

@@ -5,7 +5,8 @@ evaluation must leave the ordinary result in Y."""
 import numpy as np
 import pytest
 
-from matrox_ru_b200 import hgemm as H
+from matrox_ru_b200 import _lib, hgemm as H
+from test_f64_schedule import TILE_W, WSKEL, schedule
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +71,28 @@ def test_batch_profile(torch, small_cases):
     assert sum(x["flops"] for x in recs) == sum(c.flops(r) for c, r in cases)
     for o, w in zip(outs, want):
         torch.testing.assert_close(o, w, rtol=1e-13, atol=1e-13 * float(w.abs().max()))
+
+
+@pytest.mark.parametrize("r,width", [(1, 8), (13, 16), (100, 32)])
+@pytest.mark.parametrize("name", ["h2b", "ragged"])
+def test_fp64_profile_is_of_the_launch_that_ran(torch, small_cases, name, r, width):
+    """Width, units and issued flops of the one launch's column tiles and task list, and its passes'
+    spans, which make up the launch."""
+    cds = small_cases[name]
+    recs = H.Plan(cds, "fp64").profile(torch.randn(cds.n * r, dtype=torch.float64, device="cuda"), r)
+    tasks, items, counts = schedule(_lib.load(), cds, False, r)
+    ncol, nb = int(counts[4]), -(-r // 8)
+    assert {x["width"] for x in recs} == {width}
+    assert sum(x["units"] for x in recs) == len(tasks) * ncol
+    up = [x for x in recs if x["phase"] == "up"]
+    assert sum(x["units"] for x in up) == ncol * int(np.isin(tasks["kind"], (TILE_W, WSKEL)).sum())
+    # a warp multiplies its share of a tile's 8-row sub-blocks in pairs
+    warps = 2 if width == 32 else 4
+    issued = 0
+    for t in tasks:
+        m8 = int(t["m8"])
+        rows = sum(16 * -(-(m8 * (w + 1) // warps - m8 * w // warps) // 2) for w in range(warps))
+        issued += 2 * rows * 8 * int(items["k8"][t["item0"]:t["item0"] + t["nitem"]].sum()) * 8 * nb
+    assert sum(x["issued_flops"] for x in recs) == issued
+    assert all(x["level_ms"] > 0 for x in recs)
+    assert 0.5 * recs[0]["ms"] < sum(x["level_ms"] for x in recs) < 1.1 * recs[0]["ms"] + 0.01
