@@ -386,10 +386,10 @@ typedef struct mxb_op_profile {
     int32_t chained;      /* 1: ran inside the launch of the record before it, as a later tree
                              level that waits on the device for the level before; ms is 0 and
                              that launch's ms covers both */
-    float level_ms;       /* launches that run several passes at once (FP64 plans, one-launch
-                             batches): this pass's span inside the launch, from the kernel's own
-                             timer (last unit of the pass that ended before it to its own last unit
-                             written); 0 elsewhere */
+    float level_ms;       /* launches that run all passes at once (FP64 plans, flow launches):
+                             this pass's span inside the launch, from the kernel's own timer (last
+                             unit of the pass that ended before it to its own last unit written);
+                             0 elsewhere */
 } mxb_op_profile;
 /* `*nops` receives the number of launches; at most `cap` records are written. */
 MXB_API int32_t mxb_plan_profile(mxb_plan *plan, const double *dW, double *dY, int32_t nrhs, void *stream,

@@ -2852,9 +2852,9 @@ int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cu
     int rc = MXB_OK;
     for (cudaEvent_t &x : ev)
         if (!rc && cudaEventCreate(&x) != cudaSuccess) rc = batch_fail("profile: creating CUDA events failed", MXB_ERR_CUDA);
-    // one launch: each op's span on the device, from the kernel's own timestamps
+    // flow launch: each op's span on the device, from the kernel's own timestamps
     std::vector<unsigned long long> lns(ops.size() + 1, 0);
-    if (!rc && one_launch) {
+    if (!rc && flow_width(e->bn)) {
         if (cudaMalloc(&level_ns, lns.size() * sizeof(unsigned long long)) != cudaSuccess) {
             level_ns = nullptr;
             rc = batch_fail("profile: level timer allocation failed", MXB_ERR_NOMEM);
@@ -2908,21 +2908,15 @@ int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cu
         o.level = m.level;
         o.width = tile_width(e->bn[k]);
         o.pair = tile_pair(e->bn[k]) ? 1 : 0;
-        o.chained = one_launch ? (k > 0) : flow_width(e->bn) ? (m.phase == PH_SPLITW ? e->flow_w : (int)k != first_tc) : ((m.phase != PH_SPLITW && (e->bn[k] & TILE_CHAIN)) ? 1 : 0);
+        o.chained = one_launch ? (k > 0)
+                    : flow_width(e->bn) ? (m.phase == PH_SPLITW ? e->flow_w : (int)k != first_tc)
+                    : (m.phase != PH_SPLITW && (e->bn[k] & TILE_CHAIN)) ? 1 : 0;
         cudaEventElapsedTime(&o.ms, ev[k], ev[k + 1]);
         if (o.chained) o.ms = 0.f;
     }
-    if (!rc && one_launch && out && lns[0] != ~0ull) {
-        // the passes overlap: each gets the time from the end of the one that ended before it
-        std::vector<int> by(ops.size());
-        for (size_t k = 0; k < by.size(); ++k) by[k] = (int)k;
-        std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return lns[a + 1] < lns[b + 1]; });
-        unsigned long long last = lns[0];
-        for (int k : by) {
-            const unsigned long long end = std::max(lns[k + 1], last + 1);
-            if (k < cap) out[k].level_ms = (float)((double)(end - last) * 1e-6);
-            last = end;
-        }
+    if (!rc && flow_width(e->bn) && out) {
+        const std::vector<float> spans = pass_spans(lns);
+        for (size_t k = 0; k < ops.size() && (int)k < cap; ++k) out[k].level_ms = spans[k];
     }
     for (size_t u = 0; u < units.size() && !rc && out; ++u) {
         const TcTask &t = tasks[units[u].task];
@@ -2936,7 +2930,8 @@ int Batch::profile(const double *const *W, double *const *Y, const int *nrhs, cu
         const double cols = std::min(o.width, nr[t.plan] - units[u].col * o.width);
         for (int q = t.item0; q < t.item0 + t.nitem; ++q) {
             o.flops += 2.0 * rows * items[q].K * cols;
-            o.issued_flops += products * 2.0 * tile_rows * (64.0 * items[q].KT) * o.width;
+            o.issued_flops += products * 2.0 * tile_rows * (64.0 * items[q].KT) *
+                              (o.pair ? o.width : tile_columns(nr[t.plan], units[u].col, o.width));
         }
     }
     for (cudaEvent_t x : ev)

@@ -96,3 +96,17 @@ def test_fp64_profile_is_of_the_launch_that_ran(torch, small_cases, name, r, wid
     assert sum(x["issued_flops"] for x in recs) == issued
     assert all(x["level_ms"] > 0 for x in recs)
     assert 0.5 * recs[0]["ms"] < sum(x["level_ms"] for x in recs) < 1.1 * recs[0]["ms"] + 0.01
+
+
+def test_flow_profile_counts_what_is_issued(torch, small_cases):
+    """A flow launch: products of whole 16-column groups only, and the passes' spans inside it."""
+    cds = small_cases["ragged"]
+    plan = H.Plan(cds, "split_bf16_x6")
+    recs = {r: plan.profile(torch.randn(cds.n * r, dtype=torch.float64, device="cuda"), r) for r in (5, 16, 64)}
+    issued = {r: sum(x["issued_flops"] for x in v) for r, v in recs.items()}
+    assert issued[5] == issued[16] and issued[64] == 4 * issued[16]
+    for v in recs.values():
+        launch = sum(x["ms"] for x in v)
+        assert plan.info()["launches"] == 1
+        assert all(x["level_ms"] > 0 for x in v)
+        assert 0.3 * launch < sum(x["level_ms"] for x in v) < 1.1 * launch + 0.01
