@@ -412,7 +412,7 @@ int run_dropin(DropIn &a)
         API_CUDA(cudaStreamWaitEvent(buf->stream, buf->uploaded[b], 0));
         if (k >= 2) API_CUDA(cudaStreamWaitEvent(buf->stream, buf->downloaded[b], 0));
         // a Y known to be zero is overwritten instead of accumulated into
-        rc = plan->run(plan->launches_fwd, buf->W[b], buf->Y[b], w, nullptr, nullptr, upload_y ? 1 : 0,
+        rc = plan->run(false, buf->W[b], buf->Y[b], w, nullptr, nullptr, upload_y ? 1 : 0,
                        buf->stream);
         if (rc) {
             cudaDeviceSynchronize();
@@ -860,7 +860,7 @@ int32_t mxb_plan_evaluate(mxb_plan *plan, const double *dW, double *dY, int32_t 
         return MXB_ERR_ARG;
     }
     Plan *p = static_cast<Plan *>(plan);
-    return p->run(p->launches_fwd, dW, dY, nrhs, wptr, uptr, accumulate, (cudaStream_t)stream);
+    return p->run(false, dW, dY, nrhs, wptr, uptr, accumulate, (cudaStream_t)stream);
 }
 
 int32_t mxb_plan_adjoint(mxb_plan *plan, const double *dG, double *dGW, int32_t nrhs, const int32_t *gptr,
@@ -871,7 +871,7 @@ int32_t mxb_plan_adjoint(mxb_plan *plan, const double *dG, double *dGW, int32_t 
         return MXB_ERR_ARG;
     }
     Plan *p = static_cast<Plan *>(plan);
-    return p->run(p->launches_adj, dG, dGW, nrhs, gptr, gwptr, accumulate, (cudaStream_t)stream);
+    return p->run(true, dG, dGW, nrhs, gptr, gwptr, accumulate, (cudaStream_t)stream);
 }
 
 int32_t mxb_plan_set_permutation(mxb_plan *plan, const int32_t *perm)

@@ -67,7 +67,8 @@ struct Operands {
 
 struct Plan;
 
-// FP64 grouped GEMM (gemm_f64.cu)
+// FP64 grouped GEMM (gemm_f64.cu): a task is a tile of at most this many rows
+constexpr int F64_ROW_TILE = 64;
 cudaError_t launch_gemm_f64(const Task *tasks, const Item *items, int ntasks,
                             const Operands &ops, cudaStream_t stream);
 

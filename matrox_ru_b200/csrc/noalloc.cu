@@ -118,7 +118,7 @@ extern "C" int32_t mxb_evaluate_noalloc(const mxb_cds_desc *desc, const double *
     Plan p;
     rc = p.validate(*desc);
     if (rc) return rc;
-    p.build_tasks(row_tile_for(MXB_PREC_FP64));
+    p.build_tasks(F64_ROW_TILE);
 
     const size_t tasks_b = p.tasks.size() * sizeof(Task);
     const size_t items_b = p.items.size() * sizeof(Item);

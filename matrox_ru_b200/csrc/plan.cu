@@ -1,7 +1,5 @@
-// Plan: validated structure, device copy of the CDS and the task lists of every pass.
-//
-// FP64 plans evaluate in one dataflow launch (f64_engine.cu).  The launch-per-pass lists built
-// here are what mxb_evaluate_noalloc runs, and the pass-by-pass flop accounting of the profile.
+// Plan: validated structure, creation, and the calls that FP64 (f64_engine.cu) and split-BF16
+// (split_bf16.cu) plans share; and the launch-per-pass task lists that mxb_evaluate_noalloc runs.
 // Schedule of one such evaluation (the reference runs the same four phases,
 // symGen/HGEMM_gen.h:125-236, but as thousands of separate DGEMM calls):
 //   1. leaf up        wskel[v] = P_v W[leaf v]                          (one launch)
@@ -44,8 +42,6 @@ const char *last_error() { return g_last_error.c_str(); }
             return MXB_ERR_CUDA;                                                          \
         }                                                                                 \
     } while (0)
-
-int row_tile_for(int precision);
 
 Plan::~Plan()
 {
@@ -441,7 +437,6 @@ int Plan::create(const mxb_cds_desc &d, int prec, Plan **out)
     MXB_CUDA(cudaGetDevice(&p->device));
     int rc = p->validate(d);
     if (rc) return rc;
-    p->build_tasks(row_tile_for(prec));
     if (prec == MXB_PREC_FP64) {
         rc = f64_create(*p, d.D, d.B, d.VT);
         if (rc) return rc;
@@ -513,8 +508,8 @@ int Plan::stage_offsets(int slot, const int32_t *given, int nrhs, cudaStream_t s
     return MXB_OK;
 }
 
-int Plan::run(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs,
-              const int32_t *wofs, const int32_t *yofs, int accumulate, cudaStream_t stream)
+int Plan::run(bool adjoint, const double *dW, double *dY, int nrhs, const int32_t *wofs, const int32_t *yofs,
+              int accumulate, cudaStream_t stream)
 {
     if (nrhs < 1) {
         set_error("nrhs must be >= 1");
@@ -534,8 +529,8 @@ int Plan::run(const std::vector<Launch> &L, const double *dW, double *dY, int nr
     if (rc) return rc;
     rc = stage_offsets(1, yofs, nrhs, stream);
     if (rc) return rc;
-    if (precision != MXB_PREC_FP64) return run_split_bf16(L, dW, dY, nrhs, accumulate, stream);
-    return f64_evaluate(*this, &L == &launches_adj, dW, dY, ofs[0]->dev, ofs[1]->dev, nrhs, accumulate, stream);
+    if (precision != MXB_PREC_FP64) return run_split_bf16(adjoint, dW, dY, nrhs, accumulate, stream);
+    return f64_evaluate(*this, adjoint, dW, dY, ofs[0]->dev, ofs[1]->dev, nrhs, accumulate, stream);
 }
 
 // The caller's point order: perm[t] is the row of W / Y holding tree position t (the `lids`
@@ -578,7 +573,6 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
         return rs >= 1 && cs >= 1 && (rs >= (int64_t)nrhs * cs || cs >= n * rs);
     };
     if (!separated(w_rs, w_cs) || !separated(y_rs, y_cs)) return arg_fail("caller-order strides overlap");
-    const std::vector<Launch> &L = adjoint ? launches_adj : launches_fwd;
     if (precision != MXB_PREC_FP64) {
         int cur = -1;
         MXB_CUDA(cudaGetDevice(&cur));
@@ -587,7 +581,7 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
         if (!rc) rc = stage_offsets(1, nullptr, nrhs, stream);
         if (rc) return rc;
         const CallerOrder o{dTree, dTree + n, w_rs, w_cs, y_rs, y_cs};
-        return run_split_bf16(L, dW, dY, nrhs, accumulate, stream, &o);
+        return run_split_bf16(adjoint, dW, dY, nrhs, accumulate, stream, &o);
     }
     const size_t need = (size_t)std::max<int64_t>(n, 1) * nrhs;
     if (need > order_elems) {
@@ -608,7 +602,7 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
     int rc = stage_offsets(0, nullptr, nrhs, stream);  // packed blocks of the leaf-blocked copies
     if (rc) return rc;
     MXB_CUDA(launch_permute(dTree, dTree + n, ofs[0]->dev, nleaf, n, dW, dTW, w_rs, w_cs, nrhs, 0, 0, stream));
-    rc = run(L, dTW, dTY, nrhs, nullptr, nullptr, 0, stream);
+    rc = run(adjoint, dTW, dTY, nrhs, nullptr, nullptr, 0, stream);
     if (rc) return rc;
     MXB_CUDA(launch_permute(dTree, dTree + n, ofs[1]->dev, nleaf, n, dTY, dY, y_rs, y_cs, nrhs, 1, accumulate,
                             stream));
@@ -619,7 +613,7 @@ int Plan::run_ordered(bool adjoint, const double *dW, int64_t w_rs, int64_t w_cs
 int Plan::profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, mxb_op_profile *out, int cap,
                   int *nops)
 {
-    int rc = run(launches_fwd, dW, dY, nrhs, nullptr, nullptr, 0, stream);  // checks, offsets, graphs, tuning
+    int rc = run(false, dW, dY, nrhs, nullptr, nullptr, 0, stream);  // checks, offsets, tuning
     if (rc) return rc;
     if (precision != MXB_PREC_FP64) return batch_profile(split_bf16_batch(*this), &dW, &dY, &nrhs, stream, out, cap, nops);
     return f64_profile(*this, dW, dY, ofs[0]->dev, ofs[1]->dev, nrhs, stream, out, cap, nops);

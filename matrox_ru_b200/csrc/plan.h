@@ -36,7 +36,7 @@ struct Plan : public mxb_plan {
     int64_t rows_total = 0, skel_total = 0;
     uint64_t D_len = 0, B_len = 0, VT_len = 0;
 
-    // ---- task lists ----
+    // ---- task lists of evaluations in launches per pass (mxb_evaluate_noalloc; not built for plans) ----
     std::vector<Item> items;
     std::vector<Task> tasks;
     std::vector<Launch> launches_fwd, launches_adj;
@@ -77,8 +77,8 @@ struct Plan : public mxb_plan {
     void release(void *q, size_t bytes);  // of alloc; kept until destruction once recorded
     void record();                        // the evaluation now enqueued is being captured
     int stage_offsets(int slot, const int32_t *ofs, int nrhs, cudaStream_t stream);
-    int run(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, const int32_t *wofs,
-            const int32_t *yofs, int accumulate, cudaStream_t stream);
+    int run(bool adjoint, const double *dW, double *dY, int nrhs, const int32_t *wofs, const int32_t *yofs,
+            int accumulate, cudaStream_t stream);
     int profile(const double *dW, double *dY, int nrhs, cudaStream_t stream, mxb_op_profile *out, int cap,
                 int *nops);
     int set_permutation(const int32_t *perm);
@@ -92,7 +92,7 @@ struct Plan : public mxb_plan {
     // split-BF16 path (split_bf16.cu)
     int setup_split_bf16(const mxb_cds_desc &d);
     void clear_split_graphs();
-    int run_split_bf16(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, int accumulate,
+    int run_split_bf16(bool adjoint, const double *dW, double *dY, int nrhs, int accumulate,
                        cudaStream_t stream, const CallerOrder *order = nullptr);
     void free_split_bf16();
 };
@@ -104,7 +104,6 @@ int is_capturing(cudaStream_t stream, bool *yes);
 // before it to its own end.  ends[0]: the launch's start, ends[1 + k]: pass k (0: not in the launch), ns.
 std::vector<float> pass_spans(const std::vector<unsigned long long> &ends);
 int refuse_unprepared();  // MXB_ERR_UNSUPPORTED: preparing allocates and copies, which a capture cannot hold
-int row_tile_for(int precision);
 int split_bf16_launches(const Plan &p);
 int split_bf16_prepare();
 int batch_create(Plan *const *plans, int count, Batch **out);

@@ -67,8 +67,6 @@
 
 namespace mxb {
 
-int row_tile_for(int precision) { return precision != MXB_PREC_FP64 ? 128 : 64; }
-
 namespace {
 
 using tc::TILE_BYTES;
@@ -3271,11 +3269,11 @@ int Plan::setup_split_bf16(const mxb_cds_desc &)
     return rc;
 }
 
-int Plan::run_split_bf16(const std::vector<Launch> &L, const double *dW, double *dY, int nrhs, int accumulate,
+int Plan::run_split_bf16(bool adjoint, const double *dW, double *dY, int nrhs, int accumulate,
                          cudaStream_t stream, const CallerOrder *order)
 {
     Batch *b = bf16->self;
-    if (&L == &launches_adj) {
+    if (adjoint) {
         if (!bf16->self_adj) {
             set_error("this split-BF16 plan has no adjoint: create it with precision | MXB_PLAN_ADJOINT (or use an "
                       "FP64 plan)");
