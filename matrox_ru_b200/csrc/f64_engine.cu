@@ -35,7 +35,6 @@
 // N = 1024, 1 right-hand side 102 -> 30 us.
 #include <algorithm>
 #include <cstring>
-#include <functional>
 #include <queue>
 #include <string>
 
@@ -595,12 +594,9 @@ Shape shape_for(int nb)
     return {32, Cfg<32>::BK8, Cfg<32>::CTAS, (nb + 3) / 4};
 }
 
-// A group of the schedule: the tasks of one output block in one pass.
+// A group of the schedule: the tasks of one output block in one pass, and the groups it reads.
 struct Group {
-    std::vector<F64Task> tasks;
-    std::vector<int> deps, cons;
-    double prio = -1, ready = 0, finish = 0;
-    int unplaced = 0, cost = 0;
+    int task0, ntask, dep0, ndep;
 };
 
 }  // namespace
@@ -762,7 +758,10 @@ int f64_create(Plan &p, const double *D, const double *B, const double *VT)
 
 namespace {
 
-// Tasks in claim order for one direction and column count; see the file comment.
+// Tasks in claim order for one direction and column count; see the file comment.  Built at the first
+// evaluation of each, so the lists are flat arrays and the workers are kept by integer times: N =
+// 65536 with leaves of 256 points, 10075 tasks, 0.75 ms (2.5 ms with vectors of tasks and readers per
+// group and a heap of workers); the first product with one column after creation 2.0 ms (3.3).
 int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> &out, std::vector<F64Item> &items,
                    int &nctr, int64_t &slots)
 {
@@ -776,33 +775,48 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     const int c_w = 0, c_near = p.nleaf, c_up = 2 * p.nleaf, c_far = c_up + p.numnodes, c_u = c_far + p.numnodes;
     nctr = c_u + p.numnodes;
     std::vector<Group> G;
+    std::vector<F64Task> all;
+    std::vector<int> deps;
+    G.reserve(3 * (size_t)p.nleaf + 3 * (size_t)p.numnodes);
+    all.reserve(4 * G.capacity());
+    deps.reserve(p.near_x.size() + p.far_x.size() + 2 * G.capacity());
+    items.reserve(p.near_x.size() + p.far_x.size() + G.capacity());
     std::vector<int> g_w(p.nleaf, -1), g_near(p.nleaf, -1), g_up(p.numnodes, -1), g_far(p.numnodes, -1), g_u(p.numnodes, -1);
-    struct Src {
-        F64Block a;
-        int pool, trans, buf, dep, need, group;
-        int64_t base;
-    };
-    auto block_item = [&](const Src &s) {
-        F64Item it{};
-        it.a_off = s.a.off;
-        it.lda = s.a.m8;
-        it.k8 = s.trans ? s.a.m8 : s.a.k8;
-        it.b_base = s.base;
-        it.dep = s.dep;
-        it.need = s.need;
-        it.a_pool = (int16_t)s.pool;
-        it.trans = (int16_t)s.trans;
-        it.b_buf = (int16_t)s.buf;
-        return it;
-    };
+    const int WR = WARPS;  // every product warp of a tile counts itself
     auto stages_of = [&](int k8) { return (k8 + sh.bk8 - 1) / sh.bk8; };
-    // one group: `rows` output rows, summing the sources
-    auto add_group = [&](int kind, int64_t o, int rows, const std::vector<Src> &srcs, int beta, int sig, int old_dep,
-                         int old_need, int old_group) {
-        Group g;
+    // A group is begun, given the groups and blocks it reads, and ended with its output rows.  Every
+    // group reads only groups begun before it.
+    int item0 = 0, dep0 = 0, stages = 0;
+    auto begin_group = [&]() {
+        item0 = (int)items.size();
+        dep0 = (int)deps.size();
+        stages = 0;
+    };
+    auto reads_group = [&](int g) {
+        if (g >= 0 && std::find(deps.begin() + dep0, deps.end(), g) == deps.end()) deps.push_back(g);
+    };
+    auto reads = [&](const F64Block &a, int pool, int trans, int buf, int dep, int need, int group, int64_t base) {
+        F64Item it{};
+        it.a_off = a.off;
+        it.lda = a.m8;
+        it.k8 = trans ? a.m8 : a.k8;
+        if (it.k8 <= 0) return;
+        it.b_base = base;
+        it.dep = dep;
+        it.need = need;
+        it.a_pool = (int16_t)pool;
+        it.trans = (int16_t)trans;
+        it.b_buf = (int16_t)buf;
+        items.push_back(it);
+        stages += stages_of(it.k8);
+        reads_group(group);
+    };
+    auto end_group = [&](int kind, int64_t o, int rows, int beta, int sig, int old_dep, int old_need, int slot) {
         F64Task t{};
         t.out = o;
-        t.item0 = (int)items.size();
+        t.item0 = item0;
+        t.nitem = (int)items.size() - item0;
+        t.stages = stages;
         t.rows = rows;
         t.sig = sig;
         t.old_dep = old_dep;
@@ -811,122 +825,116 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
         t.npiece = 1;
         t.kind = (int16_t)kind;
         t.beta = (int16_t)beta;
-        for (const Src &s : srcs) {
-            const F64Item it = block_item(s);
-            if (it.k8 <= 0) continue;
-            items.push_back(it);
-            t.stages += stages_of(it.k8);
-            if (s.group >= 0 && std::find(g.deps.begin(), g.deps.end(), s.group) == g.deps.end()) g.deps.push_back(s.group);
-        }
-        t.nitem = (int)items.size() - t.item0;
-        if (old_group >= 0) g.deps.push_back(old_group);
+        t.slot = slot;
         const int m8 = ceil8(rows), T = row_tiles(rows);
+        G.push_back(Group{(int)all.size(), T, dep0, (int)deps.size() - dep0});
         for (int i = 0; i < T; ++i) {  // row tiles of nearly equal height
             t.r8 = (int)((int64_t)m8 * i / T);
             t.m8 = (int)((int64_t)m8 * (i + 1) / T) - t.r8;
-            g.tasks.push_back(t);
+            all.push_back(t);
         }
-        G.push_back(std::move(g));
         return (int)G.size() - 1;
     };
-    const int WR = WARPS;  // every product warp of a tile counts itself
+    auto reads_w = [&](const F64Block &a, int pool, int trans, int leaf) {
+        reads(a, pool, trans, BUF_W, c_w + leaf, WR * row_tiles(p.Ddim[leaf]), g_w[leaf], E.leaf8[leaf]);
+    };
+    auto reads_up = [&](const F64Block &a, int pool, int trans, int v) {  // (nothing writes the root's block)
+        reads(a, pool, trans, BUF_WSKEL, g_up[v] < 0 ? -1 : c_up + v, WR * row_tiles(p.slen[v]), g_up[v], E.node8[v]);
+    };
+    auto reads_u = [&](const F64Block &a, int pool, int trans, int v) {
+        reads(a, pool, trans, BUF_USKEL, c_u + v, WR * row_tiles(p.slen[v]), g_u[v], E.node8[v]);
+    };
     for (int i = 0; i < p.nleaf; ++i) {
-        Group g;
-        F64Task t{};
-        t.out = i;
-        t.rows = p.Ddim[i];
-        t.sig = c_w + i;
-        t.old_dep = t.piece_ctr = -1;
-        t.npiece = 1;
-        t.kind = F64_TILE_W;
-        t.slot = (int)E.leaf8[i];
-        const int m8 = ceil8(p.Ddim[i]), T = row_tiles(p.Ddim[i]);
-        for (int k = 0; k < T; ++k) {
-            t.r8 = (int)((int64_t)m8 * k / T);
-            t.m8 = (int)((int64_t)m8 * (k + 1) / T) - t.r8;
-            g.tasks.push_back(t);
-        }
-        G.push_back(std::move(g));
-        g_w[i] = (int)G.size() - 1;
+        begin_group();
+        g_w[i] = end_group(F64_TILE_W, i, p.Ddim[i], 0, c_w + i, -1, 0, (int)E.leaf8[i]);
     }
-    auto w_src = [&](const F64Block &a, int pool, int trans, int leaf) {
-        return Src{a, pool, trans, BUF_W, c_w + leaf, WR * row_tiles(p.Ddim[leaf]), g_w[leaf], E.leaf8[leaf]};
-    };
-    auto up_src = [&](const F64Block &a, int pool, int trans, int v) {  // (nothing writes the root's block)
-        return Src{a, pool, trans, BUF_WSKEL, g_up[v] < 0 ? -1 : c_up + v, WR * row_tiles(p.slen[v]), g_up[v], E.node8[v]};
-    };
-    auto u_src = [&](const F64Block &a, int pool, int trans, int v) {
-        return Src{a, pool, trans, BUF_USKEL, c_u + v, WR * row_tiles(p.slen[v]), g_u[v], E.node8[v]};
-    };
     for (auto it = p.bfs.rbegin(); it != p.bfs.rend(); ++it) {  // children before parents
         const int v = *it;
         if (!projects(v)) continue;
-        std::vector<Src> s;
+        begin_group();
         if (p.lch[v] == -1) {
-            s.push_back(w_src(E.proj_l[v], 2, 0, p.lm[v]));
+            reads_w(E.proj_l[v], 2, 0, p.lm[v]);
         } else {
-            if (p.slen[p.lch[v]] > 0) s.push_back(up_src(E.proj_l[v], 2, 0, p.lch[v]));
-            if (p.slen[p.rch[v]] > 0) s.push_back(up_src(E.proj_r[v], 2, 0, p.rch[v]));
+            if (p.slen[p.lch[v]] > 0) reads_up(E.proj_l[v], 2, 0, p.lch[v]);
+            if (p.slen[p.rch[v]] > 0) reads_up(E.proj_r[v], 2, 0, p.rch[v]);
         }
-        g_up[v] = add_group(F64_WSKEL, E.node8[v], p.slen[v], s, 0, c_up + v, -1, 0, -1);
+        g_up[v] = end_group(F64_WSKEL, E.node8[v], p.slen[v], 0, c_up + v, -1, 0, 0);
     }
-    std::vector<std::vector<int>> far_of(p.numnodes), near_of(p.nleaf);
-    for (size_t k = 0; k < p.far_x.size(); ++k) far_of[adjoint ? p.far_y[k] : p.far_x[k]].push_back((int)k);
-    for (size_t k = 0; k < p.near_x.size(); ++k) near_of[adjoint ? p.near_y[k] : p.near_x[k]].push_back((int)k);
+    // the pairs of each output block: far by node, near by leaf
+    auto by_output = [](const std::vector<int> &x, int n, std::vector<int> &first, std::vector<int> &pair) {
+        first.assign(n + 1, 0);
+        for (int v : x) ++first[v + 1];
+        for (int i = 0; i < n; ++i) first[i + 1] += first[i];
+        pair.resize(x.size());
+        std::vector<int> at(first.begin(), first.end() - 1);
+        for (size_t k = 0; k < x.size(); ++k) pair[at[x[k]]++] = (int)k;
+    };
+    std::vector<int> far0, far_of, near0, near_of;
+    by_output(adjoint ? p.far_y : p.far_x, p.numnodes, far0, far_of);
+    by_output(adjoint ? p.near_y : p.near_x, p.nleaf, near0, near_of);
     for (int v : p.bfs) {
         if (!projects(v)) continue;
-        std::vector<Src> s;
-        for (int k : far_of[v]) {
-            const int o = adjoint ? p.far_x[k] : p.far_y[k];
-            if (p.slen[o] > 0) s.push_back(up_src(E.far[k], 1, adjoint ? 1 : 0, o));
+        begin_group();
+        for (int q = far0[v]; q < far0[v + 1]; ++q) {
+            const int k = far_of[q], o = adjoint ? p.far_x[k] : p.far_y[k];
+            if (p.slen[o] > 0) reads_up(E.far[k], 1, adjoint ? 1 : 0, o);
         }
-        if (s.empty() && has_down(v)) continue;
-        g_far[v] = add_group(F64_USKEL, E.node8[v], p.slen[v], s, 0, has_down(v) ? c_far + v : c_u + v, -1, 0, -1);
+        if ((int)items.size() == item0 && has_down(v)) continue;
+        g_far[v] = end_group(F64_USKEL, E.node8[v], p.slen[v], 0, has_down(v) ? c_far + v : c_u + v, -1, 0, 0);
         if (!has_down(v)) g_u[v] = g_far[v];
     }
     for (int v : p.bfs) {  // parents before children
         if (!projects(v) || !has_down(v)) continue;
         const int q = p.parent[v];
         const bool far = g_far[v] >= 0;
-        g_u[v] = add_group(F64_USKEL, E.node8[v], p.slen[v],
-                           {u_src(v == p.rch[q] ? E.proj_r[q] : E.proj_l[q], 2, 1, q)}, far ? 1 : 0, c_u + v,
-                           far ? c_far + v : -1, WR * row_tiles(p.slen[v]), g_far[v]);
+        begin_group();
+        reads_u(v == p.rch[q] ? E.proj_r[q] : E.proj_l[q], 2, 1, q);
+        reads_group(g_far[v]);
+        g_u[v] = end_group(F64_USKEL, E.node8[v], p.slen[v], far ? 1 : 0, c_u + v, far ? c_far + v : -1,
+                           WR * row_tiles(p.slen[v]), 0);
     }
     std::vector<int> leaf_node(p.nleaf, -1);
     for (int v = 0; v < p.numnodes; ++v)
         if (p.lch[v] == -1) leaf_node[p.lm[v]] = v;
     for (int i = 0; i < p.nleaf; ++i) {
-        std::vector<Src> s;
-        for (int k : near_of[i]) s.push_back(w_src(E.near[k], 0, adjoint ? 1 : 0, adjoint ? p.near_x[k] : p.near_y[k]));
-        g_near[i] = add_group(F64_Y, i, p.Ddim[i], s, 2, c_near + i, -1, 0, -1);
+        begin_group();
+        for (int q = near0[i]; q < near0[i + 1]; ++q) {
+            const int k = near_of[q];
+            reads_w(E.near[k], 0, adjoint ? 1 : 0, adjoint ? p.near_x[k] : p.near_y[k]);
+        }
+        g_near[i] = end_group(F64_Y, i, p.Ddim[i], 2, c_near + i, -1, 0, 0);
         const int v = leaf_node[i];
-        if (projects(v))
-            add_group(F64_Y, i, p.Ddim[i], {u_src(E.proj_l[v], 2, 1, v)}, 1, -1, c_near + i, WR * row_tiles(p.Ddim[i]), g_near[i]);
+        if (!projects(v)) continue;
+        begin_group();
+        reads_u(E.proj_l[v], 2, 1, v);
+        reads_group(g_near[i]);
+        end_group(F64_Y, i, p.Ddim[i], 1, -1, c_near + i, WR * row_tiles(p.Ddim[i]), 0);
     }
 
     // Long sums are cut along K where one would keep a block busy for a large part of the
     // launch: pieces of about an eighth of a block's share of all stages, at least 256 deep
-    // (N = 32768 adjoint, 64 right-hand sides: 707 us; a third of the share: 800 us; sixteenths
-    // only add partial tiles).
-    const int blocks = sm_count() * sh.ctas;
+    // (N = 32768 adjoint, 64 right-hand sides: 707 us when this was chosen; a third of the share:
+    // 800 us; sixteenths only add partial tiles).
+    const int blocks = sm_count() * sh.ctas, ngroup = (int)G.size();
     int64_t total = 0;
-    for (const Group &g : G)
-        for (const F64Task &t : g.tasks) total += (int64_t)t.stages * sh.ncol;
+    for (const F64Task &t : all) total += (int64_t)t.stages * sh.ncol;
     const int chunk = (int)std::max<int64_t>(32 / sh.bk8, total / (8 * (int64_t)blocks));
     slots = 0;
+    std::vector<F64Item> src;
+    std::vector<F64Task> tiles, range;
     for (Group &g : G) {
-        const F64Task t0 = g.tasks[0];
+        const F64Task t0 = all[g.task0];
         if (t0.stages <= chunk + chunk / 2) continue;
         const int n = (t0.stages + chunk - 1) / chunk;
         // item ranges of the pieces, cut at stage boundaries
-        std::vector<std::pair<int, int>> range;  // item0, nitem
-        std::vector<int> len;
+        src.assign(items.begin() + t0.item0, items.begin() + t0.item0 + t0.nitem);
+        range.assign(n, t0);
         int q = 0, off = 0;
-        const std::vector<F64Item> src(items.begin() + t0.item0, items.begin() + t0.item0 + t0.nitem);
         for (int i = 0; i < n; ++i) {
+            F64Task &r = range[i];
             int want = (int)((int64_t)t0.stages * (i + 1) / n) - (int)((int64_t)t0.stages * i / n);
-            range.push_back({(int)items.size(), 0});
-            len.push_back(want);
+            r.item0 = (int)items.size();
+            r.stages = want;
             while (want > 0) {
                 F64Item it = src[q];
                 const int have = stages_of(it.k8 - off), take = std::min(want, have);
@@ -934,7 +942,6 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
                 it.b_base += off;
                 it.k8 = std::min(take * sh.bk8, it.k8 - off);
                 items.push_back(it);
-                ++range.back().second;
                 want -= take;
                 off += take * sh.bk8;
                 if (take == have) {
@@ -942,24 +949,25 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
                     off = 0;
                 }
             }
+            r.nitem = (int)items.size() - r.item0;
         }
-        std::vector<F64Task> pieces;
-        for (const F64Task &base : g.tasks) {
+        tiles.assign(all.begin() + g.task0, all.begin() + g.task0 + g.ntask);
+        g.task0 = (int)all.size();
+        g.ntask *= n;
+        for (const F64Task &base : tiles) {
             for (int i = 0; i < n; ++i) {
-                F64Task t = base;
-                t.item0 = range[i].first;
-                t.nitem = range[i].second;
-                t.stages = len[i];
+                F64Task t = range[i];
+                t.r8 = base.r8;
+                t.m8 = base.m8;
                 t.piece = i;
                 t.npiece = n;
                 t.piece_ctr = nctr;
                 t.slot = (int)slots;
-                pieces.push_back(t);
+                all.push_back(t);
             }
             nctr += WARPS;  // one arrival counter per product warp
             slots += n;
         }
-        g.tasks = std::move(pieces);
     }
 
     // List scheduling, longest remaining path first among the groups whose inputs are written.  A
@@ -968,63 +976,70 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     // Times in stages of a busy SM (1.0 - 1.5 us): writing a tile out and publishing it takes
     // about EPILOGUE, seeing it and loading from it about LATENCY.
     const int EPILOGUE = sh.bn == 8 ? 4 : 2, LATENCY = 2, DEPTH = 3;
-    for (int i = 0; i < (int)G.size(); ++i) {
-        Group &g = G[i];
-        for (const F64Task &t : g.tasks) g.cost = std::max(g.cost, t.stages + EPILOGUE + LATENCY);
-        for (int d : g.deps) G[d].cons.push_back(i);
-        g.unplaced = (int)g.deps.size();
+    std::vector<int> prio(ngroup, 0), ready_at(ngroup, 0), unplaced(ngroup), con0(ngroup + 1, 0), cons(deps.size());
+    for (int i = ngroup - 1; i >= 0; --i) {  // (readers come after what they read)
+        const Group &g = G[i];
+        int cost = 0;
+        for (int t = g.task0; t < g.task0 + g.ntask; ++t) cost = std::max(cost, all[t].stages);
+        prio[i] += cost + EPILOGUE + LATENCY;
+        unplaced[i] = g.ndep;
+        for (int d = g.dep0; d < g.dep0 + g.ndep; ++d) {
+            prio[deps[d]] = std::max(prio[deps[d]], prio[i]);
+            ++con0[deps[d] + 1];
+        }
     }
-    std::function<double(int)> prio = [&](int i) -> double {
-        Group &g = G[i];
-        if (g.prio >= 0) return g.prio;
-        double best = 0;
-        for (int c : g.cons) best = std::max(best, prio(c));
-        return g.prio = best + g.cost;
-    };
-    for (int i = 0; i < (int)G.size(); ++i) prio(i);
-    struct Worker {
-        double claim, free;
-        bool operator>(const Worker &o) const { return claim > o.claim; }
-    };
-    auto low = [&](int a, int b) { return G[a].prio != G[b].prio ? G[a].prio < G[b].prio : a > b; };
-    auto late = [&](int a, int b) { return G[a].ready != G[b].ready ? G[a].ready > G[b].ready : a > b; };
-    std::priority_queue<int, std::vector<int>, decltype(low)> ready(low);
-    std::priority_queue<int, std::vector<int>, decltype(late)> waiting(late);
-    std::priority_queue<Worker, std::vector<Worker>, std::greater<Worker>> workers;
-    for (int i = 0; i < std::max(1, blocks / sh.ncol); ++i) workers.push(Worker{0.0, 0.0});
-    for (int i = 0; i < (int)G.size(); ++i)
-        if (!G[i].unplaced) waiting.push(i);
+    for (int i = 0; i < ngroup; ++i) con0[i + 1] += con0[i];
+    {
+        std::vector<int> at(con0.begin(), con0.end() - 1);
+        for (int i = 0; i < ngroup; ++i)
+            for (int d = G[i].dep0; d < G[i].dep0 + G[i].ndep; ++d) cons[at[deps[d]]++] = i;
+    }
+    // the highest priority, then the first group; the earliest time, then the first group
+    std::priority_queue<std::pair<int, int>> ready, waiting;
+    // Workers by the time they claim at, which only grows: lists per time, walked in order.
+    const int nworker = std::max(1, blocks / sh.ncol);
+    std::vector<int> at(1, 0), next(nworker), free_at(nworker, 0);  // first worker of a time, the one after
+    for (int w = 0; w < nworker; ++w) next[w] = w + 1 < nworker ? w + 1 : -1;
+    int now = 0;
+    for (int i = 0; i < ngroup; ++i)
+        if (!unplaced[i]) waiting.push({0, -i});
     out.clear();
-    for (size_t placed = 0; placed < G.size(); ++placed) {
-        const double now = workers.top().claim;
-        while (!waiting.empty() && G[waiting.top()].ready <= now) {
-            ready.push(waiting.top());
+    out.reserve(all.size());
+    for (int placed = 0; placed < ngroup; ++placed) {
+        while (at[now] < 0) ++now;
+        while (!waiting.empty() && -waiting.top().first <= now) {
+            const int i = -waiting.top().second;
             waiting.pop();
+            ready.push({prio[i], -i});
         }
         int i;
         if (!ready.empty()) {
-            i = ready.top();
+            i = -ready.top().second;
             ready.pop();
         } else if (!waiting.empty()) {
-            i = waiting.top();
+            i = -waiting.top().second;
             waiting.pop();
         } else {
             return fail("FP64 schedule: a block's inputs are never written", MXB_ERR_STRUCTURE);
         }
-        Group &g = G[i];
-        for (const F64Task &t : g.tasks) {
-            Worker w = workers.top();
-            workers.pop();
-            const double load = std::max(w.claim, g.ready), end = std::max(load + 1, w.free) + t.stages;
-            w.claim = std::max(load, end - DEPTH);
-            w.free = end + EPILOGUE;
-            workers.push(w);
-            g.finish = std::max(g.finish, w.free);
-            out.push_back(t);
+        const Group &g = G[i];
+        int finish = 0;
+        for (int t = g.task0; t < g.task0 + g.ntask; ++t) {
+            while (at[now] < 0) ++now;
+            const int w = at[now], load = std::max(now, ready_at[i]);
+            const int end = std::max(load + 1, free_at[w]) + all[t].stages, claim = std::max(load, end - DEPTH);
+            at[now] = next[w];
+            if (claim >= (int)at.size()) at.resize(claim + claim / 2 + 1, -1);
+            next[w] = at[claim];
+            at[claim] = w;
+            free_at[w] = end + EPILOGUE;
+            finish = std::max(finish, free_at[w]);
+            out.push_back(all[t]);
         }
-        for (int c : g.cons) {
-            G[c].ready = std::max(G[c].ready, g.finish + LATENCY);
-            if (--G[c].unplaced == 0) waiting.push(c);
+        for (int q = con0[i]; q < con0[i + 1]; ++q) {
+            const int c = cons[q];
+            ready_at[c] = std::max(ready_at[c], finish + LATENCY);
+            if (--unplaced[c] == 0) waiting.push({-ready_at[c], -c});
         }
     }
     return MXB_OK;
