@@ -10,6 +10,7 @@
 from __future__ import annotations
 
 import ctypes
+from concurrent.futures import ThreadPoolExecutor
 from typing import Optional
 
 import numpy as np
@@ -259,7 +260,7 @@ def kernel_matrices(dX, kernel, row_sets, col_sets, stream=None):
     return dst, ofs
 
 
-_PINNED_RESULT_BYTES = 256 << 20
+_STAGING_BYTES = 32 << 20  # page-locked memory that results come to the host through
 
 
 def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
@@ -285,25 +286,37 @@ def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
                                      _stream_ptr(stream)), "mxb_batched_id")
     ranks = dRank.cpu().numpy()
     piv = dPiv.cpu().numpy()
-    # row-major copies of the used parts, packed on the device and brought over in one copy.  Into
-    # page-locked memory (the arrays returned are views of it) where that is a moderate amount:
-    # a pageable copy of 31 MB and the host transposes of 32 nodes took 21 ms, this 1 ms
+    # row-major copies of the used parts, packed on the device and brought over through page-locked
+    # staging into arrays of their own: a caller that keeps one P keeps no other, and no page-locked
+    # memory.  The time goes to new pages, which several threads fault in: 32 nodes of 1024 x 512, rank
+    # 256 (31 MB), with the IDs, 9.0 ms, 10.8 ms where the results are kept (one thread: 9.0 and 21 ms;
+    # views of page-locked memory: 6.4 and 19.7 ms)
     sizes = ranks.astype(np.int64) * nc
-    packed = torch.empty(int(sizes.sum()), dtype=torch.float64, device=pool.device)
-    q = p = 0
-    for b in range(len(shapes)):
-        s, c = int(ranks[b]), int(nc[b])
-        packed[q:q + s * c].view(s, c).copy_(dP[p:p + s * c].view(c, s).t())
-        q += s * c
-        p += int(pmax[b]) * c
-    host = torch.empty(packed.shape, dtype=torch.float64, pin_memory=packed.numel() * 8 <= _PINNED_RESULT_BYTES)
-    Pall = host.copy_(packed).numpy()
-    out, q, p = [], 0, 0
-    for b in range(len(shapes)):
-        s, c = int(ranks[b]), int(nc[b])
-        out.append((piv[q:q + s].astype(np.int64), Pall[p:p + s * c].reshape(s, c)))
-        q += c
-        p += s * c
+    src = np.concatenate([[0], np.cumsum(pmax * nc)]).astype(np.int64)
+    out, b, q = [], 0, 0
+    while b < len(shapes):
+        e, total = b + 1, int(sizes[b])
+        while e < len(shapes) and (total + int(sizes[e])) * 8 <= _STAGING_BYTES:
+            total += int(sizes[e])
+            e += 1
+        packed = torch.empty(total, dtype=torch.float64, device=pool.device)
+        at = 0
+        for k in range(b, e):
+            s, c = int(ranks[k]), int(nc[k])
+            packed[at:at + s * c].view(s, c).copy_(dP[src[k]:src[k] + s * c].view(c, s).t())
+            at += s * c
+        host = torch.empty(total, dtype=torch.float64, pin_memory=total * 8 <= _STAGING_BYTES)
+        parts = np.split(host.copy_(packed).numpy(), np.cumsum(sizes[b:e - 1]))
+        parts = [x.reshape(int(ranks[k]), int(nc[k])) for k, x in zip(range(b, e), parts)]
+        if total * 8 > 1 << 20:
+            with ThreadPoolExecutor(8) as threads:
+                parts = list(threads.map(np.copy, parts))
+        else:
+            parts = [x.copy() for x in parts]
+        for k, x in zip(range(b, e), parts):
+            out.append((piv[q:q + x.shape[0]].astype(np.int64), x))
+            q += x.shape[1]
+        b = e
     return out
 
 

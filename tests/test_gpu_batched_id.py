@@ -157,3 +157,19 @@ def test_batched_id_beside_other_work(torch):
         for (a, P), (b, Q) in zip(want, got):
             assert np.array_equal(a, b) and np.array_equal(P, Q)
     side.synchronize()
+
+
+@pytest.mark.parametrize("staging", [None, 40000, 8])
+def test_results_own_their_memory(torch, monkeypatch, staging):
+    """Each P is an array of its own, whatever pieces the results come over in (all at once, a few
+    nodes, each node larger than the staging)."""
+    if staging is not None:
+        monkeypatch.setattr(H, "_STAGING_BYTES", staging)
+    shapes = [(60 + b, 40 - b) for b in range(9)]
+    rng = np.random.default_rng(8)
+    mats = [rng.standard_normal(s) for s in shapes]
+    pool = torch.as_tensor(np.concatenate([m.reshape(-1, order="F") for m in mats]), device="cuda")
+    for m, (piv, P) in zip(mats, H.batched_id(pool, shapes, 1e-9, 24)):
+        hpiv, hP = S.interpolative_decomposition(np.asfortranarray(m), 1e-9, 24)
+        assert np.array_equal(piv, hpiv) and np.abs(P - hP).max() <= 1e-8 * max(1.0, np.abs(hP).max())
+        assert P.base is None and P.flags.owndata and P.flags.c_contiguous and P.flags.writeable
