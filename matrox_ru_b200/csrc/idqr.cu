@@ -732,8 +732,13 @@ void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int coun
 // Blocks per node for the cluster kernel (0: it does not take these nodes), the nodes' panel widths
 // and the shared memory: the most blocks for which every node's cluster is resident at once, each
 // with at least 16 columns.  Ranks above SOLVE_MAX, and nodes so tall that shared memory holds
-// fewer than 4 panel vectors (above ~5500 rows), stay with the kernel of one block per node.
-int choose_cluster(std::vector<IdJob> &jobs, int max_rank, int maxc, size_t &smem_doubles)
+// fewer than 4 panel vectors (above ~5500 rows), stay with the kernel of one block per node.  So do
+// levels of many small nodes, whose columns wait for one block's steps either way: that kernel's
+// blocks are half as large and a step has fewer barriers.  Kernel of one block per node / this one:
+// 256 threads and more nodes than SMs: 2048 nodes of 64 x 32 0.98 / 1.99 ms; 300 of 128 x 64 0.85 /
+// 1.44, of 160 x 80 1.26 / 1.31, of 200 x 100 2.09 / 1.92; 1024 of 200 x 100 5.04 / 6.69, of 224 x 112
+// 6.91 / 5.47; 256 of 512 x 256 34.9 / 7.0.
+int choose_cluster(std::vector<IdJob> &jobs, int max_rank, int maxc, int sms, size_t &smem_doubles)
 {
     constexpr size_t LIMIT = 225 * 1024 / sizeof(double);
     if (std::min(max_rank, maxc) > SOLVE_MAX) return 0;
@@ -742,6 +747,10 @@ int choose_cluster(std::vector<IdJob> &jobs, int max_rank, int maxc, size_t &sme
         (void)cudaGetLastError();
         return 0;
     }
+    int64_t largest = 0;
+    for (const IdJob &j : jobs) largest = std::max(largest, (int64_t)j.nrows * j.ncols);
+    const int count = (int)jobs.size();
+    const bool many_small = count >= sms && (largest <= 128 * 64 || (count > 3 * sms && largest <= 200 * 100));
     for (int C = MAX_CLUSTER; C >= 1; C >>= 1) {
         if (C > 1 && maxc < 16 * C) continue;
         smem_doubles = 0;
@@ -754,16 +763,16 @@ int choose_cluster(std::vector<IdJob> &jobs, int max_rank, int maxc, size_t &sme
             smem_doubles = std::max(smem_doubles, cl_smem_doubles(j.nrows, j.ncols, C, j.panel));
         }
         if (!fits) continue;
-        if (C == 1) return 1;
+        if (C == 1) return many_small ? 0 : 1;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
-        cluster_config(cfg, attr, (int)jobs.size(), C, smem_doubles * sizeof(double), nullptr);
+        cluster_config(cfg, attr, count, C, smem_doubles * sizeof(double), nullptr);
         int resident = 0;
         if (cudaOccupancyMaxActiveClusters(&resident, id_cluster_kernel, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             continue;
         }
-        if (resident >= (int)jobs.size()) return C;
+        if (resident >= count) return C;
     }
     return 0;
 }
@@ -801,15 +810,15 @@ extern "C" int32_t mxb_batched_id(double *dA, const int32_t *nrows, const int32_
         maxc = std::max(maxc, nc);
     }
     cudaStream_t s = (cudaStream_t)stream;
+    int dev = 0, sms = 148;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     size_t cl_smem = 0;
-    const int cluster = choose_cluster(jobs, max_rank, maxc, cl_smem);
+    const int cluster = choose_cluster(jobs, max_rank, maxc, sms, cl_smem);
     IdJob *dJobs = nullptr;
     double *dZ = nullptr;
-    cudaError_t e = cudaMallocAsync(&dJobs, jobs.size() * sizeof(IdJob), s);
+    if (e == cudaSuccess) e = cudaMallocAsync(&dJobs, jobs.size() * sizeof(IdJob), s);
     if (e == cudaSuccess) e = cudaMallocAsync(&dZ, std::max<uint64_t>(p, 1) * sizeof(double), s);
-    int dev = 0, sms = 148;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (cluster) {
         const size_t smem = cl_smem * sizeof(double);
         if (e == cudaSuccess)

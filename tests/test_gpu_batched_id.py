@@ -173,3 +173,19 @@ def test_results_own_their_memory(torch, monkeypatch, staging):
         hpiv, hP = S.interpolative_decomposition(np.asfortranarray(m), 1e-9, 24)
         assert np.array_equal(piv, hpiv) and np.abs(P - hP).max() <= 1e-8 * max(1.0, np.abs(hP).max())
         assert P.base is None and P.flags.owndata and P.flags.c_contiguous and P.flags.writeable
+
+
+@pytest.mark.parametrize("count,nr,nc", [(160, 128, 64), (160, 129, 64), (460, 200, 100), (460, 201, 100)])
+def test_batched_id_of_many_nodes(torch, count, nr, nc):
+    """Both sides of the lines between the two kernels for levels of more nodes than SMs."""
+    rng = np.random.default_rng(count + nr)
+    X = S.gaussian_mixture(2048, 5, 5, -2.0, 2.0, 0.3, 1.0, seed=nc)
+    sets = [(rng.choice(2048, nr, replace=False), rng.choice(2048, nc, replace=False)) for _ in range(count)]
+    K, _ = H.kernel_matrices(torch.as_tensor(X, device="cuda"), S.KernelSpec("imq", 0.3), [a for a, _ in sets], [b for _, b in sets])
+    mats = K[:count * nr * nc].cpu().numpy().reshape(count, nc, nr)
+    got = H.batched_id(K, [(nr, nc)] * count, 1e-9, 48)
+    for b in range(0, count, count // 3):
+        hpiv, hP = S.interpolative_decomposition(np.asfortranarray(mats[b].T), 1e-9, 48)
+        piv, P = got[b]
+        assert np.array_equal(piv, hpiv), b
+        assert float(np.abs(P - hP).max()) <= 1e-8 * max(1.0, float(np.abs(hP).max())), b
