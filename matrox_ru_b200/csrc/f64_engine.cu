@@ -18,8 +18,8 @@
 // product warps execute nothing but shared-memory reads and DMMAs.
 //
 // Schedule.  The tasks of all passes (rewriting W, up-sweep, far couplings, near field,
-// down-sweep, leaf down) form one list; a unit is a task and a column tile, claimed in list
-// order.  Units wait on per-node counters for the blocks they read, so no pass waits for the
+// down-sweep, leaf down) form one list; a unit is a task and a column tile (two where there are very
+// many), claimed in list order.  Units wait on per-node counters for the blocks they read, so no pass waits for the
 // last tile of the pass before.  The list comes from a list-scheduling simulation on the host
 // (longest remaining path first), every unit's inputs come earlier in it and a block runs its
 // units in claim order, so every wait ends; each is bounded all the same.  A long sum (a node
@@ -52,19 +52,20 @@ enum { CTL_CLAIM = 0, CTL_EXIT = 1, CTL_FIRST = 16 };
 constexpr int WARPS = 4, THREADS = (WARPS + 1) * 32, RING = 4;
 constexpr int EAGER = 64;  // polls of a node counter before the first pause
 
-// BN: right-hand sides of a column tile.  BK8: sub-block columns of A per stage.  32 is the widest
-// tile: with 64 columns a unit takes twice as long on a shared SM, which the tree sweeps wait
-// for (N = 65536, 1024 right-hand sides: 24.2 ms against 23.3 ms; N = 16384 HSS, 256: 376 against
-// 354 us), and 16 re-reads A too often (418 us).  Stages of 4 sub-block columns beat 2 (24.8 ms)
+// BN: right-hand sides of a column tile.  M8: sub-block rows of a row tile.  BK8: sub-block columns of
+// A per stage.  64 rows x 32 columns for tall blocks: with 64 columns a unit takes twice as long on a
+// shared SM, which the tree sweeps wait for (N = 65536, 1024 right-hand sides: 24.2 ms against 23.3
+// ms; N = 16384 HSS, 256: 376 against 354 us), and 16 re-reads A too often (418 us).  The same area as
+// 32 x 64 and 16 x 128 for short blocks (shape_for).  Stages of 4 sub-block columns beat 2 (24.8 ms)
 // because a warp pays ~100 cycles to move to the next stage; 3 blocks of 12 product warps per SM
 // beat 4 without fragment double-buffering (26.4 ms) and 2 (25 ms).
-template <int BN>
+template <int BN, int M8_ = 8>
 struct Cfg {
-    static constexpr int N8 = BN / 8;
-    static constexpr int WN = N8 >= 4 ? 2 : 1, WM = WARPS / WN;   // product warps: rows x columns
-    static constexpr int MI = 8 / WM, NJ = N8 / WN;               // sub-blocks per warp
-    static constexpr int BK8 = 4;
-    static constexpr int A_BYTES = BK8 * 8 * 512, B_BYTES = BK8 * N8 * 512;
+    static constexpr int M8 = M8_, N8 = BN / 8;
+    static constexpr int WN = M8 < 8 ? 4 : (N8 >= 4 ? 2 : 1), WM = WARPS / WN;  // product warps: rows x columns
+    static constexpr int MI = M8 / WM, NJ = N8 / WN;              // sub-blocks per warp
+    static constexpr int BK8 = M8 == 2 ? 2 : 4;
+    static constexpr int A_BYTES = BK8 * M8 * 512, B_BYTES = BK8 * N8 * 512;
     static constexpr int STAGE = A_BYTES + B_BYTES;
     static constexpr int STAGES = 3;
     static constexpr int CTAS = N8 >= 2 ? 3 : 4;                  // resident per SM
@@ -82,16 +83,19 @@ struct Args {
     double *partial;
     int *ctl, *err;
     long long wait_cycles;
-    int units, ncol, nb, nrhs, beta, nctr;
+    int units, ncol, group, nb, nrhs, beta, nctr;  // group: column tiles of a unit (at most 32)
     // profiling (null otherwise): [0] the earliest block's start, [1 + p] the time the last tile of
     // pass p was written (%globaltimer, ns); the pass of each task
     unsigned long long *pass_ns;
     const uint8_t *pass_of;
 };
 
-struct Unit {  // ring slot: the claimed unit
+struct Unit {  // ring slot: one column tile of the claimed unit
     F64Task task;
-    int32_t col, n8_0, n8, live, index, pad;
+    int32_t col, n8_0, n8;
+    int32_t live;   // 0: no more units, 1: more column tiles of the unit follow, 2: its last one
+    int32_t index;  // of the task
+    int32_t col0;   // the unit's first column tile
 };
 
 // Two stacked 8 x 8 sub-blocks of A (rows g and g + 8 of a lane's fragment) times one of B.
@@ -105,10 +109,10 @@ __device__ __forceinline__ void dmma(double (&c)[2], double (&d)[2], const doubl
 
 __device__ __forceinline__ int b_elem(int k, int n) { return n * 8 + (k ^ (((n >> 1) & 1) << 2)); }
 
-template <int BN>
-__global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(const Args g)
+template <int BN, int M8>
+__global__ void __launch_bounds__(THREADS, Cfg<BN, M8>::CTAS) f64_dataflow_kernel(const Args g)
 {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, M8>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::STAGES * C::STAGE);
     uint64_t *empty = full + C::STAGES;
@@ -141,89 +145,95 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
         // ---------------- producer: claims units, fills the stages ----------------
         uint32_t st = 0;  // stages filled
         int slot = 0;
-        bool ok = true;
-        while (ok) {
+        const int ngroup = (g.ncol + g.group - 1) / g.group;  // units of a task
+        bool ok = true, more = true;
+        while (ok && more) {
             // claimed once the loads of the unit before are on their way, not earlier: a unit held
             // back behind another would keep the units that read it waiting
             int u = 0;
             if (lane == 0) u = atomicAdd(g.ctl + CTL_CLAIM, 1);
             u = __shfl_sync(0xffffffffu, u, 0);
-            const int i = slot % RING;
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(&uempty[i], ((slot / RING) & 1) ^ 1, abort_word, g.wait_cycles));
-            if (!ok) break;
-            ++slot;
-            Unit &un = ring[i];
-            if (u >= g.units) {
-                if (lane == 0) un.live = 0;
+            const int t = u / ngroup, col0 = (u - t * ngroup) * g.group;
+            const bool done = u >= g.units;
+            const int col1 = done ? col0 + 1 : min(g.ncol, col0 + g.group);
+            const int word = !done && lane < 16 ? __ldg(reinterpret_cast<const int *>(g.tasks + t) + lane) : 0;
+            for (int col = col0; col < col1 && ok; ++col) {
+                const int i = slot % RING;
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(&uempty[i], ((slot / RING) & 1) ^ 1, abort_word, g.wait_cycles));
+                if (!ok) break;
+                ++slot;
+                Unit &un = ring[i];
+                // column tiles of nearly equal width: sub-blocks [n8_0, n8_0 + n8)
+                const int n8_0 = (int)((long long)g.nb * col / g.ncol);
+                const int n8 = (int)((long long)g.nb * (col + 1) / g.ncol) - n8_0;
+                if (lane < 16) reinterpret_cast<int *>(&un.task)[lane] = word;
+                if (lane == 16) un.col = col;
+                if (lane == 17) un.n8_0 = n8_0;
+                if (lane == 18) un.n8 = n8;
+                if (lane == 19) un.live = done ? 0 : 1 + (col + 1 == col1);
+                if (lane == 20) un.index = t;
+                if (lane == 21) un.col0 = col0;
                 __syncwarp();
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&ufull[i])) : "memory");
-                break;
-            }
-            const int t = u / g.ncol, col = u - t * g.ncol;
-            // column tiles of nearly equal width: sub-blocks [n8_0, n8_0 + n8)
-            const int n8_0 = (int)((long long)g.nb * col / g.ncol);
-            const int n8 = (int)((long long)g.nb * (col + 1) / g.ncol) - n8_0;
-            if (lane < 16)
-                reinterpret_cast<int *>(&un.task)[lane] = __ldg(reinterpret_cast<const int *>(g.tasks + t) + lane);
-            if (lane == 16) un.col = col;
-            if (lane == 17) un.n8_0 = n8_0;
-            if (lane == 18) un.n8 = n8;
-            if (lane == 19) un.live = 1;
-            if (lane == 20) un.index = t;
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&ufull[i])) : "memory");
-            const int item0 = un.task.item0, nitem = un.task.nitem, r8 = un.task.r8, m8 = un.task.m8;
-            for (int q = 0; q < nitem && ok; ++q) {
-                const F64Item it = g.items[item0 + q];
-                const double *a0 = it.a_pool == 0 ? g.pool[0] : (it.a_pool == 1 ? g.pool[1] : g.pool[2]);
-                const double *b0 = it.b_buf == 0 ? g.buf[0] : (it.b_buf == 1 ? g.buf[1] : g.buf[2]);
-                const uint8_t *A = reinterpret_cast<const uint8_t *>(a0 + it.a_off * 64);
-                const uint8_t *B = reinterpret_cast<const uint8_t *>(b0 + (it.b_base * g.nb + n8_0) * 64);
-                // stage f of the item: the CDS side (and the byte count of both), then B
-                auto load_a = [&](uint32_t f, int k0) {
-                    const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
-                    uint8_t *sa = smem + s * C::STAGE;
-                    if (lane == 0) {
-                        meta[s] = nk | (it.trans << 8);
-                        tc::mbar_expect_tx(&full[s], (uint32_t)(nk * (m8 + n8) * 512));
-                    }
-                    __syncwarp();
-                    if (it.trans) {  // one run per sub-block row of the tile
-                        if (lane < m8)
-                            tc::bulk_g2s(sa + lane * C::BK8 * 512, A + ((size_t)(r8 + lane) * it.lda + k0) * 512,
-                                         (uint32_t)nk * 512, &full[s]);
-                    } else if (lane < nk) {  // one run per sub-block column of the stage
-                        tc::bulk_g2s(sa + lane * 8 * 512, A + ((size_t)(k0 + lane) * it.lda + r8) * 512,
-                                     (uint32_t)m8 * 512, &full[s]);
-                    }
-                };
-                auto load_b = [&](uint32_t f, int k0) {
-                    const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
-                    if (lane < nk)
-                        tc::bulk_g2s(smem + s * C::STAGE + C::A_BYTES + lane * C::N8 * 512,
-                                     B + (size_t)(k0 + lane) * g.nb * 512, (uint32_t)n8 * 512, &full[s]);
-                };
-                int ahead = 0;  // sub-block columns whose A is on its way
-                if (it.dep >= 0) {
-                    const int *ctr = counters + it.dep * g.ncol + col;
-                    if (__any_sync(0xffffffffu, !tc::counter_reached(ctr, it.need))) {
-                        // B is not written yet: fill the free stages with A meanwhile
-                        for (uint32_t f = st; ahead < it.k8 && f < st + C::STAGES; ++f, ahead += C::BK8) {
-                            if (!__all_sync(0xffffffffu, tc::mbar_try_wait(&empty[f % C::STAGES], ((f / C::STAGES) & 1) ^ 1))) break;
-                            load_a(f, ahead);
+                if (done) {
+                    more = false;
+                    break;
+                }
+                const int item0 = un.task.item0, nitem = un.task.nitem, r8 = un.task.r8, m8 = un.task.m8;
+                for (int q = 0; q < nitem && ok; ++q) {
+                    const F64Item it = g.items[item0 + q];
+                    const double *a0 = it.a_pool == 0 ? g.pool[0] : (it.a_pool == 1 ? g.pool[1] : g.pool[2]);
+                    const double *b0 = it.b_buf == 0 ? g.buf[0] : (it.b_buf == 1 ? g.buf[1] : g.buf[2]);
+                    const uint8_t *A = reinterpret_cast<const uint8_t *>(a0 + it.a_off * 64);
+                    const uint8_t *B = reinterpret_cast<const uint8_t *>(b0 + (it.b_base * g.nb + n8_0) * 64);
+                    // stage f of the item: the CDS side (and the byte count of both), then B
+                    auto load_a = [&](uint32_t f, int k0) {
+                        const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
+                        uint8_t *sa = smem + s * C::STAGE;
+                        if (lane == 0) {
+                            meta[s] = nk | (it.trans << 8);
+                            tc::mbar_expect_tx(&full[s], (uint32_t)(nk * (m8 + n8) * 512));
+                        }
+                        __syncwarp();
+                        if (it.trans) {  // one run per sub-block row of the tile
+                            if (lane < m8)
+                                tc::bulk_g2s(sa + lane * C::BK8 * 512, A + ((size_t)(r8 + lane) * it.lda + k0) * 512,
+                                             (uint32_t)nk * 512, &full[s]);
+                        } else if (lane < nk) {  // one run per sub-block column of the stage
+                            tc::bulk_g2s(sa + lane * C::M8 * 512, A + ((size_t)(k0 + lane) * it.lda + r8) * 512,
+                                         (uint32_t)m8 * 512, &full[s]);
+                        }
+                    };
+                    auto load_b = [&](uint32_t f, int k0) {
+                        const int s = f % C::STAGES, nk = min(C::BK8, it.k8 - k0);
+                        if (lane < nk)
+                            tc::bulk_g2s(smem + s * C::STAGE + C::A_BYTES + lane * C::N8 * 512,
+                                         B + (size_t)(k0 + lane) * g.nb * 512, (uint32_t)n8 * 512, &full[s]);
+                    };
+                    int ahead = 0;  // sub-block columns whose A is on its way
+                    if (it.dep >= 0) {
+                        const int *ctr = counters + it.dep * g.ncol + col;
+                        // every lane takes its own acquire: each issues copies of its own
+                        if (__all_sync(0xffffffffu, tc::counter_reached(ctr, it.need))) {
+                            tc::fence_async_global();
+                        } else {
+                            // B is not written yet: fill the free stages with A meanwhile
+                            for (uint32_t f = st; ahead < it.k8 && f < st + C::STAGES; ++f, ahead += C::BK8) {
+                                if (!__all_sync(0xffffffffu, tc::mbar_try_wait(&empty[f % C::STAGES], ((f / C::STAGES) & 1) ^ 1))) break;
+                                load_a(f, ahead);
+                            }
+                            ok = __all_sync(0xffffffffu, tc::wait_counter(ctr, it.need, abort_word, g.wait_cycles, EAGER));
                         }
                     }
-                    // every lane takes its own acquire: each issues copies of its own
-                    ok = __all_sync(0xffffffffu, tc::wait_counter(ctr, it.need, abort_word, g.wait_cycles, EAGER));
-                }
-                for (int k0 = 0; k0 < it.k8; k0 += C::BK8, ++st) {
-                    if (k0 >= ahead) {
-                        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st % C::STAGES], ((st / C::STAGES) & 1) ^ 1,
-                                                                        abort_word, g.wait_cycles));
-                        if (!ok) break;
-                        load_a(st, k0);
+                    for (int k0 = 0; k0 < it.k8; k0 += C::BK8, ++st) {
+                        if (k0 >= ahead) {
+                            if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&empty[st % C::STAGES], ((st / C::STAGES) & 1) ^ 1,
+                                                                            abort_word, g.wait_cycles));
+                            if (!ok) break;
+                            load_a(st, k0);
+                        }
+                        load_b(st, k0);  // also after a failed wait: a stage that was begun is filled
                     }
-                    load_b(st, k0);  // also after a failed wait: a stage that was begun is filled
                 }
             }
         }
@@ -238,7 +248,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
         // ---------------- product warps ----------------
         const int wm = warp / C::WN, wn = warp % C::WN;
         const int fr = lane >> 2, fa = lane & 3;  // fragment row (A) or column (B), and k
-        uint32_t st = 0;
+        uint32_t st = 0, pend = 0;  // pend: column tiles of the unit written, not counted yet
         for (int slot = 0;; ++slot) {
             const int ri = slot % RING;
             if (!tc::mbar_wait_warp(&ufull[ri], (slot / RING) & 1, abort_word, g.wait_cycles)) {
@@ -337,7 +347,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
                                 a[h][i][0] = pa[(i * C::BK8 + k) * 64];
                                 a[h][i][1] = pa[(i * C::BK8 + k) * 64 + 32];
                             } else {
-                                const double2 v = *reinterpret_cast<const double2 *>(pa + (k * 8 + i) * 64);
+                                const double2 v = *reinterpret_cast<const double2 *>(pa + (k * C::M8 + i) * 64);
                                 a[h][i][0] = v.x;
                                 a[h][i][1] = v.y;
                             }
@@ -484,13 +494,15 @@ __global__ void __launch_bounds__(THREADS, Cfg<BN>::CTAS) f64_dataflow_kernel(co
                             }
                     }
                 }
-                if (sig >= 0) {
-                    asm volatile("fence.proxy.async.global;\n" ::: "memory");
-                    __threadfence();
-                    __syncwarp();
-                    if (lane == 0) atomicAdd(counters + sig * g.ncol + col, 1);
-                }
+                if (sig >= 0) pend |= 1u << (col - un.col0);
                 if (g.pass_ns && lane == 0) atomicMax(g.pass_ns + 1 + g.pass_of[un.index], tc::globaltimer_ns());
+            }
+            if (un.live == 2 && pend) {  // one fence for all column tiles of the unit
+                asm volatile("fence.proxy.async.global;\n" ::: "memory");
+                __threadfence();
+                __syncwarp();
+                if ((pend >> lane) & 1) atomicAdd(counters + sig * g.ncol + un.col0 + lane, 1);
+                pend = 0;
             }
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&uempty[ri])) : "memory");
@@ -562,36 +574,79 @@ int sm_count()
     return n[dev];
 }
 
-template <int BN>
+template <int BN, int M8 = 8>
 int launch(const Args &a, cudaStream_t stream)
 {
-    using C = Cfg<BN>;
+    using C = Cfg<BN, M8>;
     static bool configured[128];
     int dev = 0;
     F64_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 128) return fail("device index out of range");
     if (!configured[dev]) {
-        F64_CUDA(cudaFuncSetAttribute(f64_dataflow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        F64_CUDA(cudaFuncSetAttribute(f64_dataflow_kernel<BN, M8>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured[dev] = true;
     }
     const int grid = std::min(a.units, sm_count() * C::CTAS);
-    f64_dataflow_kernel<BN><<<grid, THREADS, C::SMEM, stream>>>(a);
+    f64_dataflow_kernel<BN, M8><<<grid, THREADS, C::SMEM, stream>>>(a);
     F64_CUDA(cudaGetLastError());
     return MXB_OK;
 }
 
-struct Shape {  // of the kernel variant that runs `nb` column sub-blocks
-    int bn, bk8, ctas, ncol;
+struct Shape {  // of the kernel variant and task list that run `nb` column sub-blocks
+    int bn, m8, bk8, ctas, wm, ncol;
+    bool fused = false;  // far and down, near and leaf down in one sum each
+    int group = 1;       // column tiles of a unit
 };
 
-// The narrowest variant that holds all columns (8, 16), else tiles of at most 32: below 17 right-hand
-// sides the launch is bound by the CDS bytes, and a wider tile only adds padding products (16
-// right-hand sides, N = 32768: 237 us; 32: 382 us).
-Shape shape_for(int nb)
+template <int BN, int M8 = 8>
+Shape shape_of(int nb)
 {
-    if (nb <= 1) return {8, Cfg<8>::BK8, Cfg<8>::CTAS, 1};
-    if (nb <= 2) return {16, Cfg<16>::BK8, Cfg<16>::CTAS, 1};
-    return {32, Cfg<32>::BK8, Cfg<32>::CTAS, (nb + 3) / 4};
+    using C = Cfg<BN, M8>;
+    return {BN, M8, C::BK8, C::CTAS, C::WM, (nb + C::N8 - 1) / C::N8};
+}
+
+// Row tiles of a block; tiles of all output blocks of an evaluation.
+int row_tiles_of(int rows, int m8) { return std::max(1, ((rows + 7) / 8 + m8 - 1) / m8); }
+int64_t tiles_of(const Plan &p, const Shape &s)
+{
+    int64_t n = 0;
+    for (int v : p.Ddim) n += 3 * row_tiles_of(v, s.m8);  // W, near field, leaf down
+    for (int v : p.slen) n += 3 * row_tiles_of(v, s.m8);  // up, far, down
+    return n * s.ncol;
+}
+
+// Columns: the narrowest variant that holds all of them (8, 16), else tiles of at most 32: below 17
+// right-hand sides the launch is bound by the CDS bytes, and a wider tile only adds padding products (16
+// right-hand sides, N = 32768: 237 us; 32: 382 us).
+//
+// Short blocks: a tile of 64 rows is mostly empty, and an evaluation is as many tiles, of 2 - 3 us each
+// whatever they hold.  Flatter, wider tiles where they cut the number of tiles by more than a quarter:
+// HSS of N = 16384, 1000 right-hand sides, leaves of 16 points 1804 -> 588 us (16 x 128), of 32 points
+// 1486 -> 917 (32 x 64; N = 65536, 512 columns 2159 -> 1309).
+//
+// Many tiles per block (of those resident): the launch is bound by tiles, not by the path through the
+// tree.  From 128 on, a block's far and down products, and its near and leaf down products, are one
+// sum, which a short path needs in two units: the far and near parts run while the sweeps arrive (N
+// = 16384 HSS, 256 columns, 41 per block: 347 us).  N = 65536 HSS, leaves of 64, 1000 columns 3273 ->
+// 2872 us, of 256 9371 -> 9106; H2-b, leaves of 256, 1024 columns (726 per block) 23.36 -> 23.14 ms.
+// From 512 on, a unit is two column tiles: one claim and one publication for both (2872 -> 2758 us,
+// 23.14 -> 23.07 ms; at 330 per block 4560 -> 4623).
+Shape shape_for(const Plan &p, int nb)
+{
+    if (nb <= 1) return shape_of<8>(nb);
+    if (nb <= 2) return shape_of<16>(nb);
+    Shape best = shape_of<32>(nb);
+    int64_t tiles = tiles_of(p, best);
+    for (const Shape &s : {shape_of<64, 4>(nb), shape_of<128, 2>(nb)}) {
+        const int64_t n = tiles_of(p, s);
+        if (4 * n >= 3 * tiles) continue;
+        best = s;
+        tiles = n;
+    }
+    const int64_t per_block = tiles / (sm_count() * best.ctas);
+    best.fused = per_block >= 128;
+    best.group = per_block >= 512 ? std::min(2, best.ncol) : 1;
+    return best;
 }
 
 // A group of the schedule: the tasks of one output block in one pass, and the groups it reads.
@@ -769,11 +824,12 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     auto projects = [&](int v) { return v != p.root && p.slen[v] > 0; };
     auto has_down = [&](int v) { return p.parent[v] >= 0 && projects(p.parent[v]); };
     auto ceil8 = [](int v) { return (v + 7) / 8; };
-    auto row_tiles = [&](int rows) { return std::max(1, (ceil8(rows) + 7) / 8); };
+    auto row_tiles = [&](int rows) { return row_tiles_of(rows, sh.m8); };
     // counters (times the column count): per leaf W tiled and near field written; per node
     // wskel, far part and uskel written
     const int c_w = 0, c_near = p.nleaf, c_up = 2 * p.nleaf, c_far = c_up + p.numnodes, c_u = c_far + p.numnodes;
     nctr = c_u + p.numnodes;
+    const bool fused = sh.fused;
     std::vector<Group> G;
     std::vector<F64Task> all;
     std::vector<int> deps;
@@ -872,13 +928,16 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
     std::vector<int> far0, far_of, near0, near_of;
     by_output(adjoint ? p.far_y : p.far_x, p.numnodes, far0, far_of);
     by_output(adjoint ? p.near_y : p.near_x, p.nleaf, near0, near_of);
-    for (int v : p.bfs) {
-        if (!projects(v)) continue;
-        begin_group();
+    auto reads_far = [&](int v) {
         for (int q = far0[v]; q < far0[v + 1]; ++q) {
             const int k = far_of[q], o = adjoint ? p.far_x[k] : p.far_y[k];
             if (p.slen[o] > 0) reads_up(E.far[k], 1, adjoint ? 1 : 0, o);
         }
+    };
+    for (int v : p.bfs) {
+        if (!projects(v) || (fused && has_down(v))) continue;
+        begin_group();
+        reads_far(v);
         if ((int)items.size() == item0 && has_down(v)) continue;
         g_far[v] = end_group(F64_USKEL, E.node8[v], p.slen[v], 0, has_down(v) ? c_far + v : c_u + v, -1, 0, 0);
         if (!has_down(v)) g_u[v] = g_far[v];
@@ -888,6 +947,7 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
         const int q = p.parent[v];
         const bool far = g_far[v] >= 0;
         begin_group();
+        if (fused) reads_far(v);
         reads_u(v == p.rch[q] ? E.proj_r[q] : E.proj_l[q], 2, 1, q);
         reads_group(g_far[v]);
         g_u[v] = end_group(F64_USKEL, E.node8[v], p.slen[v], far ? 1 : 0, c_u + v, far ? c_far + v : -1,
@@ -902,9 +962,10 @@ int build_schedule(Plan &p, bool adjoint, const Shape &sh, std::vector<F64Task> 
             const int k = near_of[q];
             reads_w(E.near[k], 0, adjoint ? 1 : 0, adjoint ? p.near_x[k] : p.near_y[k]);
         }
-        g_near[i] = end_group(F64_Y, i, p.Ddim[i], 2, c_near + i, -1, 0, 0);
         const int v = leaf_node[i];
-        if (!projects(v)) continue;
+        if (fused && projects(v)) reads_u(E.proj_l[v], 2, 1, v);
+        g_near[i] = end_group(F64_Y, i, p.Ddim[i], 2, c_near + i, -1, 0, 0);
+        if (fused || !projects(v)) continue;
         begin_group();
         reads_u(E.proj_l[v], 2, 1, v);
         reads_group(g_near[i]);
@@ -1109,7 +1170,7 @@ int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t 
 {
     F64Engine &E = *p.f64;
     const int nb = (nrhs + 7) / 8;
-    const Shape sh = shape_for(nb);
+    const Shape sh = shape_for(p, nb);
     bool capturing = false;
     int rc = is_capturing(stream, &capturing);
     if (rc) return rc;
@@ -1130,7 +1191,7 @@ int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t 
     // counters (zero between launches: each launch's last block clears what it used), then the
     // partial tiles
     const size_t ctl = ((CTL_FIRST + (size_t)s->nctr * sh.ncol) * sizeof(int) + 511) / 512 * 512;
-    const size_t partial = (size_t)s->slots * sh.ncol * 64 * sh.bn * sizeof(double);
+    const size_t partial = (size_t)s->slots * sh.ncol * 8 * sh.m8 * sh.bn * sizeof(double);
     if (ctl > E.ctl_bytes || partial > E.partial_bytes) {
         const size_t c = std::max(ctl, E.ctl_bytes), q = std::max(partial, E.partial_bytes);
         if (capturing) return refuse_unprepared();
@@ -1161,8 +1222,9 @@ int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t 
     a.err = E.err;
     // ~2 s, and longer for evaluations that themselves take that long
     a.wait_cycles = p.debug_wait_cycles > 0 ? p.debug_wait_cycles : tc::WAIT_CYCLES + (long long)(p.flops(nrhs) / 500);
-    a.units = s->ntasks * sh.ncol;
+    a.units = s->ntasks * ((sh.ncol + sh.group - 1) / sh.group);
     a.ncol = sh.ncol;
+    a.group = sh.group;
     a.nb = nb;
     a.nrhs = nrhs;
     a.beta = accumulate ? 1 : 0;
@@ -1172,17 +1234,18 @@ int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t 
     switch (sh.bn) {
     case 8: return launch<8>(a, stream);
     case 16: return launch<16>(a, stream);
-    default: return launch<32>(a, stream);
+    case 32: return launch<32>(a, stream);
+    case 64: return launch<64, 4>(a, stream);
+    default: return launch<128, 2>(a, stream);
     }
 }
 
 // Rows of the products that a variant's warps issue for a tile of m8 sub-block rows: its share of
 // them in pairs, per warp.
-int issued_rows(int bn, int m8)
+int issued_rows(const Shape &s, int m8)
 {
-    const int wm = bn >= 32 ? Cfg<32>::WM : Cfg<8>::WM;
     int rows = 0;
-    for (int w = 0; w < wm; ++w) rows += (m8 * (w + 1) / wm - m8 * w / wm + 1) / 2 * 16;
+    for (int w = 0; w < s.wm; ++w) rows += (m8 * (w + 1) / s.wm - m8 * w / s.wm + 1) / 2 * 16;
     return rows;
 }
 
@@ -1202,7 +1265,7 @@ int f64_profile(Plan &p, const double *dW, double *dY, const int32_t *wofs, cons
 {
     F64Engine &E = *p.f64;
     const int nb = (nrhs + 7) / 8;
-    const Shape sh = shape_for(nb);
+    const Shape sh = shape_for(p, nb);
     F64Engine::Schedule *s = nullptr;
     int rc = schedule_for(p, false, sh, false, &s);
     if (rc) return rc;
@@ -1261,7 +1324,7 @@ int f64_profile(Plan &p, const double *dW, double *dY, const int32_t *wofs, cons
         pass[t] = (uint8_t)std::min(k, 255);
         rec[k].units += sh.ncol;
         for (int q = tk.item0; q < tk.item0 + tk.nitem; ++q)
-            rec[k].issued_flops += 2.0 * issued_rows(sh.bn, tk.m8) * (8.0 * items[q].k8) * (8.0 * nb);
+            rec[k].issued_flops += 2.0 * issued_rows(sh, tk.m8) * (8.0 * items[q].k8) * (8.0 * nb);
     }
 
     // [start, passes], then the pass of each task
@@ -1355,7 +1418,7 @@ extern "C" int32_t mxb_debug_f64_schedule(const mxb_cds_desc *desc, int32_t adjo
     std::vector<mxb::BlockSource> blocks[3];
     uint64_t used[3] = {0, 0, 0};
     mxb::layout(p, blocks, used);
-    const mxb::Shape sh = mxb::shape_for((nrhs + 7) / 8);
+    const mxb::Shape sh = mxb::shape_for(p, (nrhs + 7) / 8);
     std::vector<mxb::F64Task> t;
     std::vector<mxb::F64Item> it;
     int nctr = 0;

@@ -104,13 +104,16 @@ __device__ __forceinline__ bool wait_counter(const int *ctr, int target, volatil
     return true;
 }
 
-// Whether such a counter has reached `target` (no wait, nothing ordered after it).
+// Whether such a counter has reached `target` (no wait); where it has, the calling thread is ordered
+// behind the counted writes as by wait_counter, but for the proxy fence.
 __device__ __forceinline__ bool counter_reached(const int *ctr, int target)
 {
     int v;
-    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(ctr) : "memory");
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(ctr) : "memory");
     return v >= target;
 }
+
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;\n" ::: "memory"); }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns()
 {

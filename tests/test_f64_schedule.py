@@ -157,3 +157,18 @@ def test_schedule_gives_the_product(lib, small_cases, r, adjoint):
         assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max(), name
         cut += int((tasks["npiece"] > 1).sum())
     assert cut > 0  # some sum was cut along K
+
+
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_schedule_of_many_tiles(lib, small_cases, adjoint):
+    """So many columns that far and down products, and near and leaf down products, are one sum: each
+    Y and each skeleton block is written once."""
+    r = 13000
+    cds = small_cases["ragged"]
+    TW = np.random.default_rng(r).standard_normal(cds.n * r)
+    got, tasks = execute(lib, cds, TW, r, adjoint)
+    want = O.adjoint(cds, TW, r) if adjoint else O.eval_h2b(cds, TW, r)
+    assert np.abs(got - want).max() <= 1e-12 * np.abs(want).max()
+    assert (tasks["old_dep"] == -1).all() and (tasks["beta"] != 1).all()
+    few = schedule(lib, cds, adjoint, 100)[0]
+    assert (few["beta"] == 1).any() and len(few) > len(tasks)

@@ -146,3 +146,52 @@ def test_infinities_stay_infinities(torch, small_cases, name, r):
             ok = np.isfinite(want)
             assert np.abs(got[ok] - want[ok]).max() <= TOL * np.abs(want[ok]).max()
     plan.status()
+
+
+@pytest.fixture(scope="module")
+def short():
+    """Blocks of at most 16 and of at most 32 rows: the variants of 128 and of 64 columns."""
+    out = {}
+    for leaf, n, budget in ((16, 1000, 0.0), (16, 999, 0.05), (32, 1990, 0.0), (32, 1001, 0.08)):
+        X = S.gaussian_mixture(n, 4, 4, 0.0, 3.0, 0.4, None, seed=n)
+        out[leaf, n] = S.build_cds(X, S.KernelSpec("gaussian", 1.0), leaf_size=leaf, budget=budget, tol=1e-7, max_rank=leaf - n % 3)
+    return out
+
+
+@pytest.mark.parametrize("r", [3, 33, 64, 65, 100, 128, 129, 200, 300])
+@pytest.mark.parametrize("key", [(16, 1000), (16, 999), (32, 1990), (32, 1001)])
+def test_short_blocks(torch, short, key, r):
+    cds = short[key]
+    rng = np.random.default_rng(r)
+    TW, Y0 = rng.standard_normal((2, cds.n * r))
+    plan = H.Plan(cds, "fp64")
+    room = torch.zeros(2 * cds.n * r + 3, dtype=torch.float64, device="cuda")
+    w, y = room[1:1 + cds.n * r], room[2 + cds.n * r:2 + 2 * cds.n * r]  # 8-byte aligned
+    w.copy_(torch.as_tensor(TW))
+    for call, want in ((plan.evaluate, O.eval_h2b(cds, TW, r)), (plan.adjoint, O.adjoint(cds, TW, r))):
+        for accumulate in (False, True):
+            y.copy_(torch.as_tensor(Y0))
+            call(w, r, out=y, accumulate=accumulate)
+            ref = want + Y0 if accumulate else want
+            assert np.abs(y.cpu().numpy() - ref).max() <= TOL * np.abs(ref).max()
+            assert room[0] == 0 and room[1 + cds.n * r] == 0 and room[-1] == 0  # nothing else written
+    plan.status()
+    width = {x["width"] for x in plan.profile(w, r)}
+    assert width == {8 if r <= 8 else 32 if r <= 32 else 64 if key[0] == 32 or r <= 64 else 128}
+
+
+@pytest.mark.parametrize("name,r", [("ragged", 13000), ("short", 13000), ("short", 52010)])
+def test_many_tiles(torch, small_cases, short, name, r):
+    """Fused sums, and units of two column tiles (the last size; an odd number of tiles)."""
+    cds = small_cases["ragged"] if name == "ragged" else short[16, 999]
+    rng = np.random.default_rng(r)
+    TW, Y0 = rng.standard_normal((2, cds.n * r))
+    plan = H.Plan(cds, "fp64")
+    w, y = torch.as_tensor(TW, device="cuda"), torch.as_tensor(Y0, device="cuda")
+    want = O.eval_h2b(cds, TW, r)
+    got = plan.evaluate(w, r).cpu().numpy()
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+    got = plan.adjoint(w, r, out=y, accumulate=True).cpu().numpy()
+    want = O.adjoint(cds, TW, r) + Y0
+    assert np.abs(got - want).max() <= TOL * np.abs(want).max()
+    plan.status()
