@@ -10,6 +10,8 @@
 from __future__ import annotations
 
 import ctypes
+import functools
+import os
 from concurrent.futures import ThreadPoolExecutor
 from typing import Optional
 
@@ -263,6 +265,12 @@ def kernel_matrices(dX, kernel, row_sets, col_sets, stream=None):
 _STAGING_BYTES = 32 << 20  # page-locked memory that results come to the host through
 
 
+@functools.lru_cache(maxsize=1)
+def _copy_threads(pid):
+    # kept: starting eight threads takes 0.4 - 0.8 ms (a forked child starts its own)
+    return ThreadPoolExecutor(8, thread_name_prefix="matrox-copy")
+
+
 def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
     """Column IDs of the packed column-major matrices in ``pool`` (a float64 CUDA tensor,
     overwritten), ``shapes`` = [(nrows, ncols), ...], on the GPU (``mxb_batched_id``).  Returns a
@@ -289,8 +297,8 @@ def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
     # row-major copies of the used parts, packed on the device and brought over through page-locked
     # staging into arrays of their own: a caller that keeps one P keeps no other, and no page-locked
     # memory.  The time goes to new pages, which several threads fault in: 32 nodes of 1024 x 512, rank
-    # 256 (31 MB), with the IDs, 9.0 ms, 10.8 ms where the results are kept (one thread: 9.0 and 21 ms;
-    # views of page-locked memory: 6.4 and 19.7 ms)
+    # 256 (31 MB), with the IDs, 8.8 ms, 9.6 ms where the results are kept (one thread: 9.0 and 21 ms;
+    # views of page-locked memory: 6.3 and 20 ms); 16 of 256 x 128 1.6 and 1.9 ms (1.4 and 1.6)
     sizes = ranks.astype(np.int64) * nc
     src = np.concatenate([[0], np.cumsum(pmax * nc)]).astype(np.int64)
     out, b, q = [], 0, 0
@@ -309,8 +317,7 @@ def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
         parts = np.split(host.copy_(packed).numpy(), np.cumsum(sizes[b:e - 1]))
         parts = [x.reshape(int(ranks[k]), int(nc[k])) for k, x in zip(range(b, e), parts)]
         if total * 8 > 1 << 20:
-            with ThreadPoolExecutor(8) as threads:
-                parts = list(threads.map(np.copy, parts))
+            parts = list(_copy_threads(os.getpid()).map(np.copy, parts))
         else:
             parts = [x.copy() for x in parts]
         for k, x in zip(range(b, e), parts):
