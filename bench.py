@@ -726,7 +726,7 @@ def main():
     roof["frac"] = round(roof["achieved"] / roof["peak"], 4)
     roof["traffic"] = traffic
     small = profile_traffic().get("small_case")
-    if traffic is None and small:
+    if traffic is None and small and small["mode"] == best:  # the bytes are of that mode's kernel
         roof["traffic_small_case"] = {"n": small["n"], "bytes_per_launch": round(
             small["tc_gemm_dram_bytes_per_evaluation"] / small["tc_gemm_launches_per_evaluation"]),
             "note": "measured at N=32768 (profiles/traffic.json); not scaled to this size"}
