@@ -1533,7 +1533,7 @@ struct Batch : public mxb_batch {
         double prio = -1, ready = 0, finish = 0;
     };
     int flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const;
-    double flow_balance(Entry &e, int w) const;
+    double flow_balance(Entry &e, int w, double *hub = nullptr) const;
     bool takes_flow(Entry &e) const;
     int flow_columns(Entry &e) const;
     int task_parts(const TcTask &t) const;
@@ -2004,8 +2004,9 @@ int Batch::flow_groups(Entry &e, int w, std::vector<FlowGroup> &G) const
 
 // Work of one SM over the longest path of a flow launch with w-column tiles: what decides the
 // tiles of a flow launch and whether to take one.  In K tiles of 6 products (a K tile of 3
-// products takes about 0.4 of one); a unit costs 3 more, a step of the path 3.5.
-double Batch::flow_balance(Entry &e, int w) const
+// products takes about 0.4 of one); a unit costs 3 more, a step of the path 3.5.  hub: the share of
+// the launch that the unit with the most inputs spends on waiting for them one by one (1.3 each).
+double Batch::flow_balance(Entry &e, int w, double *hub) const
 {
     std::vector<FlowGroup> G;
     if (flow_groups(e, w, G) <= 0) return 1e30;
@@ -2015,8 +2016,13 @@ double Batch::flow_balance(Entry &e, int w) const
     for (size_t i = 0; i < G.size(); ++i)
         if (!(open[i] = (int)G[i].deps.size())) order.push_back((int)i);
     double work = 0, longest = 1;
+    int inputs = 0;
     for (size_t q = 0; q < order.size(); ++q) {
         const FlowGroup &g = G[order[q]];
+        const TcTask &tk = tasks[g.tasks[0]];
+        int n = 0;
+        for (int k = tk.item0; k < tk.item0 + tk.nitem; ++k) n += items[k].dep >= 0 && (items[k].b_buf != BUF_W || e.flow_w);
+        inputs = std::max(inputs, n);
         double &p = path[order[q]];
         for (int d : g.deps) p = std::max(p, path[d]);
         p += ktiles(g) + 3.5;
@@ -2025,6 +2031,7 @@ double Batch::flow_balance(Entry &e, int w) const
         for (int c : g.cons)
             if (--open[c] == 0) order.push_back(c);
     }
+    if (hub) *hub = 1.3 * inputs / std::max(work / sm_count(), longest);
     return work / sm_count() / longest;
 }
 
@@ -2035,12 +2042,20 @@ double Batch::flow_balance(Entry &e, int w) const
 // 671 us at N = 30011 x 384, balance 2.9, 447 against 468 us at N = 16384 x 768, balance 3.2), and
 // timing them all takes 4 - 44 ms of the first evaluation.  Up to FLOW_TRIED it is one of the timed
 // candidates: it takes 0.83 (N = 65536 x 384 without a near field, six products) to 1.08 (N = 16384
-// x 1536) of the separate launches' time.
+// x 1536) of the separate launches' time.  A node in very many far lists (adjoints) can hold the flow
+// launch up, waiting for one short input after the other: such ones are timed as well.  Flow against
+// separate launches, 1 column: N = 131072, leaves of 64, 241 far lists (hub 0.6, balance 2.7) 856 / 637
+// us, N = 32768, leaves of 64, 75 lists (0.7, 1.4) 268 / 237.  Not where the flow launch hides it: N =
+// 65536, leaves of 256, 44 lists (0.21, 1.5) 327 / 418, and with little work besides, N = 65536, leaves
+// of 128, 58 lists (0.46, 1.15) 270 / 274, N = 16384, leaves of 64, 43 lists (0.7, 0.8) 137 / 148.
 constexpr int FLOW_COLUMNS = 128;
-constexpr double FLOW_WORK = 3.5, FLOW_TRIED = 12;
+constexpr double FLOW_WORK = 3.5, FLOW_TRIED = 12, FLOW_HUB = 0.3, FLOW_HUB_WORK = 1.2;
 bool Batch::takes_flow(Entry &e) const
 {
-    return *std::max_element(e.nrhs.begin(), e.nrhs.end()) <= FLOW_COLUMNS || flow_balance(e, 128) < FLOW_WORK;
+    double hub = 0;
+    const double balance = flow_balance(e, 128, &hub);
+    if (hub > FLOW_HUB && balance > FLOW_HUB_WORK) return false;
+    return *std::max_element(e.nrhs.begin(), e.nrhs.end()) <= FLOW_COLUMNS || balance < FLOW_WORK;
 }
 
 // Columns of a flow launch's tiles.  A step of the path is shorter on 64-column tiles and the

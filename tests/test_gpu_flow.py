@@ -6,7 +6,7 @@ import dataclasses
 import numpy as np
 import pytest
 
-from matrox_ru_b200 import _lib, hgemm as H
+from matrox_ru_b200 import _lib, hgemm as H, structure as S
 
 pytestmark = pytest.mark.gpu
 
@@ -134,3 +134,21 @@ def test_in_place_without_diagonal_blocks(torch, small_cases, hooks):
             call(x, r, out=x)
             assert torch.equal(x, want)
     plan.status()
+
+
+@pytest.mark.parametrize("r", [1, 100])
+def test_nodes_in_many_far_lists(torch, monkeypatch, r):
+    """An adjoint with a node in very many far lists, whose launches are timed instead of taken for
+    granted, and its forward product: the same as in separate launches."""
+    X = S.gaussian_mixture(24000, 8, 8, 0.0, 4.0, 0.5, None, seed=2)
+    cds = S.build_cds(X, S.KernelSpec("gaussian", 1.0), leaf_size=32, budget=0.008, tol=1e-3, max_rank=24, id_on_gpu=True)
+    assert np.bincount(cds.fpairy).max() > 60
+    W = torch.randn(cds.n * r, dtype=torch.float64, device="cuda")
+    got = []
+    for flow in ("1", "0"):
+        monkeypatch.setenv("MXB_TC_FLOW", flow)
+        plan = H.Plan(cds, "split_bf16", adjoint=True)
+        got.append([plan.evaluate(W, r), plan.adjoint(W, r), plan.adjoint(W, r)])
+        plan.status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
