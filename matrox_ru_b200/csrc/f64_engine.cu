@@ -622,7 +622,9 @@ int64_t tiles_of(const Plan &p, const Shape &s)
 // Short blocks: a tile of 64 rows is mostly empty, and an evaluation is as many tiles, of 2 - 3 us each
 // whatever they hold.  Flatter, wider tiles where they cut the number of tiles by more than a quarter:
 // HSS of N = 16384, 1000 right-hand sides, leaves of 16 points 1804 -> 588 us (16 x 128), of 32 points
-// 1486 -> 917 (32 x 64; N = 65536, 512 columns 2159 -> 1309).
+// 1486 -> 917 (32 x 64; N = 65536, 512 columns 2159 -> 1309).  Not below 8 tiles per block, where more
+// blocks at work count for more: N = 4096, leaves of 32, 64 columns (5 per block) 55.5 us against 57.8,
+// 100 columns (10) 68.6 against 65.8.
 //
 // Many tiles per block (of those resident): the launch is bound by tiles, not by the path through the
 // tree.  From 128 on, a block's far and down products, and its near and leaf down products, are one
@@ -637,9 +639,10 @@ Shape shape_for(const Plan &p, int nb)
     if (nb <= 2) return shape_of<16>(nb);
     Shape best = shape_of<32>(nb);
     int64_t tiles = tiles_of(p, best);
+    const bool many = tiles >= 8 * (int64_t)sm_count() * best.ctas;
     for (const Shape &s : {shape_of<64, 4>(nb), shape_of<128, 2>(nb)}) {
         const int64_t n = tiles_of(p, s);
-        if (4 * n >= 3 * tiles) continue;
+        if (!many || 4 * n >= 3 * tiles) continue;
         best = s;
         tiles = n;
     }

@@ -150,16 +150,17 @@ def test_infinities_stay_infinities(torch, small_cases, name, r):
 
 @pytest.fixture(scope="module")
 def short():
-    """Blocks of at most 16 and of at most 32 rows: the variants of 128 and of 64 columns."""
+    """Blocks of at most 16 and of at most 32 rows: the variants of 128 and of 64 columns (the first too
+    small for them but with very many columns)."""
     out = {}
-    for leaf, n, budget in ((16, 1000, 0.0), (16, 999, 0.05), (32, 1990, 0.0), (32, 1001, 0.08)):
+    for leaf, n, budget in ((16, 999, 0.05), (16, 8000, 0.0), (16, 7999, 0.008), (32, 16000, 0.0), (32, 15999, 0.008)):
         X = S.gaussian_mixture(n, 4, 4, 0.0, 3.0, 0.4, None, seed=n)
         out[leaf, n] = S.build_cds(X, S.KernelSpec("gaussian", 1.0), leaf_size=leaf, budget=budget, tol=1e-7, max_rank=leaf - n % 3)
     return out
 
 
 @pytest.mark.parametrize("r", [3, 33, 64, 65, 100, 128, 129, 200, 300])
-@pytest.mark.parametrize("key", [(16, 1000), (16, 999), (32, 1990), (32, 1001)])
+@pytest.mark.parametrize("key", [(16, 8000), (16, 7999), (32, 16000), (32, 15999)])
 def test_short_blocks(torch, short, key, r):
     cds = short[key]
     rng = np.random.default_rng(r)
