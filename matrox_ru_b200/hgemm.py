@@ -262,7 +262,9 @@ def kernel_matrices(dX, kernel, row_sets, col_sets, stream=None):
     return dst, ofs
 
 
-_STAGING_BYTES = 32 << 20  # page-locked memory that results come to the host through
+# results on the host: views of page-locked blocks of at most _BLOCK_BYTES (or one array's size) up to
+# _PINNED_BYTES a call, else arrays of their own, through _STAGING_BYTES of page-locked memory
+_BLOCK_BYTES, _PINNED_BYTES, _STAGING_BYTES = 4 << 20, 64 << 20, 32 << 20
 
 
 @functools.lru_cache(maxsize=1)
@@ -294,17 +296,19 @@ def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
                                      _stream_ptr(stream)), "mxb_batched_id")
     ranks = dRank.cpu().numpy()
     piv = dPiv.cpu().numpy()
-    # row-major copies of the used parts, packed on the device and brought over through page-locked
-    # staging into arrays of their own: a caller that keeps one P keeps no other, and no page-locked
-    # memory.  The time goes to new pages, which several threads fault in: 32 nodes of 1024 x 512, rank
-    # 256 (31 MB), with the IDs, 8.8 ms, 9.6 ms where the results are kept (one thread: 9.0 and 21 ms;
-    # views of page-locked memory: 6.3 and 20 ms); 16 of 256 x 128 1.6 and 1.9 ms (1.4 and 1.6)
+    # row-major copies of the used parts, packed on the device and brought over together.  A caller that
+    # keeps one P keeps the block it lies in, at most 4 MB, so a moderate amount comes as views of
+    # page-locked blocks: 32 nodes of 1024 x 512, rank 256 (31 MB), with the IDs, 6.3 ms (as arrays of
+    # their own 8.8; where every call's results are kept, and its memory is new, 20 and 9.6 ms).  Of
+    # larger amounts the time goes to new pages, which several threads fault in
     sizes = ranks.astype(np.int64) * nc
     src = np.concatenate([[0], np.cumsum(pmax * nc)]).astype(np.int64)
+    pinned = int(sizes.sum()) * 8 <= _PINNED_BYTES
+    room = _BLOCK_BYTES if pinned else _STAGING_BYTES
     out, b, q = [], 0, 0
     while b < len(shapes):
         e, total = b + 1, int(sizes[b])
-        while e < len(shapes) and (total + int(sizes[e])) * 8 <= _STAGING_BYTES:
+        while e < len(shapes) and (total + int(sizes[e])) * 8 <= room:
             total += int(sizes[e])
             e += 1
         packed = torch.empty(total, dtype=torch.float64, device=pool.device)
@@ -313,17 +317,16 @@ def batched_id(pool, shapes, tol: float, max_rank: int, stream=None):
             s, c = int(ranks[k]), int(nc[k])
             packed[at:at + s * c].view(s, c).copy_(dP[src[k]:src[k] + s * c].view(c, s).t())
             at += s * c
-        host = torch.empty(total, dtype=torch.float64, pin_memory=total * 8 <= _STAGING_BYTES)
-        parts = np.split(host.copy_(packed).numpy(), np.cumsum(sizes[b:e - 1]))
+        host = torch.empty(total, dtype=torch.float64, pin_memory=pinned or total * 8 <= room)
+        parts = np.split(host.copy_(packed, non_blocking=pinned).numpy(), np.cumsum(sizes[b:e - 1]))
         parts = [x.reshape(int(ranks[k]), int(nc[k])) for k, x in zip(range(b, e), parts)]
-        if total * 8 > 1 << 20:
+        if not pinned:
             parts = list(_copy_threads(os.getpid()).map(np.copy, parts))
-        else:
-            parts = [x.copy() for x in parts]
         for k, x in zip(range(b, e), parts):
             out.append((piv[q:q + x.shape[0]].astype(np.int64), x))
             q += x.shape[1]
         b = e
+    torch.cuda.current_stream(pool.device).synchronize()
     return out
 
 

@@ -159,20 +159,32 @@ def test_batched_id_beside_other_work(torch):
     side.synchronize()
 
 
-@pytest.mark.parametrize("staging", [None, 40000, 8])
-def test_results_own_their_memory(torch, monkeypatch, staging):
-    """Each P is an array of its own, whatever pieces the results come over in (all at once, a few
-    nodes, each node larger than the staging)."""
-    if staging is not None:
-        monkeypatch.setattr(H, "_STAGING_BYTES", staging)
+def held(P):
+    """Bytes that stay allocated while P is kept."""
+    while P.base is not None and isinstance(P.base, np.ndarray):
+        P = P.base
+    return P.nbytes if P.base is None else P.base.untyped_storage().nbytes()
+
+
+@pytest.mark.parametrize("block,pinned,staging", [(4 << 20, 64 << 20, 32 << 20), (40000, 64 << 20, 32 << 20),
+                                                  (8, 64 << 20, 32 << 20), (4 << 20, 8, 32 << 20), (4 << 20, 8, 40000),
+                                                  (4 << 20, 8, 8)])
+def test_results_keep_little_memory(torch, monkeypatch, block, pinned, staging):
+    """The results come over in blocks, or through staging into arrays of their own: in one piece, in
+    pieces of a few nodes, and with every node larger than a piece.  Keeping one of them keeps no more
+    than a block."""
+    for name, v in (("_BLOCK_BYTES", block), ("_PINNED_BYTES", pinned), ("_STAGING_BYTES", staging)):
+        monkeypatch.setattr(H, name, v)
     shapes = [(60 + b, 40 - b) for b in range(9)]
     rng = np.random.default_rng(8)
     mats = [rng.standard_normal(s) for s in shapes]
     pool = torch.as_tensor(np.concatenate([m.reshape(-1, order="F") for m in mats]), device="cuda")
-    for m, (piv, P) in zip(mats, H.batched_id(pool, shapes, 1e-9, 24)):
+    got = H.batched_id(pool, shapes, 1e-9, 24)
+    for m, (piv, P) in zip(mats, got):
         hpiv, hP = S.interpolative_decomposition(np.asfortranarray(m), 1e-9, 24)
         assert np.array_equal(piv, hpiv) and np.abs(P - hP).max() <= 1e-8 * max(1.0, np.abs(hP).max())
-        assert P.base is None and P.flags.owndata and P.flags.c_contiguous and P.flags.writeable
+        assert held(P) <= max(block if pinned > 8 else 0, P.nbytes)
+        assert P.flags.c_contiguous and P.flags.writeable
 
 
 @pytest.mark.parametrize("count,nr,nc", [(160, 128, 64), (160, 129, 64), (460, 200, 100), (460, 201, 100)])
