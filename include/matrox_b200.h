@@ -321,13 +321,13 @@ MXB_API int32_t mxb_plan_read_workspaces(mxb_plan *plan, int32_t nrhs, const int
 /* No counterpart in the reference (which evaluates one matrix per HGEMM call).  A batch merges
  * the launch sequences of several split-BF16 plans (same device; uneven N, ranks and nrhs and
  * any mix of split modes allowed -- couplings of different product counts run in separate
- * launches).  Up to 128 right-hand sides the passes of all plans run in one launch after the W
- * split, each work unit waiting on the device for the blocks it reads.  Above, one tensor-core
- * launch per level serves every plan, and the first evaluation of an nrhs signature picks by
- * timing (MXB_AUTOTUNE=0 disables the measurement) the column-tile width of every launch (64 /
- * 128 / 256 right-hand sides), which runs of up-sweep or down-sweep levels are chained into one
- * launch, and up to 512 columns whether all passes run in one.  The whole evaluation is captured
- * as one CUDA graph.
+ * launches).  Up to 128 right-hand sides, and where the products are few beside the path through
+ * the trees, the passes of all plans run in one launch after the W split, each work unit waiting on
+ * the device for the blocks it reads.  Otherwise one tensor-core launch per level serves every plan,
+ * and the first evaluation of an nrhs signature picks by timing (MXB_AUTOTUNE=0 disables the
+ * measurement) the column-tile width of every launch (64 / 128 / 256 right-hand sides), which runs
+ * of up-sweep or down-sweep levels are chained into one launch, and, unless the products are very
+ * many, whether all passes run in one.  The whole evaluation is captured as one CUDA graph.
  * The plans must outlive the batch; dW[i] / dY[i] are packed leaf-blocked device arrays of
  * plan i with nrhs[i] columns. */
 typedef struct mxb_batch mxb_batch;
@@ -348,8 +348,8 @@ MXB_API int32_t mxb_batch_info(const mxb_batch *batch, int32_t *launches, int32_
  * MXB_BATCH_ONE_LAUNCH: the whole evaluation -- the W split, up-sweep, couplings, near field,
  *   down-sweep and leaf down of every plan -- is ONE launch of the persistent kernel at every
  *   column count: each work unit waits on the device (bounded) until the blocks it reads are
- *   written.  One column-tile width (64 up to 64 right-hand sides, else 128) and 3-part stages
- *   serve every pass; units of bf16x3 couplings load 2 parts and issue 3 products.  W and Y
+ *   written.  One column-tile width (64 where the path through the trees bounds, else 128) and
+ *   3-part stages serve every pass; units of bf16x3 couplings load 2 parts and issue 3 products.  W and Y
  *   leaf-blocked (MXB_ERR_UNSUPPORTED in the caller's point order).
  * Changing the mode drops the batch's captured evaluations. */
 #define MXB_BATCH_LEVEL_LAUNCHES 0

@@ -26,12 +26,12 @@
 // in many near or far lists) is cut along K into pieces whose partial tiles the last piece
 // adds up in piece order, so the result does not depend on timing.
 //
-// What bounds it: the DMMA pipe from about 32 right-hand sides on (89 % active in the middle of a
-// launch), HBM (the CDS, read once) below, and for small matrices the chain of node to node hops
+// What bounds it: the DMMA pipe from about 32 right-hand sides on (91 % active), the number of tiles
+// where blocks are short, HBM (the CDS, read once) below, and for small matrices the chain of node to node hops
 // (2 - 3 us each: publish, poll, load, multiply).  Measured on one B200, launch per pass with
-// cp.async tiles -> one dataflow launch: N = 65536 H2-b, 1024 right-hand sides 25.6 -> 23.3 ms
-// (33.7 TFLOP/s), 1 right-hand side 2563 -> 460 us (5.8 TB/s); N = 16384 HSS, 256 right-hand
-// sides 511 -> 351 us; N = 32768 adjoint, 64 right-hand sides (long near lists) 2946 -> 690 us;
+// cp.async tiles -> one dataflow launch: N = 65536 H2-b, 1024 right-hand sides 25.6 -> 23.1 ms
+// (34.1 TFLOP/s), 1 right-hand side 2560 -> 460 us (5.8 TB/s); N = 16384 HSS, 256 right-hand
+// sides 511 -> 349 us; N = 32768 adjoint, 64 right-hand sides (long near lists) 2940 -> 695 us;
 // N = 1024, 1 right-hand side 102 -> 30 us.
 #include <algorithm>
 #include <cstring>

@@ -1,6 +1,6 @@
 // FP64 grouped variable-size GEMM on the B200's FP64 tensor path, reading the caller's CDS pools in
 // place: the kernel of mxb_evaluate_noalloc, which may not hold a re-tiled copy of the CDS.  Plans
-// run the dataflow launch of f64_engine.cu instead (N = 65536, 1024 right-hand sides: 23.3 ms
+// run the dataflow launch of f64_engine.cu instead (N = 65536, 1024 right-hand sides: 23.1 ms
 // against 25.6 ms here).
 //
 // tcgen05.mma has no f64 kind, so FP64 products use the DMMA instruction

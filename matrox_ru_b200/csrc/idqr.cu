@@ -2,8 +2,8 @@
 // CDS, matroxTest-V1/compression.h:446-523 `decomposition`, which the reference runs on the
 // host per tree node with LAPACKE_dgeqp3 followed by cblas_dtrsm.
 //
-// Two kernels do it: a cluster of blocks per node (below), and, for ranks above 512 and very tall
-// nodes, one CTA per node matrix A (nrows x ncols, column-major, nrows samples of the kernel against
+// Two kernels do it: a cluster of blocks per node (below), and, for ranks above 512, very tall nodes
+// and levels of many small ones (choose_cluster), one CTA per node matrix A (nrows x ncols, column-major, nrows samples of the kernel against
 // ncols candidate points), in place in global memory:
 //   1. Householder QR with column pivoting.  The pivot of step i is the first column of
 //      largest remaining norm; the norms are downdated after every step and recomputed where

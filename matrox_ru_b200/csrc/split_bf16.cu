@@ -1916,7 +1916,7 @@ std::vector<int> Batch::flow_tiles(int w) const
 }
 
 // Whether a flow launch splits W itself: where each block gets at most one such unit (a column tile
-// of a leaf, 19 - 30 us for 256 points x 64 - 128 columns, which the unit's 8 warps cannot hide),
+// of a leaf, 19 - 30 us for 256 points x 64 - 128 columns, which the unit's warps cannot hide),
 // the launch saved is worth more.  N = 30011, 130 columns: 102 us of the launch against 22 us in
 // split_w_kernel; N = 2048, 32 columns: 4 us against 11 us.
 bool Batch::flow_splits_w(const Entry &e, int w) const
