@@ -1136,10 +1136,14 @@ int schedule_for(Plan &p, bool adjoint, const Shape &sh, bool capturing, F64Engi
     s.bytes = tb + ib;
     size_t held = s.bytes;
     for (const F64Engine::Schedule &o : E.schedules) held += o.bytes;
-    while (!p.recorded && !E.schedules.empty() && held > SCHEDULE_BYTES) {
-        held -= E.schedules.front().bytes;
-        cudaFree(E.schedules.front().tasks);
-        E.schedules.erase(E.schedules.begin());
+    for (size_t i = 0; i < E.schedules.size() && held > SCHEDULE_BYTES;) {
+        if (E.schedules[i].recorded) {
+            ++i;
+            continue;
+        }
+        held -= E.schedules[i].bytes;
+        cudaFree(E.schedules[i].tasks);
+        E.schedules.erase(E.schedules.begin() + i);
     }
     std::vector<uint8_t> both(tb + ib);
     std::memcpy(both.data(), tasks.data(), tb);
@@ -1208,7 +1212,10 @@ int evaluate(Plan &p, bool adjoint, const double *dW, double *dY, const int32_t 
         E.ctl_bytes = c;
         E.partial_bytes = q;
     }
-    if (capturing) p.record();
+    if (capturing) {
+        s->recorded = true;
+        p.record();
+    }
     Args a{};
     for (int q = 0; q < 3; ++q) {
         a.pool[q] = E.pool[q];

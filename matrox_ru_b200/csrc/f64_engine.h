@@ -67,6 +67,7 @@ struct F64Engine {
         int ntasks = 0, nctr = 0;
         int64_t slots = 0;                          // partial slots (times ncol)
         size_t bytes = 0;                           // of tasks and items
+        bool recorded = false;                      // in a caller's capture: kept (see Plan::recorded)
         F64Task *tasks = nullptr;                   // followed by the items
         F64Item *items = nullptr;
     };

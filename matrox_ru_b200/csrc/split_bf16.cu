@@ -1458,7 +1458,6 @@ struct Batch : public mxb_batch {
     int *dNext = nullptr;  // work-unit counter per op
     int *dLevel = nullptr; // per op: epilogue warps done with its units (chained launches)
     std::vector<void *> allocations;
-    bool recorded = false;             // see Plan::recorded: what entries hold is then kept
     struct Entry {                     // one prepared evaluation
         std::vector<const double *> W;
         std::vector<double *> Y;
@@ -1481,6 +1480,7 @@ struct Batch : public mxb_batch {
         int nflow = 0;
         bool flow_w = false;           // the flow launch splits W too
         std::vector<PlanArgs> pa;
+        bool recorded = false;         // in a caller's capture: what it holds is kept (see Plan::recorded)
         cudaGraphExec_t exec = nullptr;
     };
     std::vector<Entry> entries;
@@ -1501,7 +1501,7 @@ struct Batch : public mxb_batch {
     {
         if (e.exec) cudaGraphExecDestroy(e.exec);
         for (void *q : {(void *)e.dPlans, (void *)e.dUnits, (void *)e.dDeps, (void *)e.dFlow}) {
-            if (q && recorded) allocations.push_back(q);
+            if (q && e.recorded) allocations.push_back(q);
             else if (q) cudaFree(q);
         }
         e.dFlow = nullptr;
@@ -2698,7 +2698,7 @@ int Batch::evaluate(const double *const *W, double *const *Y, const int *nrhs, i
     // preparing allocates, and uploads from temporary host memory: not while the stream captures
     if (capturing && !hit) return refuse_unprepared();
     if (capturing) {
-        recorded = true;
+        hit->recorded = true;
         for (Plan *p : plans) p->record();
     }
     if (!hit) {

@@ -86,3 +86,29 @@ def test_unprepared_evaluations_are_refused_under_capture(torch, small_cases, pr
     torch.cuda.synchronize()
     assert torch.equal(Y[:want.numel()], want)
     plan.status()
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_a_recorded_plan_does_not_grow(torch, small_cases, precision):
+    """Only what the captured evaluation uses is kept: a loop over more column counts than a plan keeps
+    entries for holds no more memory after many rounds than after a few."""
+    cds, counts = small_cases["h2b"], range(4, 64, 5)
+    plan = H.Plan(cds, precision)
+    W = torch.randn(cds.n * 64, dtype=torch.float64, device="cuda")
+    Y = torch.empty_like(W)
+    plan.evaluate(W, 24, out=Y)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        plan.evaluate(W, 24, out=Y)
+
+    def free_after(rounds):
+        for _ in range(rounds):
+            for r in counts:
+                plan.evaluate(W, r, out=Y)
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    first = free_after(3)
+    assert free_after(400) >= first - (4 << 20)
+    plan.status()
